@@ -193,7 +193,7 @@ struct GemmProblem {
   int m, n, k;
   double alpha;
   int accumulate;
-  // split-K and tile shape (filled by F64Gemm::build)
+  // split-K and kernel (filled by F64Gemm::build)
   int ksplit, kchunk, pad_;
   double* partial;
 };
@@ -201,11 +201,11 @@ struct GemmProblem {
 // Grouped FP64 GEMM: C_p (+)= alpha_p * A_p * B_p^T for all problems in one
 // persistent launch (plus a fixed-order split-K reduction when needed).
 struct F64Gemm {
-  struct Sub {  // one launch: the problems of one tile shape
+  struct Sub {  // one launch: the problems of one kernel
     GemmProblem* d_probs = nullptr;
     int* d_first = nullptr;
-    int* d_ticket = nullptr;
     int nprob = 0, total_tiles = 0, variant = 0;
+    int ts = 16, cluster = 1;  // tile kernel: tile edge, CTAs per tile
     std::vector<int> first;  // host copy of d_first (per-problem launches)
   };
   std::vector<Sub> subs;
@@ -219,11 +219,11 @@ struct F64Gemm {
   bool async_stream_set = false;
   cudaStream_t async_stream = nullptr;
   // async: allocate / upload stream-ordered on st (for one-shot leaf calls).
-  // variants: tile shape per problem (f64_variant numbering; -1 = model).
+  // variants: kernel per problem (f64_variant numbering; -1 = model).
   int build(const std::vector<GemmProblem>& probs, bool async = false, cudaStream_t st = nullptr,
             const std::vector<int>* variants = nullptr);
   int run(cudaStream_t st) const;
-  // One shape's launch (its work-queue ticket reset first).
+  // One kernel's launch.
   static int run_sub(const Sub& sb, cudaStream_t st);
   // One launch per problem (static schedule), then the split-K reduction:
   // the per-launch baseline against the single persistent launch of run().
@@ -231,17 +231,19 @@ struct F64Gemm {
   void release();
   ~F64Gemm() { release(); }
 };
+// One problem in one call, no plan: nothing is uploaded.  scratch (optional):
+// room of scratch_elems doubles for split-K partial sums, else a
+// stream-ordered temporary is allocated when they are needed.
+int run_f64_one(const GemmProblem& p, cudaStream_t st, double* scratch = nullptr, int64_t scratch_elems = 0);
 // Split-K partial-sum elements F64Gemm::build allocates for these problems
-// (model tile shapes).
+// (model kernels).
 int64_t f64_partial_elems(const std::vector<GemmProblem>& probs);
-// Tile shapes shared by the host planner and the kernels.
-int f64_variant(int m, int n);
+// Kernel choice shared by the host planner: 0 the tile kernel, 4 / 5 one
+// thread per row / column, 6 K <= 8.
 int f64_variant(int m, int n, int k);
-// As f64_variant, plus variant 7 (at most 16 x 16 outputs, long K) for planned launches.
+// As f64_variant, plus variants 7 (at most 16 x 16 outputs, long K) and 8
+// (matrix-vector) for planned launches.
 int f64_variant_planned(int m, int n, int k);
-int f64_tile_m(int variant);
-int f64_tile_n(int variant);
-int f64_tiles(int m, int n);
 
 // Device scratch allocation helpers (the library's own allocations go
 // through these so that OOM surfaces as GBX_ENOMEM).

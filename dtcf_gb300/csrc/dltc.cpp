@@ -305,7 +305,9 @@ int run_moves_once(const std::vector<MoveDesc>& v, const double* src, double* ds
 }
 
 // Runs one prepared Multiplication with workspace at ws (at least
-// ws_a + ws_b + ws_c elements); gemm (FP64) or split built by the caller.
+// ws_a + ws_b + ws_c elements); g or sp: the product planned by the caller
+// (neither: a one-shot FP64 product).
+GemmProblem gemm_problem(const Op& op, const double* A, const double* B, double* C, double* ws);
 int run_mul_op(const Op& op, const double* A, const double* B, double* C, double* ws, const MoveSet* ma,
                const MoveSet* mb, const MoveSet* mc, F64Gemm* g, SplitPlan* sp, cudaStream_t st) {
   if (op.M == 0 || op.N == 0) return GBX_OK;
@@ -315,7 +317,8 @@ int run_mul_op(const Op& op, const double* A, const double* B, double* C, double
   if (op.pack_a) GBX_TRY(ma ? run_moves(*ma, A, wa, st) : run_moves_once(op.mv_a, A, wa, st));
   if (op.pack_b) GBX_TRY(mb ? run_moves(*mb, B, wb, st) : run_moves_once(op.mv_b, B, wb, st));
   if (sp) GBX_TRY(run_split_plan(sp, true, true, st));
-  else GBX_TRY(g->run(st));
+  else if (g) GBX_TRY(g->run(st));
+  else GBX_TRY(run_f64_one(gemm_problem(op, A, B, C, ws), st));
   if (op.unpack_c) GBX_TRY(mc ? run_moves(*mc, wc, C, st) : run_moves_once(op.mv_c, wc, C, st));
   return GBX_OK;
 }
@@ -411,9 +414,7 @@ int gbx_dltc_task_mul(double coef, int rC, const int* idC, double* d_C, int rA, 
       destroy_split_plan(sp);
     }
   } else {
-    F64Gemm g;
-    rc = g.build({p}, true, st);
-    if (rc == GBX_OK) rc = run_mul_op(op, d_A, d_B, d_C, ws, nullptr, nullptr, nullptr, &g, nullptr, st);
+    rc = run_mul_op(op, d_A, d_B, d_C, ws, nullptr, nullptr, nullptr, nullptr, nullptr, st);
   }
   if (ws) cudaFreeAsync(ws, st);
   return rc;

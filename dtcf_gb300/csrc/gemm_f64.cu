@@ -1,18 +1,14 @@
 // Grouped FP64 GEMM on the FP64 tensor pipe (DMMA, mma.sync m8n8k4 f64).
 //
-// C_p (+)= alpha_p * A_p * B_p^T for every problem p of a launch.  One
-// persistent grid walks a device-side queue of work items (an atomic ticket
-// per CTA) over all problems, so a whole contraction -- every block triple,
-// every irrep -- is one launch.  A work item is a 64x64 output tile and, for
-// problems whose output is too small to fill the GPU, one K range of it
-// (split-K): those write raw partial sums to a workspace that a second
-// kernel reduces in a fixed order, so results are deterministic.  Operands
-// are read through generic element strides, which covers the transposed
-// forms of local_contraction.
-//
-// On GB300 the FP64 pipe runs near 1 TFLOP/s (DMMA and FFMA alike), so the
-// kernel is FP64-issue bound at any reasonable occupancy; the data path is
-// kept simple (register-staged shared-memory tiles, double buffered).
+// C_p (+)= alpha_p * A_p * B_p^T for every problem p of a launch: all
+// problems whose shape suits one kernel are one launch over a flat list of
+// work items, an output tile each and, for problems with long K and few
+// outputs, one K range of it (split-K): those write raw partial sums to a
+// workspace that a second kernel reduces in a fixed order, so results are
+// deterministic.  Operands are read through generic element strides, which
+// covers the transposed forms of local_contraction.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -21,16 +17,12 @@
 #include "common.h"
 #include "program.h"
 
+namespace cg = cooperative_groups;
+
 namespace gbx {
 
 namespace {
-constexpr int BK = 16;
-constexpr int kThreads = 128;
-constexpr int kPad = 1;               // pad rows to spread shared-memory banks
-constexpr int kFillTiles = 152 * 3;   // work items that keep every SM busy
-constexpr int kMinChunk = 256;        // smallest K range of a split
 constexpr int kRedThreads = dev::kRedThreads;
-constexpr int kRedChunk = dev::kRedChunk;
 constexpr int kThinN = 32, kThinK = 64, kThinMinWide = 16384;
 constexpr int kSmallK = dev::kSmallK;
 constexpr int kSmallKElems = dev::kSmallKElems;  // output elements per CTA
@@ -41,23 +33,33 @@ constexpr int kGemvDim = dev::kGemvDim;  // matrix-vector problems: one side at 
 constexpr int kGemvMinK = 64;         // ... with K above this
 constexpr int kGemvItems = 152 * 4;   // work items that keep every SM busy
 constexpr int kGemvMinChunk = 1024;   // smallest K range of a split
+constexpr int kSms = 152;
+constexpr int kQuarters = 4 * kSms;   // FP64 pipes: one per SM quarter
+
+int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 }  // namespace
 
-// Tile shapes: 64x64 for large problems, 64x16 / 16x64 / 16x16 for skinny ones
-// (output dimensions below 48), so small outputs do not waste the FP64 pipe.
-// Thin problems (one output dimension <= 32, the other at least 4x larger,
-// and either K <= 64 or at least 16384 wide rows to spread over the GPU) run
-// on CUDA-core FP64 with exact shapes: variant 4 = one thread per row of C
-// (N thin), variant 5 = one thread per column (M thin).
+// Variant 0 (tile_gemm_f64_kernel) takes any shape.  K <= 8 (outer products)
+// runs with one thread per output element (variant 6).  Thin problems (one
+// side at most 32) run with one thread per row (4) or column (5) of C, exact
+// in the thin side, where enough rows keep the 152 SMs evenly busy: the tile
+// kernel computes whole 8 x 8 x 4 blocks, so the thin kernel is taken when
+// its waves of 152 CTAs are fuller than the blocks are real (times 0.9, what
+// the tile kernel reaches on such shapes).  Measured, tile / thin kernel:
+// 5000 x 6 x 30 12 / 23 us, 100000 x 6 x 30 78 / 54, 40000 x 24 x 64 143 /
+// 207, 100000 x 24 x 64 306 / 320, 300000 x 24 x 64 883 / 825.
 int f64_variant(int m, int n, int k) {
-  // K <= 8 (outer products): one thread per output element
   if (k <= kSmallK) return 6;
-  // one thread per wide row: only with enough rows to fill the GPU, or short K
-  if (n <= kThinN && m >= 4 * n && (k <= kThinK || m >= kThinMinWide)) return 4;
-  if (m <= kThinN && n >= 4 * m && (k <= kThinK || n >= kThinMinWide)) return 5;
-  return (m < 48 ? 2 : 0) + (n < 48 ? 1 : 0);
+  const bool rows = n <= kThinN && m >= 4 * n, cols = m <= kThinN && n >= 4 * m;
+  if (rows || cols) {
+    const int wide = rows ? m : n, thin = rows ? n : m;
+    const int ctas = ceil_div(wide, 256);
+    const double filled = (double)ctas / ((double)kSms * ceil_div(ctas, kSms));
+    const double real = (double)thin / (8.0 * ceil_div(thin, 8)) * (double)k / (4.0 * ceil_div(k, 4));
+    if (filled > 0.9 * real) return rows ? 4 : 5;
+  }
+  return 0;
 }
-int f64_variant(int m, int n) { return (m < 48 ? 2 : 0) + (n < 48 ? 1 : 0); }
 // Planned launches also use variant 7: outputs of at most 16 x 16 with long
 // K, one CTA per K chunk holding the whole output (reduced in a fixed order).
 int f64_variant_planned(int m, int n, int k) {
@@ -67,21 +69,14 @@ int f64_variant_planned(int m, int n, int k) {
   if (k > kGemvMinK && ((m <= kGemvDim && n > kSmallOutDim) || (n <= kGemvDim && m > kSmallOutDim))) return 8;
   return f64_variant(m, n, k);
 }
-int f64_tile_m(int variant) { return (variant & 2) ? 16 : 64; }
-int f64_tile_n(int variant) { return (variant & 1) ? 16 : 64; }
-int f64_tiles(int m, int n) {
-  const int v = f64_variant(m, n), tm = f64_tile_m(v), tn = f64_tile_n(v);
-  return ((m + tm - 1) / tm) * ((n + tn - 1) / tn);
-}
 
 // One thread per row (variant 4) or per column (variant 5) of C; the thin
 // operand (at most kThinN rows) is staged through shared memory kThinK
 // columns at a time, so K is unbounded.  Each output is a k-ordered FMA
 // chain, so results are deterministic.
 template <bool kRows>
-__global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
-                                                            const int* __restrict__ block_first, int total_blocks) {
-  __shared__ double Ts[kThinN * kThinK];
+__device__ __forceinline__ void thin_body(const GemmProblem* __restrict__ probs, int nprob,
+                                          const int* __restrict__ block_first, int total_blocks, double* Ts) {
   for (int blk = blockIdx.x; blk < total_blocks; blk += gridDim.x) {
     int lo = 0, hi = nprob - 1;
     while (lo < hi) {
@@ -128,6 +123,13 @@ __global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* _
   }
 }
 
+template <bool kRows>
+__global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
+                                                            const int* __restrict__ block_first, int total_blocks) {
+  __shared__ double Ts[kThinN * kThinK];
+  thin_body<kRows>(probs, nprob, block_first, total_blocks, Ts);
+}
+
 // Matrix-vector shapes (variant 8): dev::gemv_body.
 __global__ void __launch_bounds__(256) gemv_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                        const int* __restrict__ block_first, int total_blocks) {
@@ -140,128 +142,200 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-template <int BM, int BN>
-__global__ void __launch_bounds__(kThreads) grouped_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
-                                                                    const int* __restrict__ tile_first,
-                                                                    int total_tiles, int* __restrict__ ticket) {
-  constexpr int WM = BM / 16, WN = BN / 16;  // m8n8 blocks per warp (2x2 warps)
-  constexpr int LA = BM * BK / kThreads, LB = BN * BK / kThreads;
-  // ticket == nullptr: static round-robin over work items; otherwise a device
-  // work queue (one atomic ticket per item) balances uneven problem sizes.
-  __shared__ double As[2][BM][BK + kPad];
-  __shared__ double Bs[2][BN][BK + kPad];
-  __shared__ int s_tile;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;  // 2x2 warps
+// ---- tile kernel (variant 0) -------------------------------------------------
+//
+// The FP64 pipe bounds this kernel and nothing else comes near: a DMMA
+// m8n8k4 occupies its quarter of the SM for 512 cycles (1.047 TFLOP/s over
+// 152 SMs, DMMA and DFMA alike, measured), against 256 bytes of operands.
+// So the operands go from L1 / L2 straight into the fragments -- no shared
+// memory stages, no barriers in the K loop -- and everything is spent on
+// keeping all 608 quarters busy to the end: output tiles of 16 x 16 or
+// 8 x 8, of which only the 8 x 8 blocks that hold real outputs are issued.
+// Very many tiles go one to a warp; else the K steps of a tile are dealt to
+// the four warps of a CTA (one per quarter) and, when the tiles are few, to a
+// cluster of up to eight CTAs, whose sums are added in a fixed order through
+// (distributed) shared memory.  Longer K still is cut into ranges that write
+// partial sums (splitk_reduce_kernel).
+constexpr int kTileWarps = 4;
+constexpr int kTileThreads = 32 * kTileWarps;
+constexpr int kTileUnroll = 4;  // K steps (of 4) per register stage, two stages
 
-  for (int iter = 0;; ++iter) {
-    if (ticket) {
-      if (tid == 0) s_tile = atomicAdd(ticket, 1);
-      __syncthreads();
-    }
-    const int tile = ticket ? s_tile : (int)blockIdx.x + iter * (int)gridDim.x;
-    if (ticket) __syncthreads();
-    if (tile >= total_tiles) break;
-    int lo = 0, hi = nprob - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (tile_first[mid] <= tile) lo = mid; else hi = mid - 1;
-    }
-    const GemmProblem p = probs[lo];
-    int local = tile - tile_first[lo];
-    const int ntn = (p.n + BN - 1) / BN, ntm = (p.m + BM - 1) / BM;
-    const int kc = local / (ntm * ntn);
-    local -= kc * ntm * ntn;
-    const int m0 = (local / ntn) * BM, n0 = (local % ntn) * BN;
-    const int kbeg = kc * p.kchunk;
-    const int kend = min(p.k, kbeg + p.kchunk);
+struct TileSmem {
+  double part[kTileWarps][256];
+  double sum[256];
+};
 
-    double acc[WM][WN][2];
+// MB x NB blocks of 8 x 8 over K steps [s0, s1) of the range [kbeg, kend);
+// out(row, col, two sums) takes the results, rows and columns within the tile.
+template <int MB, int NB, class Out>
+__device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, int kbeg, int kend, int s0, int s1,
+                                          Out&& out) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  const int64_t acs = p.a_cs, bcs = p.b_cs;
+  const double* pa[MB];
+  const double* pb[NB];
+  const int64_t k0 = kbeg + 4 * (int64_t)s0 + q;
+  // rows past the end repeat the last one: they only reach outputs that are not stored
 #pragma unroll
-    for (int i = 0; i < WM; ++i)
+  for (int i = 0; i < MB; ++i) pa[i] = p.A + (int64_t)min(m0 + 8 * i + r, p.m - 1) * p.a_rs + k0 * acs;
 #pragma unroll
-      for (int j = 0; j < WN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-    // register staging: each thread loads LA elements of A and LB of B per K step
-    double ra[LA], rb[LB];
-    auto load_regs = [&](int k0) {
+  for (int j = 0; j < NB; ++j) pb[j] = p.B + (int64_t)min(n0 + 8 * j + r, p.n - 1) * p.b_rs + k0 * bcs;
+  double acc[MB][NB][2];
 #pragma unroll
-      for (int r = 0; r < LA; ++r) {
-        int e = tid + r * kThreads;
-        int row = e / BK, col = e % BK;
-        int gm = m0 + row, gk = k0 + col;
-        ra[r] = (gm < p.m && gk < kend) ? __ldg(p.A + (int64_t)gm * p.a_rs + (int64_t)gk * p.a_cs) : 0.0;
-      }
+  for (int i = 0; i < MB; ++i)
 #pragma unroll
-      for (int r = 0; r < LB; ++r) {
-        int e = tid + r * kThreads;
-        int row = e / BK, col = e % BK;
-        int gn = n0 + row, gk = k0 + col;
-        rb[r] = (gn < p.n && gk < kend) ? __ldg(p.B + (int64_t)gn * p.b_rs + (int64_t)gk * p.b_cs) : 0.0;
-      }
-    };
-    auto store_regs = [&](int buf) {
+    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  double a[2][kTileUnroll][MB], b[2][kTileUnroll][NB];
+  auto load = [&](int buf, int s) {
 #pragma unroll
-      for (int r = 0; r < LA; ++r) {
-        int e = tid + r * kThreads;
-        As[buf][e / BK][e % BK] = ra[r];
-      }
+    for (int u = 0; u < kTileUnroll; ++u) {
+      const bool in = s + u < s1 && kbeg + 4 * (s + u) + q < kend;
+      const int64_t d = 4 * (int64_t)(s - s0 + u);
 #pragma unroll
-      for (int r = 0; r < LB; ++r) {
-        int e = tid + r * kThreads;
-        Bs[buf][e / BK][e % BK] = rb[r];
-      }
-    };
-
-    const int nk = kend > kbeg ? (kend - kbeg + BK - 1) / BK : 0;
-    if (nk > 0) {
-      load_regs(kbeg);
-      store_regs(0);
+      for (int i = 0; i < MB; ++i) a[buf][u][i] = in ? __ldg(pa[i] + d * acs) : 0.0;
+#pragma unroll
+      for (int j = 0; j < NB; ++j) b[buf][u][j] = in ? __ldg(pb[j] + d * bcs) : 0.0;
     }
-    __syncthreads();
-    for (int kt = 0; kt < nk; ++kt) {
-      const int buf = kt & 1;
-      if (kt + 1 < nk) load_regs(kbeg + (kt + 1) * BK);
+  };
+  auto mma = [&](int buf, int s) {
 #pragma unroll
-      for (int k4 = 0; k4 < BK; k4 += 4) {
-        double af[WM], bf[WN];
+    for (int u = 0; u < kTileUnroll; ++u) {
+      if (s + u >= s1) break;
 #pragma unroll
-        for (int i = 0; i < WM; ++i) af[i] = As[buf][wm * (BM / 2) + i * 8 + (lane >> 2)][k4 + (lane & 3)];
+      for (int i = 0; i < MB; ++i)
 #pragma unroll
-        for (int j = 0; j < WN; ++j) bf[j] = Bs[buf][wn * (BN / 2) + j * 8 + (lane >> 2)][k4 + (lane & 3)];
-#pragma unroll
-        for (int i = 0; i < WM; ++i)
-#pragma unroll
-          for (int j = 0; j < WN; ++j) dmma884(acc[i][j], af[i], bf[j]);
-      }
-      if (kt + 1 < nk) store_regs(buf ^ 1);
-      __syncthreads();
+        for (int j = 0; j < NB; ++j) dmma884(acc[i][j], a[buf][u][i], b[buf][u][j]);
     }
-
-    // epilogue: C (+)= alpha * acc, or the raw partial of this K range
-    double* part = p.partial ? p.partial + (int64_t)kc * p.m * p.n : nullptr;
-#pragma unroll
-    for (int i = 0; i < WM; ++i) {
-      const int gm = m0 + wm * (BM / 2) + i * 8 + (lane >> 2);
-      if (gm >= p.m) continue;
-#pragma unroll
-      for (int j = 0; j < WN; ++j) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int gn = n0 + wn * (BN / 2) + j * 8 + (lane & 3) * 2 + h;
-          if (gn >= p.n) continue;
-          if (part) {
-            part[(int64_t)gm * p.n + gn] = acc[i][j][h];
-          } else {
-            double* c = p.C + (int64_t)gm * p.c_rs + gn;
-            double v = __dmul_rn(p.alpha, acc[i][j][h]);
-            *c = p.accumulate ? __dadd_rn(*c, v) : v;
-          }
-        }
-      }
-    }
+  };
+  if (s0 < s1) load(0, s0);
+  for (int s = s0; s < s1; s += 2 * kTileUnroll) {
+    if (s + kTileUnroll < s1) load(1, s + kTileUnroll);
+    mma(0, s);
+    if (s + 2 * kTileUnroll < s1) load(0, s + 2 * kTileUnroll);
+    if (s + kTileUnroll < s1) mma(1, s + kTileUnroll);
   }
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) out(8 * i + r, 8 * j + 2 * q, acc[i][j][0], acc[i][j][1]);
+}
+
+// The 8 x 8 blocks of a 16 x 16 tile that hold real outputs.
+template <class Out>
+__device__ __forceinline__ void tile_blocks(const GemmProblem& p, bool m2, bool n2, int m0, int n0, int kbeg, int kend,
+                                            int s0, int s1, Out&& out) {
+  if (m2 && n2) tile_loop<2, 2>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else if (m2) tile_loop<2, 1>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else if (n2) tile_loop<1, 2>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else tile_loop<1, 1>(p, m0, n0, kbeg, kend, s0, s1, out);
+}
+
+// Work item `local` of problem p when every warp has a 16 x 16 tile of its own.
+__device__ __forceinline__ void warp_tile_item(const GemmProblem& p, int64_t local) {
+  const int ntn = (p.n + 15) / 16, ntm = (p.m + 15) / 16;
+  const int64_t t = local * kTileWarps + (threadIdx.x >> 5);
+  if (t >= (int64_t)ntm * ntn) return;
+  const int m0 = (int)(t / ntn) * 16, n0 = (int)(t % ntn) * 16;
+  tile_blocks(p, p.m - m0 > 8, p.n - n0 > 8, m0, n0, 0, p.k, 0, (p.k + 3) / 4, [&](int i, int j, double x, double y) {
+    const int64_t gm = m0 + i, gn = n0 + j;
+    if (gm >= p.m) return;
+    double* c = p.C + gm * p.c_rs + gn;
+    if (gn < p.n) c[0] = p.accumulate ? __dadd_rn(c[0], __dmul_rn(p.alpha, x)) : __dmul_rn(p.alpha, x);
+    if (gn + 1 < p.n) c[1] = p.accumulate ? __dadd_rn(c[1], __dmul_rn(p.alpha, y)) : __dmul_rn(p.alpha, y);
+  });
+}
+
+// One work item of problem p: output tile and K range `local`.  ts: tile
+// edge, 16 or 8; 0: a tile per warp.
+__device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, int ts, TileSmem& sm) {
+  if (ts == 0) {
+    warp_tile_item(p, local);
+    return;
+  }
+  const cg::cluster_group cl = cg::this_cluster();
+  const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
+  const int warp = threadIdx.x >> 5;
+  const int ntn = (p.n + ts - 1) / ts, ntm = (p.m + ts - 1) / ts;
+  const int64_t per_k = (int64_t)ntm * ntn;
+  const int kc = (int)(local / per_k);
+  const int t = (int)(local - kc * per_k);
+  const int m0 = t / ntn * ts, n0 = (t % ntn) * ts;
+  const int kbeg = kc * p.kchunk, kend = min(p.k, kbeg + p.kchunk);
+  const int steps = (max(kend - kbeg, 0) + 3) / 4;
+  const int per = (steps + csize * kTileWarps - 1) / (csize * kTileWarps);
+  const int s0 = min(steps, (crank * kTileWarps + warp) * per), s1 = min(steps, s0 + per);
+  const bool m2 = ts == 16 && p.m - m0 > 8, n2 = ts == 16 && p.n - n0 > 8;
+  double* part = sm.part[warp];
+  tile_blocks(p, m2, n2, m0, n0, kbeg, kend, s0, s1, [&](int i, int j, double x, double y) {
+    *reinterpret_cast<double2*>(part + i * 16 + j) = make_double2(x, y);
+  });
+  __syncthreads();
+  const int rows = min(ts, p.m - m0), cols = min(ts, p.n - n0);
+  const auto add = [&](int e) {
+    double v = sm.part[0][e];
+#pragma unroll
+    for (int w = 1; w < kTileWarps; ++w) v = __dadd_rn(v, sm.part[w][e]);
+    return v;
+  };
+  const auto store = [&](int e, double v) {
+    const int i = e >> 4, j = e & 15;
+    const int64_t gm = m0 + i, gn = n0 + j;
+    if (p.ksplit > 1) {
+      p.partial[(int64_t)kc * p.m * p.n + gm * p.n + gn] = v;
+    } else {
+      double* c = p.C + gm * p.c_rs + gn;
+      v = __dmul_rn(p.alpha, v);
+      *c = p.accumulate ? __dadd_rn(*c, v) : v;
+    }
+  };
+  const auto real = [&](int e) { return (e >> 4) < rows && (e & 15) < cols; };
+  if (csize == 1) {
+    for (int e = threadIdx.x; e < 256; e += kTileThreads)
+      if (real(e)) store(e, add(e));
+    return;
+  }
+  for (int e = threadIdx.x; e < 256; e += kTileThreads)
+    if (real(e)) sm.sum[e] = add(e);
+  cl.sync();
+  // output e is summed over the cluster, in rank order, by rank e % csize
+  for (int e = (int)threadIdx.x * csize + crank; e < 256; e += kTileThreads * csize)
+    if (real(e)) {
+      double v = *cl.map_shared_rank(&sm.sum[e], 0);
+      for (int c = 1; c < csize; ++c) v = __dadd_rn(v, *cl.map_shared_rank(&sm.sum[e], c));
+      store(e, v);
+    }
+  cl.sync();  // no CTA leaves while another reads its sums
+}
+
+// All problems of a launch, one work item per cluster: the item's problem is
+// found by a 32-way search of the first-item table.
+__global__ void __launch_bounds__(kTileThreads, 4)
+    tile_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob, const int* __restrict__ first, int ts) {
+  __shared__ TileSmem sm;
+  const int item = (int)(blockIdx.x / cg::this_cluster().num_blocks());
+  int lo = 0, n = nprob;
+  while (n > 1) {
+    const int step = (n + 31) / 32, at = lo + (int)(threadIdx.x & 31) * step;
+    const unsigned le = __ballot_sync(0xffffffffu, at < lo + n && __ldg(first + min(at, nprob - 1)) <= item);
+    const int hit = 31 - __clz(le);  // the first entry of the range is always <= item
+    const int nlo = lo + hit * step;
+    n = min(step, lo + n - nlo);
+    lo = nlo;
+  }
+  tile_item(probs[lo], item - first[lo], ts, sm);
+}
+
+// A one-problem launch with its descriptor in the kernel's arguments: nothing to upload, no search.
+struct OneProblem {
+  GemmProblem p;
+  int zero;            // the problem's first work item
+  int red_prob;        // split-K reduction: problem index (0)
+  uint32_t red_first;  // and its first chunk (0)
+};
+
+__global__ void __launch_bounds__(kTileThreads, 4) tile_one_f64_kernel(const __grid_constant__ OneProblem a, int ts) {
+  __shared__ TileSmem sm;
+  tile_item(a.p, blockIdx.x / cg::this_cluster().num_blocks(), ts, sm);
 }
 
 // K <= 8 (dev::small_k_body).
@@ -282,7 +356,23 @@ __global__ void __launch_bounds__(kRedThreads) splitk_reduce_kernel(const GemmPr
                                                                     const int* __restrict__ red_prob,
                                                                     const uint32_t* __restrict__ red_first, int nred,
                                                                     uint32_t nchunks) {
-  dev::splitk_reduce_body<false>(probs, red_prob, red_first, nred, nchunks, blockIdx.x, gridDim.x);
+  __shared__ double red[kRedThreads];
+  dev::splitk_reduce_body<false>(probs, red_prob, red_first, nred, nchunks, blockIdx.x, gridDim.x, red);
+}
+
+// The one-problem forms of the kernels above.
+template <bool kRows>
+__global__ void __launch_bounds__(256) thin_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  __shared__ double Ts[kThinN * kThinK];
+  thin_body<kRows>(&a.p, 1, &a.zero, total, Ts);
+}
+__global__ void __launch_bounds__(256) small_k_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  dev::small_k_body<false>(&a.p, 1, &a.zero, total, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(kRedThreads) splitk_reduce_one_kernel(const __grid_constant__ OneProblem a,
+                                                                        uint32_t nchunks) {
+  __shared__ double red[kRedThreads];
+  dev::splitk_reduce_body<false>(&a.p, &a.red_prob, &a.red_first, 1, nchunks, blockIdx.x, gridDim.x, red);
 }
 
 void F64Gemm::release() {
@@ -293,7 +383,6 @@ void F64Gemm::release() {
   for (auto& sb : subs) {
     fr(sb.d_probs);
     fr(sb.d_first);
-    fr(sb.d_ticket);
   }
   subs.clear();
   fr(d_all);
@@ -309,52 +398,147 @@ void F64Gemm::release() {
 }
 
 namespace {
-// K split of a DMMA problem: only when the output tiles of the whole launch
-// leave the GPU idle; ranges are multiples of the K step.
-void f64_ksplit(int k, int64_t out_tiles, int* ks_out, int* chunk_out) {
-  int ks = 1;
-  if (out_tiles < kFillTiles && k > 2 * kMinChunk) {
-    int want = (int)((kFillTiles + out_tiles - 1) / out_tiles);
-    ks = std::max(1, std::min(want, (k + kMinChunk - 1) / kMinChunk));
-  }
-  int chunk = (k + ks - 1) / ks;
-  chunk = ((chunk + BK - 1) / BK) * BK;
-  ks = std::max(1, (k + chunk - 1) / chunk);
-  *ks_out = ks;
-  *chunk_out = chunk;
-}
-}  // namespace
 
-int64_t f64_partial_elems(const std::vector<GemmProblem>& probs) {
-  int64_t out_tiles = 0, part = 0;
-  for (auto& q : probs)
-    if (q.m > 0 && q.n > 0) out_tiles += f64_tiles(q.m, q.n);
-  for (auto& q : probs) {
-    if (q.m <= 0 || q.n <= 0) continue;
-    const int v = f64_variant_planned(q.m, q.n, q.k);
-    if (v == 7) {
-      const int64_t ks7 = (q.k + kSmallOutChunk - 1) / kSmallOutChunk;
-      if (ks7 > 1) part += ks7 * q.m * q.n;
-      continue;
+// Schedule of one launch of the tile kernel: the tile edge (0: a 16 x 16
+// tile per warp) and the cluster size.  16 x 16 tiles read half the operand
+// bytes per product of 8 x 8 ones, but only many tiles keep the last wave
+// short: a tile per warp where the waves of warps are many or full (no
+// reduction through shared memory: 300000 x 32 x 30 722 -> 612 us), a tile
+// per CTA from eight per SM on, else 8 x 8, and with fewer than four of those
+// per SM clusters share a tile's K steps, at least three for every warp.
+// 64 x 48 x 96 takes 9 us a call so (one 64 x 64 tile: 129 us), 1021 x 765 x
+// 1531 2.29 ms, 1.045 TFLOP/s (64 x 64 tiles: 2.36 ms).
+struct TilePlan {
+  int ts = 16, cluster = 1;
+};
+
+int64_t tile_count(const GemmProblem& q, int ts) { return (int64_t)ceil_div(q.m, ts) * ceil_div(q.n, ts); }
+
+TilePlan tile_plan(const std::vector<const GemmProblem*>& probs) {
+  TilePlan t;
+  int64_t n16 = 0, n8 = 0;
+  int kmax = 0;
+  for (const GemmProblem* q : probs) {
+    n16 += tile_count(*q, 16);
+    n8 += tile_count(*q, 8);
+    kmax = std::max(kmax, q->k);
+  }
+  const int64_t waves = (n16 + kQuarters - 1) / kQuarters;
+  if (waves >= 16 || (waves >= 4 && n16 >= 0.92 * (double)(waves * kQuarters))) t.ts = 0;
+  if (n16 >= 8 * kSms) return t;
+  t.ts = 8;
+  while (t.cluster < 8 && n8 * t.cluster < 4 * kSms && ceil_div(kmax, 4) >= 12 * t.cluster) t.cluster *= 2;
+  return t;
+}
+
+// K ranges of one problem: cut where one CTA's share of a tile would outlast
+// an even share of the whole launch (of `dmmas` DMMAs) and `least` DMMAs per
+// warp, the cost that the partial sums and their reduction have to be worth.
+void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
+  const int steps = ceil_div(q.k, 4), workers = 4 * t.cluster;
+  if (t.ts == 0) return;
+  const int64_t blocks = t.ts == 16 ? std::min(2, ceil_div(q.m, 8)) * std::min(2, ceil_div(q.n, 8)) : 1;
+  const int64_t item = blocks * ceil_div(steps, workers);
+  const int64_t share = std::max<int64_t>(dmmas / kQuarters, least);
+  int64_t ks = std::max<int64_t>(1, std::min<int64_t>((item + share / 2) / share, steps / (8 * workers)));
+  const int chunk = 4 * ceil_div(steps, ks);
+  q.ksplit = std::max(1, ceil_div(q.k, std::max(chunk, 4)));
+  q.kchunk = std::max(chunk, 4);
+}
+
+int64_t dmma_count(const GemmProblem& q) { return tile_count(q, 8) * ceil_div(q.k, 4); }
+
+constexpr int kPlannedLeast = 96;   // about 25 us of one quarter: two reduction launches
+constexpr int kOneShotLeast = 512;  // a one-shot call also allocates the partial sums
+
+// Variant, K ranges and tile schedule of every problem; partial sums are
+// numbered from 0 in q.partial (offset + 1, 0 = none).  Returns their count.
+int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& want, TilePlan& tp) {
+  std::vector<const GemmProblem*> tiles;
+  int64_t dmmas = 0, small_k = 0;
+  for (size_t i = 0; i < probs.size(); ++i) {
+    GemmProblem& q = probs[i];
+    q.pad_ = want[i] >= 0 ? want[i] : f64_variant_planned(q.m, q.n, q.k);
+    if (q.pad_ == 0) {
+      tiles.push_back(&q);
+      dmmas += dmma_count(q);
     }
-    if (v == 8) {
+    if (q.pad_ == 7) small_k += q.k;
+  }
+  tp = tile_plan(tiles);
+  // small outputs: chunks of up to 2048, shorter where all problems together
+  // would leave CTAs without one
+  const int chunk7 = (int)std::max<int64_t>(64, std::min<int64_t>(kSmallOutChunk, small_k / (4 * kSms) / 64 * 64));
+  int64_t part = 0;
+  for (GemmProblem& q : probs) {
+    q.ksplit = 1;
+    q.kchunk = std::max(q.k, 4);
+    q.partial = nullptr;
+    if (q.pad_ == 7) {
+      q.ksplit = std::max(1, ceil_div(q.k, chunk7));
+      q.kchunk = chunk7;
+    } else if (q.pad_ == 8) {  // matrix-vector: K ranges when the outputs are few
       const int64_t wide = q.m <= kGemvDim && q.m <= q.n ? q.n : q.m;
       const int64_t groups = (wide + 7) / 8;
-      int64_t ks8 = 1;
+      int ks = 1;
       if (groups < kGemvItems && q.k > 2 * kGemvMinChunk)
-        ks8 = std::min<int64_t>((kGemvItems + groups - 1) / groups, (q.k + kGemvMinChunk - 1) / kGemvMinChunk);
-      int64_t chunk = (q.k + ks8 - 1) / ks8;
-      chunk = (chunk + 31) / 32 * 32;
-      ks8 = std::max<int64_t>(1, (q.k + chunk - 1) / chunk);
-      if (ks8 > 1) part += ks8 * q.m * q.n;
-      continue;
+        ks = (int)std::min<int64_t>((kGemvItems + groups - 1) / groups, ceil_div(q.k, kGemvMinChunk));
+      q.kchunk = ceil_div(ceil_div(q.k, ks), 32) * 32;
+      q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
+    } else if (q.pad_ == 0) {
+      tile_ksplit(q, tp, dmmas, kPlannedLeast);
     }
-    if (v >= 4) continue;
-    int ks = 1, chunk = 0;
-    f64_ksplit(q.k, out_tiles, &ks, &chunk);
-    if (ks > 1) part += (int64_t)ks * q.m * q.n;
+    if (q.ksplit > 1) {
+      q.partial = (double*)(intptr_t)(part + 1);
+      part += (int64_t)q.ksplit * q.m * q.n;
+    }
   }
   return part;
+}
+
+// Work items of a problem's variant.
+int64_t f64_items(const GemmProblem& q, int ts) {
+  switch (q.pad_) {
+    case 4: return ceil_div(q.m, 256);
+    case 5: return ceil_div(q.n, 256);
+    case 6: return ((int64_t)q.m * q.n + kSmallKElems - 1) / kSmallKElems;
+    case 7: return q.ksplit;
+    case 8: return (int64_t)ceil_div(q.m <= kGemvDim && q.m <= q.n ? q.n : q.m, 8) * q.ksplit;
+    default: return ts == 0 ? (tile_count(q, 16) + kTileWarps - 1) / kTileWarps : tile_count(q, ts) * q.ksplit;
+  }
+}
+
+uint64_t red_chunks_of(const GemmProblem& q) {
+  const int per = q.ksplit >= dev::kRedDeep ? dev::kRedDeepChunk : dev::kRedChunk;
+  return ((uint64_t)q.m * q.n + per - 1) / per;
+}
+
+// Launch of a tile kernel over `items` work items, one cluster each.
+template <class K, class... A>
+int launch_tiles(K kernel, const TilePlan& t, int64_t items, cudaStream_t st, A... args) {
+  if (items * t.cluster >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "FP64 GEMM has too many work items");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(items * t.cluster));
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = t.cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = t.cluster > 1 ? 1 : 0;
+  GBX_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return GBX_OK;
+}
+
+}  // namespace
+
+int64_t f64_partial_elems(const std::vector<GemmProblem>& in) {
+  std::vector<GemmProblem> probs;
+  for (auto& q : in)
+    if (q.m > 0 && q.n > 0) probs.push_back(q);
+  TilePlan tp;
+  return f64_schedule(probs, std::vector<int>(probs.size(), -1), tp);
 }
 
 int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t st, const std::vector<int>* variants) {
@@ -368,84 +552,27 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
     if (q.m <= 0 || q.n <= 0) continue;
     probs.push_back(q);
     int v = variants && i < variants->size() ? (*variants)[i] : -1;
-    if (v < -1 || v > 8) return fail(GBX_EINVAL, "FP64 tile variant %d", v);
+    if (v < -1 || (v > 0 && v < 4) || v > 8) return fail(GBX_EINVAL, "FP64 variant %d", v);
     // the thin kernels need their shape limits
     if ((v == 4 && q.n > kThinN) || (v == 5 && q.m > kThinN) || (v == 6 && q.k > kSmallK) ||
         (v == 7 && (q.m > kSmallOutDim || q.n > kSmallOutDim)) || (v == 8 && q.m > kGemvDim && q.n > kGemvDim))
-      return fail(GBX_EINVAL, "FP64 tile variant %d does not fit %d x %d x %d", v, q.m, q.n, q.k);
+      return fail(GBX_EINVAL, "FP64 variant %d does not fit %d x %d x %d", v, q.m, q.n, q.k);
     want.push_back(v);
   }
   nprob = (int)probs.size();
   if (nprob == 0) return GBX_OK;
-  // total output tiles decide how much K splitting the small problems get
-  int64_t out_tiles = 0;
-  for (auto& q : probs) out_tiles += f64_tiles(q.m, q.n);
-  int64_t part_elems = 0;
+  TilePlan tp;
+  const int64_t part_elems = f64_schedule(probs, want, tp);
   std::vector<int> red;
   std::vector<uint32_t> red_first;
   uint64_t rc = 0;
-  for (int i = 0; i < nprob; ++i) {
-    GemmProblem& q = probs[i];
-    int ks = 1;
-    const int thin = want[i] >= 0 ? want[i] : f64_variant_planned(q.m, q.n, q.k);
-    if (thin == 7) {  // small output: one work item per K chunk, fixed-order reduction
-      ks = std::max(1, (q.k + kSmallOutChunk - 1) / kSmallOutChunk);
-      q.ksplit = ks;
-      q.kchunk = kSmallOutChunk;
-      q.partial = nullptr;
-      q.pad_ = 7;
-      if (ks > 1) {
-        q.partial = (double*)(intptr_t)(part_elems + 1);  // offset + 1, patched below
-        part_elems += (int64_t)ks * q.m * q.n;
-        red.push_back(i);
-        red_first.push_back((uint32_t)rc);
-        rc += ((uint64_t)q.m * q.n + kRedChunk - 1) / kRedChunk;
-      }
-      continue;
-    }
-    if (thin == 8) {  // matrix-vector: K ranges when the outputs are few
-      const int64_t wide = q.m <= kGemvDim && q.m <= q.n ? q.n : q.m;
-      const int64_t groups = (wide + 7) / 8;
-      ks = 1;
-      if (groups < kGemvItems && q.k > 2 * kGemvMinChunk)
-        ks = (int)std::min<int64_t>((kGemvItems + groups - 1) / groups, (q.k + kGemvMinChunk - 1) / kGemvMinChunk);
-      int chunk = (q.k + ks - 1) / ks;
-      chunk = (chunk + 31) / 32 * 32;
-      ks = std::max(1, (q.k + chunk - 1) / chunk);
-      q.ksplit = ks;
-      q.kchunk = chunk;
-      q.partial = nullptr;
-      q.pad_ = 8;
-      if (ks > 1) {
-        q.partial = (double*)(intptr_t)(part_elems + 1);  // offset + 1, patched below
-        part_elems += (int64_t)ks * q.m * q.n;
-        red.push_back(i);
-        red_first.push_back((uint32_t)rc);
-        rc += ((uint64_t)q.m * q.n + kRedChunk - 1) / kRedChunk;
-      }
-      continue;
-    }
-    if (thin >= 4) {  // thin and small-K kernels: no split-K
-      q.ksplit = 1;
-      q.kchunk = std::max(q.k, BK);
-      q.partial = nullptr;
-      q.pad_ = thin;
-      continue;
-    }
-    int chunk = 0;
-    f64_ksplit(q.k, out_tiles, &ks, &chunk);
-    q.ksplit = ks;
-    q.kchunk = std::max(chunk, BK);
-    q.partial = nullptr;
-    q.pad_ = want[i] >= 0 ? want[i] : f64_variant(q.m, q.n);
-    if (ks > 1) {
-      q.partial = (double*)(intptr_t)(part_elems + 1);  // offset + 1, patched below
-      part_elems += (int64_t)ks * q.m * q.n;
+  for (int i = 0; i < nprob; ++i)
+    if (probs[i].ksplit > 1) {
       red.push_back(i);
       red_first.push_back((uint32_t)rc);
-      rc += ((uint64_t)q.m * q.n + kRedChunk - 1) / kRedChunk;
+      rc += red_chunks_of(probs[i]);
     }
-  }
+  if (rc >= (1ull << 31)) return fail(GBX_EUNSUPPORTED, "grouped GEMM has too many partial sums");
   nred = (int)red.size();
   red_chunks = (uint32_t)rc;
   auto alloc = [&](void** q, size_t bytes) -> int {
@@ -468,8 +595,8 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
   GBX_TRY(alloc((void**)&d_partial, sizeof(double) * part_elems));
   for (auto& q : probs)
     if (q.partial) q.partial = d_partial + ((intptr_t)q.partial - 1);
-  // one launch per tile shape
-  for (int v = 0; v < 9; ++v) {
+  // one launch per kernel
+  for (int v : {0, 4, 5, 6, 7, 8}) {
     std::vector<GemmProblem> vp;
     std::vector<int> first;
     int64_t tiles = 0;
@@ -477,22 +604,18 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
       if (q.pad_ != v) continue;
       vp.push_back(q);
       first.push_back((int)tiles);
-      if (v == 4) tiles += (q.m + 255) / 256;
-      else if (v == 5) tiles += (q.n + 255) / 256;
-      else if (v == 6) tiles += ((int64_t)q.m * q.n + kSmallKElems - 1) / kSmallKElems;
-      else if (v == 7) tiles += q.ksplit;
-      else if (v == 8) tiles += ((q.m <= kGemvDim && q.m <= q.n ? (int64_t)q.n : (int64_t)q.m) + 7) / 8 * q.ksplit;
-      else tiles += (int64_t)((q.m + f64_tile_m(v) - 1) / f64_tile_m(v)) * ((q.n + f64_tile_n(v) - 1) / f64_tile_n(v)) * q.ksplit;
+      tiles += f64_items(q, tp.ts);
+      if (tiles >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "grouped GEMM has too many work items");
     }
     if (vp.empty()) continue;
-    if (tiles >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "grouped GEMM has too many work items");
     Sub sb;
     sb.variant = v;
     sb.nprob = (int)vp.size();
     sb.total_tiles = (int)tiles;
+    sb.ts = tp.ts;
+    sb.cluster = tp.cluster;
     GBX_TRY(alloc((void**)&sb.d_probs, sizeof(GemmProblem) * vp.size()));
     GBX_TRY(alloc((void**)&sb.d_first, sizeof(int) * vp.size()));
-    GBX_TRY(alloc((void**)&sb.d_ticket, sizeof(int)));
     GBX_TRY(copy(sb.d_probs, vp.data(), sizeof(GemmProblem) * vp.size()));
     GBX_TRY(copy(sb.d_first, first.data(), sizeof(int) * vp.size()));
     sb.first = first;
@@ -515,8 +638,7 @@ int F64Gemm::run(cudaStream_t st) const {
   if (nprob == 0) return GBX_OK;
   if (ProgRecorder* rec = prog_recording()) {
     // the CUDA-core shapes become records of the persistent program (static
-    // schedule over their work items); the DMMA tile shapes and the thin
-    // kernels keep their own launches
+    // schedule over their work items); the tile and thin kernels keep their own launches
     for (const Sub& sb : subs) {
       const int kind = sb.variant == 6 ? PK_SMALLK : sb.variant == 7 ? PK_SMALLOUT : sb.variant == 8 ? PK_GEMV : -1;
       if (kind >= 0) {
@@ -544,71 +666,30 @@ int F64Gemm::run(cudaStream_t st) const {
   return GBX_OK;
 }
 
-int F64Gemm::run_sub(const Sub& sb, cudaStream_t st) {
-  GBX_CUDA(cudaMemsetAsync(sb.d_ticket, 0, sizeof(int), st));
-  int grid = std::min(sb.total_tiles, 152 * 4);
-  switch (sb.variant) {
-    case 0:
-      grouped_gemm_f64_kernel<64, 64><<<grid, kThreads, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles,
-                                                                 sb.d_ticket);
-      break;
-    case 1:
-      grouped_gemm_f64_kernel<64, 16><<<grid, kThreads, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles,
-                                                                 sb.d_ticket);
-      break;
-    case 2:
-      grouped_gemm_f64_kernel<16, 64><<<grid, kThreads, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles,
-                                                                 sb.d_ticket);
-      break;
-    case 3:
-      grouped_gemm_f64_kernel<16, 16><<<grid, kThreads, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles,
-                                                                 sb.d_ticket);
-      break;
-    case 4:
-      thin_gemm_f64_kernel<true><<<std::min(sb.total_tiles, 152 * 8), 256, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first,
-                                                                                    sb.total_tiles);
-      break;
-    case 6:
-      small_k_gemm_f64_kernel<<<std::min(sb.total_tiles, 152 * 8), 256, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first,
-                                                                                 sb.total_tiles);
-      break;
-    case 7:
-      small_out_gemm_f64_kernel<<<std::min(sb.total_tiles, 152 * 8), 256, 0, st>>>(sb.d_probs, sb.nprob,
-                                                                                   sb.d_first, sb.total_tiles);
-      break;
-    case 8:
-      gemv_f64_kernel<<<std::min(sb.total_tiles, 152 * 8), 256, 0, st>>>(sb.d_probs, sb.nprob, sb.d_first,
-                                                                         sb.total_tiles);
-      break;
-    default:
-      thin_gemm_f64_kernel<false><<<std::min(sb.total_tiles, 152 * 8), 256, 0, st>>>(sb.d_probs, sb.nprob,
-                                                                                     sb.d_first, sb.total_tiles);
-      break;
-  }
-  GBX_CUDA(cudaGetLastError());
-  return GBX_OK;
-}
-
-
 namespace {
-// A single-problem launch of variant v over work items [0, tiles).
-int launch_one(int v, const GemmProblem* prob, const int* zero, int tiles, cudaStream_t st) {
-  const int grid = std::min(tiles, 152 * 4), tgrid = std::min(tiles, 152 * 8);
+// The kernel of variant v over problems [probs, probs + nprob) and their `tiles` work items.
+int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first, int tiles, const TilePlan& tp,
+                   cudaStream_t st) {
+  const int grid = std::min(tiles, kSms * 8);
   switch (v) {
-    case 0: grouped_gemm_f64_kernel<64, 64><<<grid, kThreads, 0, st>>>(prob, 1, zero, tiles, nullptr); break;
-    case 1: grouped_gemm_f64_kernel<64, 16><<<grid, kThreads, 0, st>>>(prob, 1, zero, tiles, nullptr); break;
-    case 2: grouped_gemm_f64_kernel<16, 64><<<grid, kThreads, 0, st>>>(prob, 1, zero, tiles, nullptr); break;
-    case 3: grouped_gemm_f64_kernel<16, 16><<<grid, kThreads, 0, st>>>(prob, 1, zero, tiles, nullptr); break;
-    case 4: thin_gemm_f64_kernel<true><<<tgrid, 256, 0, st>>>(prob, 1, zero, tiles); break;
-    case 6: small_k_gemm_f64_kernel<<<tgrid, 256, 0, st>>>(prob, 1, zero, tiles); break;
-    case 7: small_out_gemm_f64_kernel<<<tgrid, 256, 0, st>>>(prob, 1, zero, tiles); break;
-    case 8: gemv_f64_kernel<<<tgrid, 256, 0, st>>>(prob, 1, zero, tiles); break;
-    default: thin_gemm_f64_kernel<false><<<tgrid, 256, 0, st>>>(prob, 1, zero, tiles); break;
+    case 0: return launch_tiles(tile_gemm_f64_kernel, tp, tiles, st, probs, nprob, first, tp.ts);
+    case 4: thin_gemm_f64_kernel<true><<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
+    case 6: small_k_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
+    case 7: small_out_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
+    case 8: gemv_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
+    default: thin_gemm_f64_kernel<false><<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
   }
   GBX_CUDA(cudaGetLastError());
   return GBX_OK;
 }
 }  // namespace
+
+int F64Gemm::run_sub(const Sub& sb, cudaStream_t st) {
+  TilePlan tp;
+  tp.ts = sb.ts;
+  tp.cluster = sb.cluster;
+  return launch_variant(sb.variant, sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles, tp, st);
+}
 
 int F64Gemm::run_each(cudaStream_t st) const {
   if (nprob == 0) return GBX_OK;
@@ -616,7 +697,12 @@ int F64Gemm::run_each(cudaStream_t st) const {
     // d_first[0] is 0: problem i is launched as a one-problem group whose
     // first-work-item table is that zero
     for (int i = 0; i < sb.nprob; ++i)
-      GBX_TRY(launch_one(sb.variant, sb.d_probs + i, sb.d_first, sb.first[i + 1] - sb.first[i], st));
+    {
+      TilePlan tp;
+      tp.ts = sb.ts;
+      tp.cluster = sb.cluster;
+      GBX_TRY(launch_variant(sb.variant, sb.d_probs + i, 1, sb.d_first, sb.first[i + 1] - sb.first[i], tp, st));
+    }
   }
   if (nred) {
     int rg = (int)std::min<uint32_t>(red_chunks, 152u * 8u);
@@ -624,6 +710,54 @@ int F64Gemm::run_each(cudaStream_t st) const {
     GBX_CUDA(cudaGetLastError());
   }
   return GBX_OK;
+}
+
+// One problem, one call: the descriptor travels in the kernel's arguments.
+// The partial sums of long K with few outputs come from `scratch` (at most
+// scratch_elems) when given, else from a stream-ordered temporary.
+int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t scratch_elems) {
+  OneProblem a;
+  std::memset(&a, 0, sizeof(a));
+  GemmProblem& q = a.p;
+  q = in;
+  if (q.m <= 0 || q.n <= 0) return GBX_OK;
+  q.pad_ = f64_variant(q.m, q.n, q.k);
+  q.ksplit = 1;
+  q.kchunk = std::max(q.k, 4);
+  q.partial = nullptr;
+  const TilePlan tp = tile_plan({&q});
+  double* own = nullptr;
+  if (q.pad_ == 0) {
+    tile_ksplit(q, tp, dmma_count(q), kOneShotLeast);
+    if (scratch && (int64_t)q.ksplit * q.m * q.n > scratch_elems) {
+      const int64_t ks = std::max<int64_t>(1, scratch_elems / ((int64_t)q.m * q.n));
+      q.kchunk = 4 * ceil_div(ceil_div(q.k, 4), ks);
+      q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
+    }
+    if (q.ksplit > 1) {
+      if (!scratch) GBX_CUDA(cudaMallocAsync((void**)&own, sizeof(double) * q.ksplit * q.m * q.n, st));
+      q.partial = scratch ? scratch : own;
+    }
+  }
+  const int64_t items = f64_items(q, tp.ts);
+  if (items >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "FP64 GEMM has too many work items");
+  const int grid = (int)std::min<int64_t>(items, kSms * 8);
+  int rc = GBX_OK;
+  switch (q.pad_) {
+    case 0: rc = launch_tiles(tile_one_f64_kernel, tp, items, st, a, tp.ts); break;
+    case 4: thin_one_f64_kernel<true><<<grid, 256, 0, st>>>(a, (int)items); break;
+    case 6: small_k_one_f64_kernel<<<grid, 256, 0, st>>>(a, (int)items); break;
+    default: thin_one_f64_kernel<false><<<grid, 256, 0, st>>>(a, (int)items); break;
+  }
+  cudaError_t e = cudaGetLastError();
+  if (rc == GBX_OK && e == cudaSuccess && q.ksplit > 1) {
+    const uint32_t chunks = (uint32_t)red_chunks_of(q);
+    splitk_reduce_one_kernel<<<std::min<uint32_t>(chunks, kSms * 8u), kRedThreads, 0, st>>>(a, chunks);
+    e = cudaGetLastError();
+  }
+  if (own) cudaFreeAsync(own, st);
+  if (rc == GBX_OK && e != cudaSuccess) rc = cuda_fail(e, "FP64 GEMM launch", __FILE__, __LINE__);
+  return rc;
 }
 }  // namespace gbx
 
@@ -634,37 +768,18 @@ int F64Gemm::run_each(cudaStream_t st) const {
 // library cudaMalloc then fails, or forces the pool to give memory back), and
 // latency-bound loops that keep other streams busy (cudaFree synchronises the
 // device and stalls them).  For them gbx_local_contraction_noalloc runs the
-// same FP64 GEMM with its descriptor and split-K partial sums in one
-// file-scope device array of kNoAllocBytes, which every GPU that loads the
-// library holds until the process exits.  What must start at zero: the
-// work-queue ticket, written (with the whole descriptor, by a one-thread
-// kernel on the caller's stream) by every call before its GEMM runs.  The
-// partial-sum slabs need no clearing: every split-K range overwrites its slab
-// in full before the reduction reads it.
+// same FP64 GEMM with its split-K partial sums in one file-scope device
+// array of kNoAllocBytes, which every GPU that loads the library holds until
+// the process exits; the descriptor travels in the kernel's arguments.
+// Nothing of the array needs clearing: every split-K range overwrites its
+// slab in full before the reduction reads it.
 namespace gbx {
 namespace {
-constexpr size_t kNoAllocHeader = 4096;                   // descriptor, schedule words
-constexpr size_t kNoAllocPartialBytes = 32ull << 20;      // split-K partial sums
-constexpr size_t kNoAllocBytes = kNoAllocHeader + kNoAllocPartialBytes;
-constexpr int64_t kNoAllocMaxElems = (int64_t)(kNoAllocPartialBytes / sizeof(double));
-
-struct NoAllocHeader {
-  GemmProblem prob;
-  int first;         // first work item of the problem (always 0)
-  int ticket;        // work-queue counter, reset by every call
-  int red_prob;      // split-K reduction: problem index (0)
-  uint32_t red_first;
-};
-static_assert(sizeof(NoAllocHeader) <= kNoAllocHeader, "header does not fit");
+constexpr size_t kNoAllocBytes = 32ull << 20;  // split-K partial sums
+constexpr int64_t kNoAllocMaxElems = (int64_t)(kNoAllocBytes / sizeof(double));
 }  // namespace
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
-
-// Writes the call's descriptor (ticket 0 included) into the scratch array
-// ahead of the GEMM on the same stream: the descriptor travels as a kernel
-// argument, so the call needs no host staging buffer and never waits for the
-// stream.
-__global__ void noalloc_header_kernel(NoAllocHeader h, NoAllocHeader* dst) { *dst = h; }
 
 // Device address of the scratch array, looked up once per device (the host
 // symbol is only a stand-in for it).
@@ -697,10 +812,8 @@ extern "C" int gbx_local_contraction_noalloc(int n_a, int n_b, int n_k, const do
                 (long long)n_a * n_b, (long long)kNoAllocMaxElems);
   unsigned char* scratch = nullptr;
   GBX_TRY(noalloc_scratch(&scratch));
-  cudaStream_t st = (cudaStream_t)stream;
-  NoAllocHeader h;
-  std::memset(&h, 0, sizeof(h));
-  GemmProblem& p = h.prob;
+  GemmProblem p;
+  std::memset(&p, 0, sizeof(p));
   p.A = d_A;
   p.B = d_B;
   p.C = d_C;
@@ -714,54 +827,5 @@ extern "C" int gbx_local_contraction_noalloc(int n_a, int n_b, int n_k, const do
   p.k = n_k;
   p.alpha = alpha;
   p.accumulate = 1;
-  // same schedule as the allocating path, split-K capped by the workspace
-  const int variant = f64_variant(n_a, n_b, n_k);
-  int ks = 1;
-  const int out_tiles = f64_tiles(n_a, n_b);
-  if (variant < 4 && out_tiles < kFillTiles && n_k > 2 * kMinChunk) {
-    int want = (kFillTiles + out_tiles - 1) / out_tiles;
-    ks = std::max(1, std::min(want, (n_k + kMinChunk - 1) / kMinChunk));
-    ks = (int)std::min<int64_t>(ks, kNoAllocMaxElems / ((int64_t)n_a * n_b));
-  }
-  int chunk = (n_k + ks - 1) / ks;
-  chunk = ((chunk + BK - 1) / BK) * BK;
-  ks = std::max(1, (n_k + chunk - 1) / chunk);
-  p.ksplit = ks;
-  p.kchunk = std::max(chunk, BK);
-  p.pad_ = variant;
-  p.partial = ks > 1 ? (double*)(scratch + kNoAllocHeader) : nullptr;
-  h.first = 0;
-  h.ticket = 0;
-  h.red_prob = 0;
-  h.red_first = 0;
-  NoAllocHeader* dh = (NoAllocHeader*)scratch;
-  // the descriptor is written on the stream by a one-thread kernel; the ticket starts at 0
-  noalloc_header_kernel<<<1, 1, 0, st>>>(h, dh);
-  GBX_CUDA(cudaGetLastError());
-  int tiles;
-  if (variant == 4) tiles = (n_a + 255) / 256;
-  else if (variant == 5) tiles = (n_b + 255) / 256;
-  else if (variant == 6) tiles = (int)(((int64_t)n_a * n_b + kSmallKElems - 1) / kSmallKElems);
-  else tiles = f64_tiles(n_a, n_b) * ks;
-  const GemmProblem* dp = &dh->prob;
-  const int* df = &dh->first;
-  int* dt = &dh->ticket;
-  const int grid = std::min(tiles, 152 * 4);
-  switch (variant) {
-    case 0: grouped_gemm_f64_kernel<64, 64><<<grid, kThreads, 0, st>>>(dp, 1, df, tiles, dt); break;
-    case 1: grouped_gemm_f64_kernel<64, 16><<<grid, kThreads, 0, st>>>(dp, 1, df, tiles, dt); break;
-    case 2: grouped_gemm_f64_kernel<16, 64><<<grid, kThreads, 0, st>>>(dp, 1, df, tiles, dt); break;
-    case 3: grouped_gemm_f64_kernel<16, 16><<<grid, kThreads, 0, st>>>(dp, 1, df, tiles, dt); break;
-    case 4: thin_gemm_f64_kernel<true><<<std::min(tiles, 152 * 8), 256, 0, st>>>(dp, 1, df, tiles); break;
-    case 6: small_k_gemm_f64_kernel<<<std::min(tiles, 152 * 8), 256, 0, st>>>(dp, 1, df, tiles); break;
-    default: thin_gemm_f64_kernel<false><<<std::min(tiles, 152 * 8), 256, 0, st>>>(dp, 1, df, tiles); break;
-  }
-  GBX_CUDA(cudaGetLastError());
-  if (ks > 1) {
-    const uint32_t chunks = (uint32_t)(((int64_t)n_a * n_b + kRedChunk - 1) / kRedChunk);
-    const int rg = (int)std::min<uint32_t>(chunks, 152u * 8u);
-    splitk_reduce_kernel<<<rg, kRedThreads, 0, st>>>(dp, &dh->red_prob, &dh->red_first, 1, chunks);
-    GBX_CUDA(cudaGetLastError());
-  }
-  return GBX_OK;
+  return run_f64_one(p, (cudaStream_t)stream, (double*)scratch, kNoAllocMaxElems);
 }

@@ -1,8 +1,8 @@
 // Grouped block triples: every (A-block, B-block -> C-block) product of one
 // launch set, C_t (+)= alpha_t A_t B_t^T, planned once and run as one
-// persistent launch per kernel kind (FP64 tile shapes on the FP64 pipe, or
+// launch per kernel kind (tile and thin kernels on the FP64 pipe, or
 // split-precision slices on tcgen05), with an autotuner that picks the
-// engine, orientation and tile shape per class of triple shapes by timing.
+// engine, orientation and width per class of triple shapes by timing.
 //
 // This is the leaf GEMM work of DTCF's transpose_and_dgemm
 // (contraction.cc:1779-1976) and of DLTC's task_mul (DLTC/task.cc:83-137)
@@ -367,12 +367,7 @@ int gbx_group_autotune(gbx_group* g, int reps, void* stream) {
       maxk = std::max(maxk, P.tri[i].k);
     }
     std::vector<Choice> cand;
-    if (g->mode != GBX_MODE_SPLIT)
-      for (int v = 0; v < 4; ++v) {
-        Choice c;
-        c.variant = v;
-        cand.push_back(c);
-      }
+    if (g->mode != GBX_MODE_SPLIT) cand.push_back(Choice());
     if (splittable)
       for (int sw = 0; sw < 2; ++sw)
         for (int w : {32, 64, 128, 256}) {

@@ -348,10 +348,7 @@ int gbx_local_contraction(int n_a, int n_b, int n_k, const double* d_A, const do
   p.k = n_k;
   p.alpha = alpha;
   p.accumulate = 1;
-  cudaStream_t st = (cudaStream_t)stream;
-  F64Gemm g;
-  GBX_TRY(g.build({p}, true, st));
-  return g.run(st);
+  return run_f64_one(p, (cudaStream_t)stream);
 }
 
 int gbx_dltc_compute(double* d_c, const double* d_a, const double* d_b, int m, int n, int k, void* stream) {

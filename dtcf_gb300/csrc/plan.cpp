@@ -241,6 +241,24 @@ void sub_strides(const std::vector<int64_t>& ext, int64_t base, std::vector<int6
 
 }  // namespace
 
+namespace {
+// FP64 seconds of an m x n x k product for the engine choice, as an FP64
+// engine of 64- and 16-wide output tiles would take them.  The FP64 kernels
+// have since become faster than this on small and ragged shapes, but the
+// line between the engines stays: a group that moved from slices to FP64 or
+// back would change a job's results by the slices' error, not by rounding.
+double f64_model_seconds(int64_t M, int64_t N, int64_t K) {
+  auto up = [](int64_t x, int64_t m) { return (double)((x + m - 1) / m * m); };
+  const double flops = 2.0 * (double)M * (double)N * (double)K, wide = (double)std::max(M, N) * (double)K * 8.0;
+  const int64_t lo = std::min(M, N), hi = std::max(M, N);
+  if (hi <= 16 && K >= 4096) return std::max(flops / 0.9e12, (double)(M + N) * (double)K * 8.0 / 5e12) + 4e-6;
+  if (K > 64 && lo <= 2 && hi > 16) return std::max(flops / 0.9e12, wide / 5e12) + 2e-6;
+  if (K <= 8) return std::max(flops / 0.9e12, (double)M * (double)N * 8.0 / 5e12) + 2e-6;
+  if (lo <= 32 && hi >= 4 * lo && (K <= 64 || hi >= 16384)) return std::max(flops / 0.9e12, wide / 5e12) + 2e-6;
+  return 2.0 * up(M, M < 48 ? 16 : 64) * up(N, N < 48 ? 16 : 64) * up(K, 16) / 0.95e12;
+}
+}  // namespace
+
 void choose_engine(GroupBlock& g, bool split_engine, bool split_all, int slices) {
   g.engine = 0;
   g.swap = false;
@@ -260,17 +278,7 @@ void choose_engine(GroupBlock& g, bool split_engine, bool split_all, int slices)
   };
   const double t_split = split_cost(g.M, g.N);
   const double t_split_sw = split_cost(g.N, g.M);
-  const int mi = (int)std::min<int64_t>(g.M, 1 << 30), ni = (int)std::min<int64_t>(g.N, 1 << 30);
-  const int v = f64_variant_planned(mi, ni, (int)std::min<int64_t>(g.K, 1 << 30));
-  // thin FP64: exact flops, or streaming the wide operand once, whichever binds
-  const double wide = (double)std::max(g.M, g.N) * (double)g.K * 8.0;
-  const double outs = (double)g.M * (double)g.N * 8.0;
-  const double t_f64 =
-      v == 7 ? std::max(2.0 * (double)g.M * (double)g.N * (double)g.K / 0.9e12,
-                        (double)(g.M + g.N) * (double)g.K * 8.0 / 5e12) + 4e-6
-      : v == 6 ? std::max(2.0 * (double)g.M * (double)g.N * (double)g.K / 0.9e12, outs / 5e12) + 2e-6
-      : v >= 4 ? std::max(2.0 * (double)g.M * (double)g.N * (double)g.K / 0.9e12, wide / 5e12) + 2e-6
-               : 2.0 * up(g.M, f64_tile_m(v)) * up(g.N, f64_tile_n(v)) * up(g.K, 16) / 0.95e12;
+  const double t_f64 = f64_model_seconds(g.M, g.N, g.K);
   const double best_split = std::min(t_split, t_split_sw) + 4e-6;  // + split and launch overhead
   if (split_all || best_split < t_f64) {
     g.engine = 1;

@@ -128,7 +128,7 @@ __device__ __forceinline__ void run_record(const ProgRec& r, uint32_t vb, ProgSm
       break;
     case PK_SPLITKRED:
       dev::splitk_reduce_body<true>(a.kred.probs, a.kred.red_prob, a.kred.red_first, a.kred.nred, a.kred.nchunks, vb,
-                                    g);
+                                    g, sm.red);
       break;
     case PK_AMP:
       dev::cc_amp_body<true>(a.amp.tiles, a.amp.items, a.amp.nitems, a.amp.t1, a.amp.t2, a.amp.tau, a.amp.taut,

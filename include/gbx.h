@@ -77,9 +77,9 @@ GBX_API int gbx_local_contraction(int n_a, int n_b, int n_k, const double* d_A, 
  * the GPU's memory to its own caching pool, or a latency-bound loop whose
  * other streams must not be stalled by the device synchronisation of
  * cudaFree.  This entry point calls no cudaMalloc, cudaMallocAsync, cudaFree
- * or allocating library routine.  Its descriptor and split-K partial sums
- * live in one fixed device array of 32 MiB + 4 KiB that the library defines
- * and every GPU that loads the library holds until the process exits.
+ * or allocating library routine.  Its split-K partial sums live in one fixed
+ * device array of 32 MiB that the library defines and every GPU that loads
+ * the library holds until the process exits.
  * Outputs larger than 4,194,304 elements (n_a * n_b) are rejected with
  * GBX_EINVAL.  The first call on a device looks up that array's device
  * address (cudaGetSymbolAddress); make it before any stream capture.  All
@@ -237,8 +237,8 @@ typedef struct {
     int accumulate; /* 1: C += ..., 0: C = ... */
 } gbx_triple;
 
-/* Run all triples in one persistent launch driven by a device-side work
- * queue of 64x64 output tiles.  triples is a host array; it is uploaded with
+/* Run all triples in one launch per kernel kind over a flat list of output
+ * tiles.  triples is a host array; it is uploaded with
  * stream-ordered temporaries.  Triples whose C overlap must not share a call. */
 GBX_API int gbx_grouped_gemm_f64(const gbx_triple* triples, int num_triples, void* stream);
 
@@ -251,8 +251,7 @@ typedef struct gbx_group gbx_group;
 /* Plan a set of triples once (the per-block-pair dgemm calls of
  * transpose_and_dgemm, contraction.cc:1779-1976, and of DLTC task_mul,
  * DLTC/task.cc:83-137, as one batch).  mode GBX_MODE_FP64 runs every triple
- * on the FP64 pipe (DMMA tile shapes 64x64 / 64x16 / 16x64 / 16x16, thin and
- * small-K kernels), GBX_MODE_SPLIT on the split engine (needs a_cs = b_cs =
+ * on the FP64 pipe (the DMMA tile kernel, thin and small-K kernels), GBX_MODE_SPLIT on the split engine (needs a_cs = b_cs =
  * 1; GBX_EUNSUPPORTED otherwise), GBX_MODE_AUTO picks per triple.  slices:
  * split slices (0 = 6).  The triple array is copied; operand memory must
  * stay valid while the group exists.  Triples whose C overlap must not share
@@ -264,14 +263,13 @@ GBX_API int gbx_group_create(const gbx_triple* triples, int num_triples, int mod
  * run batched). */
 GBX_API int gbx_group_execute(gbx_group* g, int per_triple, void* stream);
 /* Autotuner: triples are classed by shape (log4 bins of m, n, k); for each
- * class every candidate (the four FP64 tile shapes; split output widths 32 to
+ * class every candidate (the FP64 model's kernel; split output widths 32 to
  * 256 in both orientations, as the mode allows) is timed with CUDA events on
  * scratch outputs (marginal cost of 4 copies over 1, best of reps) and the
  * fastest is kept; the group is then re-planned.  Synchronises the stream;
  * writes no triple's C. */
 GBX_API int gbx_group_autotune(gbx_group* g, int reps, void* stream);
-/* Per triple: engine (0 FP64, 1 split) and parameter (FP64 tile variant, -1
- * = model; split: 2 * width + swapped); flops = 2 * sum m*n*k.  Any pointer
+/* Per triple: engine (0 FP64, 1 split) and parameter (FP64: -1, the model's kernel; split: 2 * width + swapped); flops = 2 * sum m*n*k.  Any pointer
  * may be NULL. */
 GBX_API int gbx_group_info(const gbx_group* g, int* engines, int* params, double* flops);
 GBX_API int gbx_group_destroy(gbx_group* g);
