@@ -114,6 +114,18 @@ struct MoveSet {
 int run_moves(const MoveSet& ms, const double* src, double* dst, cudaStream_t st);
 int run_moves_scaled(const MoveSet& ms, const double* src, double* dst, double alpha, cudaStream_t st);
 
+// One-call moves (permute.cu): nothing is allocated or uploaded.
+// One move; an accumulating one uses scale * alpha.
+int run_move_one(const MoveDesc& md, const double* src, double* dst, double alpha, cudaStream_t st);
+// nblocks blocks of block_elems elements, block b moved by moves[which[b]]
+// (at most 16 moves, offsets relative to the block; which unused for one).
+int run_block_moves(const std::vector<MoveDesc>& moves, const uint8_t* which, int64_t nblocks, int64_t block_elems,
+                    const double* src, double* dst, cudaStream_t st);
+// Tiles of rows x cols elements into (or out of) one row-major matrix of
+// nrows x ncols tiles; position i of the grid holds tile slots[i].
+int run_pack(int64_t rows, int64_t cols, int64_t nrows, int64_t ncols, const std::vector<int>& slots, bool to_big,
+             const double* src, double* dst, cudaStream_t st);
+
 // Fused permuted sum over one destination layout of rank 2..4: every
 // destination element is formed in one pass as
 //   out = (0 + coef_0 * x_0 + coef_1 * x_1 + ...) [* scale]

@@ -280,28 +280,9 @@ using namespace gbx;
 // ---- one-shot task calls -------------------------------------------------
 
 namespace {
-// Stream-ordered run of a small move list (descriptors uploaded, freed on
-// the stream).
+// The (single) move of a prepared expression.
 int run_moves_once(const std::vector<MoveDesc>& v, const double* src, double* dst, cudaStream_t st) {
-  if (v.empty() || v[0].n == 0) return GBX_OK;
-  MoveSet ms;
-  ms.host = v;
-  uint32_t first[2] = {0, (uint32_t)((v[0].n + 2047) / 2048)};
-  void *dd = nullptr, *df = nullptr;
-  GBX_CUDA(cudaMallocAsync(&dd, sizeof(MoveDesc), st));
-  GBX_CUDA(cudaMemcpyAsync(dd, v.data(), sizeof(MoveDesc), cudaMemcpyHostToDevice, st));
-  GBX_CUDA(cudaMallocAsync(&df, sizeof(first), st));
-  GBX_CUDA(cudaMemcpyAsync(df, first, sizeof(first), cudaMemcpyHostToDevice, st));
-  ms.d_desc = (MoveDesc*)dd;
-  ms.d_first = (uint32_t*)df;
-  ms.ndesc = 1;
-  ms.nchunks = first[1];
-  int rc = run_moves(ms, src, dst, st);
-  cudaFreeAsync(dd, st);
-  cudaFreeAsync(df, st);
-  ms.d_desc = nullptr;
-  ms.d_first = nullptr;
-  return rc;
+  return v.empty() ? GBX_OK : run_move_one(v[0], src, dst, 1.0, st);
 }
 
 // Runs one prepared Multiplication with workspace at ws (at least

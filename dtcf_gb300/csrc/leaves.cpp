@@ -1,8 +1,8 @@
 // Error state, device allocation helpers, and the leaf entry points of the C
 // ABI: block permutes (RRR and DLTC), big-matrix pack / unpack, and the FP64
-// local contraction.  Each leaf builds its tile moves or GEMM problem on the
-// host and runs them with stream-ordered temporaries, so a call never
-// synchronises the host with the device.
+// local contraction.  Each leaf builds its moves or GEMM problem on the host
+// and launches with the descriptors in the kernel's arguments, so a call
+// never synchronises the host with the device.
 #include <algorithm>
 #include <atomic>
 #include <mutex>
@@ -120,42 +120,6 @@ void dev_free(void* p) {
   else cudaFree(p);
 }
 
-// Stream-ordered temporary upload of host data (freed on the same stream).
-static int upload_async(const void* host, size_t bytes, cudaStream_t st, void** dptr) {
-  GBX_CUDA(cudaMallocAsync(dptr, bytes, st));
-  GBX_CUDA(cudaMemcpyAsync(*dptr, host, bytes, cudaMemcpyHostToDevice, st));
-  return GBX_OK;
-}
-
-// Run a small set of moves with stream-ordered descriptor storage.
-static int run_moves_async(const std::vector<MoveDesc>& moves, const double* src, double* dst, cudaStream_t st) {
-  if (moves.empty()) return GBX_OK;
-  MoveSet ms;
-  ms.host = moves;
-  // build the chunk schedule like MoveSet::upload, but stream-ordered
-  std::vector<uint32_t> first(moves.size() + 1);
-  uint64_t c = 0;
-  for (size_t i = 0; i < moves.size(); ++i) {
-    first[i] = (uint32_t)c;
-    c += (moves[i].n + 2047) / 2048;
-  }
-  first[moves.size()] = (uint32_t)c;
-  if (c == 0) return GBX_OK;
-  void *dd = nullptr, *df = nullptr;
-  GBX_TRY(upload_async(moves.data(), sizeof(MoveDesc) * moves.size(), st, &dd));
-  GBX_TRY(upload_async(first.data(), sizeof(uint32_t) * first.size(), st, &df));
-  ms.d_desc = (MoveDesc*)dd;
-  ms.d_first = (uint32_t*)df;
-  ms.ndesc = (int)moves.size();
-  ms.nchunks = (uint32_t)c;
-  int rc = run_moves(ms, src, dst, st);
-  cudaFreeAsync(dd, st);
-  cudaFreeAsync(df, st);
-  ms.d_desc = nullptr;
-  ms.d_first = nullptr;
-  return rc;
-}
-
 // Move describing "source dim i lands at output position perm[i]" for one
 // dense row-major block.
 static MoveDesc permute_move(int dims, const int* perm, const int* widths, int64_t src, int64_t dst) {
@@ -212,15 +176,54 @@ static int big_matrix_order(int dims, const int* vgrid, const int* p_map, int nu
     }
     return r;
   };
+  order.clear();
+  nrows = 0;
+  ncols = -1;
+  // Addresses inside a grid not much larger than the tile count: one pass
+  // over the grid in rank order, the first tile of every position.
+  int64_t cells = 1, row_cells = 1;
+  for (int d = 0; d < dims && cells <= 8ll * num_tiles + 4096; ++d) {
+    cells *= std::max(grid_T[d], 0);
+    if (d < num_row_dim) row_cells = cells;
+  }
+  bool dense = cells <= 8ll * num_tiles + 4096;
+  std::vector<int> at;
+  if (dense) {
+    at.assign((size_t)cells, -1);
+    for (int t = 0; t < num_tiles && dense; ++t) {
+      const int* a = paddr + (int64_t)t * dims;
+      int64_t r = 0;
+      for (int d = 0; d < dims; ++d) {
+        dense = dense && a[d] >= 0 && a[d] < grid_T[d];
+        r = r * grid_T[d] + a[d];
+      }
+      if (dense && at[r] < 0) at[r] = t;
+    }
+  }
+  if (dense) {
+    order.reserve(num_tiles);
+    const int64_t col_cells = row_cells ? cells / row_cells : 0;
+    for (int64_t i = 0; i < row_cells; ++i) {
+      int cur = 0;
+      for (int64_t j = 0; j < col_cells; ++j)
+        if (at[i * col_cells + j] >= 0) {
+          order.push_back(at[i * col_cells + j]);
+          ++cur;
+        }
+      if (cur == 0) continue;
+      if (ncols >= 0 && cur != ncols) return fail(GBX_EINVAL, "tile pattern is not rectangular");
+      ncols = cur;
+      ++nrows;
+    }
+    if (ncols < 0) ncols = 0;
+    return GBX_OK;
+  }
   std::vector<std::tuple<int64_t, int64_t, int>> pl(num_tiles);
   for (int t = 0; t < num_tiles; ++t) {
     const int* a = paddr + (int64_t)t * dims;
     pl[t] = std::make_tuple(rank_of(a, 0, num_row_dim), rank_of(a, num_row_dim, dims), t);
   }
   std::sort(pl.begin(), pl.end());
-  order.clear();
-  nrows = 0;
-  ncols = -1;
   int cur = 0;
   for (int i = 0; i < num_tiles; ++i) {
     if (i > 0 && std::get<0>(pl[i]) == std::get<0>(pl[i - 1]) && std::get<1>(pl[i]) == std::get<1>(pl[i - 1]))
@@ -256,32 +259,20 @@ static int big_matrix_order(int dims, const int* vgrid, const int* p_map, int nu
 
 // loc (optional): the tile data of placement entry t sits at tile slot
 // loc[t] instead of t (create_big_matrix_nl's address_to_location).
-static int big_matrix_moves(int dims, const int* vgrid, const int* p_map, int num_tiles, const int* paddr,
-                            int rpb, int cpb, int nrd, bool to_big, std::vector<MoveDesc>& moves, int* nrows_out,
-                            int* ncols_out, const std::vector<int>* loc = nullptr) {
+static int big_matrix(int dims, const int* vgrid, const int* p_map, int num_tiles, const int* paddr, int rpb, int cpb,
+                      int nrd, bool to_big, const double* src, double* dst, int* nrows_out, int* ncols_out,
+                      cudaStream_t st, const std::vector<int>* loc = nullptr) {
   if (dims < 1 || dims > kMaxDims || num_tiles < 0 || rpb < 0 || cpb < 0 || nrd < 0 || nrd > dims)
     return fail(GBX_EINVAL, "bad big-matrix arguments");
   GBX_TRY(check_perm(dims, p_map));
   std::vector<int> order;
   int nrows = 0, ncols = 0;
   GBX_TRY(big_matrix_order(dims, vgrid, p_map, num_tiles, paddr, nrd, order, nrows, ncols));
-  const int64_t bs = (int64_t)rpb * cpb;
-  const int64_t total_col = (int64_t)ncols * cpb;
-  for (int r = 0; r < nrows; ++r)
-    for (int c = 0; c < ncols; ++c) {
-      int t = order[(size_t)r * ncols + c];
-      int64_t tile_off = (int64_t)(loc ? (*loc)[t] : t) * bs;
-      int64_t big_off = (int64_t)r * rpb * total_col + (int64_t)c * cpb;
-      int64_t ext[2] = {rpb, cpb};
-      int64_t ts[2] = {cpb, 1}, bstr[2] = {total_col, 1};
-      if (to_big)
-        moves.push_back(make_move(2, ext, ts, bstr, tile_off, big_off, 0, 1.0));
-      else
-        moves.push_back(make_move(2, ext, bstr, ts, big_off, tile_off, 0, 1.0));
-    }
+  if (loc)
+    for (int& t : order) t = (*loc)[t];
   if (nrows_out) *nrows_out = nrows;
   if (ncols_out) *ncols_out = ncols;
-  return GBX_OK;
+  return run_pack(rpb, cpb, nrows, ncols, order, to_big, src, dst, st);
 }
 
 }  // namespace gbx
@@ -297,8 +288,7 @@ const char* gbx_version(void) { return "dtcf_gb300 0.1 (sm_103a)"; }
 int gbx_transpose(const double* d_in, double* d_out, const int* perm, int dims, const int* widths, void* stream) {
   GBX_TRY(check_perm(dims, perm));
   GBX_TRY(check_widths(dims, widths));
-  std::vector<MoveDesc> mv{permute_move(dims, perm, widths, 0, 0)};
-  return run_moves_async(mv, d_in, d_out, (cudaStream_t)stream);
+  return run_move_one(permute_move(dims, perm, widths, 0, 0), d_in, d_out, 1.0, (cudaStream_t)stream);
 }
 
 int gbx_transpose_blocks(const double* d_in, double* d_out, int num_blocks, const int* perms, int dims,
@@ -307,13 +297,51 @@ int gbx_transpose_blocks(const double* d_in, double* d_out, int num_blocks, cons
   GBX_TRY(check_widths(dims, widths));
   int64_t bs = 1;
   for (int i = 0; i < dims; ++i) bs *= widths[i];
-  std::vector<MoveDesc> mv;
-  mv.reserve(num_blocks);
+  // every permutation as one word (three bits a dimension), checked when it
+  // first occurs
+  std::vector<uint32_t> key(num_blocks);
+  std::vector<uint32_t> known;
+  uint32_t prev = ~0u;
   for (int b = 0; b < num_blocks; ++b) {
-    GBX_TRY(check_perm(dims, perms + (int64_t)b * dims));
-    mv.push_back(permute_move(dims, perms + (int64_t)b * dims, widths, b * bs, b * bs));
+    const int* p = perms + (int64_t)b * dims;
+    if (b == 0) GBX_TRY(check_perm(dims, p));  // dims too
+    uint32_t k = 0;
+    int stray = 0;
+    for (int d = 0; d < dims; ++d) {
+      k = k << 3 | ((uint32_t)p[d] & 7u);
+      stray |= p[d] & ~7;
+    }
+    if (stray) return check_perm(dims, p);
+    if (k != prev && std::find(known.begin(), known.end(), k) == known.end()) {
+      GBX_TRY(check_perm(dims, p));
+      known.push_back(k);
+    }
+    key[b] = prev = k;
   }
-  return run_moves_async(mv, d_in, d_out, (cudaStream_t)stream);
+  // the blocks' numbers among the permutations of a launch; more than 16 go
+  // out in several launches of consecutive blocks
+  std::vector<MoveDesc> mv;
+  std::vector<uint32_t> seen;
+  std::vector<uint8_t> which(num_blocks);
+  cudaStream_t st = (cudaStream_t)stream;
+  int b0 = 0;
+  for (int b = 0; b < num_blocks; ++b) {
+    size_t i = 0;
+    while (i < seen.size() && seen[i] != key[b]) ++i;
+    if (i == 16) {
+      GBX_TRY(run_block_moves(mv, which.data() + b0, b - b0, bs, d_in + b0 * bs, d_out + b0 * bs, st));
+      mv.clear();
+      seen.clear();
+      b0 = b;
+      i = 0;
+    }
+    if (i == seen.size()) {
+      seen.push_back(key[b]);
+      mv.push_back(permute_move(dims, perms + (int64_t)b * dims, widths, 0, 0));
+    }
+    which[b] = (uint8_t)i;
+  }
+  return run_block_moves(mv, which.data() + b0, num_blocks - b0, bs, d_in + b0 * bs, d_out + b0 * bs, st);
 }
 
 int gbx_dltc_transpose(const double* d_x, const int* ids_x, double* d_y, const int* ids_y, int dim,
@@ -358,10 +386,8 @@ int gbx_dltc_compute(double* d_c, const double* d_a, const double* d_b, int m, i
 int gbx_create_big_matrix(int dims, const int* vgrid, const int* p_map, int num_tiles, const double* d_tiles,
                           const int* permuted_address, int row_per_block, int col_per_block, int num_row_dim,
                           double* d_big, int* nrows, int* ncols, void* stream) {
-  std::vector<MoveDesc> mv;
-  GBX_TRY(big_matrix_moves(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block,
-                           num_row_dim, true, mv, nrows, ncols));
-  return run_moves_async(mv, d_tiles, d_big, (cudaStream_t)stream);
+  return big_matrix(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block, num_row_dim, true,
+                    d_tiles, d_big, nrows, ncols, (cudaStream_t)stream);
 }
 
 int gbx_create_big_matrix_nl(int dims, const int* vgrid, const int* p_map, int num_tiles, const double* d_tiles,
@@ -393,19 +419,15 @@ int gbx_create_big_matrix_nl(int dims, const int* vgrid, const int* p_map, int n
       return fail(GBX_EINVAL, "location %d of tile %d outside [0, %d)", it->second, t, num_slots);
     loc[t] = it->second;
   }
-  std::vector<MoveDesc> mv;
-  GBX_TRY(big_matrix_moves(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block,
-                           num_row_dim, true, mv, nrows, ncols, &loc));
-  return run_moves_async(mv, d_tiles, d_big, (cudaStream_t)stream);
+  return big_matrix(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block, num_row_dim, true,
+                    d_tiles, d_big, nrows, ncols, (cudaStream_t)stream, &loc);
 }
 
 int gbx_revert_big_matrix(int dims, const int* vgrid, const int* p_map, int num_tiles, const int* permuted_address,
                           int row_per_block, int col_per_block, int num_row_dim, const double* d_big, double* d_tiles,
                           void* stream) {
-  std::vector<MoveDesc> mv;
-  GBX_TRY(big_matrix_moves(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block,
-                           num_row_dim, false, mv, nullptr, nullptr));
-  return run_moves_async(mv, d_big, d_tiles, (cudaStream_t)stream);
+  return big_matrix(dims, vgrid, p_map, num_tiles, permuted_address, row_per_block, col_per_block, num_row_dim, false,
+                    d_big, d_tiles, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int gbx_grouped_gemm_f64(const gbx_triple* triples, int num_triples, void* stream) {
