@@ -107,6 +107,14 @@ def lib():
     return _lib
 
 
+def stream_ptr(stream):
+    """The raw handle of a torch stream; the current one when None."""
+    if stream is not None:
+        return stream.cuda_stream
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+
+
 def check(rc):
     if rc != 0:
         raise GbxError(rc, lib().gbx_last_error().decode())

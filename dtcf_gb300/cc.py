@@ -4,7 +4,7 @@ import ctypes
 import numpy as np
 import torch
 
-from ._lib import lib, check
+from ._lib import lib, check, stream_ptr
 
 CCD, CCSD = 0, 1
 FP64, SPLIT = 0, 1
@@ -40,9 +40,7 @@ def config(**kw):
     return c
 
 
-def _stream(stream):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+_stream = stream_ptr
 
 
 class Job:

@@ -912,8 +912,8 @@ __device__ __forceinline__ void small_out_body(const GemmProblem* __restrict__ p
 // Fixed-order reduction of split-K partials into C.  Few partials: one
 // output per thread.  Many (kRedDeep or more): a CTA takes 16 outputs, 16
 // threads each adding every 16th partial, so that the chain of dependent
-// loads and adds is a sixteenth as long (243 partials of 144 outputs:
-// 18.9 us with one thread per output, 5.1 us so).
+// loads and adds is a sixteenth as long (243 partials of 144 outputs, cold:
+// 18.9 us with one thread per output, 10.0 us so).
 template <bool kCoh>
 __device__ __forceinline__ void splitk_reduce_body(const GemmProblem* __restrict__ probs,
                                                    const int* __restrict__ red_prob,

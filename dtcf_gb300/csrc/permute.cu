@@ -122,7 +122,7 @@ struct BoxWalk {
 // What happens to an element on its way out: the two forms are separate code,
 // since a select between x and scale * x issues the multiply either way and
 // FP64 instructions are scarce (2 per clock and SM: the multiplies alone made
-// 2000 8^4 blocks 43 us instead of 26).
+// 2000 8^4 blocks 43 us instead of 24).
 struct BoxCopy {  // +-x
   long long flip;
   __device__ __forceinline__ double sign(double x) const { return __longlong_as_double(__double_as_longlong(x) ^ flip); }

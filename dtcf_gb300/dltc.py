@@ -6,7 +6,7 @@ import ctypes
 import numpy as np
 import torch
 
-from ._lib import lib, check
+from ._lib import lib, check, stream_ptr
 
 MUL, SUM = 0, 1
 CCD_T2, CCSD_T1, CCSD_T2 = 0, 1, 2
@@ -40,9 +40,7 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr())
 
 
-def _stream(stream):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+_stream = stream_ptr
 
 
 def dims(O, V, wbO, wbV, nocc_names=12):

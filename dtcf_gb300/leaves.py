@@ -4,27 +4,33 @@ Arguments that the reference passes as device-resident buffers are torch CUDA
 tensors (float64, contiguous); index arrays are Python sequences.  Each
 function names the reference function it mirrors.
 """
+import array
 import ctypes
 
 import numpy as np
 import torch
 
-from ._lib import lib, check
+from ._lib import lib, check, stream_ptr
 
 
 def _ptr(t):
     assert t.is_cuda and t.dtype == torch.float64 and t.is_contiguous(), "need a contiguous float64 CUDA tensor"
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _iarr(seq):
+    """(holder of the int32 values, their address)."""
+    if isinstance(seq, (list, tuple)):
+        try:
+            a = array.array("i", seq)
+            return a, a.buffer_info()[0]
+        except TypeError:  # nested or not integers: as numpy takes them
+            pass
     a = np.ascontiguousarray(np.asarray(seq, dtype=np.int32).reshape(-1))
-    return a, a.ctypes.data_as(ctypes.c_void_p)
+    return a, a.__array_interface__["data"][0]
 
 
-def _stream(stream):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+_stream = stream_ptr
 
 
 def transpose(inp, out, perm, widths, stream=None):

@@ -12,7 +12,7 @@ import ctypes
 import numpy as np
 import torch
 
-from ._lib import lib, check
+from ._lib import lib, check, stream_ptr
 
 MODES = {"fp64": 0, "split": 1}
 
@@ -23,9 +23,7 @@ class TensorDesc(ctypes.Structure):
                 ("vgrid", ctypes.c_void_p), ("num_tiles", ctypes.c_int), ("tile_address", ctypes.c_void_p)]
 
 
-def _stream(stream):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+_stream = stream_ptr
 
 
 def unique_blocks(sym, vgrid, stream=None):
@@ -89,9 +87,8 @@ class Plan:
         return lib().gbx_plan_flops(self.handle)
 
     def execute(self, A, B, C, alpha=1.0, stream=None):
-        s = stream if stream is not None else torch.cuda.current_stream()
-        check(lib().gbx_execute(self.handle, ctypes.c_void_p(A.tiles.data_ptr()), ctypes.c_void_p(B.tiles.data_ptr()),
-                                ctypes.c_void_p(C.tiles.data_ptr()), alpha, ctypes.c_void_p(s.cuda_stream)))
+        check(lib().gbx_execute(self.handle, A.tiles.data_ptr(), B.tiles.data_ptr(), C.tiles.data_ptr(), alpha,
+                                _stream(stream)))
 
     def __del__(self):
         if getattr(self, "handle", None) and self.handle.value:
