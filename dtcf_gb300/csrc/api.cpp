@@ -51,8 +51,12 @@ int gbx_plan_create(const gbx_tensor_desc* A, const gbx_tensor_desc* B, const gb
   GBX_TRY(layout_from_desc(B, sign, LB));
   GBX_TRY(layout_from_desc(C, sign, LC));
   auto h = std::make_unique<gbx_plan>();
-  GBX_TRY(plan_contraction(LA, LB, LC, split_labels(idxA), split_labels(idxB), split_labels(idxC),
-                           mode == GBX_MODE_SPLIT ? Engine::Split : Engine::F64, slices, h->p));
+  const auto la = split_labels(idxA), lb = split_labels(idxB), lc = split_labels(idxC);
+  ContractionPair pair;
+  // (the split engine's slices would lose a bit of the weighted blocks)
+  const bool paired = mode == GBX_MODE_FP64 && find_contraction_pair(LA, LB, la, lb, pair);
+  GBX_TRY(plan_contraction(LA, LB, LC, la, lb, lc, mode == GBX_MODE_SPLIT ? Engine::Split : Engine::F64, slices, h->p,
+                           false, false, paired ? &pair : nullptr));
   *plan = h.release();
   return GBX_OK;
 }

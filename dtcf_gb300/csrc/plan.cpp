@@ -295,6 +295,33 @@ ContractionPlan::~ContractionPlan() {
   dev_free(d_own_arena);
 }
 
+bool find_contraction_pair(const TensorLayout& A, const TensorLayout& B, const std::vector<std::string>& la,
+                           const std::vector<std::string>& lb, ContractionPair& out) {
+  if ((int)la.size() != A.rank || (int)lb.size() != B.rank) return false;
+  // dims i and j are a whole symmetry group of T, and T stores only its canonical tiles in them
+  auto canonical = [](const TensorLayout& T, int i, int j) {
+    if (i > j) std::swap(i, j);
+    if (T.group[i] < 0 || T.group[i] != T.group[j] || !T.dims[i]->same_as(*T.dims[j])) return false;
+    for (int d = 0; d < T.rank; ++d)
+      if (d != i && d != j && T.group[d] == T.group[i]) return false;
+    for (const Coords& c : T.tiles)
+      if (c[i] < c[j]) return false;
+    return true;
+  };
+  auto in_b = [&](int i) { return (int)(std::find(lb.begin(), lb.end(), la[i]) - lb.begin()); };
+  for (int i = 0; i < A.rank; ++i)
+    for (int j = i + 1; j < A.rank; ++j) {
+      const int bi = in_b(i), bj = in_b(j);
+      if (bi >= B.rank || bj >= B.rank || !canonical(A, i, j) || !canonical(B, bi, bj)) continue;
+      out.x = la[i];
+      out.y = la[j];
+      out.scale_b = B.nelem <= A.nelem;
+      out.half_diagonal = true;
+      return true;
+    }
+  return false;
+}
+
 int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorLayout& C,
                      const std::vector<std::string>& la, const std::vector<std::string>& lb,
                      const std::vector<std::string>& lc, Engine e, int nslices,
@@ -393,6 +420,7 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
   p->b_elems = bo;
   p->c_elems = co;
   for (auto& g : p->groups) choose_engine(g, e == Engine::Split, split_all, nslices);
+  if (pair && pair->half_diagonal) p->alpha_factor = 2.0;
 
   // pack moves: A (rows = extA tuples of irrep h, cols = K tuples of irrep h)
   auto pack = [&](const TensorLayout& T, const std::vector<int>& ext_dims, const std::vector<int>& contr_dims,
@@ -439,7 +467,11 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
           for (size_t i = 0; i < contr_dims.size(); ++i) dstr[contr_dims[i]] = sK[i];
           int64_t dst = (isA ? g.a_off : g.b_off) + rv.second * g.K + kvv.second;
           // off-diagonal block pairs of a symmetric contracted pair count twice
-          if (pair_scaled && px >= 0 && kvv.first[px] > kvv.first[py]) factor *= 2.0;
+          // (or the diagonal ones half)
+          if (pair_scaled && px >= 0) {
+            if (pair->half_diagonal) factor *= kvv.first[px] == kvv.first[py] ? 0.5 : 1.0;
+            else if (kvv.first[px] > kvv.first[py]) factor *= 2.0;
+          }
           ms.host.push_back(make_move(T.rank, ext, sstr, dstr, T.off[id], dst, 0, factor));
         }
       }
@@ -890,7 +922,7 @@ int ContractionPlan::execute(const double* dA, const double* dB, double* dC, dou
   }
   GBX_TRY(f64.run(st));
   if (split) GBX_TRY(run_split_plan(split, !skipA, !skipB, st));
-  return run_moves_scaled(unpackC, d_Cbig, dC, alpha, st);
+  return run_moves_scaled(unpackC, d_Cbig, dC, alpha * alpha_factor, st);
 }
 
 bool ContractionPlan::set_overwrite(double alpha, int64_t c_elems) {
@@ -910,7 +942,7 @@ bool ContractionPlan::set_overwrite(double alpha, int64_t c_elems) {
     // stores of alpha * the product (a store move ignores the run-time factor)
     for (MoveDesc& m : unpackC.host) {
       m.op = 0;
-      m.scale = alpha;
+      m.scale = alpha * alpha_factor;
     }
     store_scale = alpha;
   }

@@ -156,6 +156,7 @@ struct ContractionPlan {
   // Nonzero: the unpack stores store_scale * A B into C, whatever factor
   // execute is given (set_overwrite on a packed plan).
   double store_scale = 0.0;
+  double alpha_factor = 1.0;  // of the unpack (half_diagonal pairs)
   // Makes the plan write C = alpha A B instead of accumulating, when it writes
   // every element of C (the direct items, or the unpack moves: one per C
   // tile); call before build.  false: nothing changed.
@@ -202,10 +203,22 @@ constexpr double kDirectMaxK = 16.0;
 // so the packed GEMMs run over block pairs X >= Y only, the off-diagonal ones
 // weighted 2 in one operand's pack (scale_b: B's, else A's) -- close to half
 // the contracted extent.  Both indices must have the same blocking.
+// half_diagonal: the same sum as 2 (sum_{X>Y} + 1/2 sum_{X=Y}): the diagonal
+// pairs weighted 1/2 in the pack, the unpack's factor doubled, so that no
+// packed value grows (the FP64 ladder at o = 16, v = 48 in blocks of 8: 1193
+// -> 710 us).
 struct ContractionPair {
   std::string x, y;
   bool scale_b = true;
+  bool half_diagonal = false;
 };
+
+// The pair of a contraction over RRR layouts: two contracted indices that are
+// one symmetry group's two indices in A and in B, of which only block pairs
+// x >= y are stored, so that every other block is the stored one permuted,
+// times the sign, in both.
+bool find_contraction_pair(const TensorLayout& A, const TensorLayout& B, const std::vector<std::string>& la,
+                           const std::vector<std::string>& lb, ContractionPair& out);
 
 int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorLayout& C,
                      const std::vector<std::string>& la, const std::vector<std::string>& lb,
