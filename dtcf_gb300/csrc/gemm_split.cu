@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <utility>
 
 #include "bodies.cuh"
 #include "program.h"
@@ -215,10 +216,10 @@ struct SplitCfg {
   static constexpr int kStageBytes = (BM + BN) * BK * 2;
   // narrow tiles: two CTAs per SM (half the shared memory each) and deeper
   // TMEM buffering, since their chunks are short and drains come often
-  static constexpr int kCtasPerSm = BN <= 64 ? 2 : 1;
-  static constexpr int kSmemBudget = (BN <= 64 ? 100 : 200) * 1024;
+  static constexpr int kCtasPerSm = BN <= 32 ? 2 : 1;
+  static constexpr int kSmemBudget = (BN <= 32 ? 100 : 200) * 1024;
   static constexpr int kStages = (kSmemBudget / kStageBytes) < 8 ? (kSmemBudget / kStageBytes) : 8;
-  static constexpr int kAccBufs = BN <= 32 ? 8 : (BN <= 64 ? 4 : 2);
+  static constexpr int kAccBufs = BN <= 32 ? 8 : 2;
   static constexpr uint32_t kTmemCols = (kAccBufs * BN <= 32) ? 32 : (kAccBufs * BN <= 64) ? 64
                                         : (kAccBufs * BN <= 128) ? 128 : (kAccBufs * BN <= 256) ? 256 : 512;
   // drain warps: 4 per 64 columns (one per TMEM lane quarter), at least 4
@@ -740,54 +741,94 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
   }
 }
 
-// ---- k-stationary kernel: S <= 4, 64-column output tiles -----------------
+// ---- k-stationary kernel: 64-column output tiles, any slice count -------------
 //
 // The pair-by-pair kernel above streams a k-block's A and B slices once per
 // slice pair that uses them (2 S (S + 1) / 2 tile loads per k-block).  Here
-// every k-block's S A slices and S B slices are loaded once into a ring of
-// (A_s, B_s) slots and all S (S + 1) / 2 products are issued from there into
-// per-level TMEM accumulators (level l at columns l * 64 of a buffer, two
-// buffers).  A level sums at most S products of 64 K-elements per k-block,
-// each below 2^20 in magnitude, so 16 / S k-blocks fit below 2^24 and the
-// FP32 sums are exact; the drain warps then combine the levels into an exact
-// int64 Y = sum_l X_l 2^(8 (L - l)) per output (|Y| <= K 2^(14 + 8 L) < 2^63
-// for L <= 3 and K < 2^24) and scale it to FP64 once per tile.
+// every k-block's S A slices and S B slices are loaded once and all
+// S (S + 1) / 2 products are issued from there into per-level TMEM accumulators of 64 columns: B slices
+// sit back to back in the stage, so one instruction of A slice s covers
+// every level it contributes to (product (s, t) lands in level s + t - 2's
+// columns when D starts at level s - 1's).
+//
+// What bounds it is shared memory: at S = 4 a K step of 16 reads 16 KB of A
+// and 20 KB of B and TMA writes 24 KB, 60 KB at 128 bytes a clock against 320
+// clocks of MMAs.  9216 x 768 x 4096 runs at 1305 TFLOP/s of slice products
+// at S = 4 (58% of the tensor pipe; the bound above is 68%), 1250 at 5, 1240
+// at 6 and 1180 at 7, where the pair-by-pair kernel reaches 940.
+//
+// A k-block is 64 elements up to four slices (two stages or more); beyond
+// only one such stage would fit, so 32 (S = 4 takes 453 us with 32, 441 with
+// 64).
+//
+// TMEM holds eight such accumulators.  Level l sums l + 1 products of at
+// most 2^14 per element, so 1024 / (l + 1) elements fit below 2^24 and are
+// exact.  The high levels, which fill up first, have two buffers and are
+// drained every kHiBlocks k-blocks behind the MMAs of the next ones; the low
+// ones have one and are drained more rarely, the MMAs of a k-block starting
+// with its high levels while they are.  S = 4: four high levels; 5: three
+// and two low ones; 6: two and four; 7: one and six.
+//
+// The drains add the levels exactly into 64-bit sums (levels apart by 2^8;
+// two sums 2^32 apart from five slices on), which become one FP64 value per
+// output at the end of a tile.  (Rounding and scaling by integer instructions
+// instead of a conversion and a multiply: 20000 x 64 x 256 at 6 slices 80
+// instead of 66 us.)
 constexpr int kKsBN = 64;
-constexpr int kKsSlots = 8;        // (A slice, B slice) pairs, 24 KB each: two k-blocks of 4 slices
-constexpr int kKsDrainWarps = 8;   // 4 TMEM lane quarters x 2 column halves
+constexpr int ks_bk(int S) { return S <= 4 ? 64 : 32; }  // elements of a k-block
+constexpr int kKsDrainWarps = 8;     // 4 TMEM lane quarters x 2 column halves
 constexpr int kKsThreads = 64 + 32 * kKsDrainWarps;
-constexpr int kKsMaxS = 4;
+constexpr int kKsMinS = 2, kKsMaxS = 7;
 
+template <int S>
+struct KsCfg {
+  static constexpr int L = S - 1;
+  static constexpr int kHi = S <= 4 ? S : 8 - S;  // levels with two buffers
+  static constexpr int kLo = S - kHi;             // levels with one (kLo + 2 kHi <= 8)
+  static constexpr int kBK = ks_bk(S);
+  static constexpr int kHiBlocks = 1024 / S / kBK;
+  static constexpr int kLoBlocks = kLo ? 1024 / (kLo ? kLo : 1) / kBK : 1;
+  static constexpr int kStageBytes = S * (BM + kKsBN) * kBK * 2;
+  static constexpr int kStages = (220 * 1024 / kStageBytes) < 8 ? 220 * 1024 / kStageBytes : 8;
+  static constexpr int kCut = S <= 4 ? 0 : S - 4;  // levels below this go to the upper sum
+  // the drains' level loops: unrolled, their TMEM reads overlap the sums
+  // before (S = 6: 978 instead of 1019 us); at S = 4 that spills
+  static constexpr int kUnroll = S <= 4 ? 1 : S;
+};
+
+template <int S>
 struct KsSmem {
-  alignas(1024) __nv_bfloat16 a[kKsSlots][BM * BK];
-  alignas(1024) __nv_bfloat16 b[kKsSlots][kKsBN * BK];
-  uint64_t full[kKsSlots], empty[kKsSlots], accfull[2], accempty[2], done;
+  using Cfg = KsCfg<S>;
+  struct alignas(1024) Stage {
+    __nv_bfloat16 a[S][BM * Cfg::kBK];
+    __nv_bfloat16 b[S][kKsBN * Cfg::kBK];
+  };
+  Stage st[Cfg::kStages];
+  uint64_t full[Cfg::kStages], empty[Cfg::kStages], hifull[2], hiempty[2], lofull, loempty, done;
   uint32_t tmem_base;
 };
 
-// S is a template parameter so that the slice-pair loops of the MMA issuer
-// (one thread issuing every tcgen05.mma) unroll completely.
 template <int S>
 __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParams P) {
+  using Cfg = KsCfg<S>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  KsSmem& sm = *reinterpret_cast<KsSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  KsSmem<S>& sm = *reinterpret_cast<KsSmem<S>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int L = S - 1;
-  constexpr int D = 16 / S;  // k-blocks per exact accumulation group
-  constexpr uint32_t kTx = (BM + kKsBN) * BK * 2;
-  // a stage is one k-block's S slot pairs behind one full and one empty
-  // barrier: one wait and one commit per k-block for the MMA-issuing thread
-  constexpr int kStages = kKsSlots / S;
+  constexpr int L = Cfg::L, kStages = Cfg::kStages;
   constexpr uint32_t kCols = 512;
+  // accumulator columns: the low levels, then the two buffers of the high ones
+  constexpr uint32_t kHiCol = Cfg::kLo * kKsBN, kHiCols = Cfg::kHi * kKsBN;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&sm.full[i], 1);
       mbar_init(&sm.empty[i], 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&sm.accfull[b], 1);
-      mbar_init(&sm.accempty[b], kKsDrainWarps);
+      mbar_init(&sm.hifull[b], 1);
+      mbar_init(&sm.hiempty[b], kKsDrainWarps);
     }
+    mbar_init(&sm.lofull, 1);
+    mbar_init(&sm.loempty, kKsDrainWarps);
     mbar_init(&sm.done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -800,10 +841,9 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  const uint32_t buf_cols = (uint32_t)(S * kKsBN);
 
   if (warp == 0) {
-    // ---------------- TMA producer: a k-block's S slice pairs ----------------
+    // ---------------- TMA producer: a k-block's slices ----------------
     if (lane == 0) {
       int st = 0;
       uint32_t phase = 0;
@@ -812,16 +852,16 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
         const TileInfo ti = decode_tile<kKsBN>(P, tile);
         const CUtensorMap* ma = P.maps + 2 * ti.p;
         const CUtensorMap* mb = P.maps + 2 * ti.p + 1;
-        for (int kb = ti.kb0; kb < ti.kb0 + ti.nkb && ok; ++kb) {
+        for (int kb = ti.kb0; kb < ti.kb0 + ti.nkb; ++kb) {
           if (!mbar_wait(&sm.empty[st], phase ^ 1, P.err, 21)) {
             ok = false;
             break;
           }
-          mbar_expect_tx(&sm.full[st], (uint32_t)S * kTx);
+          mbar_expect_tx(&sm.full[st], (uint32_t)Cfg::kStageBytes);
 #pragma unroll
           for (int s = 0; s < S; ++s) {
-            tma_load_3d(sm.a[st * S + s], ma, &sm.full[st], kb * BK, ti.m0, s);
-            tma_load_3d(sm.b[st * S + s], mb, &sm.full[st], kb * BK, ti.n0, s);
+            tma_load_3d(sm.st[st].a[s], ma, &sm.full[st], kb * Cfg::kBK, ti.m0, s);
+            tma_load_3d(sm.st[st].b[s], mb, &sm.full[st], kb * Cfg::kBK, ti.n0, s);
           }
           if (++st == kStages) {
             st = 0;
@@ -829,6 +869,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
           }
         }
       }
+      // wait (bounded) for the copies this warp issued to land before leaving
       for (int i = 0; i < kStages; ++i) {
         if (--st < 0) {
           st = kStages - 1;
@@ -846,58 +887,81 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      int st = 0, buf = 0;
-      uint32_t phase = 0, aphase = 0;
+      int st = 0, hb = 0;
+      uint32_t phase = 0, hphase = 0, lphase = 0;
       bool ok = true;
-      // slot descriptors: slot 0's plus the slot offset in 16-byte units
+      // stage descriptors: stage 0's plus the stage offset in 16-byte units
       // (the address field holds shared-memory address / 16, below 2^14)
-      const uint64_t ad0 = sdesc(smem_u32(sm.a[0])), bd0 = sdesc(smem_u32(sm.b[0]));
-      constexpr uint64_t kAStep = (uint64_t)(BM * BK * 2) >> 4, kBStep = (uint64_t)(kKsBN * BK * 2) >> 4;
+      const auto desc = [](const void* p) { return Cfg::kBK == 64 ? sdesc(smem_u32(p)) : sdesc64(smem_u32(p)); };
+      const uint64_t ad0 = desc(sm.st[0].a), bd0 = desc(sm.st[0].b);
+      constexpr uint64_t kStep = (uint64_t)sizeof(typename KsSmem<S>::Stage) >> 4;
+      constexpr uint64_t kAStep = (uint64_t)(BM * Cfg::kBK * 2) >> 4, kBStep = (uint64_t)(kKsBN * Cfg::kBK * 2) >> 4;
       for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
         const int nkb = decode_tile<kKsBN>(P, tile).nkb;
-        for (int g0 = 0; g0 < nkb && ok; g0 += D) {
-          if (!mbar_wait(&sm.accempty[buf], aphase ^ 1, P.err, 22)) {
+        int hn = 0, ln = 0;  // k-blocks in the current accumulators
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (hn == 0 && !mbar_wait(&sm.hiempty[hb], hphase ^ 1, P.err, 22)) {
+            ok = false;
+            break;
+          }
+          if (!mbar_wait(&sm.full[st], phase, P.err, 23)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const int g1 = min(nkb, g0 + D);
-          for (int kb = g0; kb < g1 && ok; ++kb) {
-            if (!mbar_wait(&sm.full[st], phase, P.err, 23)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const int base = st * S;
-            const uint32_t fresh = kb == g0 ? 0u : 1u;
-            // One UMMA per A slice s and K step: B slices 1 .. S + 1 - s sit
-            // back to back in the stage (64 rows each), so one instruction of
-            // N = 64 (S + 1 - s) forms every product (s, t) with t <= S + 1 - s
-            // at once; with D at column 64 (s - 1) of the buffer, product
-            // (s, t) lands in columns 64 (s + t - 2), its level's accumulator.
-            // The first instruction of a group (s = 1, N = 64 S) spans every
-            // level and starts them all from zero.
-            const uint64_t b0 = bd0 + (uint64_t)base * kBStep;
+          const uint64_t as = ad0 + (uint64_t)st * kStep, bs = bd0 + (uint64_t)st * kStep;
+          // high levels kLo .. L: A slice s with B slices max(1, kLo + 2 - s) .. S + 1 - s
+          const uint32_t hcol = tmem + kHiCol + (uint32_t)hb * kHiCols;
 #pragma unroll
-            for (int s = 1; s <= S; ++s) {
-              const uint32_t d = tmem + (uint32_t)buf * buf_cols + (uint32_t)((s - 1) * kKsBN);
-              const uint64_t a0 = ad0 + (uint64_t)(base + s - 1) * kAStep;
+          for (int s = 1; s <= S; ++s) {
+            const int l0 = s - 1 > Cfg::kLo ? s - 1 : Cfg::kLo;  // first high level of slice s
+            const int t0 = l0 + 2 - s;
 #pragma unroll
-              for (int k = 0; k < BK / 16; ++k)
-                umma(d, a0 + (uint64_t)(k * 2), b0 + (uint64_t)(k * 2), idesc_bf16_n(kKsBN * (S + 1 - s)),
-                     (s == 1 && k == 0) ? fresh : 1u);
-            }
-            umma_commit(&sm.empty[st]);
-            if (++st == kStages) {
-              st = 0;
-              phase ^= 1;
+            for (int k = 0; k < Cfg::kBK / 16; ++k)
+              umma(hcol + (uint32_t)((l0 - Cfg::kLo) * kKsBN), as + (uint64_t)(s - 1) * kAStep + (uint64_t)(k * 2),
+                   bs + (uint64_t)(t0 - 1) * kBStep + (uint64_t)(k * 2), idesc_bf16_n(kKsBN * (S - l0)),
+                   (s == 1 && k == 0 && hn == 0) ? 0u : 1u);
+          }
+          if (Cfg::kLo == 0) umma_commit(&sm.empty[st]);
+          if (++hn == Cfg::kHiBlocks || kb == nkb - 1) {
+            umma_commit(&sm.hifull[hb]);
+            hn = 0;
+            if (++hb == 2) {
+              hb = 0;
+              hphase ^= 1;
             }
           }
-          if (!ok) break;
-          umma_commit(&sm.accfull[buf]);
-          if (++buf == 2) {
-            buf = 0;
-            aphase ^= 1;
+          if constexpr (Cfg::kLo > 0) {
+            if (ln == 0) {
+              if (!mbar_wait(&sm.loempty, lphase ^ 1, P.err, 27)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+            }
+            // low levels 0 .. kLo - 1: A slice s with B slices 1 .. kLo + 1 - s,
+            // at most 256 columns to an instruction
+#pragma unroll
+            for (int s = 1; s <= Cfg::kLo; ++s) {
+              const int n = Cfg::kLo + 1 - s;
+#pragma unroll
+              for (int k = 0; k < Cfg::kBK / 16; ++k)
+#pragma unroll
+                for (int c = 0; c < n; c += 4)
+                  umma(tmem + (uint32_t)((s - 1 + c) * kKsBN), as + (uint64_t)(s - 1) * kAStep + (uint64_t)(k * 2),
+                       bs + (uint64_t)c * kBStep + (uint64_t)(k * 2), idesc_bf16_n(kKsBN * (n - c < 4 ? n - c : 4)),
+                       (s == 1 && k == 0 && ln == 0) ? 0u : 1u);
+            }
+            if (++ln == Cfg::kLoBlocks || kb == nkb - 1) {
+              umma_commit(&sm.lofull);
+              ln = 0;
+              lphase ^= 1;
+            }
+            umma_commit(&sm.empty[st]);
+          }
+          if (++st == kStages) {
+            st = 0;
+            phase ^= 1;
           }
         }
       }
@@ -905,45 +969,82 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
       mbar_wait(&sm.done, 0, P.err, 26);
     }
   } else {
-    // ---------------- drain: exact int64 level recombination ----------------
+    // ---------------- drain: exact 64-bit level recombination ----------------
     const int quarter = warp & 3;               // TMEM lanes this warp may read
     const int half = (warp - 2) >> 2;           // which 32 of the 64 columns
-    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    int buf = 0;
-    uint32_t aphase = 0;
+    const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 32);
+    int hb = 0;
+    uint32_t hphase = 0, lphase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
       const TileInfo ti = decode_tile<kKsBN>(P, tile);
       const DevProblem& pr = P.probs[ti.p];
-      long long Y[32];
+      long long Y[32], U[Cfg::kCut ? 32 : 1];
 #pragma unroll
       for (int j = 0; j < 32; ++j) Y[j] = 0;
-      for (int g0 = 0; g0 < ti.nkb; g0 += D) {
-        int w_ok = lane == 0 ? (int)mbar_wait(&sm.accfull[buf], aphase, P.err, 24) : 1;
-        w_ok = __shfl_sync(0xffffffffu, w_ok, 0);
-        if (!w_ok) {
-          ok = false;
-          break;
-        }
-        __syncwarp();
-        tc_fence_after();
-        for (int l = 0; l <= L; ++l) {
-          uint32_t r[2][16];
-          const uint32_t col = (uint32_t)buf * buf_cols + (uint32_t)(l * kKsBN + half * 32);
-          tmem_ld16(tmem + lane_addr + col, r[0]);
-          tmem_ld16(tmem + lane_addr + col + 16, r[1]);
-          tmem_wait_ld();
-          const int sh = 8 * (L - l);
-          const long long w = 1ll << sh;
+      if (Cfg::kCut) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) U[Cfg::kCut ? j : 0] = 0;
+      }
+      // adds level l's 32 columns at col, weighted 2^(8 (L - l)) (below the
+      // cut 2^(8 (kCut - 1 - l)) of the upper sum)
+      auto add = [&](int l, uint32_t col) {
+        uint32_t r[2][16];
+        tmem_ld16(base + col, r[0]);
+        tmem_ld16(base + col + 16, r[1]);
+        tmem_wait_ld();
+        if (Cfg::kCut && l < Cfg::kCut) {
+          const int w = 1 << (8 * (Cfg::kCut - 1 - l));
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            U[Cfg::kCut ? j : 0] += (long long)__float2int_rn(__uint_as_float(r[j >> 4][j & 15])) * w;
+        } else {
+          const int w = 1 << (8 * (L - l));
 #pragma unroll
           for (int j = 0; j < 32; ++j) Y[j] += (long long)__float2int_rn(__uint_as_float(r[j >> 4][j & 15])) * w;
         }
+      };
+      auto wait = [&](uint64_t* bar, uint32_t parity) {
+        int w_ok = lane == 0 ? (int)mbar_wait(bar, parity, P.err, 24) : 1;
+        w_ok = __shfl_sync(0xffffffffu, w_ok, 0);
+        __syncwarp();
+        tc_fence_after();
+        return w_ok != 0;
+      };
+      auto release = [&](uint64_t* bar) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.accempty[buf]);
-        if (++buf == 2) {
-          buf = 0;
-          aphase ^= 1;
+        if (lane == 0) mbar_arrive(bar);
+      };
+      int hn = 0, ln = 0;
+      for (int kb = 0; kb < ti.nkb; ++kb) {
+        if (++hn == Cfg::kHiBlocks || kb == ti.nkb - 1) {
+          if (!wait(&sm.hifull[hb], hphase)) {
+            ok = false;
+            break;
+          }
+#pragma unroll(Cfg::kUnroll)
+          for (int l = Cfg::kLo; l <= L; ++l)
+            add(l, kHiCol + (uint32_t)hb * kHiCols + (uint32_t)((l - Cfg::kLo) * kKsBN));
+          release(&sm.hiempty[hb]);
+          hn = 0;
+          if (++hb == 2) {
+            hb = 0;
+            hphase ^= 1;
+          }
+        }
+        if constexpr (Cfg::kLo > 0) {
+          if (++ln == Cfg::kLoBlocks || kb == ti.nkb - 1) {
+            if (!wait(&sm.lofull, lphase)) {
+              ok = false;
+              break;
+            }
+#pragma unroll(Cfg::kUnroll)
+            for (int l = 0; l < Cfg::kLo; ++l) add(l, (uint32_t)(l * kKsBN));
+            release(&sm.loempty);
+            ln = 0;
+            lphase ^= 1;
+          }
         }
       }
       if (!ok) break;
@@ -957,7 +1058,9 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
           if (col < pr.N) {
             int ex = ea + pr.eB[col] - 2 * 1022 - 14 - 8 * L + 1023;
             ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-            crow[col] = (double)Y[j] * __longlong_as_double((long long)ex << 52);
+            double v = (double)Y[j];
+            if (Cfg::kCut) v = __fma_rn((double)U[Cfg::kCut ? j : 0], 0x1.0p32, v);
+            crow[col] = v * __longlong_as_double((long long)ex << 52);
           }
         }
       }
@@ -1033,35 +1136,16 @@ int encode_slices(CUtensorMap* map, const __nv_bfloat16* base, int64_t S, int64_
 
 }  // namespace
 
-// Output tile width per problem: the smallest modelled time over the
-// instantiated widths.  A k-block costs the largest of: tensor 2.72 * BN
-// cycles (128 x BN x 64 MACs at ~3000 MAC/clk), shared-memory reads
-// (16 KB of A + BN * 128 B of B at 128 B/clk) and L2 -> SM traffic (same
-// bytes at ~76 B/clk per SM).  The 256 width spills a little and is de-rated.
-// gbx_split_set_width() overrides the choice (tuning).
-constexpr int kWidths[4] = {32, 64, 128, 256};
+// Output tile width of a problem: 64 columns, the k-stationary kernel.
+// gbx_split_set_width() and the autotuners may take another (the
+// pair-by-pair kernel).
 static int g_width_override = 0;
 
-int choose_width(int64_t N, int S) {
-  if (g_width_override) return g_width_override;
-  // up to 4 slices the k-stationary kernel (64 columns) loads every slice
-  // once per k-block and keeps its sums in registers
-  if (S <= kKsMaxS) return kKsBN;
-  int best = 256;
-  double best_cost = 1e300;
-  for (int bn : kWidths) {
-    const double tiles = (double)((N + bn - 1) / bn);
-    const double bytes = 16384.0 + 128.0 * bn;
-    double per_kb = std::max(std::max(2.72 * bn, 128.0 + bn), bytes / 76.0);
-    if (bn == 256) per_kb *= 1.15;
-    const double cost = tiles * per_kb;
-    if (cost < best_cost * 0.999) {
-      best_cost = cost;
-      best = bn;
-    }
-  }
-  return best;
-}
+int choose_width() { return g_width_override ? g_width_override : kKsBN; }
+
+// The k-stationary kernel's exact 64-bit sums: 2^(14 + 24) a level sum and
+// element from four slices on, S products to a level.
+int64_t ks_max_k(int S) { return S <= 4 ? 1 << 24 : 1 << 22; }
 
 struct SplitLaunch {  // the problems of one output tile width
   int bn = 0;
@@ -1080,6 +1164,7 @@ struct SplitPlan {
   std::vector<SplitProblem> host;
   std::vector<int> width;  // per problem
   std::vector<int> thin;  // per problem: 0, or the thin-K kernel with a 64 (1) or 32 (2) element k-block
+  std::vector<int> kb;    // per problem: k-block
   unsigned char* d_persist = nullptr;    // slices and exponents of constant plan operands
   unsigned char* d_own_arena = nullptr;  // the per-run region when no arena was given
   SplitRowSet* d_sets_a = nullptr;  // long rows from the plan's packed A
@@ -1129,6 +1214,14 @@ int set_smem_attr() {
   return GBX_OK;
 }
 
+template <int... I>
+int set_ks_attr(std::integer_sequence<int, I...>) {
+  for (cudaError_t e : {cudaFuncSetAttribute(split_ks_kernel<kKsMinS + I>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(sizeof(KsSmem<kKsMinS + I>) + 1024))...})
+    GBX_CUDA(e);
+  return GBX_OK;
+}
+
 namespace {
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -1141,8 +1234,8 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 struct SplitLayout {
   struct Prob {
     int bn = 0;
-    bool thin = false;
-    int kb = BK;  // k-block: 64, or 32 for thin problems with K <= 32
+    bool thin = false, ks_kernel = false;
+    int kb = BK;  // k-block: 64; 32 from five slices on in the k-stationary kernel and for thin problems with K <= 32
     int64_t Mp = 0, Np = 0, Kp = 0;
     int ra = 0, rb = 0;      // region of the GEMM's A and B slices
     int64_t sa = 0, sb = 0;  // slice offsets
@@ -1172,14 +1265,14 @@ int split_layout(const std::vector<SplitProblem>& probs, int S, bool static_a, b
     SplitLayout::Prob o;
     // thin-K problems (one k-block, at most 32 columns) take the thin kernel
     o.thin = q.K <= BK && q.N <= kThinBN && S <= 7;
-    o.bn = o.thin ? kThinBN : (q.width ? q.width : choose_width(q.N, S));
-    // the k-stationary kernel's exact int64 sums need K < 2^24
-    if (!o.thin && S <= kKsMaxS && o.bn == kKsBN && q.K >= (1 << 24)) o.bn = 128;
+    o.bn = o.thin ? kThinBN : (q.width ? q.width : choose_width());
+    if (!o.thin && o.bn == kKsBN && q.K >= ks_max_k(S)) o.bn = 128;
+    o.ks_kernel = !o.thin && o.bn == kKsBN;
     if (!o.thin && o.bn != 32 && o.bn != 64 && o.bn != 128 && o.bn != 256)
       return fail(GBX_EINVAL, "split tile width %d", o.bn);
     o.Mp = (q.M + BM - 1) / BM * BM;
     o.Np = (q.N + o.bn - 1) / o.bn * o.bn;
-    o.kb = o.thin && q.K <= 32 ? 32 : BK;
+    o.kb = o.ks_kernel ? ks_bk(S) : o.thin && q.K <= 32 ? 32 : BK;
     o.Kp = (q.K + o.kb - 1) / o.kb * o.kb;
     // the GEMM's A rows come from plan operand B when swapped
     const bool a_const = q.a_is_plan_b ? static_b : static_a;
@@ -1203,10 +1296,10 @@ int split_layout(const std::vector<SplitProblem>& probs, int S, bool static_a, b
     if (nkb < 1) return fail(GBX_EINVAL, "split problem without a k-block");
     // split K when the output tiles of all problems leave SMs idle; ranges are
     // whole exact-accumulation chunks: 16 k-blocks for the pair-by-pair
-    // kernel, 16 / S for the k-stationary one (whose exact groups are that
-    // short, so few-tile problems -- matrix-vector shapes, small outputs with
-    // long K -- spread over many more CTAs instead of walking K serially)
-    const int chunk = (!o.thin && S <= kKsMaxS && o.bn == kKsBN) ? 16 / S : kChunkKb;
+    // kernel, 256 elements for the k-stationary one (so few-tile problems --
+    // matrix-vector shapes, small outputs with long K -- spread over many more
+    // CTAs instead of walking K serially)
+    const int chunk = o.ks_kernel ? 256 / o.kb : kChunkKb;
     int ks = 1;
     if (!o.thin && out_tiles < kSplitFill && nkb > 2 * chunk) {
       int want = (int)((kSplitFill + out_tiles - 1) / out_tiles);
@@ -1250,6 +1343,7 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
   for (auto& o : lay.p) {
     sp->width.push_back(o.bn);
     sp->thin.push_back(o.thin ? (o.kb == 32 ? 2 : 1) : 0);
+    sp->kb.push_back(o.kb);
   }
   unsigned char* base[2] = {nullptr, nullptr};
   const size_t b0 = lay.bytes(0), b1 = lay.bytes(1);
@@ -1414,15 +1508,9 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
   GBX_TRY(dev_alloc((void**)&sp->d_err, sizeof(int)));
   GBX_CUDA(cudaMemset(sp->d_err, 0, sizeof(int)));
   GBX_TRY(set_smem_attr<32>());
-  GBX_TRY(set_smem_attr<64>());
   GBX_TRY(set_smem_attr<128>());
   GBX_TRY(set_smem_attr<256>());
-  GBX_CUDA(cudaFuncSetAttribute(split_ks_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(KsSmem) + 1024)));
-  GBX_CUDA(cudaFuncSetAttribute(split_ks_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(KsSmem) + 1024)));
-  GBX_CUDA(cudaFuncSetAttribute(split_ks_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(KsSmem) + 1024)));
+  GBX_TRY(set_ks_attr(std::make_integer_sequence<int, kKsMaxS - kKsMinS + 1>()));
   GBX_CUDA(cudaFuncSetAttribute(split_thin_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(ThinSmem<64>) + 1024)));
   GBX_CUDA(cudaFuncSetAttribute(split_thin_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1496,9 +1584,16 @@ int launch_width(const GemmParams& P, int nsm, cudaStream_t st) {
   return GBX_OK;
 }
 
+template <int S>
+int launch_ks(const GemmParams& P, int nsm, cudaStream_t st) {
+  split_ks_kernel<S><<<std::min(P.total_tiles, nsm), kKsThreads, sizeof(KsSmem<S>) + 1024, st>>>(P);
+  GBX_CUDA(cudaGetLastError());
+  return GBX_OK;
+}
+
 // The GEMM kernel of one launch class -- bn 0 / 1: thin-K with a 64 / 32
-// element k-block; 64 with S <= 4: k-stationary; else the pair-by-pair
-// kernel of that output tile width -- over the problems of P.
+// element k-block; 64: k-stationary; else the pair-by-pair kernel of that
+// output tile width -- over the problems of P.
 int launch_split_gemm(int bn, const GemmParams& P, cudaStream_t st) {
   if (P.total_tiles <= 0) return GBX_OK;
   int dev = 0, nsm = 152;
@@ -1523,16 +1618,14 @@ int launch_split_gemm(int bn, const GemmParams& P, cudaStream_t st) {
   switch (bn) {
     case 32: return launch_width<32>(P, nsm, st);
     case 64:
-      if (P.S <= kKsMaxS) {
-        const int g = std::min(P.total_tiles, nsm);
-        const size_t sh = sizeof(KsSmem) + 1024;
-        if (P.S == 2) split_ks_kernel<2><<<g, kKsThreads, sh, st>>>(P);
-        else if (P.S == 3) split_ks_kernel<3><<<g, kKsThreads, sh, st>>>(P);
-        else split_ks_kernel<4><<<g, kKsThreads, sh, st>>>(P);
-        GBX_CUDA(cudaGetLastError());
-        return GBX_OK;
+      switch (P.S) {
+        case 2: return launch_ks<2>(P, nsm, st);
+        case 3: return launch_ks<3>(P, nsm, st);
+        case 4: return launch_ks<4>(P, nsm, st);
+        case 5: return launch_ks<5>(P, nsm, st);
+        case 6: return launch_ks<6>(P, nsm, st);
+        default: return launch_ks<7>(P, nsm, st);
       }
-      return launch_width<64>(P, nsm, st);
     case 128: return launch_width<128>(P, nsm, st);
     default: return launch_width<256>(P, nsm, st);
   }
@@ -1657,7 +1750,7 @@ double split_plan_tensor_flops(const SplitPlan* sp) {
     const SplitProblem& p = sp->host[i];
     const int bn = sp->width[i];  // thin-K problems: 32
     double Mp = (double)((p.M + BM - 1) / BM * BM), Np = (double)((p.N + bn - 1) / bn * bn);
-    const int kb = sp->thin[i] == 2 ? 32 : BK;
+    const int kb = sp->kb[i];
     double Kp = (double)((p.K + kb - 1) / kb * kb);
     f += 2.0 * pairs * Mp * Np * Kp;
   }

@@ -110,8 +110,7 @@ GBX_API int gbx_cc_read_energy(gbx_cc_job* job, double* energy, void* stream);
 GBX_API int gbx_cc_profile(gbx_cc_job* job, int cap, float* ms, double* flops, double* bytes, int* kind, int* plan,
                            char* names, int name_len, int* count, void* stream);
 /* Kernel choice of one contraction's packed GEMMs: the split output tile
- * width (64 with at most 4 slices: the k-stationary kernel; 0: the width
- * model's choice per GEMM), the number of split and FP64 GEMMs (both 0 for a
+ * width (64: the k-stationary kernel; 0: the default, 64), the number of split and FP64 GEMMs (both 0 for a
  * contraction on the direct engine), the slices. */
 GBX_API int gbx_cc_plan_info(const gbx_cc_job* job, int contraction, int* split_width, int* n_split, int* n_f64,
                              int* slices);
