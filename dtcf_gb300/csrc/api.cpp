@@ -53,8 +53,7 @@ int gbx_plan_create(const gbx_tensor_desc* A, const gbx_tensor_desc* B, const gb
   auto h = std::make_unique<gbx_plan>();
   const auto la = split_labels(idxA), lb = split_labels(idxB), lc = split_labels(idxC);
   ContractionPair pair;
-  // (the split engine's slices would lose a bit of the weighted blocks)
-  const bool paired = mode == GBX_MODE_FP64 && find_contraction_pair(LA, LB, la, lb, pair);
+  const bool paired = find_contraction_pair(LA, LB, la, lb, pair);
   GBX_TRY(plan_contraction(LA, LB, LC, la, lb, lc, mode == GBX_MODE_SPLIT ? Engine::Split : Engine::F64, slices, h->p,
                            false, false, paired ? &pair : nullptr));
   *plan = h.release();

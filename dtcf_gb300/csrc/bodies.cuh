@@ -509,19 +509,20 @@ __device__ __forceinline__ void locate_chunk(const SplitRowSet* __restrict__ set
 // significant in slice S - 1.  For S <= 4 (F <= 31) |X| <= 2^31 and the
 // digits come from 32-bit arithmetic: d = ((U + 128) & 255) - 128 and
 // U <- (U + 128) >> 8, since U - d = (U + 128) rounded down to a multiple of
-// 256.  Larger S keeps 64-bit arithmetic.
+// 256.  Larger S keeps 64-bit arithmetic.  dbl: the digits of 2 X (one bit
+// more, the leading digit up to 256, which bf16 holds too).
 __device__ __forceinline__ void write_digits(long long bits, uint32_t emax, int F, int S, __nv_bfloat16* out,
-                                             int64_t stride) {
+                                             int64_t stride, bool dbl) {
   const uint32_t e = (uint32_t)((bits >> 52) & 0x7FF);
   const bool neg = bits < 0;
   unsigned long long U = 0;
   if (e != 0 && emax != 0) {
     const unsigned long long mant = ((unsigned long long)bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int sh = 53 + (int)(emax - e) - F;  // U = mant * 2^-sh, rounded half up
+    const int sh = 53 + (int)(emax - e) - F - (dbl ? 1 : 0);  // U = mant * 2^-sh, rounded half up
     if (sh <= 0) U = mant << (-sh);
     else if (sh < 64) U = (mant + (1ull << (sh - 1))) >> sh;
   }
-  if (F <= 31) {
+  if (F <= 31 && (!dbl || F <= 30)) {
     uint32_t u = (uint32_t)U;  // <= 2^31
     for (int s = S - 1; s >= 1; --s) {
       const int d = (int)((u + 128u) & 255u) - 128;
@@ -591,7 +592,7 @@ __device__ __forceinline__ void digits_body(const SplitRowSet* __restrict__ sets
       for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < k1 ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (k + u * 256 < k1) write_digits(v[u], emax, F, S, dst + k + u * 256, rs.slice_stride);
+        if (k + u * 256 < k1) write_digits(v[u], emax, F, S, dst + k + u * 256, rs.slice_stride, k + u * 256 >= rs.dbl);
     }
     // the row's last chunk also clears its K padding (the slice buffers may be
     // an arena shared with other plans, so nothing else keeps it zero)
@@ -636,7 +637,7 @@ __device__ __forceinline__ void split_row_in_registers(const SplitRowSet& rs, in
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = (int)threadIdx.x + u * 256;
-    if (k < K) write_digits(v[u], m, F, S, dst + k, rs.slice_stride);
+    if (k < K) write_digits(v[u], m, F, S, dst + k, rs.slice_stride, k >= rs.dbl);
   }
   for (int64_t k = K + threadIdx.x; k < rs.Kp; k += 256)
     for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
@@ -687,7 +688,7 @@ __device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ 
       for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < K ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (k + u * 256 < K) write_digits(v[u], m, F, S, dst + k + u * 256, rs.slice_stride);
+        if (k + u * 256 < K) write_digits(v[u], m, F, S, dst + k + u * 256, rs.slice_stride, k + u * 256 >= rs.dbl);
     }
     for (int64_t k = K + threadIdx.x; k < rs.Kp; k += 256)
       for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
@@ -717,7 +718,7 @@ __device__ __forceinline__ void short_rows_body(const SplitRowSet* __restrict__ 
     if (lane == 0) rs.exps[row] = (int)emax;
     __nv_bfloat16* dst = rs.dst + row * rs.Kp;
     for (int64_t k = lane; k < rs.K; k += 32)
-      write_digits(__double_as_longlong(ldin<kCoh>(src + k)), emax, F, S, dst + k, rs.slice_stride);
+      write_digits(__double_as_longlong(ldin<kCoh>(src + k)), emax, F, S, dst + k, rs.slice_stride, k >= rs.dbl);
     for (int64_t k = rs.K + lane; k < rs.Kp; k += 32)
       for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
   }

@@ -50,7 +50,7 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 64;             // bf16 elements per 128-byte swizzled row
-constexpr int kChunkKb = 16;       // k-blocks per exact FP32 chunk (16 * 64 = 1024)
+constexpr int kChunkKb = 16;       // k-blocks per exact FP32 chunk (16 * 64 = 1024; half with doubled digits)
 constexpr int kFoldChunks = 127;   // int32 drain sums fold into FP64 before overflow
 
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at 2 GHz
@@ -181,7 +181,7 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 struct TileInfo {
-  int p, m0, n0, kb0, nkb, kc;
+  int p, m0, n0, kb0, nkb, kc, dbl;
 };
 
 template <int BN>
@@ -202,6 +202,7 @@ __device__ __forceinline__ TileInfo decode_tile(const GemmParams& P, int tile) {
   t.n0 = (local % pr.tiles_n) * BN;
   t.kb0 = t.kc * pr.kb_per_split;
   t.nkb = min(pr.nkb, t.kb0 + pr.kb_per_split) - t.kb0;
+  t.dbl = pr.dbl;
   return t;
 }
 
@@ -327,13 +328,14 @@ __global__ void __launch_bounds__(SplitCfg<BN>::kThreads, SplitCfg<BN>::kCtasPer
       bool ok = true;
       constexpr uint32_t idesc = idesc_bf16<BN>();
       for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
-        const int nkb = decode_tile<BN>(P, tile).nkb;
+        const TileInfo ti = decode_tile<BN>(P, tile);
+        const int nkb = ti.nkb, chunk_kb = ti.dbl ? kChunkKb / 2 : kChunkKb;
         for (int l = L; l >= 0 && ok; --l) {
           const int items = level_pairs(l, S) * nkb;
           int item = 0;
           for (int s = max(1, l + 2 - S); s <= min(S, l + 1) && ok; ++s) {
             for (int kb = 0; kb < nkb && ok; ++kb, ++item) {
-              const int in_chunk = item % kChunkKb;
+              const int in_chunk = item % chunk_kb;
               if (in_chunk == 0 && !mbar_wait(&sm.accempty[buf], aphase ^ 1, P.err, 2)) {
                 ok = false;
                 break;
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(SplitCfg<BN>::kThreads, SplitCfg<BN>::kCtasPer
                 stage = 0;
                 phase ^= 1;
               }
-              if (in_chunk == kChunkKb - 1 || item == items - 1) {
+              if (in_chunk == chunk_kb - 1 || item == items - 1) {
                 umma_commit(&sm.accfull[buf]);
                 if (++buf == kAcc) {
                   buf = 0;
@@ -396,7 +398,8 @@ __global__ void __launch_bounds__(SplitCfg<BN>::kThreads, SplitCfg<BN>::kCtasPer
       bool first_fold = true;
       for (int l = L; l >= 0 && ok; --l) {
         const int items = level_pairs(l, S) * ti.nkb;
-        const int chunks = (items + kChunkKb - 1) / kChunkKb;
+        const int chunk_kb = ti.dbl ? kChunkKb / 2 : kChunkKb;
+        const int chunks = (items + chunk_kb - 1) / chunk_kb;
         bool scale_pending = l != L;  // Horner: acc = acc * 2^-8 + X_l at the first fold of level l
         int since_fold = 0;
         for (int c = 0; c < chunks; ++c) {
@@ -764,7 +767,7 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
 // TMEM holds eight such accumulators.  Level l sums l + 1 products of at
 // most 2^14 per element, so 1024 / (l + 1) elements fit below 2^24 and are
 // exact.  The high levels, which fill up first, have two buffers and are
-// drained every kHiBlocks k-blocks behind the MMAs of the next ones; the low
+// drained every few k-blocks behind the MMAs of the next ones; the low
 // ones have one and are drained more rarely, the MMAs of a k-block starting
 // with its high levels while they are.  S = 4: four high levels; 5: three
 // and two low ones; 6: two and four; 7: one and six.
@@ -786,8 +789,9 @@ struct KsCfg {
   static constexpr int kHi = S <= 4 ? S : 8 - S;  // levels with two buffers
   static constexpr int kLo = S - kHi;             // levels with one (kLo + 2 kHi <= 8)
   static constexpr int kBK = ks_bk(S);
-  static constexpr int kHiBlocks = 1024 / S / kBK;
-  static constexpr int kLoBlocks = kLo ? 1024 / (kLo ? kLo : 1) / kBK : 1;
+  // k-blocks of an accumulator (a doubled leading digit counts as a product more)
+  static constexpr int kHiBlocks = 1024 / S / kBK, kHiBlocksDbl = 1024 / (S + 1) / kBK;
+  static constexpr int kLoBlocks = kLo ? 1024 / (kLo ? kLo : 1) / kBK : 1, kLoBlocksDbl = kLo ? 1024 / (kLo + 1) / kBK : 1;
   static constexpr int kStageBytes = S * (BM + kKsBN) * kBK * 2;
   static constexpr int kStages = (220 * 1024 / kStageBytes) < 8 ? 220 * 1024 / kStageBytes : 8;
   static constexpr int kCut = S <= 4 ? 0 : S - 4;  // levels below this go to the upper sum
@@ -897,7 +901,9 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
       constexpr uint64_t kStep = (uint64_t)sizeof(typename KsSmem<S>::Stage) >> 4;
       constexpr uint64_t kAStep = (uint64_t)(BM * Cfg::kBK * 2) >> 4, kBStep = (uint64_t)(kKsBN * Cfg::kBK * 2) >> 4;
       for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
-        const int nkb = decode_tile<kKsBN>(P, tile).nkb;
+        const TileInfo ti = decode_tile<kKsBN>(P, tile);
+        const int nkb = ti.nkb, hmax = ti.dbl ? Cfg::kHiBlocksDbl : Cfg::kHiBlocks,
+                  lmax = ti.dbl ? Cfg::kLoBlocksDbl : Cfg::kLoBlocks;
         int hn = 0, ln = 0;  // k-blocks in the current accumulators
         for (int kb = 0; kb < nkb; ++kb) {
           if (hn == 0 && !mbar_wait(&sm.hiempty[hb], hphase ^ 1, P.err, 22)) {
@@ -923,7 +929,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
                    (s == 1 && k == 0 && hn == 0) ? 0u : 1u);
           }
           if (Cfg::kLo == 0) umma_commit(&sm.empty[st]);
-          if (++hn == Cfg::kHiBlocks || kb == nkb - 1) {
+          if (++hn == hmax || kb == nkb - 1) {
             umma_commit(&sm.hifull[hb]);
             hn = 0;
             if (++hb == 2) {
@@ -952,7 +958,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
                        bs + (uint64_t)c * kBStep + (uint64_t)(k * 2), idesc_bf16_n(kKsBN * (n - c < 4 ? n - c : 4)),
                        (s == 1 && k == 0 && ln == 0) ? 0u : 1u);
             }
-            if (++ln == Cfg::kLoBlocks || kb == nkb - 1) {
+            if (++ln == lmax || kb == nkb - 1) {
               umma_commit(&sm.lofull);
               ln = 0;
               lphase ^= 1;
@@ -1016,9 +1022,11 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
         __syncwarp();
         if (lane == 0) mbar_arrive(bar);
       };
+      const int hmax = ti.dbl ? Cfg::kHiBlocksDbl : Cfg::kHiBlocks,
+                  lmax = ti.dbl ? Cfg::kLoBlocksDbl : Cfg::kLoBlocks;
       int hn = 0, ln = 0;
       for (int kb = 0; kb < ti.nkb; ++kb) {
-        if (++hn == Cfg::kHiBlocks || kb == ti.nkb - 1) {
+        if (++hn == hmax || kb == ti.nkb - 1) {
           if (!wait(&sm.hifull[hb], hphase)) {
             ok = false;
             break;
@@ -1034,7 +1042,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
           }
         }
         if constexpr (Cfg::kLo > 0) {
-          if (++ln == Cfg::kLoBlocks || kb == ti.nkb - 1) {
+          if (++ln == lmax || kb == ti.nkb - 1) {
             if (!wait(&sm.lofull, lphase)) {
               ok = false;
               break;
@@ -1144,7 +1152,8 @@ static int g_width_override = 0;
 int choose_width() { return g_width_override ? g_width_override : kKsBN; }
 
 // The k-stationary kernel's exact 64-bit sums: 2^(14 + 24) a level sum and
-// element from four slices on, S products to a level.
+// element from four slices on, up to S products to a level, one bit more for
+// doubled digits.
 int64_t ks_max_k(int S) { return S <= 4 ? 1 << 24 : 1 << 22; }
 
 struct SplitLaunch {  // the problems of one output tile width
@@ -1266,7 +1275,7 @@ int split_layout(const std::vector<SplitProblem>& probs, int S, bool static_a, b
     // thin-K problems (one k-block, at most 32 columns) take the thin kernel
     o.thin = q.K <= BK && q.N <= kThinBN && S <= 7;
     o.bn = o.thin ? kThinBN : (q.width ? q.width : choose_width());
-    if (!o.thin && o.bn == kKsBN && q.K >= ks_max_k(S)) o.bn = 128;
+    if (!o.thin && o.bn == kKsBN && q.K >= ks_max_k(S) / 2) o.bn = 128;
     o.ks_kernel = !o.thin && o.bn == kKsBN;
     if (!o.thin && o.bn != 32 && o.bn != 64 && o.bn != 128 && o.bn != 256)
       return fail(GBX_EINVAL, "split tile width %d", o.bn);
@@ -1381,11 +1390,12 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
     // row sets are grouped by the plan operand they come from, so constant
     // plan operands can be split once
     SplitRowSet a{p.A, p.M, p.K, slice_ptr(o.ra, o.sa), p.M * o.Kp, o.Kp, exp_ptr(o.ra, o.ea), 0,
-                  p.lda ? p.lda : p.K};
+                  p.lda ? p.lda : p.K, p.K};
     SplitRowSet b{p.B, p.N, p.K, slice_ptr(o.rb, o.sb), p.N * o.Kp, o.Kp, exp_ptr(o.rb, o.eb), 0,
-                  p.ldb ? p.ldb : p.K};
+                  p.ldb ? p.ldb : p.K, p.K};
     SplitRowSet& to_a = p.a_is_plan_b ? b : a;  // rows that come from plan A
     SplitRowSet& to_b = p.a_is_plan_b ? a : b;
+    if (p.dbl_from >= 0) (p.dbl_plan_b ? to_b : to_a).dbl = p.dbl_from;
     if (to_a.K <= kShortRow) {
       to_a.first_row = sra;
       sra += to_a.rows;
@@ -1434,6 +1444,7 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
       red_total += p.M * p.N;
     }
     d.ldc = p.ldc ? p.ldc : p.N;
+    d.dbl = p.dbl_from >= 0 ? 1 : 0;
     dp.push_back(d);
     CUtensorMap ma, mb;
     // slices hold only the real rows: a tile's rows past M (or N) lie outside

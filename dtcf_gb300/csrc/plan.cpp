@@ -316,7 +316,7 @@ bool find_contraction_pair(const TensorLayout& A, const TensorLayout& B, const s
       out.x = la[i];
       out.y = la[j];
       out.scale_b = B.nelem <= A.nelem;
-      out.half_diagonal = true;
+      out.exact = true;
       return true;
     }
   return false;
@@ -395,6 +395,22 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
   for (auto& kv : rows) assign(kv.second, dA);
   for (auto& kv : cols) assign(kv.second, dB);
   for (auto& kv : ks) assign(kv.second, dK);
+  // the diagonal block pairs' columns first
+  int64_t k_diag = 0;
+  if (pair && pair->exact) {
+    if (rows.size() > 1 || ks.size() > 1) return fail(GBX_EINVAL, "symmetric pair over several irreps");
+    for (auto& kv : ks) {
+      int64_t off = 0;
+      for (bool diag : {true, false}) {
+        for (auto& t : kv.second.off)
+          if ((t.first[px] == t.first[py]) == diag) {
+            t.second = off;
+            off += tuple_size(dK, t.first);
+          }
+        if (diag) k_diag = off;
+      }
+    }
+  }
   for (auto& kv : ks_full) assign(kv.second, dK);
   // irrep groups present in rows, cols and K
   int64_t ao = 0, bo = 0, co = 0;
@@ -419,8 +435,23 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
   p->a_elems = ao;
   p->b_elems = bo;
   p->c_elems = co;
-  for (auto& g : p->groups) choose_engine(g, e == Engine::Split, split_all, nslices);
-  if (pair && pair->half_diagonal) p->alpha_factor = 2.0;
+  for (auto& g : p->groups) {
+    GroupBlock whole = g;
+    if (pair && pair->exact) whole.K = ks_full.count(g.h) ? ks_full[g.h].total : 0;
+    choose_engine(whole, e == Engine::Split, split_all, nslices);
+    g.engine = whole.engine;
+    g.swap = whole.swap;
+  }
+  bool halve = false;  // the diagonal pairs in one operand's pack
+  if (pair && pair->exact && !p->groups.empty()) {
+    if (p->groups[0].engine == 1) {
+      p->dbl_from = k_diag;
+      p->dbl_plan_b = pair->scale_b;
+    } else {
+      halve = true;
+      p->alpha_factor = 2.0;
+    }
+  }
 
   // pack moves: A (rows = extA tuples of irrep h, cols = K tuples of irrep h)
   auto pack = [&](const TensorLayout& T, const std::vector<int>& ext_dims, const std::vector<int>& contr_dims,
@@ -469,7 +500,7 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
           // off-diagonal block pairs of a symmetric contracted pair count twice
           // (or the diagonal ones half)
           if (pair_scaled && px >= 0) {
-            if (pair->half_diagonal) factor *= kvv.first[px] == kvv.first[py] ? 0.5 : 1.0;
+            if (pair->exact) factor *= halve && kvv.first[px] == kvv.first[py] ? 0.5 : 1.0;
             else if (kvv.first[px] > kvv.first[py]) factor *= 2.0;
           }
           ms.host.push_back(make_move(T.rank, ext, sstr, dstr, T.off[id], dst, 0, factor));
@@ -677,6 +708,8 @@ void ContractionPlan::split_problems(std::vector<SplitProblem>& sp) const {
     q.C = d_Cbig + g.c_off;
     q.K = g.K;
     q.width = split_width;
+    q.dbl_from = dbl_from;
+    q.dbl_plan_b = dbl_plan_b;
     sp.push_back(q);
   }
 }

@@ -156,7 +156,11 @@ struct ContractionPlan {
   // Nonzero: the unpack stores store_scale * A B into C, whatever factor
   // execute is given (set_overwrite on a packed plan).
   double store_scale = 0.0;
-  double alpha_factor = 1.0;  // of the unpack (half_diagonal pairs)
+  // exact pairs: the unpack's factor (FP64 groups), the columns whose
+  // products count twice (split groups; -1: none)
+  double alpha_factor = 1.0;
+  int64_t dbl_from = -1;
+  bool dbl_plan_b = true;
   // Makes the plan write C = alpha A B instead of accumulating, when it writes
   // every element of C (the direct items, or the unpack moves: one per C
   // tile); call before build.  false: nothing changed.
@@ -203,14 +207,16 @@ constexpr double kDirectMaxK = 16.0;
 // so the packed GEMMs run over block pairs X >= Y only, the off-diagonal ones
 // weighted 2 in one operand's pack (scale_b: B's, else A's) -- close to half
 // the contracted extent.  Both indices must have the same blocking.
-// half_diagonal: the same sum as 2 (sum_{X>Y} + 1/2 sum_{X=Y}): the diagonal
-// pairs weighted 1/2 in the pack, the unpack's factor doubled, so that no
-// packed value grows (the FP64 ladder at o = 16, v = 48 in blocks of 8: 1193
-// -> 710 us).
+// exact: no value is scaled up for it.  The FP64 engine computes 2 (sum_{X>Y}
+// + 1/2 sum_{X=Y}), the diagonal pairs weighted 1/2 in the pack and the
+// unpack's factor doubled (the FP64 ladder at o = 16, v = 48 in blocks of 8:
+// 1193 -> 710 us); the split engine doubles the off-diagonal columns' digits
+// (SplitProblem::dbl_from; o = 32, v = 128, blocks of 16: 5033 -> 3132 us).
+// Needs operands of one irrep; the engine is chosen as for the whole sum.
 struct ContractionPair {
   std::string x, y;
   bool scale_b = true;
-  bool half_diagonal = false;
+  bool exact = false;
 };
 
 // The pair of a contraction over RRR layouts: two contracted indices that are

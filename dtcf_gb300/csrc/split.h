@@ -21,7 +21,13 @@ struct SplitProblem {
   // orientation); split_operands(plan_a, plan_b) maps accordingly
   bool a_is_plan_b = false;
   int64_t lda = 0, ldb = 0, ldc = 0;
-  int width = 0;  // output tile width 32/64/128/256; 0 = the built-in model
+  int width = 0;  // output tile width 32/64/128/256; 0 = the default
+  // The products of columns dbl_from .. K - 1 count twice (-1: none): plan
+  // operand B's digits (dbl_plan_b, else A's) there are those of twice the
+  // value at the row's own scale, so nothing of either operand is rounded
+  // coarser for it.
+  int64_t dbl_from = -1;
+  bool dbl_plan_b = true;
 };
 
 struct SplitPlan;

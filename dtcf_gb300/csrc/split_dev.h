@@ -15,6 +15,7 @@ struct SplitRowSet {   // one operand of one problem for the split kernels
   int* exps;
   int64_t first_row;   // first (row, K chunk) work item of this set
   int64_t ld;          // source row stride (elements)
+  int64_t dbl;         // from this column on the digits are those of twice the value (K: none)
 };
 
 struct DevProblem {
@@ -26,6 +27,7 @@ struct DevProblem {
   double* C;        // ksplit == 1: output
   double* partial;  // ksplit > 1: ksplit x M x N raw contributions
   int64_t ldc;
+  int dbl;  // one operand has doubled digits: its leading ones reach 256, not 128
 };
 
 }  // namespace gbx

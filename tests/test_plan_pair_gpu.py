@@ -98,3 +98,27 @@ def test_extreme_values(scale):
     C = make("aabb", (n, n, 16, 16), (g, g, 2, 2), rng)
     got, want, bound = run(A, B, C, "a,b,e,f", "e,f,i,j", "a,b,i,j", "fp64", -1)
     assert np.max(np.abs(got - want)) <= bound
+
+
+@pytest.mark.parametrize("slices,width", [(4, 0), (5, 0), (6, 0), (7, 0), (6, 32), (6, 128), (4, 256)])
+def test_doubled_digits_are_exact(slices, width):
+    """Integers of one leading digit near its maximum, all of one sign, so that every accumulator comes as close to
+    2^24 as it can: the split engine's result is the exact integer one."""
+    from dtcf_gb300._lib import lib
+    rng = np.random.default_rng(slices + width)
+    n, g = 48, 6
+    A, B, C = (make("aabb", s, v, rng) for s, v in (((n,) * 4, (g,) * 4), ((n, n, 16, 16), (g, g, 2, 2)),
+                                                   ((n, n, 16, 16), (g, g, 2, 2))))
+    for t in (A, B):
+        t.tiles.copy_(torch.from_numpy(rng.integers(100, 128, t.tiles.numel()).astype(np.float64)).cuda())
+    C.tiles.zero_()
+    from dtcf_gb300.rrr import Plan
+    want = oracle.rrr.contract(as_oracle(A), as_oracle(B), as_oracle(C), "a,b,e,f", "e,f,i,j", "a,b,i,j", 1.0, 1)
+    assert lib().gbx_split_set_width(width) == 0
+    try:
+        plan = Plan(A, B, C, "a,b,e,f", "e,f,i,j", "a,b,i,j", mode="split", sign=1, slices=slices)
+    finally:
+        lib().gbx_split_set_width(0)
+    plan.execute(A, B, C, 1.0)
+    torch.cuda.synchronize()
+    assert np.array_equal(C.tiles.cpu().numpy().reshape(want.shape), want)
