@@ -503,42 +503,82 @@ __device__ __forceinline__ void locate_chunk(const SplitRowSet* __restrict__ set
   k0 = (local - row * per_row) * kSplitChunk;
 }
 
-// One element's S slices: X = the element scaled by 2^-(emax - 1022 - F +
-// 53) and rounded half up to an integer of F = 7 + 8 (S - 1) bits, cut into
-// balanced base-256 digits (the digits of |X|, with X's sign), least
-// significant in slice S - 1.  For S <= 4 (F <= 31) |X| <= 2^31 and the
-// digits come from 32-bit arithmetic: d = ((U + 128) & 255) - 128 and
-// U <- (U + 128) >> 8, since U - d = (U + 128) rounded down to a multiple of
-// 256.  Larger S keeps 64-bit arithmetic.  dbl: the digits of 2 X (one bit
-// more, the leading digit up to 256, which bf16 holds too).
-__device__ __forceinline__ void write_digits(long long bits, uint32_t emax, int F, int S, __nv_bfloat16* out,
-                                             int64_t stride, bool dbl) {
-  const uint32_t e = (uint32_t)((bits >> 52) & 0x7FF);
-  const bool neg = bits < 0;
-  unsigned long long U = 0;
-  if (e != 0 && emax != 0) {
-    const unsigned long long mant = ((unsigned long long)bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int sh = 53 + (int)(emax - e) - F - (dbl ? 1 : 0);  // U = mant * 2^-sh, rounded half up
-    if (sh <= 0) U = mant << (-sh);
-    else if (sh < 64) U = (mant + (1ull << (sh - 1))) >> sh;
-  }
-  if (F <= 31 && (!dbl || F <= 30)) {
-    uint32_t u = (uint32_t)U;  // <= 2^31
-    for (int s = S - 1; s >= 1; --s) {
-      const int d = (int)((u + 128u) & 255u) - 128;
-      u = (u + 128u) >> 8;
-      out[s * stride] = __int2bfloat16_rn(neg ? -d : d);
+// W consecutive elements of a row from column k on (zeros past K); al: the
+// row starts on a 16-byte boundary (k is a multiple of W).
+template <bool kCoh, int W>
+__device__ __forceinline__ void load_group(const double* src, int64_t k, int64_t K, bool al, long long (&v)[W]) {
+  if (al && k + W <= K) {
+#pragma unroll
+    for (int i = 0; i < W; i += 2) {
+      const double2 x = ldin<kCoh>(reinterpret_cast<const double2*>(src + k + i));
+      v[i] = __double_as_longlong(x.x);
+      v[i + 1] = __double_as_longlong(x.y);
     }
-    out[0] = __int2bfloat16_rn(neg ? -(int)u : (int)u);
   } else {
-    unsigned long long u = U;
-    for (int s = S - 1; s >= 1; --s) {
-      const int d = (int)((u + 128ull) & 255ull) - 128;
-      u = (u + 128ull) >> 8;
-      out[s * stride] = __int2bfloat16_rn(neg ? -d : d);
-    }
-    out[0] = __int2bfloat16_rn(neg ? -(int)u : (int)u);
+#pragma unroll
+    for (int i = 0; i < W; ++i) v[i] = k + i < K ? __double_as_longlong(ldin<kCoh>(src + k + i)) : 0ll;
   }
+}
+
+template <int W>
+__device__ __forceinline__ uint32_t max_exponent(uint32_t m, const long long (&v)[W]) {
+#pragma unroll
+  for (int i = 0; i < W; ++i) m = max(m, (uint32_t)((v[i] >> 52) & 0x7FF));
+  return m;
+}
+
+// The S slices of W (2 or 4) consecutive elements.  X = the element scaled by
+// 2^-(emax - 1022 - F + 53) and rounded half up to an integer of F = 7 + 8 (S
+// - 1) bits, cut into balanced base-256 digits (the digits of |X|, with X's
+// sign), least significant in slice S - 1.  Adding 128 at every digit but the
+// leading one makes them plain bytes: digit = byte - 128.  A byte becomes a
+// float by placing it under 2^23's bits and subtracting (one multiply-add
+// with the sign, exact), two floats' upper halves are a bf16 pair, and a
+// group's digits of one slice leave in one store: the splits were bound by
+// their instructions (one digit at a time through integer conversions and
+// 2-byte stores, 9216 rows of 9216 at 6 slices took 615 us; 335 us so).
+// from: columns from it on have the digits of 2 X (one bit more, the leading
+// digit up to 256, which bf16 holds too).
+template <int W>
+__device__ __forceinline__ void write_digits(const long long (&bits)[W], uint32_t emax, int F, int S,
+                                             __nv_bfloat16* out, int64_t stride, int64_t k, int64_t from) {
+  uint32_t lo[W], hi[W], top[W];
+  float sgn[W];
+  const unsigned long long bias = 0x0080808080808080ull & ((1ull << (8 * (S - 1))) - 1ull);
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    const uint32_t h = (uint32_t)(bits[i] >> 32), e = (h >> 20) & 0x7FFu;
+    sgn[i] = __uint_as_float(0x3F800000u | (h & 0x80000000u));
+    unsigned long long U = 0;
+    if (e != 0 && emax != 0) {
+      const unsigned long long mant = ((unsigned long long)bits[i] & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+      const int sh = 53 + (int)(emax - e) - F - (k + i >= from ? 1 : 0);  // U = mant * 2^-sh, rounded half up
+      if (sh <= 0) U = mant << (-sh);
+      else if (sh < 64) U = (mant + (1ull << (sh - 1))) >> sh;
+    }
+    U += bias;
+    lo[i] = (uint32_t)U;
+    hi[i] = (uint32_t)(U >> 32);
+    top[i] = (uint32_t)(U >> (8 * (S - 1)));
+  }
+  const auto put = [&](__nv_bfloat16* p, const float (&f)[W]) {
+    const uint32_t a = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632);
+    if constexpr (W == 2) *reinterpret_cast<uint32_t*>(p) = a;
+    else *reinterpret_cast<uint2*>(p) = make_uint2(a, __byte_perm(__float_as_uint(f[2]), __float_as_uint(f[3]), 0x7632));
+  };
+  float f[W];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {  // byte j: slice S - 1 - j
+    if (j >= S - 1) break;
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      f[i] = __fmaf_rn(__uint_as_float(__byte_perm(j < 4 ? lo[i] : hi[i], 0x4B000000u, 0x7650 | (j & 3))), sgn[i],
+                       -8388736.0f * sgn[i]);
+    put(out + (S - 1 - j) * stride, f);
+  }
+#pragma unroll
+  for (int i = 0; i < W; ++i) f[i] = __fmaf_rn(__uint_as_float(0x4B000000u | top[i]), sgn[i], -8388608.0f * sgn[i]);
+  put(out, f);
 }
 
 template <bool kCoh>
@@ -551,14 +591,14 @@ __device__ __forceinline__ void row_exponent_body(const SplitRowSet* __restrict_
     const SplitRowSet& rs = sets[set];
     const double* src = rs.src + row * rs.ld;
     const int64_t k1 = min(rs.K, k0 + kSplitChunk);
+    const bool al = ((uintptr_t)src & 15) == 0;
     uint32_t emax = 0;
-    // four loads in flight per thread (the loop is bound by load latency)
-    for (int64_t k = k0 + threadIdx.x; k < k1; k += 4 * 256) {
-      long long v[4];
+    for (int64_t k = k0 + 4 * threadIdx.x; k < k1; k += 2 * 1024) {
+      long long v[2][4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < k1 ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
+      for (int u = 0; u < 2; ++u) load_group<kCoh>(src, k + u * 1024, k1, al, v[u]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) emax = max(emax, (uint32_t)((v[u] >> 52) & 0x7FF));
+      for (int u = 0; u < 2; ++u) emax = max_exponent(emax, v[u]);
     }
     for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = emax;
@@ -583,22 +623,21 @@ __device__ __forceinline__ void digits_body(const SplitRowSet* __restrict__ sets
     locate_chunk(sets, nsets, chunk, set, row, k0);
     const SplitRowSet& rs = sets[set];
     const double* src = rs.src + row * rs.ld;
+    const bool al = ((uintptr_t)src & 15) == 0;
     __nv_bfloat16* dst = rs.dst + row * rs.Kp;
     const uint32_t emax = (uint32_t)ldrw<kCoh>(rs.exps + row);
-    const int64_t k1 = min(rs.K, k0 + kSplitChunk);
-    for (int64_t k = k0 + threadIdx.x; k < k1; k += 4 * 256) {
-      long long v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < k1 ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (k + u * 256 < k1) write_digits(v[u], emax, F, S, dst + k + u * 256, rs.slice_stride, k + u * 256 >= rs.dbl);
-    }
     // the row's last chunk also clears its K padding (the slice buffers may be
     // an arena shared with other plans, so nothing else keeps it zero)
-    if (k1 == rs.K)
-      for (int64_t k = rs.K + threadIdx.x; k < rs.Kp; k += 256)
-        for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
+    const int64_t k1 = k0 + kSplitChunk >= rs.K ? rs.Kp : k0 + kSplitChunk;
+    for (int64_t k = k0 + 4 * threadIdx.x; k < k1; k += 2 * 4 * 256) {
+      long long v[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) load_group<kCoh>(src, k + u * 1024, rs.K, al, v[u]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (k + u * 1024 < k1)
+          write_digits(v[u], emax, F, S, dst + k + u * 1024, rs.slice_stride, k + u * 1024, rs.dbl);
+    }
   }
 }
 
@@ -609,41 +648,48 @@ __device__ __forceinline__ void digits_body(const SplitRowSet* __restrict__ sets
 // once.  The row sets here carry first_row in rows.
 constexpr int64_t kMidRow = 16384;
 
-// A row of at most kPer * 256 elements: every element loaded at once (one
-// HBM round trip per row instead of one per 1024 elements and pass), the
-// exponent reduced across the CTA, the digits written from the registers.
-template <bool kCoh, int kPer>
-__device__ __forceinline__ void split_row_in_registers(const SplitRowSet& rs, int64_t row, const double* src, int F,
-                                                       int S, uint32_t* red) {
-  const int K = (int)rs.K;
-  long long v[kPer];
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int k = (int)threadIdx.x + u * 256;
-    v[u] = k < K ? __double_as_longlong(ldin<kCoh>(src + k)) : 0;
-  }
-  uint32_t emax = 0;
-#pragma unroll
-  for (int u = 0; u < kPer; ++u) emax = max(emax, (uint32_t)((v[u] >> 52) & 0x7FF));
-  for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+// The largest of the CTA's 256 values.
+__device__ __forceinline__ uint32_t block_max(uint32_t m, uint32_t* red) {
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
   __syncthreads();  // the previous row is done with red
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = emax;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
-  uint32_t m = 0;
 #pragma unroll
   for (int w = 0; w < 8; ++w) m = max(m, red[w]);
+  return m;
+}
+
+// A row of at most kGroups * 1024 elements: every element loaded at once (one
+// HBM round trip per row instead of one per 1024 elements and pass), the
+// exponent reduced across the CTA, the digits written from the registers.
+template <bool kCoh, int kGroups>
+__device__ __forceinline__ void split_row_in_registers(const SplitRowSet& rs, int64_t row, const double* src, bool al,
+                                                       int F, int S, uint32_t* red) {
+  long long v[kGroups][4];
+  uint32_t m = 0;
+#pragma unroll
+  for (int u = 0; u < kGroups; ++u) load_group<kCoh>(src, 4 * threadIdx.x + u * 1024, rs.K, al, v[u]);
+#pragma unroll
+  for (int u = 0; u < kGroups; ++u) m = max_exponent(m, v[u]);
+  m = block_max(m, red);
   if (threadIdx.x == 0) rs.exps[row] = (int)m;
   __nv_bfloat16* dst = rs.dst + row * rs.Kp;
 #pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int k = (int)threadIdx.x + u * 256;
-    if (k < K) write_digits(v[u], m, F, S, dst + k, rs.slice_stride, k >= rs.dbl);
+  for (int u = 0; u < kGroups; ++u) {
+    const int k = 4 * threadIdx.x + u * 1024;
+    if (k < rs.Kp) write_digits(v[u], m, F, S, dst + k, rs.slice_stride, k, rs.dbl);
   }
-  for (int64_t k = K + threadIdx.x; k < rs.Kp; k += 256)
-    for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
+  // padding beyond the groups (K just below their end)
+  for (int64_t k = 4 * threadIdx.x + kGroups * 1024; k < rs.Kp; k += 1024) {
+    const long long z[4] = {0, 0, 0, 0};
+    write_digits(z, 0, F, S, dst + k, rs.slice_stride, k, rs.dbl);
+  }
 }
 
-template <bool kCoh>
+// kFour: with the path that holds rows of 2049 .. 4096 elements in registers,
+// which takes registers from the others (20000 rows of 4000 at 4 slices: 232
+// us with it, 278 without; of 2000: 137 and 121; of 8000 at 6: 709 and 632).
+template <bool kCoh, bool kFour>
 __device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows,
                                                 int S, uint32_t bid, uint32_t nblk, uint32_t* red) {
   const int F = 7 + 8 * (S - 1);
@@ -656,71 +702,82 @@ __device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ 
     const SplitRowSet& rs = sets[lo];
     const int64_t row = rg - rs.first_row;
     const double* src = rs.src + row * rs.ld;
+    const bool al = ((uintptr_t)src & 15) == 0;
     const int64_t K = rs.K;
-    if (K <= 8 * 256) {
-      split_row_in_registers<kCoh, 8>(rs, row, src, F, S, red);
+    if (K <= 2 * 1024) {
+      split_row_in_registers<kCoh, 2>(rs, row, src, al, F, S, red);
       continue;
     }
-    if (K <= 16 * 256) {
-      split_row_in_registers<kCoh, 16>(rs, row, src, F, S, red);
+    if (kFour && K <= 4 * 1024) {
+      split_row_in_registers<kCoh, 4>(rs, row, src, al, F, S, red);
       continue;
     }
-    uint32_t emax = 0;
-    for (int64_t k = threadIdx.x; k < K; k += 4 * 256) {
-      long long v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < K ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) emax = max(emax, (uint32_t)((v[u] >> 52) & 0x7FF));
-    }
-    for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-    __syncthreads();  // the previous row is done with red
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = emax;
-    __syncthreads();
     uint32_t m = 0;
+    for (int64_t k = 4 * threadIdx.x; k < K; k += 2 * 1024) {
+      long long v[2][4];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) m = max(m, red[w]);
+      for (int u = 0; u < 2; ++u) load_group<kCoh>(src, k + u * 1024, K, al, v[u]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) m = max_exponent(m, v[u]);
+    }
+    m = block_max(m, red);
     if (threadIdx.x == 0) rs.exps[row] = (int)m;
     __nv_bfloat16* dst = rs.dst + row * rs.Kp;
-    for (int64_t k = threadIdx.x; k < K; k += 4 * 256) {
-      long long v[4];
+    for (int64_t k = 4 * threadIdx.x; k < rs.Kp; k += 2 * 1024) {
+      long long v[2][4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = k + u * 256 < K ? __double_as_longlong(ldin<kCoh>(src + k + u * 256)) : 0;
+      for (int u = 0; u < 2; ++u) load_group<kCoh>(src, k + u * 1024, K, al, v[u]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (k + u * 256 < K) write_digits(v[u], m, F, S, dst + k + u * 256, rs.slice_stride, k + u * 256 >= rs.dbl);
+      for (int u = 0; u < 2; ++u)
+        if (k + u * 1024 < rs.Kp)
+          write_digits(v[u], m, F, S, dst + k + u * 1024, rs.slice_stride, k + u * 1024, rs.dbl);
     }
-    for (int64_t k = K + threadIdx.x; k < rs.Kp; k += 256)
-      for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
   }
 }
 
-// Short rows: one warp handles a whole row (exponent by warp shuffles, then
-// the digits); the row sets here carry first_row in rows.
+// Short rows: 2^lg lanes of a warp (8, 16 or 32) handle a whole row, two
+// elements to a lane and step: the exponent by shuffles, then the digits,
+// from registers where the row takes one step (every row of a launch with lg
+// < 5 does).  The row sets here carry first_row in rows.
 template <bool kCoh>
 __device__ __forceinline__ void short_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows,
-                                                int S, uint32_t bid, uint32_t nblk) {
+                                                int S, int lg, uint32_t bid, uint32_t nblk) {
   const int F = 7 + 8 * (S - 1);
-  const int lane = threadIdx.x & 31;
-  for (int64_t rg = (int64_t)bid * 8 + (threadIdx.x >> 5); rg < total_rows; rg += (int64_t)nblk * 8) {
-    int lo = 0, hi = nsets - 1;
+  const int lanes = 1 << lg, lane = threadIdx.x & (lanes - 1), step = 2 * lanes;
+  const int64_t per = (int64_t)(256 >> lg);  // rows of a CTA
+  int lo = 0;
+  for (int64_t r0 = (int64_t)bid * per; r0 < total_rows; r0 += (int64_t)nblk * per) {
+    // rows past the end repeat the last one without storing (the shuffles need every lane)
+    const int64_t want = r0 + (threadIdx.x >> lg), rg = min(want, total_rows - 1);
+    const bool real = want < total_rows;
+    int hi = nsets - 1;  // rows only grow
     while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
+      const int mid = (lo + hi + 1) >> 1;
       if (sets[mid].first_row <= rg) lo = mid; else hi = mid - 1;
     }
     const SplitRowSet& rs = sets[lo];
     const int64_t row = rg - rs.first_row;
     const double* src = rs.src + row * rs.ld;
-    uint32_t emax = 0;
-    for (int64_t k = lane; k < rs.K; k += 32)
-      emax = max(emax, (uint32_t)((__double_as_longlong(ldin<kCoh>(src + k)) >> 52) & 0x7FF));
-    for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-    if (lane == 0) rs.exps[row] = (int)emax;
+    const bool al = ((uintptr_t)src & 15) == 0;
+    const int64_t K = rs.K;
+    long long v[2];
+    load_group<kCoh>(src, 2 * lane, K, al, v);
+    uint32_t m = max_exponent(0u, v);
+    if (lg == 5)
+      for (int64_t k = 2 * lane + step; k < K; k += step) {
+        long long w[2];
+        load_group<kCoh>(src, k, K, al, w);
+        m = max_exponent(m, w);
+      }
+    for (int o = lanes / 2; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (!real) continue;
+    if (lane == 0) rs.exps[row] = (int)m;
     __nv_bfloat16* dst = rs.dst + row * rs.Kp;
-    for (int64_t k = lane; k < rs.K; k += 32)
-      write_digits(__double_as_longlong(ldin<kCoh>(src + k)), emax, F, S, dst + k, rs.slice_stride, k >= rs.dbl);
-    for (int64_t k = rs.K + lane; k < rs.Kp; k += 32)
-      for (int s = 0; s < S; ++s) dst[s * rs.slice_stride + k] = __int2bfloat16_rn(0);
+    if (2 * lane < rs.Kp) write_digits(v, m, F, S, dst + 2 * lane, rs.slice_stride, 2 * lane, rs.dbl);
+    for (int64_t k = 2 * lane + step; k < rs.Kp; k += step) {
+      load_group<kCoh>(src, k, K, al, v);
+      write_digits(v, m, F, S, dst + k, rs.slice_stride, k, rs.dbl);
+    }
   }
 }
 

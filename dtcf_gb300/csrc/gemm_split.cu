@@ -1103,15 +1103,16 @@ __global__ void __launch_bounds__(256) digits_kernel(const SplitRowSet* __restri
   dev::digits_body<false>(sets, nsets, total_chunks, S, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(256) split_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets,
-                                                         int64_t total_rows, int S) {
+template <bool kFour>
+__global__ void __launch_bounds__(256, kFour ? 3 : 4)
+    split_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows, int S) {
   __shared__ uint32_t red[8];
-  dev::split_rows_body<false>(sets, nsets, total_rows, S, blockIdx.x, gridDim.x, red);
+  dev::split_rows_body<false, kFour>(sets, nsets, total_rows, S, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void __launch_bounds__(256) split_short_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets,
-                                                               int64_t total_rows, int S) {
-  dev::short_rows_body<false>(sets, nsets, total_rows, S, blockIdx.x, gridDim.x);
+                                                               int64_t total_rows, int S, int lg) {
+  dev::short_rows_body<false>(sets, nsets, total_rows, S, lg, blockIdx.x, gridDim.x);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -1184,6 +1185,8 @@ struct SplitPlan {
   SplitRowSet* d_mid_b = nullptr;
   int nlong_a = 0, nlong_b = 0, nshort_a = 0, nshort_b = 0, nmid_a = 0, nmid_b = 0;
   int64_t short_rows_a = 0, short_rows_b = 0, mid_rows_a = 0, mid_rows_b = 0;
+  bool mid_four_a = false, mid_four_b = false;  // a medium row of 2049 .. 4096 elements
+  int short_lg_a = 3, short_lg_b = 3;  // log2 of a short row's lanes: the longest row's elements in one step, or 5
   int nsets = 0;
   int64_t rows_a = 0, rows_b = 0;  // (row, K chunk) work items per side
   std::vector<std::pair<void*, size_t>> exp_ranges_a, exp_ranges_b;  // exponent words reset before a split
@@ -1399,10 +1402,12 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
     if (to_a.K <= kShortRow) {
       to_a.first_row = sra;
       sra += to_a.rows;
+      while (sp->short_lg_a < 5 && to_a.K > (2ll << sp->short_lg_a)) ++sp->short_lg_a;
       ssa.push_back(to_a);
     } else if (to_a.K <= kMidRow) {
       to_a.first_row = mra;
       mra += to_a.rows;
+      sp->mid_four_a = sp->mid_four_a || (to_a.K > 2048 && to_a.K <= 4096);
       msa.push_back(to_a);
     } else {
       to_a.first_row = ra;
@@ -1413,10 +1418,12 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
     if (to_b.K <= kShortRow) {
       to_b.first_row = srb;
       srb += to_b.rows;
+      while (sp->short_lg_b < 5 && to_b.K > (2ll << sp->short_lg_b)) ++sp->short_lg_b;
       ssb.push_back(to_b);
     } else if (to_b.K <= kMidRow) {
       to_b.first_row = mrb;
       mrb += to_b.rows;
+      sp->mid_four_b = sp->mid_four_b || (to_b.K > 2048 && to_b.K <= 4096);
       msb.push_back(to_b);
     } else {
       to_b.first_row = rb;
@@ -1543,7 +1550,7 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
       const int grid = (int)std::min<int64_t>(chunks, 152 * 16);
       if (rec) {
         ProgArgs a;
-        a.sets = {sets, chunks, nsets, sp->S};
+        a.sets = {sets, chunks, nsets, sp->S, 0};
         GBX_TRY(prog_mem(rec, PK_ROWEXP, (uint32_t)grid, a, {}));
         GBX_TRY(prog_mem(rec, PK_DIGITS, (uint32_t)grid, a, {}));
       } else {
@@ -1560,10 +1567,13 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
       const int grid = (int)std::min<int64_t>(mrows, 152 * 8);
       if (rec) {
         ProgArgs a;
-        a.sets = {sets, mrows, nsets, sp->S};
+        a.sets = {sets, mrows, nsets, sp->S, 0};
         GBX_TRY(prog_mem(rec, PK_SPLITROWS, (uint32_t)grid, a, {}));
       } else {
-        split_rows_kernel<<<grid, 256, 0, st>>>(sets, nsets, mrows, sp->S);
+        if (side == 0 ? sp->mid_four_a : sp->mid_four_b)
+          split_rows_kernel<true><<<grid, 256, 0, st>>>(sets, nsets, mrows, sp->S);
+        else
+          split_rows_kernel<false><<<grid, 256, 0, st>>>(sets, nsets, mrows, sp->S);
         GBX_CUDA(cudaGetLastError());
       }
     }
@@ -1571,14 +1581,15 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
     if (srows > 0) {
       const SplitRowSet* sets = side == 0 ? sp->d_short_a : sp->d_short_b;
       const int nsets = side == 0 ? sp->nshort_a : sp->nshort_b;
-      const int grid = (int)std::min<int64_t>((srows + 7) / 8, 152 * 32);
+      const int lg = side == 0 ? sp->short_lg_a : sp->short_lg_b;
+      const int grid = (int)std::min<int64_t>((srows + (256 >> lg) - 1) / (256 >> lg), 152 * 32);
       if (rec) {
         ProgArgs a;
-        a.sets = {sets, srows, nsets, sp->S};
+        a.sets = {sets, srows, nsets, sp->S, lg};
         GBX_TRY(prog_mem(rec, PK_SHORTROWS, (uint32_t)grid, a, {}));
         continue;
       }
-      split_short_rows_kernel<<<grid, 256, 0, st>>>(sets, nsets, srows, sp->S);
+      split_short_rows_kernel<<<grid, 256, 0, st>>>(sets, nsets, srows, sp->S, lg);
       GBX_CUDA(cudaGetLastError());
     }
   }

@@ -108,10 +108,10 @@ __device__ __forceinline__ void run_record(const ProgRec& r, uint32_t vb, ProgSm
       dev::digits_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g);
       break;
     case PK_SHORTROWS:
-      dev::short_rows_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g);
+      dev::short_rows_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, a.sets.lg, vb, g);
       break;
     case PK_SPLITROWS:
-      dev::split_rows_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g, sm.red8);
+      dev::split_rows_body<true, true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g, sm.red8);
       break;
     case PK_SPLITRED:
       dev::split_reduce_body<true>(a.splitred.probs, a.splitred.red_prob, a.splitred.red_first, a.splitred.nred,
