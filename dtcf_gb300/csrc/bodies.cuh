@@ -49,7 +49,8 @@ constexpr int kBodyThreads = 256;
 
 constexpr int kMoveThreads = 256;
 constexpr int kMoveChunk = 2048;   // elements per work item (general moves)
-constexpr int kMove4Chunk = 4096;  // elements per work item (moves of at most four dimensions)
+constexpr int kMove4Chunk = 4096;  // elements per work item (moves of at most four dimensions) ...
+constexpr int kMove4Small = 1024;  // ... in sets that would not fill the GPU with such chunks
 
 template <bool kCoh>
 __device__ __forceinline__ void move_body(const MoveDesc* __restrict__ descs, const uint32_t* __restrict__ first,
@@ -122,21 +123,21 @@ __device__ __forceinline__ void move_body(const MoveDesc* __restrict__ descs, co
 // table, its fields are read once per chunk into registers and the index
 // decode is fully unrolled (three multiply-high divisions per element), so
 // the kernel issues a few tens of instructions per element and streams at
-// memory speed.  Each thread handles kMove4Chunk / kMoveThreads elements in
-// two batches, addresses first, then every load, then every store.  A move
+// memory speed.  Each thread handles kChunk / kMoveThreads elements in
+// batches, addresses first, then every load, then every store.  A move
 // marked for pairs (contiguous even inner runs at even offsets) goes two
 // elements per index decode with 16-byte loads and stores.
-template <bool kCoh, int kPer = 8>
+template <bool kCoh, int kPer = 8, int kChunk = kMove4Chunk>
 __device__ __forceinline__ void move4_body(const MoveDesc4* __restrict__ descs, const uint32_t* __restrict__ chunk_desc,
                                            uint32_t nchunks, const double* __restrict__ src, double* __restrict__ dst,
                                            double alpha, int allow_pairs, uint32_t bid, uint32_t nblk) {
-  constexpr int kBatches = kMove4Chunk / (kMoveThreads * kPer);
-  constexpr int kPairBatches = kMove4Chunk / (2 * kMoveThreads * kPer);
-  static_assert(kPairBatches * 2 * kMoveThreads * kPer == kMove4Chunk, "chunk size");
+  constexpr int kBatches = kChunk / (kMoveThreads * kPer);
+  constexpr int kPairBatches = kChunk / (2 * kMoveThreads * kPer);
+  static_assert(kPairBatches * 2 * kMoveThreads * kPer == kChunk, "chunk size");
   for (uint32_t chunk = bid; chunk < nchunks; chunk += nblk) {
     const MoveDesc4* __restrict__ md = descs + __ldg(chunk_desc + chunk);
     const uint32_t n = md->n;
-    const uint32_t base = (chunk - md->first) * kMove4Chunk;
+    const uint32_t base = (chunk - md->first) * kChunk;
     const int op = md->op;
     const double scale = op == 0 ? md->scale : __dmul_rn(md->scale, alpha);
     const FastDiv d1 = md->div[1], d2 = md->div[2], d3 = md->div[3];
@@ -151,7 +152,7 @@ __device__ __forceinline__ void move4_body(const MoveDesc4* __restrict__ descs, 
     const bool unit = op == 0 && (sb & 0x7FFFFFFFFFFFFFFFull) == 0x3FF0000000000000ull;
     const long long flip = (long long)(sb & 0x8000000000000000ull);
     if (allow_pairs && md->pad == 1) {
-      // pairs (2e, 2e + 1): the chunk's kMove4Chunk elements in batches of
+      // pairs (2e, 2e + 1): the chunk's elements in batches of
       // kPer pairs per thread
 #pragma unroll 1
       for (int bt = 0; bt < kPairBatches; ++bt) {
@@ -395,14 +396,95 @@ struct DirSmem {
   DirPair pairs[kDirMaxPairs];
 };
 
-// One CTA per work item (grid-stride), kThr threads.  Each thread holds
-// kDirPer output elements per pass (kDirItemElems / (kThr kDirPer) passes),
-// in output order; for every tile pair it forms their operand base offsets,
-// then walks the contracted indices with all kDirPer loads of A and of B in
+// kPer output elements of a thread, from element e0 of the item on, kThr
+// apart: for every tile pair their operand base offsets, then the contracted
+// indices with the loads of kUnroll of them in flight.
+template <int kThr, int kPer, int kUnroll, bool kCoh, bool kStore>
+__device__ __forceinline__ void direct_elements(const DirSmem& sm, uint32_t e0, const double* __restrict__ A,
+                                                const double* __restrict__ B, double* __restrict__ C, double alpha) {
+  const DirItem& it = sm.item;
+  const uint32_t e1 = it.f1.d, e2 = it.f2.d, e3 = it.f3.d;
+  double acc[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) acc[k] = 0.0;
+  for (uint32_t p = 0; p < it.npair; ++p) {
+    const DirPair& pr = sm.pairs[p];
+    // offsets inside the operand tiles (a tile holds fewer than 2^31 elements)
+    uint32_t ba[kPer], bb[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      // lanes past the end repeat the last element (valid addresses, no store)
+      const uint32_t f = it.f0 + min(e0 + (uint32_t)(k * kThr), it.n - 1);
+      const uint32_t q3 = it.f3.div(f), c3 = f - q3 * e3;
+      const uint32_t q2 = it.f2.div(q3), c2 = q3 - q2 * e2;
+      const uint32_t c0 = it.f1.div(q2), c1 = q2 - c0 * e1;
+      ba[k] = (uint32_t)(c0 * pr.sA[0] + c1 * pr.sA[1] + c2 * pr.sA[2] + c3 * pr.sA[3]);
+      bb[k] = (uint32_t)(c0 * pr.sB[0] + c1 * pr.sB[1] + c2 * pr.sB[2] + c3 * pr.sB[3]);
+    }
+    // the pair's loop fields in registers; its sign flips the sign bit of
+    // the A values on the integer pipe (written as a floating-point
+    // negation it costs a second DFMA per product: both signs computed,
+    // then selected)
+    const uint32_t ek0 = pr.ek[0], ek1 = pr.ek[1];
+    const int64_t sak0 = pr.sAk[0], sak1 = pr.sAk[1], sbk0 = pr.sBk[0], sbk1 = pr.sBk[1];
+    const double* __restrict__ A0 = A + pr.offA;
+    const double* __restrict__ B0 = B + pr.offB;
+    const long long flip = pr.neg != 0 ? (long long)0x8000000000000000ull : 0ll;
+    for (uint32_t k1 = 0; k1 < ek1; ++k1) {
+      const double* __restrict__ pa = A0 + (int64_t)k1 * sak1;
+      const double* __restrict__ pb = B0 + (int64_t)k1 * sbk1;
+      uint32_t k0 = 0;
+      if constexpr (kUnroll > 1) {
+        for (; k0 + kUnroll <= ek0; k0 += kUnroll) {
+          long long x[kUnroll][kPer];
+          double y[kUnroll][kPer];
+#pragma unroll
+          for (int u = 0; u < kUnroll; ++u)
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+              x[u][k] = __double_as_longlong(ldin<kCoh>(pa + (int64_t)(k0 + u) * sak0 + ba[k]));
+              y[u][k] = ldin<kCoh>(pb + (int64_t)(k0 + u) * sbk0 + bb[k]);
+            }
+#pragma unroll
+          for (int u = 0; u < kUnroll; ++u)
+#pragma unroll
+            for (int k = 0; k < kPer; ++k)
+              acc[k] = __fma_rn(__longlong_as_double(x[u][k] ^ flip), y[u][k], acc[k]);
+        }
+      }
+      for (; k0 < ek0; ++k0) {
+        long long x[kPer];
+        double y[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+          x[k] = __double_as_longlong(ldin<kCoh>(pa + (int64_t)k0 * sak0 + ba[k]));
+          y[k] = ldin<kCoh>(pb + (int64_t)k0 * sbk0 + bb[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) acc[k] = __fma_rn(__longlong_as_double(x[k] ^ flip), y[k], acc[k]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = e0 + (uint32_t)(k * kThr);
+    if (e < it.n) {
+      double* c = C + it.coff + e;
+      if constexpr (kStore) *c = __dmul_rn(alpha, acc[k]);
+      else *c = __fma_rn(alpha, acc[k], ldrw<kCoh>(c));
+    }
+  }
+}
+
+// One CTA per work item (grid-stride), kThr threads, kDirPer output elements
+// per thread and pass in output order, with all their loads of A and of B in
 // flight.  Consecutive lanes hold consecutive output elements, so the
 // operand that carries the output's last dimension is read coalesced and the
-// other one is (mostly) a broadcast.  Every output element is the same
-// sequence of fused multiply-adds whatever kThr is.
+// other one is (mostly) a broadcast.  Items of at most kThr elements (the
+// planner cuts small outputs so, see direct_step) take one element per
+// thread, warps beyond the end none, and several contracted indices at once.
+// Every output element is the same sequence of fused multiply-adds either
+// way.
 // kStore: C = alpha * sum (the items cover every element of C, which holds
 // no earlier value), else C += alpha * sum -- a template parameter, so that
 // the accumulating kernel's C loads are scheduled as without the choice.
@@ -420,62 +502,14 @@ __device__ __forceinline__ void direct_body(const DirItem* __restrict__ items, i
     const DirItem& it = sm.item;
     if (threadIdx.x < it.npair) sm.pairs[threadIdx.x] = pairs[it.pair0 + threadIdx.x];
     __syncthreads();
-    const uint32_t e1 = it.f1.d, e2 = it.f2.d, e3 = it.f3.d;
-#pragma unroll 1
-    for (int pass = 0; pass < kPasses; ++pass) {
-      const uint32_t e0 = (uint32_t)(pass * kThr * kDirPer) + threadIdx.x;
-      double acc[kDirPer];
-#pragma unroll
-      for (int k = 0; k < kDirPer; ++k) acc[k] = 0.0;
-      for (uint32_t p = 0; p < it.npair; ++p) {
-        const DirPair& pr = sm.pairs[p];
-        // offsets inside the operand tiles (a tile holds fewer than 2^31 elements)
-        uint32_t ba[kDirPer], bb[kDirPer];
-#pragma unroll
-        for (int k = 0; k < kDirPer; ++k) {
-          // lanes past the end repeat the last element (valid addresses, no store)
-          const uint32_t f = it.f0 + min(e0 + (uint32_t)(k * kThr), it.n - 1);
-          const uint32_t q3 = it.f3.div(f), c3 = f - q3 * e3;
-          const uint32_t q2 = it.f2.div(q3), c2 = q3 - q2 * e2;
-          const uint32_t c0 = it.f1.div(q2), c1 = q2 - c0 * e1;
-          ba[k] = (uint32_t)(c0 * pr.sA[0] + c1 * pr.sA[1] + c2 * pr.sA[2] + c3 * pr.sA[3]);
-          bb[k] = (uint32_t)(c0 * pr.sB[0] + c1 * pr.sB[1] + c2 * pr.sB[2] + c3 * pr.sB[3]);
-        }
-        // the pair's loop fields in registers; its sign flips the sign bit of
-        // the A values on the integer pipe (written as a floating-point
-        // negation it costs a second DFMA per product: both signs computed,
-        // then selected)
-        const uint32_t ek0 = pr.ek[0], ek1 = pr.ek[1];
-        const int64_t sak0 = pr.sAk[0], sak1 = pr.sAk[1], sbk0 = pr.sBk[0], sbk1 = pr.sBk[1];
-        const double* __restrict__ A0 = A + pr.offA;
-        const double* __restrict__ B0 = B + pr.offB;
-        const long long flip = pr.neg != 0 ? (long long)0x8000000000000000ull : 0ll;
-        for (uint32_t k1 = 0; k1 < ek1; ++k1) {
-          for (uint32_t k0 = 0; k0 < ek0; ++k0) {
-            const double* __restrict__ pa = A0 + (int64_t)k0 * sak0 + (int64_t)k1 * sak1;
-            const double* __restrict__ pb = B0 + (int64_t)k0 * sbk0 + (int64_t)k1 * sbk1;
-            long long x[kDirPer];
-            double y[kDirPer];
-#pragma unroll
-            for (int k = 0; k < kDirPer; ++k) {
-              x[k] = __double_as_longlong(ldin<kCoh>(pa + ba[k]));
-              y[k] = ldin<kCoh>(pb + bb[k]);
-            }
-#pragma unroll
-            for (int k = 0; k < kDirPer; ++k) acc[k] = __fma_rn(__longlong_as_double(x[k] ^ flip), y[k], acc[k]);
-          }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kDirPer; ++k) {
-        const uint32_t e = e0 + (uint32_t)(k * kThr);
-        if (e < it.n) {
-          double* c = C + it.coff + e;
-          if constexpr (kStore) *c = __dmul_rn(alpha, acc[k]);
-          else *c = __fma_rn(alpha, acc[k], ldrw<kCoh>(c));
-        }
-      }
+    if (it.n <= (uint32_t)kThr) {
+      if ((threadIdx.x & ~31u) < it.n)
+        direct_elements<kThr, 1, 8, kCoh, kStore>(sm, threadIdx.x, A, B, C, alpha);
+      continue;
     }
+#pragma unroll 1
+    for (int pass = 0; pass < kPasses; ++pass)
+      direct_elements<kThr, kDirPer, 1, kCoh, kStore>(sm, (uint32_t)(pass * kThr * kDirPer) + threadIdx.x, A, B, C, alpha);
   }
 }
 
@@ -1090,27 +1124,26 @@ __device__ __forceinline__ void dot_partial_body(const double* __restrict__ x, c
   if (threadIdx.x == 0) partial[bid] = red[0];
 }
 
-// The partials are staged through shared memory by all threads, 256 at a
-// time, and added by one thread in index order (the same sum as one thread
-// reading them one by one, without its chain of dependent global loads).
+// The partials are added by all threads, each every 256th in order, and the
+// 256 sums pairwise: a fixed order, without one thread's chain of np
+// dependent additions (608 partials: 25 us so, 5 now).
 template <bool kCoh>
 __device__ __forceinline__ void energy_final_body(const double* __restrict__ partial, int np, double scale,
                                                   double* __restrict__ hist, int* __restrict__ count, int cap,
                                                   uint32_t bid, double* stage) {
   if (bid != 0) return;
   double s = 0.0;
-  for (int i0 = 0; i0 < np; i0 += kCcThreads) {
+  for (int i = (int)threadIdx.x; i < np; i += kCcThreads) s += ldrw<kCoh>(partial + i);
+  __syncthreads();
+  stage[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = kCcThreads / 2; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) stage[threadIdx.x] += stage[threadIdx.x + w];
     __syncthreads();
-    if (i0 + (int)threadIdx.x < np) stage[threadIdx.x] = ldrw<kCoh>(partial + i0 + threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int n = min(kCcThreads, np - i0);
-      for (int i = 0; i < n; ++i) s += stage[i];
-    }
   }
   if (threadIdx.x == 0) {
     int k = ldrw<kCoh>(count);
-    if (k < cap) hist[k] = s * scale;
+    if (k < cap) hist[k] = stage[0] * scale;
     *count = k + 1;
   }
 }

@@ -102,7 +102,9 @@ struct MoveSet {
   MoveDesc4* d_desc4 = nullptr;
   uint32_t* d_chunk_desc = nullptr;  // descriptor of each chunk
   uint32_t nchunks = 0;
+  uint32_t chunk = 0;  // elements of a chunk (compact descriptors)
   int ndesc = 0;
+  uint32_t chunk4() const;
   int upload();   // copies host -> device (allocates)
   void release();
   size_t device_bytes() const;  // what upload() allocates
@@ -174,7 +176,7 @@ int run_fused_sum(const FsItem* items, int nitems, const FsTerm* terms, const Fs
 // with one fused multiply-add per product (FP64 instructions are the bound
 // on this part, so no separate pack, GEMM and unpack passes).
 constexpr int kDirMaxPairs = 32;     // operand tile pairs of one output tile
-constexpr int kDirItemElems = 2048;  // output elements per work item
+constexpr int kDirItemElems = 2048;  // output elements per work item (at most)
 
 struct DirPair {
   int64_t offA, offB;      // stored operand tiles

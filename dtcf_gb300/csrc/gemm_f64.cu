@@ -245,13 +245,15 @@ __device__ __forceinline__ void warp_tile_item(const GemmProblem& p, int64_t loc
   });
 }
 
-// One work item of problem p: output tile and K range `local`.  ts: tile
+// One work item of problem p: output tile and K range `local`.  TS: tile
 // edge, 16 or 8; 0: a tile per warp.
-__device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, int ts, TileSmem& sm) {
-  if (ts == 0) {
+template <int TS>
+__device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, TileSmem& sm) {
+  if constexpr (TS == 0) {
     warp_tile_item(p, local);
     return;
   }
+  constexpr int ts = TS;
   const cg::cluster_group cl = cg::this_cluster();
   const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
   const int warp = threadIdx.x >> 5;
@@ -266,9 +268,11 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, i
   const int s0 = min(steps, (crank * kTileWarps + warp) * per), s1 = min(steps, s0 + per);
   const bool m2 = ts == 16 && p.m - m0 > 8, n2 = ts == 16 && p.n - n0 > 8;
   double* part = sm.part[warp];
-  tile_blocks(p, m2, n2, m0, n0, kbeg, kend, s0, s1, [&](int i, int j, double x, double y) {
+  const auto keep = [&](int i, int j, double x, double y) {
     *reinterpret_cast<double2*>(part + i * 16 + j) = make_double2(x, y);
-  });
+  };
+  if constexpr (TS == 8) tile_loop<1, 1>(p, m0, n0, kbeg, kend, s0, s1, keep);
+  else tile_blocks(p, m2, n2, m0, n0, kbeg, kend, s0, s1, keep);
   __syncthreads();
   const int rows = min(ts, p.m - m0), cols = min(ts, p.n - n0);
   const auto add = [&](int e) {
@@ -309,8 +313,9 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, i
 
 // All problems of a launch, one work item per cluster: the item's problem is
 // found by a 32-way search of the first-item table.
-__global__ void __launch_bounds__(kTileThreads, 4)
-    tile_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob, const int* __restrict__ first, int ts) {
+template <int TS>
+__global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
+    tile_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob, const int* __restrict__ first) {
   __shared__ TileSmem sm;
   const int item = (int)(blockIdx.x / cg::this_cluster().num_blocks());
   int lo = 0, n = nprob;
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(kTileThreads, 4)
     n = min(step, lo + n - nlo);
     lo = nlo;
   }
-  tile_item(probs[lo], item - first[lo], ts, sm);
+  tile_item<TS>(probs[lo], item - first[lo], sm);
 }
 
 // A one-problem launch with its descriptor in the kernel's arguments: nothing to upload, no search.
@@ -333,9 +338,11 @@ struct OneProblem {
   uint32_t red_first;  // and its first chunk (0)
 };
 
-__global__ void __launch_bounds__(kTileThreads, 4) tile_one_f64_kernel(const __grid_constant__ OneProblem a, int ts) {
+template <int TS>
+__global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
+    tile_one_f64_kernel(const __grid_constant__ OneProblem a) {
   __shared__ TileSmem sm;
-  tile_item(a.p, blockIdx.x / cg::this_cluster().num_blocks(), ts, sm);
+  tile_item<TS>(a.p, blockIdx.x / cg::this_cluster().num_blocks(), sm);
 }
 
 // K <= 8 (dev::small_k_body).
@@ -403,11 +410,13 @@ namespace {
 // tile per warp) and the cluster size.  16 x 16 tiles read half the operand
 // bytes per product of 8 x 8 ones, but only many tiles keep the last wave
 // short: a tile per warp where the waves of warps are many or full (no
-// reduction through shared memory: 300000 x 32 x 30 722 -> 612 us), a tile
-// per CTA from eight per SM on, else 8 x 8, and with fewer than four of those
-// per SM clusters share a tile's K steps, at least three for every warp.
-// 64 x 48 x 96 takes 9 us a call so (one 64 x 64 tile: 129 us), 1021 x 765 x
-// 1531 2.29 ms, 1.045 TFLOP/s (64 x 64 tiles: 2.36 ms).
+// reduction through shared memory: 300000 x 32 x 30 722 -> 612 us), 16 x 16
+// per CTA from twelve per SM on, else 8 x 8 (500 x 500 x 100: 57 us, 65 with
+// 16 x 16).  While those leave fewer than two CTAs per SM, clusters share a
+// tile's K steps, at least six for every warp (64 x 64 x 432: 10.3 us without,
+// 8.3 with four; 192 x 192 x 192, 576 tiles: 17.2 without, 18.7 with two).
+// 64 x 48 x 96 takes 3.9 us on the GPU so (one 64 x 64 tile: 125), 1021 x 765
+// x 1531 2.29 ms, 1.045 TFLOP/s (64 x 64 tiles: 2.36 ms).
 struct TilePlan {
   int ts = 16, cluster = 1;
 };
@@ -425,9 +434,9 @@ TilePlan tile_plan(const std::vector<const GemmProblem*>& probs) {
   }
   const int64_t waves = (n16 + kQuarters - 1) / kQuarters;
   if (waves >= 16 || (waves >= 4 && n16 >= 0.92 * (double)(waves * kQuarters))) t.ts = 0;
-  if (n16 >= 8 * kSms) return t;
+  if (t.ts == 0 || n16 >= 12 * kSms) return t;
   t.ts = 8;
-  while (t.cluster < 8 && n8 * t.cluster < 4 * kSms && ceil_div(kmax, 4) >= 12 * t.cluster) t.cluster *= 2;
+  while (t.cluster < 8 && n8 * t.cluster <= kSms && ceil_div(kmax, 4) >= 48 * t.cluster) t.cluster *= 2;
   return t;
 }
 
@@ -672,7 +681,9 @@ int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first,
                    cudaStream_t st) {
   const int grid = std::min(tiles, kSms * 8);
   switch (v) {
-    case 0: return launch_tiles(tile_gemm_f64_kernel, tp, tiles, st, probs, nprob, first, tp.ts);
+    case 0:
+      return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8> : tp.ts ? tile_gemm_f64_kernel<16> : tile_gemm_f64_kernel<0>,
+                          tp, tiles, st, probs, nprob, first);
     case 4: thin_gemm_f64_kernel<true><<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
     case 6: small_k_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
     case 7: small_out_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
@@ -744,7 +755,10 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
   const int grid = (int)std::min<int64_t>(items, kSms * 8);
   int rc = GBX_OK;
   switch (q.pad_) {
-    case 0: rc = launch_tiles(tile_one_f64_kernel, tp, items, st, a, tp.ts); break;
+    case 0:
+      rc = launch_tiles(tp.ts == 8 ? tile_one_f64_kernel<8> : tp.ts ? tile_one_f64_kernel<16> : tile_one_f64_kernel<0>, tp,
+                        items, st, a);
+      break;
     case 4: thin_one_f64_kernel<true><<<grid, 256, 0, st>>>(a, (int)items); break;
     case 6: small_k_one_f64_kernel<<<grid, 256, 0, st>>>(a, (int)items); break;
     default: thin_one_f64_kernel<false><<<grid, 256, 0, st>>>(a, (int)items); break;

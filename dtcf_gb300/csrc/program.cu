@@ -89,6 +89,10 @@ __device__ __forceinline__ void run_record(const ProgRec& r, uint32_t vb, ProgSm
       dev::move4_body<true, kProgMovePer>(a.move4.descs, a.move4.chunk_desc, a.move4.nchunks, a.move4.src,
                                           a.move4.dst, a.move4.alpha, a.move4.pairs, vb, g);
       break;
+    case PK_MOVE4S:
+      dev::move4_body<true, 2, dev::kMove4Small>(a.move4.descs, a.move4.chunk_desc, a.move4.nchunks, a.move4.src,
+                                                 a.move4.dst, a.move4.alpha, a.move4.pairs, vb, g);
+      break;
     case PK_FUSED:
       dev::fused_sum_body<true>(a.fused.items, a.fused.nitems, a.fused.terms, a.fused.src, a.fused.scale, a.fused.out,
                                 vb, g, sm.fs);

@@ -53,6 +53,7 @@ enum ProgKind : int32_t {
   PK_ZERO,
   PK_MOVE,
   PK_MOVE4,
+  PK_MOVE4S,
   PK_FUSED,
   PK_DIRECT,
   PK_ROWEXP,
