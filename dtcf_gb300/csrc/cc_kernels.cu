@@ -9,6 +9,7 @@
 
 #include "bodies.cuh"
 #include "cc.h"
+#include "launch.h"
 #include "program.h"
 
 namespace gbx {
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kThreads) cc_tile_kernel(const CCTile* __restr
 
 __global__ void __launch_bounds__(kThreads) mul_kernel(const double* __restrict__ a, const double* __restrict__ b,
                                                        double* __restrict__ out, int64_t n) {
+  begin_dependent();
   dev::mul_body<false>(a, b, out, n, blockIdx.x, gridDim.x);
 }
 
@@ -97,11 +99,13 @@ __global__ void __launch_bounds__(kThreads) mul_kernel(const double* __restrict_
 __global__ void __launch_bounds__(kThreads) dot_partial_kernel(const double* __restrict__ x,
                                                                const double* __restrict__ y, int64_t n,
                                                                double* __restrict__ partial) {
+  begin_dependent();
   __shared__ double red[kThreads];
   dev::dot_partial_body<false>(x, y, n, partial, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void dot_final_kernel(const double* __restrict__ partial, int np, double scale, double* __restrict__ out) {
+  begin_dependent();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     double s = 0.0;
     for (int i = 0; i < np; ++i) s += partial[i];
@@ -112,6 +116,7 @@ __global__ void dot_final_kernel(const double* __restrict__ partial, int np, dou
 __global__ void __launch_bounds__(kThreads) energy_final_kernel(const double* __restrict__ partial, int np,
                                                                 double scale, double* __restrict__ hist,
                                                                 int* __restrict__ count, int cap) {
+  begin_dependent();
   __shared__ double stage[kThreads];
   dev::energy_final_body<false>(partial, np, scale, hist, count, cap, blockIdx.x, stage);
 }
@@ -125,10 +130,8 @@ int run_energy(const double* V, const double* tau, int64_t n, double* partial, i
     a.efin = {partial, hist, count, 0.25, npartial, cap};
     return prog_mem(rec, PK_ENERGYFIN, 1, a, {{partial, false}, {hist, true}, {count, true}});
   }
-  dot_partial_kernel<<<npartial, kThreads, 0, st>>>(V, tau, n, partial);
-  GBX_CUDA(cudaGetLastError());
-  energy_final_kernel<<<1, kThreads, 0, st>>>(partial, npartial, 0.25, hist, count, cap);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(dot_partial_kernel, (unsigned)npartial, kThreads, st, V, tau, n, partial));
+  GBX_TRY(launch(energy_final_kernel, 1u, kThreads, st, partial, npartial, 0.25, hist, count, cap));
   return GBX_OK;
 }
 
@@ -165,6 +168,7 @@ __global__ void __launch_bounds__(kThreads) cc_amp_kernel(const CCAmpTile* __res
                                                          const double* __restrict__ t1,
                                                          const double* __restrict__ t2, double* __restrict__ tau,
                                                          double* __restrict__ taut, double* __restrict__ Q) {
+  begin_dependent();
   dev::cc_amp_body<false>(tiles, items, nitems, t1, t2, tau, taut, Q, blockIdx.x, gridDim.x);
 }
 
@@ -198,8 +202,7 @@ int run_cc_amp(const CCAmpSet& s, const double* t1, const double* t2, double* ta
     return prog_mem(rec, PK_AMP, (uint32_t)grid, a,
                     {{t1, false}, {t2, false}, {tau, true}, {taut, true}, {Q, true}});
   }
-  cc_amp_kernel<<<grid, kThreads, 0, st>>>(s.d_tiles, s.d_items, s.nitems, t1, t2, tau, taut, Q);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(cc_amp_kernel, (unsigned)grid, kThreads, st, s.d_tiles, s.d_items, s.nitems, t1, t2, tau, taut, Q));
   return GBX_OK;
 }
 
@@ -211,8 +214,7 @@ int run_mul(const double* a, const double* b, double* out, int64_t n, cudaStream
     pa.mul = {a, b, out, n};
     return prog_mem(rec, PK_MUL, (uint32_t)grid, pa, {{a, false}, {b, false}, {out, true}});
   }
-  mul_kernel<<<grid, kThreads, 0, st>>>(a, b, out, n);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(mul_kernel, (unsigned)grid, kThreads, st, a, b, out, n));
   return GBX_OK;
 }
 
@@ -227,10 +229,8 @@ int run_cc_tiles(const CCTileSet& ts, int op, const CCDeviceTables& tab, const d
 
 int run_dot(const double* x, const double* y, int64_t n, double scale, double* partial, int npartial, double* out,
             cudaStream_t st) {
-  dot_partial_kernel<<<npartial, kThreads, 0, st>>>(x, y, n, partial);
-  GBX_CUDA(cudaGetLastError());
-  dot_final_kernel<<<1, 32, 0, st>>>(partial, npartial, scale, out);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(dot_partial_kernel, (unsigned)npartial, kThreads, st, x, y, n, partial));
+  GBX_TRY(launch(dot_final_kernel, 1u, 32, st, partial, npartial, scale, out));
   return GBX_OK;
 }
 

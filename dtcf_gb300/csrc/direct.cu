@@ -9,6 +9,7 @@
 
 #include "bodies.cuh"
 #include "common.h"
+#include "launch.h"
 #include "program.h"
 
 namespace gbx {
@@ -23,6 +24,7 @@ __global__ void __launch_bounds__(kDirThreads, 2)
     direct_contract_kernel(const DirItem* __restrict__ items, int nitems, const DirPair* __restrict__ pairs,
                            const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
                            double alpha) {
+  begin_dependent();
   __shared__ dev::DirSmem sm;
   dev::direct_body<kDirThreads, false, kStore>(items, nitems, pairs, A, B, C, alpha, blockIdx.x, gridDim.x, sm);
 }
@@ -36,9 +38,10 @@ int run_direct(const DirItem* items, int nitems, const DirPair* pairs, const dou
     a.direct = {items, pairs, A, B, C, alpha, nitems, overwrite ? 1 : 0};
     return prog_mem(rec, PK_DIRECT, (uint32_t)grid, a, {{A, false}, {B, false}, {C, true}});
   }
-  if (overwrite) direct_contract_kernel<true><<<grid, kDirThreads, 0, st>>>(items, nitems, pairs, A, B, C, alpha);
-  else direct_contract_kernel<false><<<grid, kDirThreads, 0, st>>>(items, nitems, pairs, A, B, C, alpha);
-  GBX_CUDA(cudaGetLastError());
+  if (overwrite) GBX_TRY(launch(direct_contract_kernel<true>, (unsigned)grid, kDirThreads, st, items, nitems, pairs, A,
+                                B, C, alpha));
+  else GBX_TRY(launch(direct_contract_kernel<false>, (unsigned)grid, kDirThreads, st, items, nitems, pairs, A, B, C,
+                      alpha));
   return GBX_OK;
 }
 

@@ -15,6 +15,7 @@
 
 #include "bodies.cuh"
 #include "common.h"
+#include "launch.h"
 #include "program.h"
 
 namespace cg = cooperative_groups;
@@ -126,6 +127,7 @@ __device__ __forceinline__ void thin_body(const GemmProblem* __restrict__ probs,
 template <bool kRows>
 __global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                             const int* __restrict__ block_first, int total_blocks) {
+  begin_dependent();
   __shared__ double Ts[kThinN * kThinK];
   thin_body<kRows>(probs, nprob, block_first, total_blocks, Ts);
 }
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* _
 // Matrix-vector shapes (variant 8): dev::gemv_body.
 __global__ void __launch_bounds__(256) gemv_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                        const int* __restrict__ block_first, int total_blocks) {
+  begin_dependent();
   dev::gemv_body<false>(probs, nprob, block_first, total_blocks, blockIdx.x, gridDim.x);
 }
 
@@ -316,6 +319,7 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, T
 template <int TS>
 __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
     tile_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob, const int* __restrict__ first) {
+  begin_dependent();
   __shared__ TileSmem sm;
   const int item = (int)(blockIdx.x / cg::this_cluster().num_blocks());
   int lo = 0, n = nprob;
@@ -341,6 +345,7 @@ struct OneProblem {
 template <int TS>
 __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
     tile_one_f64_kernel(const __grid_constant__ OneProblem a) {
+  begin_dependent();
   __shared__ TileSmem sm;
   tile_item<TS>(a.p, blockIdx.x / cg::this_cluster().num_blocks(), sm);
 }
@@ -348,12 +353,14 @@ __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
 // K <= 8 (dev::small_k_body).
 __global__ void __launch_bounds__(256) small_k_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                                const int* __restrict__ block_first, int total_blocks) {
+  begin_dependent();
   dev::small_k_body<false>(probs, nprob, block_first, total_blocks, blockIdx.x, gridDim.x);
 }
 
 // Small output, long K (variant 7, dev::small_out_body).
 __global__ void __launch_bounds__(256) small_out_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                                  const int* __restrict__ item_first, int total) {
+  begin_dependent();
   __shared__ dev::SmallOutSmem sm;
   dev::small_out_body<false>(probs, nprob, item_first, total, blockIdx.x, gridDim.x, sm);
 }
@@ -363,6 +370,7 @@ __global__ void __launch_bounds__(kRedThreads) splitk_reduce_kernel(const GemmPr
                                                                     const int* __restrict__ red_prob,
                                                                     const uint32_t* __restrict__ red_first, int nred,
                                                                     uint32_t nchunks) {
+  begin_dependent();
   __shared__ double red[kRedThreads];
   dev::splitk_reduce_body<false>(probs, red_prob, red_first, nred, nchunks, blockIdx.x, gridDim.x, red);
 }
@@ -370,14 +378,17 @@ __global__ void __launch_bounds__(kRedThreads) splitk_reduce_kernel(const GemmPr
 // The one-problem forms of the kernels above.
 template <bool kRows>
 __global__ void __launch_bounds__(256) thin_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  begin_dependent();
   __shared__ double Ts[kThinN * kThinK];
   thin_body<kRows>(&a.p, 1, &a.zero, total, Ts);
 }
 __global__ void __launch_bounds__(256) small_k_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  begin_dependent();
   dev::small_k_body<false>(&a.p, 1, &a.zero, total, blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(kRedThreads) splitk_reduce_one_kernel(const __grid_constant__ OneProblem a,
                                                                         uint32_t nchunks) {
+  begin_dependent();
   __shared__ double red[kRedThreads];
   dev::splitk_reduce_body<false>(&a.p, &a.red_prob, &a.red_first, 1, nchunks, blockIdx.x, gridDim.x, red);
 }
@@ -524,20 +535,9 @@ uint64_t red_chunks_of(const GemmProblem& q) {
 
 // Launch of a tile kernel over `items` work items, one cluster each.
 template <class K, class... A>
-int launch_tiles(K kernel, const TilePlan& t, int64_t items, cudaStream_t st, A... args) {
+int launch_tiles(K kernel, const TilePlan& t, int64_t items, cudaStream_t st, const A&... args) {
   if (items * t.cluster >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "FP64 GEMM has too many work items");
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(items * t.cluster));
-  cfg.blockDim = dim3(kTileThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = t.cluster;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = t.cluster > 1 ? 1 : 0;
-  GBX_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-  return GBX_OK;
+  return launch_dependent(kernel, (unsigned)(items * t.cluster), kTileThreads, st, (unsigned)t.cluster, args...);
 }
 
 }  // namespace
@@ -669,8 +669,8 @@ int F64Gemm::run(cudaStream_t st) const {
   for (const Sub& sb : subs) GBX_TRY(run_sub(sb, st));
   if (nred) {
     int rg = (int)std::min<uint32_t>(red_chunks, 152u * 8u);
-    splitk_reduce_kernel<<<rg, kRedThreads, 0, st>>>(d_all, d_red_prob, d_red_first, nred, red_chunks);
-    GBX_CUDA(cudaGetLastError());
+    GBX_TRY(launch(splitk_reduce_kernel, (unsigned)rg, kRedThreads, st, d_all, d_red_prob, d_red_first, nred,
+                   red_chunks));
   }
   return GBX_OK;
 }
@@ -684,14 +684,12 @@ int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first,
     case 0:
       return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8> : tp.ts ? tile_gemm_f64_kernel<16> : tile_gemm_f64_kernel<0>,
                           tp, tiles, st, probs, nprob, first);
-    case 4: thin_gemm_f64_kernel<true><<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
-    case 6: small_k_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
-    case 7: small_out_gemm_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
-    case 8: gemv_f64_kernel<<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
-    default: thin_gemm_f64_kernel<false><<<grid, 256, 0, st>>>(probs, nprob, first, tiles); break;
+    case 4: return launch(thin_gemm_f64_kernel<true>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
+    case 6: return launch(small_k_gemm_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
+    case 7: return launch(small_out_gemm_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
+    case 8: return launch(gemv_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
+    default: return launch(thin_gemm_f64_kernel<false>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
   }
-  GBX_CUDA(cudaGetLastError());
-  return GBX_OK;
 }
 }  // namespace
 
@@ -717,8 +715,8 @@ int F64Gemm::run_each(cudaStream_t st) const {
   }
   if (nred) {
     int rg = (int)std::min<uint32_t>(red_chunks, 152u * 8u);
-    splitk_reduce_kernel<<<rg, kRedThreads, 0, st>>>(d_all, d_red_prob, d_red_first, nred, red_chunks);
-    GBX_CUDA(cudaGetLastError());
+    GBX_TRY(launch(splitk_reduce_kernel, (unsigned)rg, kRedThreads, st, d_all, d_red_prob, d_red_first, nred,
+                   red_chunks));
   }
   return GBX_OK;
 }
@@ -759,18 +757,15 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
       rc = launch_tiles(tp.ts == 8 ? tile_one_f64_kernel<8> : tp.ts ? tile_one_f64_kernel<16> : tile_one_f64_kernel<0>, tp,
                         items, st, a);
       break;
-    case 4: thin_one_f64_kernel<true><<<grid, 256, 0, st>>>(a, (int)items); break;
-    case 6: small_k_one_f64_kernel<<<grid, 256, 0, st>>>(a, (int)items); break;
-    default: thin_one_f64_kernel<false><<<grid, 256, 0, st>>>(a, (int)items); break;
+    case 4: rc = launch(thin_one_f64_kernel<true>, (unsigned)grid, 256, st, a, (int)items); break;
+    case 6: rc = launch(small_k_one_f64_kernel, (unsigned)grid, 256, st, a, (int)items); break;
+    default: rc = launch(thin_one_f64_kernel<false>, (unsigned)grid, 256, st, a, (int)items); break;
   }
-  cudaError_t e = cudaGetLastError();
-  if (rc == GBX_OK && e == cudaSuccess && q.ksplit > 1) {
+  if (rc == GBX_OK && q.ksplit > 1) {
     const uint32_t chunks = (uint32_t)red_chunks_of(q);
-    splitk_reduce_one_kernel<<<std::min<uint32_t>(chunks, kSms * 8u), kRedThreads, 0, st>>>(a, chunks);
-    e = cudaGetLastError();
+    rc = launch(splitk_reduce_one_kernel, std::min<uint32_t>(chunks, kSms * 8u), kRedThreads, st, a, chunks);
   }
   if (own) cudaFreeAsync(own, st);
-  if (rc == GBX_OK && e != cudaSuccess) rc = cuda_fail(e, "FP64 GEMM launch", __FILE__, __LINE__);
   return rc;
 }
 }  // namespace gbx

@@ -40,6 +40,7 @@
 #include <utility>
 
 #include "bodies.cuh"
+#include "launch.h"
 #include "program.h"
 #include "split.h"
 #include "split_dev.h"
@@ -1088,30 +1089,35 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const DevProblem* __r
                                                            const int* __restrict__ red_prob,
                                                            const int64_t* __restrict__ red_first, int nred,
                                                            int64_t total) {
+  begin_dependent();
   dev::split_reduce_body<false>(probs, red_prob, red_first, nred, total, blockIdx.x, gridDim.x);
 }
 
 // Operand splits (dev::row_exponent_body, dev::digits_body, dev::short_rows_body).
 __global__ void __launch_bounds__(256) row_exponent_kernel(const SplitRowSet* __restrict__ sets, int nsets,
                                                            int64_t total_chunks) {
+  begin_dependent();
   __shared__ uint32_t red[8];
   dev::row_exponent_body<false>(sets, nsets, total_chunks, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void __launch_bounds__(256) digits_kernel(const SplitRowSet* __restrict__ sets, int nsets,
                                                      int64_t total_chunks, int S) {
+  begin_dependent();
   dev::digits_body<false>(sets, nsets, total_chunks, S, blockIdx.x, gridDim.x);
 }
 
 template <bool kFour>
 __global__ void __launch_bounds__(256, kFour ? 3 : 4)
     split_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows, int S) {
+  begin_dependent();
   __shared__ uint32_t red[8];
   dev::split_rows_body<false, kFour>(sets, nsets, total_rows, S, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void __launch_bounds__(256) split_short_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets,
                                                                int64_t total_rows, int S, int lg) {
+  begin_dependent();
   dev::short_rows_body<false>(sets, nsets, total_rows, S, lg, blockIdx.x, gridDim.x);
 }
 
@@ -1554,10 +1560,8 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
         GBX_TRY(prog_mem(rec, PK_ROWEXP, (uint32_t)grid, a, {}));
         GBX_TRY(prog_mem(rec, PK_DIGITS, (uint32_t)grid, a, {}));
       } else {
-        row_exponent_kernel<<<grid, 256, 0, st>>>(sets, nsets, chunks);
-        GBX_CUDA(cudaGetLastError());
-        digits_kernel<<<grid, 256, 0, st>>>(sets, nsets, chunks, sp->S);
-        GBX_CUDA(cudaGetLastError());
+        GBX_TRY(launch(row_exponent_kernel, (unsigned)grid, 256, st, sets, nsets, chunks));
+        GBX_TRY(launch(digits_kernel, (unsigned)grid, 256, st, sets, nsets, chunks, sp->S));
       }
     }
     const int64_t mrows = side == 0 ? sp->mid_rows_a : sp->mid_rows_b;
@@ -1571,10 +1575,9 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
         GBX_TRY(prog_mem(rec, PK_SPLITROWS, (uint32_t)grid, a, {}));
       } else {
         if (side == 0 ? sp->mid_four_a : sp->mid_four_b)
-          split_rows_kernel<true><<<grid, 256, 0, st>>>(sets, nsets, mrows, sp->S);
+          GBX_TRY(launch(split_rows_kernel<true>, (unsigned)grid, 256, st, sets, nsets, mrows, sp->S));
         else
-          split_rows_kernel<false><<<grid, 256, 0, st>>>(sets, nsets, mrows, sp->S);
-        GBX_CUDA(cudaGetLastError());
+          GBX_TRY(launch(split_rows_kernel<false>, (unsigned)grid, 256, st, sets, nsets, mrows, sp->S));
       }
     }
     const int64_t srows = side == 0 ? sp->short_rows_a : sp->short_rows_b;
@@ -1589,8 +1592,7 @@ int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
         GBX_TRY(prog_mem(rec, PK_SHORTROWS, (uint32_t)grid, a, {}));
         continue;
       }
-      split_short_rows_kernel<<<grid, 256, 0, st>>>(sets, nsets, srows, sp->S, lg);
-      GBX_CUDA(cudaGetLastError());
+      GBX_TRY(launch(split_short_rows_kernel, (unsigned)grid, 256, st, sets, nsets, srows, sp->S, lg));
     }
   }
   return GBX_OK;
@@ -1685,8 +1687,8 @@ int run_split_plan(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
       a.splitred = {sp->d_all, sp->d_red_prob, sp->d_red_first, sp->red_total, sp->nred};
       return prog_mem(rec, PK_SPLITRED, (uint32_t)rg, a, {});
     }
-    split_reduce_kernel<<<rg, 256, 0, st>>>(sp->d_all, sp->d_red_prob, sp->d_red_first, sp->nred, sp->red_total);
-    GBX_CUDA(cudaGetLastError());
+    GBX_TRY(launch(split_reduce_kernel, (unsigned)rg, 256, st, sp->d_all, sp->d_red_prob, sp->d_red_first, sp->nred,
+                   sp->red_total));
   }
   return GBX_OK;
 }

@@ -17,6 +17,7 @@
 
 #include "../../include/gbx.h"
 #include "common.h"
+#include "launch.h"
 #include "plan.h"
 #include "split.h"
 
@@ -37,6 +38,7 @@ struct ApplyDesc {
 __global__ void __launch_bounds__(256) apply_kernel(const ApplyDesc* __restrict__ d, int nd,
                                                     const int64_t* __restrict__ first, int64_t total,
                                                     const double* __restrict__ W) {
+  begin_dependent();
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     int lo = 0, hi = nd - 1;
     while (lo < hi) {
@@ -222,8 +224,7 @@ struct GroupPlan {
     if (split) GBX_TRY(run_split_plan(split, true, true, st));
     if (napply) {
       const int grid = (int)std::min<int64_t>((apply_total + 255) / 256, 152 * 8);
-      apply_kernel<<<grid, 256, 0, st>>>(d_apply, napply, d_apply_first, apply_total, d_w);
-      GBX_CUDA(cudaGetLastError());
+      GBX_TRY(launch(apply_kernel, (unsigned)grid, 256, st, d_apply, napply, d_apply_first, apply_total, d_w));
     }
     return GBX_OK;
   }

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.h"
+#include "launch.h"
 
 namespace gbx {
 
@@ -284,6 +285,7 @@ __device__ __forceinline__ void box_move(const BoxMove& m, uint32_t box, const d
 __global__ void __launch_bounds__(kBoxThreads) box_one_kernel(const __grid_constant__ OneMove a,
                                                               const double* __restrict__ src, double* __restrict__ dst,
                                                               double alpha) {
+  begin_dependent();
   __shared__ double stage[kBoxSmem];
   __shared__ BoxPlace place;
   const uint32_t b = a.per.div(blockIdx.x);
@@ -294,6 +296,7 @@ template <int kBlocks>
 __global__ void __launch_bounds__(kBoxThreads) box_set_kernel(const __grid_constant__ MoveTable<kBlocks> a,
                                                               const double* __restrict__ src,
                                                               double* __restrict__ dst) {
+  begin_dependent();
   __shared__ double stage[kBoxSmem];
   __shared__ BoxPlace place;
   const uint32_t b = a.per.div(blockIdx.x);
@@ -465,8 +468,7 @@ int run_move_one(const MoveDesc& md, const double* src, double* dst, double alph
   a.m = make_box(md, box_target(md.n), (((uintptr_t)src | (uintptr_t)dst) & 15) == 0);
   a.per = FastDiv::make(a.m.boxes);
   a.block = 0;
-  box_one_kernel<<<a.m.boxes, kBoxThreads, 0, st>>>(a, src, dst, alpha);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(box_one_kernel, a.m.boxes, kBoxThreads, st, a, src, dst, alpha));
   return GBX_OK;
 }
 
@@ -498,23 +500,22 @@ int run_block_moves(const std::vector<MoveDesc>& moves, const uint8_t* which, in
       OneMove a;
       a.m = b[0];
       fill(a);
-      box_one_kernel<<<grid, kBoxThreads, 0, st>>>(a, s, d, 1.0);
+      GBX_TRY(launch(box_one_kernel, grid, kBoxThreads, st, a, s, d, 1.0));
     } else {
-      const auto launch = [&](auto& a, auto kernel) {
+      const auto run = [&](auto& a, auto kernel) {
         std::copy(b.begin(), b.end(), a.m);
         fill(a);
         std::copy(which + b0, which + b0 + nb, a.which);
-        kernel<<<grid, kBoxThreads, 0, st>>>(a, s, d);
+        return launch(kernel, grid, kBoxThreads, st, a, s, d);
       };
       if (nb <= 2048) {
         MoveTable<2048> a;
-        launch(a, box_set_kernel<2048>);
+        GBX_TRY(run(a, box_set_kernel<2048>));
       } else {
         MoveTable<kSetBlocks> a;
-        launch(a, box_set_kernel<kSetBlocks>);
+        GBX_TRY(run(a, box_set_kernel<kSetBlocks>));
       }
     }
-    GBX_CUDA(cudaGetLastError());
   }
   return GBX_OK;
 }
@@ -541,6 +542,7 @@ constexpr int kPackChunk = 2048;  // elements of a work item
 template <typename T, bool kToBig, class Table>
 __global__ void __launch_bounds__(kBoxThreads) pack_kernel(const __grid_constant__ Table a,
                                                            const double* __restrict__ src, double* __restrict__ dst) {
+  begin_dependent();
   constexpr int kPer = kPackChunk / kBoxThreads / (int)(sizeof(T) / sizeof(double));
   const uint32_t tile = a.per.div(blockIdx.x), e0 = (blockIdx.x - tile * a.per.d) * a.chunk;
   const uint32_t at = a.first + tile, r = at / a.ncols, c = at - r * a.ncols;
@@ -567,11 +569,10 @@ __global__ void __launch_bounds__(kBoxThreads) pack_kernel(const __grid_constant
 template <class Table>
 int launch_pack(const Table& a, unsigned grid, bool pairs, bool to_big, const double* src, double* dst,
                 cudaStream_t st) {
-  if (pairs && to_big) pack_kernel<double2, true><<<grid, kBoxThreads, 0, st>>>(a, src, dst);
-  else if (pairs) pack_kernel<double2, false><<<grid, kBoxThreads, 0, st>>>(a, src, dst);
-  else if (to_big) pack_kernel<double, true><<<grid, kBoxThreads, 0, st>>>(a, src, dst);
-  else pack_kernel<double, false><<<grid, kBoxThreads, 0, st>>>(a, src, dst);
-  GBX_CUDA(cudaGetLastError());
+  if (pairs && to_big) GBX_TRY(launch(pack_kernel<double2, true, Table>, grid, kBoxThreads, st, a, src, dst));
+  else if (pairs) GBX_TRY(launch(pack_kernel<double2, false, Table>, grid, kBoxThreads, st, a, src, dst));
+  else if (to_big) GBX_TRY(launch(pack_kernel<double, true, Table>, grid, kBoxThreads, st, a, src, dst));
+  else GBX_TRY(launch(pack_kernel<double, false, Table>, grid, kBoxThreads, st, a, src, dst));
   return GBX_OK;
 }
 

@@ -13,6 +13,7 @@
 
 #include "bodies.cuh"
 #include "common.h"
+#include "launch.h"
 #include "program.h"
 
 namespace gbx {
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kMoveThreads) tile_move_kernel(const MoveDesc*
                                                                  const uint32_t* __restrict__ first, int ndesc,
                                                                  uint32_t nchunks, const double* __restrict__ src,
                                                                  double* __restrict__ dst, double alpha) {
+  begin_dependent();
   dev::move_body<false>(descs, first, ndesc, nchunks, src, dst, alpha, blockIdx.x, gridDim.x);
 }
 
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(kMoveThreads) tile_move4_kernel(const MoveDesc
                                                                   uint32_t nchunks, const double* __restrict__ src,
                                                                   double* __restrict__ dst, double alpha,
                                                                   int allow_pairs) {
+  begin_dependent();
   dev::move4_body<false, kPer, kChunk>(descs, chunk_desc, nchunks, src, dst, alpha, allow_pairs, blockIdx.x,
                                        gridDim.x);
 }
@@ -210,12 +213,11 @@ int run_moves_scaled(const MoveSet& ms, const double* src, double* dst, double a
                       {{src, false}, {dst, true}});
     }
     if (ms.chunk == (uint32_t)kMove4Chunk)
-      tile_move4_kernel<8, kMove4Chunk><<<grid, kMoveThreads, 0, st>>>(ms.d_desc4, ms.d_chunk_desc, ms.nchunks, src,
-                                                                       dst, alpha, pairs);
+      GBX_TRY(launch(tile_move4_kernel<8, kMove4Chunk>, (unsigned)grid, kMoveThreads, st, ms.d_desc4, ms.d_chunk_desc,
+                     ms.nchunks, src, dst, alpha, pairs));
     else
-      tile_move4_kernel<2, dev::kMove4Small><<<grid, kMoveThreads, 0, st>>>(ms.d_desc4, ms.d_chunk_desc, ms.nchunks,
-                                                                            src, dst, alpha, pairs);
-    GBX_CUDA(cudaGetLastError());
+      GBX_TRY(launch(tile_move4_kernel<2, dev::kMove4Small>, (unsigned)grid, kMoveThreads, st, ms.d_desc4,
+                     ms.d_chunk_desc, ms.nchunks, src, dst, alpha, pairs));
     return GBX_OK;
   }
   int grid = (int)std::min<uint32_t>(ms.nchunks, 152u * 16u);
@@ -224,8 +226,8 @@ int run_moves_scaled(const MoveSet& ms, const double* src, double* dst, double a
     a.move = {ms.d_desc, ms.d_first, ms.ndesc, ms.nchunks, src, dst, alpha};
     return prog_mem(rec, PK_MOVE, (uint32_t)grid, a, {{src, false}, {dst, true}});
   }
-  tile_move_kernel<<<grid, kMoveThreads, 0, st>>>(ms.d_desc, ms.d_first, ms.ndesc, ms.nchunks, src, dst, alpha);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(tile_move_kernel, (unsigned)grid, kMoveThreads, st, ms.d_desc, ms.d_first, ms.ndesc, ms.nchunks, src,
+                 dst, alpha));
   return GBX_OK;
 }
 
@@ -237,6 +239,7 @@ int run_moves(const MoveSet& ms, const double* src, double* dst, cudaStream_t st
 __global__ void __launch_bounds__(dev::kFsThreads, 3)
     fused_sum_kernel(const FsItem* __restrict__ items, int nitems, const FsTerm* __restrict__ terms, FsSrc src,
                      const double* __restrict__ scale, double* __restrict__ out) {
+  begin_dependent();
   __shared__ dev::FsSmem sm;
   dev::fused_sum_body<false>(items, nitems, terms, src, scale, out, blockIdx.x, gridDim.x, sm);
 }
@@ -257,8 +260,7 @@ int run_fused_sum(const FsItem* items, int nitems, const FsTerm* terms, const Fs
     for (int k = 0; k < kFsMaxSlots; ++k) t.push_back({src.p[k], false});
     return prog_mem(rec, PK_FUSED, (uint32_t)grid, a, t);
   }
-  fused_sum_kernel<<<grid, dev::kFsThreads, 0, st>>>(items, nitems, terms, src, scale, out);
-  GBX_CUDA(cudaGetLastError());
+  GBX_TRY(launch(fused_sum_kernel, (unsigned)grid, dev::kFsThreads, st, items, nitems, terms, src, scale, out));
   return GBX_OK;
 }
 
