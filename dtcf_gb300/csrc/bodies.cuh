@@ -515,6 +515,8 @@ __device__ __forceinline__ void direct_body(const DirItem* __restrict__ items, i
 
 // ---- split-precision operand preparation -------------------------------------
 
+// A launch takes the work items first .. end - 1 of its row sets: one
+// operand's, or both's (A's sets before B's).
 // Splitting runs in two passes over (row, K chunk) work items so that rows
 // with very long K spread over the whole GPU.  Pass 1 takes the largest biased
 // exponent of each row chunk and folds it into the row with atomicMax (exact,
@@ -616,9 +618,9 @@ __device__ __forceinline__ void write_digits(const long long (&bits)[W], uint32_
 }
 
 template <bool kCoh>
-__device__ __forceinline__ void row_exponent_body(const SplitRowSet* __restrict__ sets, int nsets,
-                                                  int64_t total_chunks, uint32_t bid, uint32_t nblk, uint32_t* red) {
-  for (int64_t chunk = bid; chunk < total_chunks; chunk += nblk) {
+__device__ __forceinline__ void row_exponent_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t first,
+                                                  int64_t end, uint32_t bid, uint32_t nblk, uint32_t* red) {
+  for (int64_t chunk = first + bid; chunk < end; chunk += nblk) {
     int set;
     int64_t row, k0;
     locate_chunk(sets, nsets, chunk, set, row, k0);
@@ -648,10 +650,10 @@ __device__ __forceinline__ void row_exponent_body(const SplitRowSet* __restrict_
 
 // exps hold the largest biased exponent of each row (0 for an all-zero row).
 template <bool kCoh>
-__device__ __forceinline__ void digits_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_chunks,
+__device__ __forceinline__ void digits_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t first, int64_t end,
                                             int S, uint32_t bid, uint32_t nblk) {
   const int F = 7 + 8 * (S - 1);
-  for (int64_t chunk = bid; chunk < total_chunks; chunk += nblk) {
+  for (int64_t chunk = first + bid; chunk < end; chunk += nblk) {
     int set;
     int64_t row, k0;
     locate_chunk(sets, nsets, chunk, set, row, k0);
@@ -724,10 +726,10 @@ __device__ __forceinline__ void split_row_in_registers(const SplitRowSet& rs, in
 // which takes registers from the others (20000 rows of 4000 at 4 slices: 232
 // us with it, 278 without; of 2000: 137 and 121; of 8000 at 6: 709 and 632).
 template <bool kCoh, bool kFour>
-__device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows,
-                                                int S, uint32_t bid, uint32_t nblk, uint32_t* red) {
+__device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t first,
+                                                int64_t end, int S, uint32_t bid, uint32_t nblk, uint32_t* red) {
   const int F = 7 + 8 * (S - 1);
-  for (int64_t rg = bid; rg < total_rows; rg += nblk) {
+  for (int64_t rg = first + bid; rg < end; rg += nblk) {
     int lo = 0, hi = nsets - 1;
     while (lo < hi) {
       int mid = (lo + hi + 1) >> 1;
@@ -774,16 +776,16 @@ __device__ __forceinline__ void split_rows_body(const SplitRowSet* __restrict__ 
 // from registers where the row takes one step (every row of a launch with lg
 // < 5 does).  The row sets here carry first_row in rows.
 template <bool kCoh>
-__device__ __forceinline__ void short_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows,
-                                                int S, int lg, uint32_t bid, uint32_t nblk) {
+__device__ __forceinline__ void short_rows_body(const SplitRowSet* __restrict__ sets, int nsets, int64_t first,
+                                                int64_t end, int S, int lg, uint32_t bid, uint32_t nblk) {
   const int F = 7 + 8 * (S - 1);
   const int lanes = 1 << lg, lane = threadIdx.x & (lanes - 1), step = 2 * lanes;
   const int64_t per = (int64_t)(256 >> lg);  // rows of a CTA
   int lo = 0;
-  for (int64_t r0 = (int64_t)bid * per; r0 < total_rows; r0 += (int64_t)nblk * per) {
+  for (int64_t r0 = first + (int64_t)bid * per; r0 < end; r0 += (int64_t)nblk * per) {
     // rows past the end repeat the last one without storing (the shuffles need every lane)
-    const int64_t want = r0 + (threadIdx.x >> lg), rg = min(want, total_rows - 1);
-    const bool real = want < total_rows;
+    const int64_t want = r0 + (threadIdx.x >> lg), rg = min(want, end - 1);
+    const bool real = want < end;
     int hi = nsets - 1;  // rows only grow
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;

@@ -115,6 +115,10 @@ struct MoveSet {
 // scale * alpha.
 int run_moves(const MoveSet& ms, const double* src, double* dst, cudaStream_t st);
 int run_moves_scaled(const MoveSet& ms, const double* src, double* dst, double alpha, cudaStream_t st);
+// Two sets with nothing in common but their readers (a contraction's operand
+// packs), in one launch where both allow it.
+int run_moves_two(const MoveSet& ma, const double* srcA, double* dstA, const MoveSet& mb, const double* srcB,
+                  double* dstB, cudaStream_t st);
 
 // One-call moves (permute.cu): nothing is allocated or uploaded.
 // One move; an accumulating one uses scale * alpha.

@@ -295,8 +295,12 @@ int run_mul_op(const Op& op, const double* A, const double* B, double* C, double
   double* wa = ws;
   double* wb = ws + op.ws_a;
   double* wc = ws + op.ws_a + op.ws_b;
-  if (op.pack_a) GBX_TRY(ma ? run_moves(*ma, A, wa, st) : run_moves_once(op.mv_a, A, wa, st));
-  if (op.pack_b) GBX_TRY(mb ? run_moves(*mb, B, wb, st) : run_moves_once(op.mv_b, B, wb, st));
+  if (op.pack_a && op.pack_b && ma && mb) {
+    GBX_TRY(run_moves_two(*ma, A, wa, *mb, B, wb, st));
+  } else {
+    if (op.pack_a) GBX_TRY(ma ? run_moves(*ma, A, wa, st) : run_moves_once(op.mv_a, A, wa, st));
+    if (op.pack_b) GBX_TRY(mb ? run_moves(*mb, B, wb, st) : run_moves_once(op.mv_b, B, wb, st));
+  }
   if (sp) GBX_TRY(run_split_plan(sp, true, true, st));
   else if (g) GBX_TRY(g->run(st));
   else GBX_TRY(run_f64_one(gemm_problem(op, A, B, C, ws), st));

@@ -537,7 +537,7 @@ uint64_t red_chunks_of(const GemmProblem& q) {
 template <class K, class... A>
 int launch_tiles(K kernel, const TilePlan& t, int64_t items, cudaStream_t st, const A&... args) {
   if (items * t.cluster >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "FP64 GEMM has too many work items");
-  return launch_dependent(kernel, (unsigned)(items * t.cluster), kTileThreads, st, (unsigned)t.cluster, args...);
+  return launch_dependent(kernel, (unsigned)(items * t.cluster), kTileThreads, st, (unsigned)t.cluster, 0, args...);
 }
 
 }  // namespace

@@ -253,6 +253,7 @@ __global__ void __launch_bounds__(SplitCfg<BN>::kThreads, SplitCfg<BN>::kCtasPer
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem<BN>& sm = *reinterpret_cast<Smem<BN>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  begin_dependent();
   constexpr uint32_t kTxBytes = (BM + BN) * BK * 2;
 
   if (threadIdx.x == 0) {
@@ -593,6 +594,7 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Sm& sm = *reinterpret_cast<Sm*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  begin_dependent();
   const int S = P.S, L = P.L;
   // a stage holds one tile's S (A slice, B slice) pairs, the B slices back
   // to back, behind one full and one empty barrier
@@ -819,6 +821,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   KsSmem<S>& sm = *reinterpret_cast<KsSmem<S>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  begin_dependent();
   constexpr int L = Cfg::L, kStages = Cfg::kStages;
   constexpr uint32_t kCols = 512;
   // accumulator columns: the low levels, then the two buffers of the high ones
@@ -1093,32 +1096,40 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const DevProblem* __r
   dev::split_reduce_body<false>(probs, red_prob, red_first, nred, total, blockIdx.x, gridDim.x);
 }
 
+// Rows up to this length go a warp to a row in plans of few rows (both
+// operands' rows fit one wave of the CTA-per-row kernel), up to kShortRow in
+// others: a warp walks a long row 64 elements at a time (a plan of 975 rows
+// of 900 at 4 slices: 52.1 us with a warp to a row, 45.8 with a CTA; 800 rows
+// of 400: 35.5 and 33.5).
+constexpr int64_t kFewRows = 152 * 8;
+constexpr int64_t kFewShortRow = 128;
+
 // Operand splits (dev::row_exponent_body, dev::digits_body, dev::short_rows_body).
 __global__ void __launch_bounds__(256) row_exponent_kernel(const SplitRowSet* __restrict__ sets, int nsets,
-                                                           int64_t total_chunks) {
+                                                           int64_t first, int64_t end) {
   begin_dependent();
   __shared__ uint32_t red[8];
-  dev::row_exponent_body<false>(sets, nsets, total_chunks, blockIdx.x, gridDim.x, red);
+  dev::row_exponent_body<false>(sets, nsets, first, end, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void __launch_bounds__(256) digits_kernel(const SplitRowSet* __restrict__ sets, int nsets,
-                                                     int64_t total_chunks, int S) {
+                                                     int64_t first, int64_t end, int S) {
   begin_dependent();
-  dev::digits_body<false>(sets, nsets, total_chunks, S, blockIdx.x, gridDim.x);
+  dev::digits_body<false>(sets, nsets, first, end, S, blockIdx.x, gridDim.x);
 }
 
 template <bool kFour>
 __global__ void __launch_bounds__(256, kFour ? 3 : 4)
-    split_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets, int64_t total_rows, int S) {
+    split_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets, int64_t first, int64_t end, int S) {
   begin_dependent();
   __shared__ uint32_t red[8];
-  dev::split_rows_body<false, kFour>(sets, nsets, total_rows, S, blockIdx.x, gridDim.x, red);
+  dev::split_rows_body<false, kFour>(sets, nsets, first, end, S, blockIdx.x, gridDim.x, red);
 }
 
 __global__ void __launch_bounds__(256) split_short_rows_kernel(const SplitRowSet* __restrict__ sets, int nsets,
-                                                               int64_t total_rows, int S, int lg) {
+                                                               int64_t first, int64_t end, int S, int lg) {
   begin_dependent();
-  dev::short_rows_body<false>(sets, nsets, total_rows, S, lg, blockIdx.x, gridDim.x);
+  dev::short_rows_body<false>(sets, nsets, first, end, S, lg, blockIdx.x, gridDim.x);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -1183,19 +1194,21 @@ struct SplitPlan {
   std::vector<int> kb;    // per problem: k-block
   unsigned char* d_persist = nullptr;    // slices and exponents of constant plan operands
   unsigned char* d_own_arena = nullptr;  // the per-run region when no arena was given
-  SplitRowSet* d_sets_a = nullptr;  // long rows from the plan's packed A
-  SplitRowSet* d_sets_b = nullptr;  // long rows from the plan's packed B
-  SplitRowSet* d_short_a = nullptr;  // short rows (first_row counts rows)
-  SplitRowSet* d_short_b = nullptr;
-  SplitRowSet* d_mid_a = nullptr;  // medium rows, one CTA per row (first_row counts rows)
-  SplitRowSet* d_mid_b = nullptr;
-  int nlong_a = 0, nlong_b = 0, nshort_a = 0, nshort_b = 0, nmid_a = 0, nmid_b = 0;
-  int64_t short_rows_a = 0, short_rows_b = 0, mid_rows_a = 0, mid_rows_b = 0;
-  bool mid_four_a = false, mid_four_b = false;  // a medium row of 2049 .. 4096 elements
-  int short_lg_a = 3, short_lg_b = 3;  // log2 of a short row's lanes: the longest row's elements in one step, or 5
+  // row sets of one kernel: those of the plan's packed A, then those of its
+  // packed B (first_row counts on), so one launch covers either or both
+  struct Rows {
+    SplitRowSet* d = nullptr;
+    int n[2] = {0, 0};
+    int64_t items[2] = {0, 0};
+  };
+  Rows lng;   // (row, K chunk) work items
+  Rows mid;   // one CTA per row
+  Rows shrt;  // a warp or less per row
+  bool mid_four = false;  // a medium row of 2049 .. 4096 elements
+  int short_lg = 3;       // log2 of a short row's lanes: the longest row's elements in one step, or 5
   int nsets = 0;
-  int64_t rows_a = 0, rows_b = 0;  // (row, K chunk) work items per side
-  std::vector<std::pair<void*, size_t>> exp_ranges_a, exp_ranges_b;  // exponent words reset before a split
+  // exponent words of the long rows, reset before a split of A (1), B (2) or both (3)
+  std::vector<std::pair<void*, size_t>> exp_ranges[4];
   std::vector<SplitLaunch> launches;
   DevProblem* d_all = nullptr;  // every problem, for the split-K reduction
   int* d_err = nullptr;
@@ -1209,12 +1222,9 @@ struct SplitPlan {
     dev_free(d_red_first);
     dev_free(d_persist);
     dev_free(d_own_arena);
-    dev_free(d_sets_a);
-    dev_free(d_sets_b);
-    dev_free(d_short_a);
-    dev_free(d_short_b);
-    dev_free(d_mid_a);
-    dev_free(d_mid_b);
+    dev_free(lng.d);
+    dev_free(mid.d);
+    dev_free(shrt.d);
     dev_free(d_all);
     for (auto& l : launches) {
       dev_free(l.d_probs);
@@ -1384,11 +1394,18 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
   auto exp_ptr = [&](int r, int64_t off) { return (int*)(base[r] + lay.exps_at(r)) + off; };
   double* part_base = b1 ? (double*)(base[1] + lay.part_at()) : nullptr;
   sp->bytes = (double)b0 + (double)b1;
-  std::vector<SplitRowSet> sa, sb, ssa, ssb, msa, msb;
-  int64_t sra = 0, srb = 0, mra = 0, mrb = 0;
+  std::vector<SplitRowSet> sets[3][2];  // long, medium, short rows of plan A and B
+  SplitPlan::Rows* const rows_of[3] = {&sp->lng, &sp->mid, &sp->shrt};
+  int64_t all_rows = 0;
+  for (const SplitProblem& p : probs) all_rows += p.M + p.N;
+  const int64_t short_row = all_rows <= kFewRows ? kFewShortRow : kShortRow;
+  struct ExpRange {
+    int region, side;
+    int64_t at, n;
+  };
+  std::vector<ExpRange> ranges;
   std::vector<DevProblem> dp;
   std::vector<CUtensorMap> maps;
-  int64_t ra = 0, rb = 0;
   std::vector<int> red;
   std::vector<int64_t> red_first;
   int64_t red_total = 0;
@@ -1405,38 +1422,18 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
     SplitRowSet& to_a = p.a_is_plan_b ? b : a;  // rows that come from plan A
     SplitRowSet& to_b = p.a_is_plan_b ? a : b;
     if (p.dbl_from >= 0) (p.dbl_plan_b ? to_b : to_a).dbl = p.dbl_from;
-    if (to_a.K <= kShortRow) {
-      to_a.first_row = sra;
-      sra += to_a.rows;
-      while (sp->short_lg_a < 5 && to_a.K > (2ll << sp->short_lg_a)) ++sp->short_lg_a;
-      ssa.push_back(to_a);
-    } else if (to_a.K <= kMidRow) {
-      to_a.first_row = mra;
-      mra += to_a.rows;
-      sp->mid_four_a = sp->mid_four_a || (to_a.K > 2048 && to_a.K <= 4096);
-      msa.push_back(to_a);
-    } else {
-      to_a.first_row = ra;
-      ra += to_a.rows * ((to_a.K + kSplitChunk - 1) / kSplitChunk);
-      sa.push_back(to_a);
-      sp->exp_ranges_a.push_back({(void*)to_a.exps, sizeof(int) * (size_t)to_a.rows});
+    for (int side = 0; side < 2; ++side) {
+      SplitRowSet& rs = side == 0 ? to_a : to_b;
+      const int cls = p.K <= short_row ? 2 : p.K <= kMidRow ? 1 : 0;
+      int64_t& items = rows_of[cls]->items[side];
+      rs.first_row = items;
+      items += cls == 0 ? rs.rows * ((p.K + kSplitChunk - 1) / kSplitChunk) : rs.rows;
+      sets[cls][side].push_back(rs);
+      const bool gemm_a = (side == 0) != p.a_is_plan_b;
+      if (cls == 0) ranges.push_back({gemm_a ? o.ra : o.rb, side, gemm_a ? o.ea : o.eb, rs.rows});
     }
-    if (to_b.K <= kShortRow) {
-      to_b.first_row = srb;
-      srb += to_b.rows;
-      while (sp->short_lg_b < 5 && to_b.K > (2ll << sp->short_lg_b)) ++sp->short_lg_b;
-      ssb.push_back(to_b);
-    } else if (to_b.K <= kMidRow) {
-      to_b.first_row = mrb;
-      mrb += to_b.rows;
-      sp->mid_four_b = sp->mid_four_b || (to_b.K > 2048 && to_b.K <= 4096);
-      msb.push_back(to_b);
-    } else {
-      to_b.first_row = rb;
-      rb += to_b.rows * ((to_b.K + kSplitChunk - 1) / kSplitChunk);
-      sb.push_back(to_b);
-      sp->exp_ranges_b.push_back({(void*)to_b.exps, sizeof(int) * (size_t)to_b.rows});
-    }
+    while (p.K <= short_row && sp->short_lg < 5 && p.K > (2ll << sp->short_lg)) ++sp->short_lg;
+    sp->mid_four = sp->mid_four || (p.K > 2048 && p.K <= 4096);
     DevProblem d;
     d.M = (int)p.M;
     d.N = (int)p.N;
@@ -1476,30 +1473,45 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
     sp->red_total = red_total;
   }
   sp->nsets = (int)probs.size();
-  sp->rows_a = ra;
-  sp->rows_b = rb;
-  sp->short_rows_a = sra;
-  sp->short_rows_b = srb;
-  sp->nlong_a = (int)sa.size();
-  sp->nlong_b = (int)sb.size();
-  sp->nshort_a = (int)ssa.size();
-  sp->nshort_b = (int)ssb.size();
-  sp->mid_rows_a = mra;
-  sp->mid_rows_b = mrb;
-  sp->nmid_a = (int)msa.size();
-  sp->nmid_b = (int)msb.size();
   auto up = [&](const void* h, size_t bytes, void** d) -> int {
     if (bytes == 0) return GBX_OK;
     GBX_TRY(dev_alloc(d, bytes));
     GBX_CUDA(cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice));
     return GBX_OK;
   };
-  GBX_TRY(up(sa.data(), sizeof(SplitRowSet) * sa.size(), (void**)&sp->d_sets_a));
-  GBX_TRY(up(sb.data(), sizeof(SplitRowSet) * sb.size(), (void**)&sp->d_sets_b));
-  GBX_TRY(up(ssa.data(), sizeof(SplitRowSet) * ssa.size(), (void**)&sp->d_short_a));
-  GBX_TRY(up(ssb.data(), sizeof(SplitRowSet) * ssb.size(), (void**)&sp->d_short_b));
-  GBX_TRY(up(msa.data(), sizeof(SplitRowSet) * msa.size(), (void**)&sp->d_mid_a));
-  GBX_TRY(up(msb.data(), sizeof(SplitRowSet) * msb.size(), (void**)&sp->d_mid_b));
+  for (int cls = 0; cls < 3; ++cls) {
+    SplitPlan::Rows& R = *rows_of[cls];
+    std::vector<SplitRowSet> v = sets[cls][0];
+    for (SplitRowSet rs : sets[cls][1]) {
+      rs.first_row += R.items[0];
+      v.push_back(rs);
+    }
+    for (int side = 0; side < 2; ++side) R.n[side] = (int)sets[cls][side].size();
+    GBX_TRY(up(v.data(), sizeof(SplitRowSet) * v.size(), (void**)&R.d));
+  }
+  // the exponent words of a region lie one after another: a split that
+  // writes all of them (every row's exponent, once the reset is done) resets
+  // them as one range, another one each problem's
+  int in_region[2] = {0, 0};
+  for (const SplitLayout::Prob& o : lay.p) {
+    const SplitProblem& p = probs[&o - lay.p.data()];
+    in_region[o.ra] |= p.a_is_plan_b ? 2 : 1;
+    in_region[o.rb] |= p.a_is_plan_b ? 1 : 2;
+  }
+  for (int sides = 1; sides < 4; ++sides)
+    for (int r = 0; r < 2; ++r) {
+      int64_t lo = -1, hi = 0;
+      for (const ExpRange& x : ranges) {
+        if (x.region != r || !(sides & (1 << x.side))) continue;
+        if ((in_region[r] & ~sides) != 0) {
+          sp->exp_ranges[sides].push_back({(void*)exp_ptr(r, x.at), sizeof(int) * (size_t)x.n});
+          continue;
+        }
+        lo = lo < 0 ? x.at : std::min(lo, x.at);
+        hi = std::max(hi, x.at + x.n);
+      }
+      if (lo >= 0) sp->exp_ranges[sides].push_back({(void*)exp_ptr(r, lo), sizeof(int) * (size_t)(hi - lo)});
+    }
   GBX_TRY(up(dp.data(), sizeof(DevProblem) * dp.size(), (void**)&sp->d_all));
   // one launch per output tile width, plus one for the thin-K problems of
   // each k-block (bn 0: 64, bn 1: 32)
@@ -1545,55 +1557,50 @@ int create_split_plan(const std::vector<SplitProblem>& probs, int slices, SplitP
 
 int split_operands(SplitPlan* sp, bool plan_a, bool plan_b, cudaStream_t st) {
   if (!sp || sp->nsets == 0) return GBX_OK;
+  const int sides = (plan_a ? 1 : 0) | (plan_b ? 2 : 0);
+  if (sides == 0) return GBX_OK;
   ProgRecorder* rec = prog_recording();
-  for (int side = 0; side < 2; ++side) {
-    if ((side == 0 && !plan_a) || (side == 1 && !plan_b)) continue;
-    const int64_t chunks = side == 0 ? sp->rows_a : sp->rows_b;
-    if (chunks > 0) {
-      const SplitRowSet* sets = side == 0 ? sp->d_sets_a : sp->d_sets_b;
-      const int nsets = side == 0 ? sp->nlong_a : sp->nlong_b;
-      for (auto& z : (side == 0 ? sp->exp_ranges_a : sp->exp_ranges_b)) GBX_TRY(zero_async(z.first, z.second, st));
-      const int grid = (int)std::min<int64_t>(chunks, 152 * 16);
-      if (rec) {
-        ProgArgs a;
-        a.sets = {sets, chunks, nsets, sp->S, 0};
-        GBX_TRY(prog_mem(rec, PK_ROWEXP, (uint32_t)grid, a, {}));
-        GBX_TRY(prog_mem(rec, PK_DIGITS, (uint32_t)grid, a, {}));
-      } else {
-        GBX_TRY(launch(row_exponent_kernel, (unsigned)grid, 256, st, sets, nsets, chunks));
-        GBX_TRY(launch(digits_kernel, (unsigned)grid, 256, st, sets, nsets, chunks, sp->S));
-      }
+  const int S = sp->S;
+  // the launch's part of a class: its first set, set count and work items
+  const auto part = [&](const SplitPlan::Rows& R, int lg) {
+    PaSplitSets a;
+    a.sets = R.d + (plan_a ? 0 : R.n[0]);
+    a.first = plan_a ? 0 : R.items[0];
+    a.end = R.items[0] + (plan_b ? R.items[1] : 0);
+    a.nsets = (plan_a ? R.n[0] : 0) + (plan_b ? R.n[1] : 0);
+    a.S = S;
+    a.lg = lg;
+    return a;
+  };
+  const auto record = [&](int kind, int64_t grid, const PaSplitSets& a) {
+    ProgArgs pa;
+    pa.sets = a;
+    return prog_mem(rec, kind, (uint32_t)grid, pa, {});
+  };
+  const PaSplitSets l = part(sp->lng, 0), m = part(sp->mid, 0), s = part(sp->shrt, sp->short_lg);
+  if (l.end > l.first) {
+    for (auto& z : sp->exp_ranges[sides]) GBX_TRY(zero_async(z.first, z.second, st));
+    const int64_t grid = std::min<int64_t>(l.end - l.first, 152 * 16);
+    if (rec) {
+      GBX_TRY(record(PK_ROWEXP, grid, l));
+      GBX_TRY(record(PK_DIGITS, grid, l));
+    } else {
+      GBX_TRY(launch(row_exponent_kernel, (unsigned)grid, 256, st, l.sets, l.nsets, l.first, l.end));
+      GBX_TRY(launch(digits_kernel, (unsigned)grid, 256, st, l.sets, l.nsets, l.first, l.end, S));
     }
-    const int64_t mrows = side == 0 ? sp->mid_rows_a : sp->mid_rows_b;
-    if (mrows > 0) {
-      const SplitRowSet* sets = side == 0 ? sp->d_mid_a : sp->d_mid_b;
-      const int nsets = side == 0 ? sp->nmid_a : sp->nmid_b;
-      const int grid = (int)std::min<int64_t>(mrows, 152 * 8);
-      if (rec) {
-        ProgArgs a;
-        a.sets = {sets, mrows, nsets, sp->S, 0};
-        GBX_TRY(prog_mem(rec, PK_SPLITROWS, (uint32_t)grid, a, {}));
-      } else {
-        if (side == 0 ? sp->mid_four_a : sp->mid_four_b)
-          GBX_TRY(launch(split_rows_kernel<true>, (unsigned)grid, 256, st, sets, nsets, mrows, sp->S));
-        else
-          GBX_TRY(launch(split_rows_kernel<false>, (unsigned)grid, 256, st, sets, nsets, mrows, sp->S));
-      }
-    }
-    const int64_t srows = side == 0 ? sp->short_rows_a : sp->short_rows_b;
-    if (srows > 0) {
-      const SplitRowSet* sets = side == 0 ? sp->d_short_a : sp->d_short_b;
-      const int nsets = side == 0 ? sp->nshort_a : sp->nshort_b;
-      const int lg = side == 0 ? sp->short_lg_a : sp->short_lg_b;
-      const int grid = (int)std::min<int64_t>((srows + (256 >> lg) - 1) / (256 >> lg), 152 * 32);
-      if (rec) {
-        ProgArgs a;
-        a.sets = {sets, srows, nsets, sp->S, lg};
-        GBX_TRY(prog_mem(rec, PK_SHORTROWS, (uint32_t)grid, a, {}));
-        continue;
-      }
-      GBX_TRY(launch(split_short_rows_kernel, (unsigned)grid, 256, st, sets, nsets, srows, sp->S, lg));
-    }
+  }
+  if (m.end > m.first) {
+    const int64_t grid = std::min<int64_t>(m.end - m.first, 152 * 8);
+    if (rec) GBX_TRY(record(PK_SPLITROWS, grid, m));
+    else
+      GBX_TRY(launch(sp->mid_four ? split_rows_kernel<true> : split_rows_kernel<false>, (unsigned)grid, 256, st, m.sets,
+                     m.nsets, m.first, m.end, S));
+  }
+  if (s.end > s.first) {
+    const int64_t per = 256 >> s.lg, grid = std::min<int64_t>((s.end - s.first + per - 1) / per, 152 * 32);
+    if (rec) GBX_TRY(record(PK_SHORTROWS, grid, s));
+    else
+      GBX_TRY(launch(split_short_rows_kernel, (unsigned)grid, 256, st, s.sets, s.nsets, s.first, s.end, S, s.lg));
   }
   return GBX_OK;
 }
@@ -1603,16 +1610,13 @@ namespace {
 template <int BN>
 int launch_width(const GemmParams& P, int nsm, cudaStream_t st) {
   const int grid = std::min(P.total_tiles, nsm * SplitCfg<BN>::kCtasPerSm);
-  split_gemm_kernel<BN><<<grid, SplitCfg<BN>::kThreads, sizeof(Smem<BN>) + 1024, st>>>(P);
-  GBX_CUDA(cudaGetLastError());
-  return GBX_OK;
+  return launch_dependent(split_gemm_kernel<BN>, (unsigned)grid, SplitCfg<BN>::kThreads, st, 1u, sizeof(Smem<BN>) + 1024, P);
 }
 
 template <int S>
 int launch_ks(const GemmParams& P, int nsm, cudaStream_t st) {
-  split_ks_kernel<S><<<std::min(P.total_tiles, nsm), kKsThreads, sizeof(KsSmem<S>) + 1024, st>>>(P);
-  GBX_CUDA(cudaGetLastError());
-  return GBX_OK;
+  return launch_dependent(split_ks_kernel<S>, (unsigned)std::min(P.total_tiles, nsm), kKsThreads, st, 1u,
+                          sizeof(KsSmem<S>) + 1024, P);
 }
 
 // The GEMM kernel of one launch class -- bn 0 / 1: thin-K with a 64 / 32
@@ -1624,17 +1628,16 @@ int launch_split_gemm(int bn, const GemmParams& P, cudaStream_t st) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (bn <= 1) {
-    if (bn == 0)
-      split_thin_kernel<64><<<std::min(P.total_tiles, nsm), kThinThreads, sizeof(ThinSmem<64>) + 1024, st>>>(P);
-    else
-      split_thin_kernel<32><<<std::min(P.total_tiles, nsm), kThinThreads, sizeof(ThinSmem<32>) + 1024, st>>>(P);
-    const cudaError_t le = cudaGetLastError();
+    const unsigned grid = (unsigned)std::min(P.total_tiles, nsm);
+    const size_t smem = (bn == 0 ? sizeof(ThinSmem<64>) : sizeof(ThinSmem<32>)) + 1024;
+    const cudaError_t le = try_launch_dependent(bn == 0 ? split_thin_kernel<64> : split_thin_kernel<32>, grid,
+                                                kThinThreads, st, 1u, smem, P);
     if (le != cudaSuccess) {
       cudaFuncAttributes fa;
       std::memset(&fa, 0, sizeof(fa));
       cudaFuncGetAttributes(&fa, bn == 0 ? (const void*)split_thin_kernel<64> : (const void*)split_thin_kernel<32>);
       return fail(GBX_ECUDA, "thin-K launch (k-block %d): %s; dynamic smem %zu (max %d), static %zu, regs %d, max threads %d",
-                  bn == 0 ? 64 : 32, cudaGetErrorString(le), (bn == 0 ? sizeof(ThinSmem<64>) : sizeof(ThinSmem<32>)) + 1024,
+                  bn == 0 ? 64 : 32, cudaGetErrorString(le), smem,
                   fa.maxDynamicSharedSizeBytes, fa.sharedSizeBytes, fa.numRegs, fa.maxThreadsPerBlock);
     }
     return GBX_OK;

@@ -915,16 +915,17 @@ int ContractionPlan::tune_split(cudaStream_t st, int reps) {
   return rc;
 }
 
+int ContractionPlan::pack(bool a, bool b, const double* dA, const double* dB, cudaStream_t st) {
+  if (a && a_needs_zero) GBX_TRY(zero_async(d_Abig, sizeof(double) * a_elems, st));
+  if (b && b_needs_zero) GBX_TRY(zero_async(d_Bbig, sizeof(double) * b_elems, st));
+  if (a && b) return run_moves_two(packA, dA, d_Abig, packB, dB, d_Bbig, st);
+  if (a) return run_moves(packA, dA, d_Abig, st);
+  return b ? run_moves(packB, dB, d_Bbig, st) : GBX_OK;
+}
+
 int ContractionPlan::prepare_static(const double* dA, const double* dB, cudaStream_t st) {
   if (direct) return GBX_OK;  // reads its operands where they are stored
-  if (a_static) {
-    if (a_needs_zero) GBX_TRY(zero_async(d_Abig, sizeof(double) * a_elems, st));
-    GBX_TRY(run_moves(packA, dA, d_Abig, st));
-  }
-  if (b_static) {
-    if (b_needs_zero) GBX_TRY(zero_async(d_Bbig, sizeof(double) * b_elems, st));
-    GBX_TRY(run_moves(packB, dB, d_Bbig, st));
-  }
+  GBX_TRY(pack(a_static, b_static, dA, dB, st));
   if (split) GBX_TRY(split_operands(split, a_static, b_static, st));
   static_ready = a_static || b_static;
   return GBX_OK;
@@ -934,14 +935,7 @@ int ContractionPlan::stage(const double* dA, const double* dB, cudaStream_t st) 
   if (direct) return GBX_OK;
   const bool skipA = a_static && static_ready, skipB = b_static && static_ready;
   if ((!skipA && !dA) || (!skipB && !dB)) return fail(GBX_EINVAL, "contraction operand without device memory");
-  if (!skipA) {
-    if (a_needs_zero) GBX_TRY(zero_async(d_Abig, sizeof(double) * a_elems, st));
-    GBX_TRY(run_moves(packA, dA, d_Abig, st));
-  }
-  if (!skipB) {
-    if (b_needs_zero) GBX_TRY(zero_async(d_Bbig, sizeof(double) * b_elems, st));
-    GBX_TRY(run_moves(packB, dB, d_Bbig, st));
-  }
+  GBX_TRY(pack(!skipA, !skipB, dA, dB, st));
   if (split) GBX_TRY(split_operands(split, !skipA, !skipB, st));
   return GBX_OK;
 }
@@ -954,14 +948,7 @@ int ContractionPlan::execute(const double* dA, const double* dB, double* dC, dou
   if (f64.nprob == 0 && !split) return GBX_OK;
   const bool skipA = a_static && static_ready, skipB = b_static && static_ready;
   if ((!skipA && !dA) || (!skipB && !dB)) return fail(GBX_EINVAL, "contraction operand without device memory");
-  if (!skipA) {
-    if (a_needs_zero) GBX_TRY(zero_async(d_Abig, sizeof(double) * a_elems, st));
-    GBX_TRY(run_moves(packA, dA, d_Abig, st));
-  }
-  if (!skipB) {
-    if (b_needs_zero) GBX_TRY(zero_async(d_Bbig, sizeof(double) * b_elems, st));
-    GBX_TRY(run_moves(packB, dB, d_Bbig, st));
-  }
+  GBX_TRY(pack(!skipA, !skipB, dA, dB, st));
   GBX_TRY(f64.run(st));
   if (split) GBX_TRY(run_split_plan(split, !skipA, !skipB, st));
   return run_moves_scaled(unpackC, d_Cbig, dC, alpha * alpha_factor, st);

@@ -177,6 +177,8 @@ struct ContractionPlan {
   // own) and the static scratch (nullptr: after the arena), uploads the
   // launch descriptors.
   int build(unsigned char* arena = nullptr, unsigned char* static_scratch = nullptr);
+  // Packs A and / or B into their scratch.
+  int pack(bool a, bool b, const double* dA, const double* dB, cudaStream_t st);
   int prepare_static(const double* dA, const double* dB, cudaStream_t st);
   // Packs and splits the changing operands without running the GEMM (so a
   // GEMM can be timed alone on current data).

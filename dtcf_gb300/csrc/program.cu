@@ -6,6 +6,7 @@
 #include <memory>
 
 #include "bodies.cuh"
+#include "launch.h"
 #include "program.h"
 #include "split.h"
 
@@ -106,16 +107,16 @@ __device__ __forceinline__ void run_record(const ProgRec& r, uint32_t vb, ProgSm
                                                     a.direct.B, a.direct.C, a.direct.alpha, vb, g, sm.dir);
       break;
     case PK_ROWEXP:
-      dev::row_exponent_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, vb, g, sm.red8);
+      dev::row_exponent_body<true>(a.sets.sets, a.sets.nsets, a.sets.first, a.sets.end, vb, g, sm.red8);
       break;
     case PK_DIGITS:
-      dev::digits_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g);
+      dev::digits_body<true>(a.sets.sets, a.sets.nsets, a.sets.first, a.sets.end, a.sets.S, vb, g);
       break;
     case PK_SHORTROWS:
-      dev::short_rows_body<true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, a.sets.lg, vb, g);
+      dev::short_rows_body<true>(a.sets.sets, a.sets.nsets, a.sets.first, a.sets.end, a.sets.S, a.sets.lg, vb, g);
       break;
     case PK_SPLITROWS:
-      dev::split_rows_body<true, true>(a.sets.sets, a.sets.nsets, a.sets.total, a.sets.S, vb, g, sm.red8);
+      dev::split_rows_body<true, true>(a.sets.sets, a.sets.nsets, a.sets.first, a.sets.end, a.sets.S, vb, g, sm.red8);
       break;
     case PK_SPLITRED:
       dev::split_reduce_body<true>(a.splitred.probs, a.splitred.red_prob, a.splitred.red_first, a.splitred.nred,
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(kProgThreads, kProgCtasPerSm) prog_mem_kernel(
   __shared__ uint32_t seen[kSeenWords];
   __shared__ uint32_t s_t, s_next;
   __shared__ int s_r, s_ok;
+  begin_dependent();
   const int tid = threadIdx.x;
   for (int i = tid; i < kSeenWords; i += kProgThreads) seen[i] = 0u;
   if (tid == 0) s_t = atomicAdd(L.ticket, (uint32_t)kProgBatch);
@@ -617,8 +619,7 @@ int prog_run(const Program& P, cudaStream_t st) {
       L.limit = P.limit;
       L.nrec = m.nrec;
       L.total = m.total;
-      prog_mem_kernel<<<m.grid, kProgThreads, 0, st>>>(L);
-      GBX_CUDA(cudaGetLastError());
+      GBX_TRY(launch(prog_mem_kernel, (unsigned)m.grid, kProgThreads, st, L));
     } else if (op.type == 1) {
       GBX_TRY(split_merged_run(P.merged[op.idx], st));
     } else {

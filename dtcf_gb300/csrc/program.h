@@ -110,7 +110,7 @@ struct PaDirect {
 };
 struct PaSplitSets {  // row exponents, digits, short rows
   const SplitRowSet* sets;
-  int64_t total;
+  int64_t first, end;  // work items
   int nsets, S, lg;  // lg: log2 of the lanes of a short row
 };
 struct PaSplitRed {
