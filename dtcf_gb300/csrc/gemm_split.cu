@@ -468,14 +468,53 @@ __global__ void __launch_bounds__(SplitCfg<BN>::kThreads, SplitCfg<BN>::kCtasPer
   }
 }
 
+// x * 2^(ex - 1023), the exponent moved by an integer addition: a multiply is
+// one of the FP64 instructions that bound the drains (an SM issues 1.8 a
+// clock).  x is 0 or of magnitude 2^-60 .. 2^70, ex one of plain_exponent.
+__device__ __forceinline__ double scaled(double x, int ex) {
+  const int hi = __double2hiint(x);
+  return __hiloint2double((hi & 0x7FFFFFFF) ? hi + (ex - 1023) * (1 << 20) : hi, __double2loint(x));
+}
+__device__ __forceinline__ bool plain_exponent(int ex) { return ex >= 64 && ex <= 1900; }
+
+// T * 2^(ex - 1023), rounded to nearest even, without an FP64 instruction (the
+// conversion is one): T normalised, its bits below the 53rd rounded off, the
+// exponent set (plain_exponent(ex)).
+__device__ __forceinline__ double scaled_int(long long T, int ex) {
+  const unsigned long long u = (unsigned long long)(T < 0 ? -T : T);
+  const int z = __clzll((long long)u);
+  const unsigned long long n = (u << (z & 63)) & 0x7FFFFFFFFFFFFFFFull;  // without its leading 1
+  const unsigned long long m = (n + (0x3FFull + ((uint32_t)(n >> 11) & 1u))) >> 11;  // a carry moves the exponent
+  const uint32_t hi = (uint32_t)(m >> 32) + ((uint32_t)(ex + 63 - z) << 20);
+  return __hiloint2double((int)((u ? hi : 0u) | ((uint32_t)(T >> 32) & 0x80000000u)), (int)(uint32_t)m);
+}
+
+// No scale of a warp's elements near the ends of the range: each lane's row
+// exponent with each of the column exponents the lanes hold (ebl).  A zero
+// row or column (exponent word 0) has sums of 0, which scaled() leaves alone.
+__device__ __forceinline__ bool plain_exponents(int ea, int ebl, int offset) {
+  const int emin = (int)__reduce_min_sync(0xffffffffu, ebl ? (uint32_t)ebl : 4000u);
+  const int emax = (int)__reduce_max_sync(0xffffffffu, (uint32_t)ebl);
+  return __all_sync(0xffffffffu, ea == 0 || emax == 0 ||
+                                     (plain_exponent(ea + emin + offset) && plain_exponent(ea + emax + offset)));
+}
+
+// The 16 or 32 bytes at p (aligned so).
+__device__ __forceinline__ void store_vec(double* p, const double (&v)[2]) {
+  *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+}
+__device__ __forceinline__ void store_vec(double* p, const double (&v)[4]) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3]) : "memory");
+}
+
 // ---- thin-K kernel: K <= 64, N <= 32 -----------------------------------
 //
 // One k-block per problem, so every slice is loaded once per 128-row tile
 // and all S(S+1)/2 slice products go into per-level TMEM accumulators
 // (level l at columns l*32 of a buffer; two buffers alternate between tiles).
 // A level sums at most S products of 64 K-elements, below 2^24, so no drains
-// are needed mid-tile: the drain warps read the levels from S-1 down to 0 and
-// recombine them with FP64 Horner steps directly.  The k-block is TBK = 64
+// are needed mid-tile: the drain warps read the levels and recombine them,
+// in integers up to six slices, with FP64 Horner steps beyond.  The k-block is TBK = 64
 // (128-byte swizzled rows) or, for K <= 32, TBK = 32 (64-byte rows): slices
 // are padded to the k-block, so short K (a virtual block of ~30 orbitals)
 // streams half the bytes with the narrow block.
@@ -497,31 +536,52 @@ struct ThinSmem {
 // levels in exact int64 fixed point, Y = sum_l X_l 2^(8 (L - l)), from level
 // 0 up (|X_l| <= 7 * 64 * 2^14 < 2^23, so |Y| < 2^63 for L <= 5; S = 7 keeps
 // the FP64 recombination); the accumulator buffer is released before the
-// scaled results are stored.
-// ea: the row's exponent, eb8: the first 8 column exponents, both loaded
-// by the caller before it waited for the accumulator (their latency hidden
-// behind the wait); columns past 8 are read here.
-// Stores of one drained row: v[j] * 2^(its exponent), columns < ncol.
-template <int NC>
-__device__ __forceinline__ void thin_store(const double (&v)[NC], int L, int ncol, const DevProblem& pr, int row,
-                                           int ea, const int* eb8) {
-  if (row >= pr.M) return;
-  double* crow = pr.C + (int64_t)row * pr.ldc;
-  const int lshift = L <= 5 ? 8 * L : 0;  // the int64 path carries 2^(8L)
+// results are rounded, scaled and stored (in integers, as in the k-stationary
+// kernel: the nine thin launches of a CCSD iteration at o = 48, v = 240 take
+// 546 us with a conversion and a multiply to each output, 475 so).
+// ea: the row's exponent, ebl: the lane's column's, both loaded by the caller
+// before it waited for the accumulator (their latency hidden behind the wait).
+// Stores of one drained row: v[j] * 2^(its exponent), columns < ncol.  All
+// lanes of the warp call it.
+__device__ __forceinline__ double plain_value(long long x, int ex) { return scaled_int(x, ex); }
+__device__ __forceinline__ double plain_value(double x, int ex) { return scaled(x, ex); }
+
+template <int NC, typename T>
+__device__ __forceinline__ void thin_store(const T (&v)[NC], int L, int ncol, const DevProblem& pr, int row,
+                                           int ea, int ebl) {
+  const int64_t ld = pr.ldc;
+  double* crow = pr.C + (int64_t)row * ld;
+  const int e0 = ea + 1023 - 2 * 1022 - 14 - (L <= 5 ? 8 * L : 0);  // the int64 path carries 2^(8L)
+  const bool real = row < pr.M;
+  if (plain_exponents(ea, ebl, e0 - ea)) {
+    const bool pairs = (((uintptr_t)pr.C | (uintptr_t)(ld * 8)) & 15) == 0;
+#pragma unroll
+    for (int j = 0; j < NC; j += 2) {
+      if (j >= ncol) break;
+      const int ex0 = e0 + __shfl_sync(0xffffffffu, ebl, j), ex1 = e0 + __shfl_sync(0xffffffffu, ebl, j + 1);
+      const double x[2] = {plain_value(v[j], ex0), plain_value(v[j + 1], ex1)};
+      if (!real) continue;
+      if (pairs && j + 1 < ncol) {
+        store_vec(crow + j, x);
+      } else {
+        crow[j] = x[0];
+        if (j + 1 < ncol) crow[j + 1] = x[1];
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < NC; ++j) {
-    if (j < ncol) {
-      int ex = ea + (j < 8 ? eb8[j] : pr.eB[j]) - 2 * 1022 - 14 - lshift + 1023;
-      ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-      crow[j] = v[j] * __longlong_as_double((long long)ex << 52);
-    }
+    if (j >= ncol) break;
+    int ex = e0 + __shfl_sync(0xffffffffu, ebl, j);
+    ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
+    if (real) crow[j] = (double)v[j] * __longlong_as_double((long long)ex << 52);
   }
 }
 
 template <int NC>
 __device__ __forceinline__ void thin_drain(uint32_t tb, int L, int ncol, const DevProblem& pr, int row,
-                                           uint64_t* accempty, int lane, int ea, const int* eb8) {
-  double v[NC];
+                                           uint64_t* accempty, int lane, int ea, int ebl) {
   if (L <= 5) {
     long long Y[NC];
 #pragma unroll
@@ -560,9 +620,9 @@ __device__ __forceinline__ void thin_drain(uint32_t tb, int L, int ncol, const D
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(accempty);
-#pragma unroll
-    for (int j = 0; j < NC; ++j) v[j] = (double)Y[j];
+    thin_store<NC>(Y, L, ncol, pr, row, ea, ebl);
   } else {
+    double v[NC];
 #pragma unroll
     for (int j = 0; j < NC; ++j) v[j] = 0.0;
     for (int l = L; l >= 0; --l) {
@@ -582,8 +642,8 @@ __device__ __forceinline__ void thin_drain(uint32_t tb, int L, int ncol, const D
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(accempty);
+    thin_store<NC>(v, L, ncol, pr, row, ea, ebl);
   }
-  thin_store<NC>(v, L, ncol, pr, row, ea, eb8);
 }
 
 template <int TBK>
@@ -723,18 +783,16 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
       const int ncol = min(kThinBN, pr.N - ti.n0);
       const int row = ti.m0 + quarter * 32 + lane;
       const int ea = row < pr.M ? pr.eA[row] : 0;
-      int eb8[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) eb8[j] = j < ncol ? pr.eB[j] : 0;  // thin tiles start at column 0
+      const int ebl = lane < ncol ? pr.eB[lane] : 0;  // thin tiles start at column 0
       int w_ok = lane == 0 ? (int)mbar_wait(&sm.accfull[buf], aphase, P.err, 14) : 1;
       w_ok = __shfl_sync(0xffffffffu, w_ok, 0);
       if (!w_ok) break;
       __syncwarp();
       tc_fence_after();
       const uint32_t tb = tmem + lane_addr + (uint32_t)buf * buf_cols;
-      if (ncol <= 8) thin_drain<8>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, eb8);
-      else if (ncol <= 16) thin_drain<16>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, eb8);
-      else thin_drain<32>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, eb8);
+      if (ncol <= 8) thin_drain<8>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, ebl);
+      else if (ncol <= 16) thin_drain<16>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, ebl);
+      else thin_drain<32>(tb, L, ncol, pr, row, &sm.accempty[buf], lane, ea, ebl);
       aphase ^= 1;
     }
   }
@@ -776,10 +834,16 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
 // and two low ones; 6: two and four; 7: one and six.
 //
 // The drains add the levels exactly into 64-bit sums (levels apart by 2^8;
-// two sums 2^32 apart from five slices on), which become one FP64 value per
-// output at the end of a tile.  (Rounding and scaling by integer instructions
-// instead of a conversion and a multiply: 20000 x 64 x 256 at 6 slices 80
-// instead of 66 us.)
+// two sums 2^32 apart from six slices on), which become one FP64 value per
+// output at the end of a tile.  That end is what bounds short K: an SM issues
+// 1.8 FP64 instructions a clock, so each one to an output is 2.4 us of a
+// tile.  So the values are rounded and scaled by integer instructions (from
+// six slices on one FP64 multiply-add is left; near the ends of the FP64
+// range the plain conversion and multiply), full rows of four go out in one
+// store, and warps without real elements skip their part.  Conversions,
+// multiplies and 8-byte stores / so, with the operand splits: 2000 x 2000 x 66
+// 62.5 / 29.4 us at 4 slices and 99.6 / 42.4 at 6, 400 x 400 x 400 26.1 / 17.5
+// and 44.5 / 27.8, 2000 x 2000 x 3200 279 / 248 and 578 / 529.
 constexpr int kKsBN = 64;
 constexpr int ks_bk(int S) { return S <= 4 ? 64 : 32; }  // elements of a k-block
 constexpr int kKsDrainWarps = 8;     // 4 TMEM lane quarters x 2 column halves
@@ -797,7 +861,7 @@ struct KsCfg {
   static constexpr int kLoBlocks = kLo ? 1024 / (kLo ? kLo : 1) / kBK : 1, kLoBlocksDbl = kLo ? 1024 / (kLo + 1) / kBK : 1;
   static constexpr int kStageBytes = S * (BM + kKsBN) * kBK * 2;
   static constexpr int kStages = (220 * 1024 / kStageBytes) < 8 ? 220 * 1024 / kStageBytes : 8;
-  static constexpr int kCut = S <= 4 ? 0 : S - 4;  // levels below this go to the upper sum
+  static constexpr int kCut = S <= 5 ? 0 : S - 4;  // levels below this go to the upper sum
   // the drains' level loops: unrolled, their TMEM reads overlap the sums
   // before (S = 6: 978 instead of 1019 us); at S = 4 that spills
   static constexpr int kUnroll = S <= 4 ? 1 : S;
@@ -988,7 +1052,14 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
     bool ok = true;
     for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
       const TileInfo ti = decode_tile<kKsBN>(P, tile);
-      const DevProblem& pr = P.probs[ti.p];
+      const int M = P.probs[ti.p].M, N = P.probs[ti.p].N;
+      const int row = ti.m0 + quarter * 32 + lane, col0 = ti.n0 + half * 32;
+      // a warp whose 32 x 32 elements lie outside the matrix only keeps the
+      // accumulators turning
+      const bool idle = ti.m0 + quarter * 32 >= M || col0 >= N;
+      // the exponents, read ahead of the waits: the row's, and a column's to a lane
+      const int ea = row < M ? P.probs[ti.p].eA[row] : 0;
+      const int ebl = col0 + lane < N ? P.probs[ti.p].eB[col0 + lane] : 0;
       long long Y[32], U[Cfg::kCut ? 32 : 1];
 #pragma unroll
       for (int j = 0; j < 32; ++j) Y[j] = 0;
@@ -999,6 +1070,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
       // adds level l's 32 columns at col, weighted 2^(8 (L - l)) (below the
       // cut 2^(8 (kCut - 1 - l)) of the upper sum)
       auto add = [&](int l, uint32_t col) {
+        if (idle) return;
         uint32_t r[2][16];
         tmem_ld16(base + col, r[0]);
         tmem_ld16(base + col + 16, r[1]);
@@ -1009,7 +1081,7 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
           for (int j = 0; j < 32; ++j)
             U[Cfg::kCut ? j : 0] += (long long)__float2int_rn(__uint_as_float(r[j >> 4][j & 15])) * w;
         } else {
-          const int w = 1 << (8 * (L - l));
+          const long long w = 1ll << (8 * (L - l));
 #pragma unroll
           for (int j = 0; j < 32; ++j) Y[j] += (long long)__float2int_rn(__uint_as_float(r[j >> 4][j & 15])) * w;
         }
@@ -1060,22 +1132,60 @@ __global__ void __launch_bounds__(kKsThreads, 1) split_ks_kernel(const GemmParam
         }
       }
       if (!ok) break;
-      const int row = ti.m0 + quarter * 32 + lane;
-      if (row < pr.M) {
-        const int ea = pr.eA[row];
-        double* crow = pr.ksplit > 1 ? pr.partial + ((int64_t)ti.kc * pr.M + row) * pr.N : pr.C + (int64_t)row * pr.ldc;
+      if (idle) continue;
+      const DevProblem& pr = P.probs[ti.p];
+      const int64_t ld = pr.ksplit > 1 ? N : pr.ldc;
+      double* cbase = (pr.ksplit > 1 ? pr.partial + (int64_t)ti.kc * M * N : pr.C) + col0;
+      double* crow = cbase + (int64_t)row * ld;
+      const uintptr_t at = (uintptr_t)cbase | (uintptr_t)(ld * 8);
+      const int vec = (at & 31) == 0 ? 4 : (at & 15) == 0 ? 2 : 1;
+      constexpr int kE = 1023 - 2 * 1022 - 14 - 8 * L;
+      auto store = [&](auto is_plain) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int col = ti.n0 + half * 32 + j;
-          if (col < pr.N) {
-            int ex = ea + pr.eB[col] - 2 * 1022 - 14 - 8 * L + 1023;
-            ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
-            double v = (double)Y[j];
-            if (Cfg::kCut) v = __fma_rn((double)U[Cfg::kCut ? j : 0], 0x1.0p32, v);
-            crow[col] = v * __longlong_as_double((long long)ex << 52);
+        for (int j0 = 0; j0 < 32; j0 += 4) {
+          if (col0 + j0 >= N) break;
+          double v[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int j = j0 + i;
+            int ex = ea + __shfl_sync(0xffffffffu, ebl, j) + kE;
+            constexpr bool kPlain = decltype(is_plain)::value;
+            if constexpr (kPlain && !Cfg::kCut) {
+              v[i] = scaled_int(Y[j], ex);
+            } else {
+              double x;
+              if constexpr (Cfg::kCut) {
+                // U 2^32 + Y = V 2^32 + (2^52 + the low 32 bits of Y), the
+                // bracket a double's bits as it stands; V is below 2^53
+                const long long V = U[j] + (Y[j] >> 32) - (1 << 20);
+                x = __fma_rn(kPlain ? scaled_int(V, 1023) : (double)V, 0x1.0p32,
+                             __hiloint2double(0x43300000, (int)(uint32_t)Y[j]));
+              } else {
+                x = (double)Y[j];
+              }
+              if constexpr (kPlain) {
+                v[i] = scaled(x, ex);
+              } else {
+                ex = ex < 1 ? 1 : (ex > 2046 ? 2046 : ex);
+                v[i] = x * __longlong_as_double((long long)ex << 52);
+              }
+            }
+          }
+          if (row >= M) continue;
+          if (vec == 4 && col0 + j0 + 4 <= N) {
+            store_vec(crow + j0, v);
+          } else if (vec == 2 && col0 + j0 + 4 <= N) {
+            store_vec(crow + j0, {v[0], v[1]});
+            store_vec(crow + j0 + 2, {v[2], v[3]});
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (col0 + j0 + i < N) crow[j0 + i] = v[i];
           }
         }
-      }
+      };
+      if (plain_exponents(ea, ebl, kE)) store(std::true_type());
+      else store(std::false_type());
     }
   }
   tc_fence_before();
@@ -1173,6 +1283,9 @@ int choose_width() { return g_width_override ? g_width_override : kKsBN; }
 // element from four slices on, up to S products to a level, one bit more for
 // doubled digits.
 int64_t ks_max_k(int S) { return S <= 4 ? 1 << 24 : 1 << 22; }
+// At five slices they are one sum each, 2^(14 + 32) an element: longer rows
+// are cut into ranges (as rows are where output tiles are few).
+constexpr int64_t kFiveRange = 1 << 15;
 
 struct SplitLaunch {  // the problems of one output tile width
   int bn = 0;
@@ -1333,6 +1446,7 @@ int split_layout(const std::vector<SplitProblem>& probs, int S, bool static_a, b
       int want = (int)((kSplitFill + out_tiles - 1) / out_tiles);
       ks = std::max(1, std::min(want, nkb / chunk));
     }
+    if (o.ks_kernel && S == 5) ks = std::max(ks, (int)((probs[i].K + kFiveRange - 1) / kFiveRange));
     int per = (nkb + ks - 1) / ks;
     per = (per + chunk - 1) / chunk * chunk;
     ks = (nkb + per - 1) / per;
