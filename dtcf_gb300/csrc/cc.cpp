@@ -129,7 +129,10 @@ struct gbx_cc_job {
   ProgramPtr prog;
 
   bool persistent() const { return cfg.use_graph == 2; }
+  bool branched = false;  // use_graph 1: independent steps are branches of the graph
+  int record_steps(ProgRecorder** rec);
   int record_program();
+  int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps);
 
   ~gbx_cc_job() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -610,6 +613,21 @@ int gbx_cc_job::plan_all() {
 
 namespace {
 double up256d(double x) { return std::ceil(x / 256.0) * 256.0; }
+
+// Whether contractions may run side by side, each in its own region of the
+// arena (`regions` bytes together): always in a persistent program, in a
+// graph up to 2 GB of regions (under 1% of the GPU's memory).  Larger jobs
+// share one region and run in a chain: their kernels fill the GPU one after
+// another and their memory counts.  Per iteration, chain / branches: CCSD at
+// o = 8, v = 24, FP64 300 / 179 us (12 / 15 MB resident); o = 16, v = 64 in 8
+// irreps at 6 slices 486 / 277 (54 / 63 MB); o = 16, v = 64 at 5 slices 1219 /
+// 843 (457 / 721 MB); o = 32, v = 160 in 8 irreps at 4 slices 1691 / 1325 (1.4 /
+// 1.9 GB); o = 48, v = 240 in 8 irreps 5945 / 5722 (6.6 / 8.6 GB, beyond the
+// line).
+constexpr double kBranchBytes = 2e9;
+bool side_by_side(int use_graph, double regions) {
+  return use_graph == 2 || (use_graph == 1 && regions <= kBranchBytes);
+}
 }  // namespace
 
 // An integral tensor read only as constant plan operands: released once those
@@ -621,7 +639,7 @@ bool gbx_cc_job_static_only(const gbx_cc_job& j, const std::string& name) {
 // Device bytes of the built job: what stays resident, and the peak while it
 // is being built (integral tiles and constant-operand scratch included).
 int gbx_cc_job::footprint(double* resident, double* peak) const {
-  double keep = 0.0, transient = 0.0, ws = 0.0, scratch = 0.0;
+  double keep = 0.0, transient = 0.0, ws = 0.0, widest = 0.0, scratch = 0.0;
   for (auto& kv : T) {
     const double b = up256d(8.0 * (double)std::max<int64_t>(1, kv.second->L.nelem));
     if (gbx_cc_job_static_only(*this, kv.first)) transient += b; else keep += b;
@@ -630,11 +648,12 @@ int gbx_cc_job::footprint(double* resident, double* peak) const {
     size_t k = 0, w = 0, sc = 0;
     GBX_TRY(p->sizes(&k, &w, &sc));
     keep += (double)k + p->f64_workspace_estimate();
-    // a persistent program runs contractions side by side: each plan keeps
-    // its own region of the arena
-    ws = persistent() ? ws + up256d((double)w) : std::max(ws, (double)w);
+    // contractions that run side by side keep their own regions of the arena
+    ws += up256d((double)w);
+    widest = std::max(widest, (double)w);
     scratch = std::max(scratch, (double)sc);
   }
+  if (!side_by_side(cfg.use_graph, ws)) ws = widest;
   for (auto& p : fplans) keep += up256d((double)(p->items.size() * sizeof(FsItem))) + up256d((double)(p->terms.size() * sizeof(FsTerm)));
   for (auto& m : expansions) keep += up256d((double)m->device_bytes());
   keep += up256d((double)(amp_tiles.size() * sizeof(CCAmpTile))) + up256d((double)(amp_items.size() * sizeof(CCAmpItem)));
@@ -694,22 +713,25 @@ int gbx_cc_job::materialize(cudaStream_t st) {
   den2 = tileset(get("t2"));
   if (sd) den1 = tileset(get("t1"));
   if (!den2 || (sd && !den1)) return fail(GBX_ENOMEM, "tile set upload failed");
-  // one arena for every plan's per-run buffers (the steps run in order on one
-  // stream); constant operands are packed into scratch, split, and the
+  // one arena for every plan's per-run buffers: a region to each where plans
+  // run side by side, one for all where the steps run in order on one
+  // stream; constant operands are packed into scratch, split, and the
   // scratch is released
-  arena_bytes = 0;
-  size_t scratch_bytes = 0;
+  size_t scratch_bytes = 0, widest = 0;
   std::vector<size_t> arena_off(cplans.size(), 0);
+  arena_bytes = 0;
   for (size_t i = 0; i < cplans.size(); ++i) {
     size_t k = 0, w = 0, sc = 0;
     GBX_TRY(cplans[i]->sizes(&k, &w, &sc));
-    if (persistent()) {  // a region per plan (they run side by side)
-      arena_off[i] = arena_bytes;
-      arena_bytes += (w + 255) / 256 * 256;
-    } else {
-      arena_bytes = std::max(arena_bytes, w);
-    }
+    arena_off[i] = arena_bytes;
+    arena_bytes += (w + 255) / 256 * 256;
+    widest = std::max(widest, w);
     scratch_bytes = std::max(scratch_bytes, sc);
+  }
+  branched = cfg.use_graph == 1 && side_by_side(1, (double)arena_bytes);
+  if (!side_by_side(cfg.use_graph, (double)arena_bytes)) {
+    arena_bytes = widest;
+    arena_off.assign(cplans.size(), 0);
   }
   if (arena_bytes) {
     GBX_TRY(dev_alloc((void**)&d_arena, arena_bytes));
@@ -827,20 +849,26 @@ int gbx_cc_create(const gbx_cc_config* cfg, void* stream, gbx_cc_job** out) {
   return GBX_OK;
 }
 
-// Records the iteration's steps into the persistent program: the job's
-// tensors are the buffers whose conflicts order the records of different
-// steps (every other buffer a step touches belongs to that step's plan).
-int gbx_cc_job::record_program() {
+// Records the iteration's steps: the job's tensors are the buffers whose
+// conflicts order the records of different steps (every other buffer a step
+// touches belongs to that step's plan).
+int gbx_cc_job::record_steps(ProgRecorder** rec) {
   std::vector<ProgBuffer> bufs;
   for (auto& kv : T)
     if (kv.second->d) bufs.push_back({kv.second->d, sizeof(double) * (size_t)std::max<int64_t>(1, kv.second->L.nelem)});
-  ProgRecorder* rec = nullptr;
-  GBX_TRY(prog_begin(bufs, &rec));
+  GBX_TRY(prog_begin(bufs, rec));
   int rc = GBX_OK;
   for (size_t i = 0; i < steps.size() && rc == GBX_OK; ++i) {
-    prog_step(rec, (int)i);
-    rc = steps[i](prog_stream(rec));
+    prog_step(*rec, (int)i);
+    rc = steps[i](prog_stream(*rec));
   }
+  return rc;
+}
+
+int gbx_cc_job::record_program() {
+  ProgRecorder* rec = nullptr;
+  const int rc = record_steps(&rec);
+  if (!rec) return rc;
   ProgramPtr p;
   const int frc = prog_finish(rec, p);
   if (rc != GBX_OK) return rc;
@@ -849,16 +877,75 @@ int gbx_cc_job::record_program() {
   return GBX_OK;
 }
 
+// Captures the steps as branches: each on a stream that ends in a step it
+// waits for, or on one of its own, with events for its other dependencies.
+// The streams and events serve the capture alone.
+int gbx_cc_job::capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps) {
+  struct Streams {
+    std::vector<cudaStream_t> s;
+    std::vector<cudaEvent_t> e;
+    ~Streams() {
+      for (cudaEvent_t x : e) cudaEventDestroy(x);
+      for (size_t i = 1; i < s.size(); ++i) cudaStreamDestroy(s[i]);
+    }
+    int event(cudaEvent_t* out) {
+      GBX_CUDA(cudaEventCreateWithFlags(out, cudaEventDisableTiming));
+      e.push_back(*out);
+      return GBX_OK;
+    }
+  } use;
+  use.s.push_back(cap);
+  cudaEvent_t begin;
+  GBX_TRY(use.event(&begin));
+  GBX_CUDA(cudaEventRecord(begin, cap));
+  const int n = (int)steps.size();
+  std::vector<int> last(1, -1), at(n, 0);  // a stream's last step; a step's stream
+  std::vector<cudaEvent_t> done(n);
+  for (int i = 0; i < n; ++i) {
+    int q = -1;
+    for (int d : deps[i])
+      if (last[at[d]] == d) q = at[d];  // the latest of them
+    if (q < 0 && i == 0) q = 0;
+    if (q < 0) {
+      cudaStream_t st;
+      GBX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      q = (int)use.s.size();
+      use.s.push_back(st);
+      last.push_back(-1);
+      if (deps[i].empty()) GBX_CUDA(cudaStreamWaitEvent(st, begin, 0));
+    }
+    for (int d : deps[i])
+      if (last[q] != d) GBX_CUDA(cudaStreamWaitEvent(use.s[q], done[d], 0));
+    GBX_TRY(steps[i](use.s[q]));
+    GBX_TRY(use.event(&done[i]));
+    GBX_CUDA(cudaEventRecord(done[i], use.s[q]));
+    last[q] = i;
+    at[i] = q;
+  }
+  for (size_t q = 1; q < use.s.size(); ++q) GBX_CUDA(cudaStreamWaitEvent(cap, done[last[q]], 0));
+  return GBX_OK;
+}
+
 int gbx_cc_capture(gbx_cc_job* job) {
   if (!job) return fail(GBX_EINVAL, "null job");
   if (!job->cfg.use_graph || job->exec) return GBX_OK;
   if (job->persistent() && !job->prog) GBX_TRY(job->record_program());
+  std::vector<std::vector<int>> deps;
+  if (job->branched) {
+    ProgRecorder* rec = nullptr;
+    const int rrc = job->record_steps(&rec);
+    const int frc = rec ? prog_finish_steps(rec, (int)job->steps.size(), deps) : GBX_OK;
+    GBX_TRY(rrc);
+    GBX_TRY(frc);
+  }
   cudaStream_t cap;
   GBX_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   GBX_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   int rc = GBX_OK;
   if (job->prog) {
     rc = prog_run(*job->prog, cap);
+  } else if (job->branched) {
+    rc = job->capture_branches(cap, deps);
   } else {
     for (auto& s : job->steps) {
       rc = s(cap);

@@ -39,6 +39,10 @@
 
 namespace gbx {
 
+// use_graph of a server's jobs: the kernel graph with its steps in one chain
+// (every value but 0, 1 and 2 means so).
+constexpr int kGraphChain = 3;
+
 struct CCTile {
   int64_t off;
   uint32_t n;

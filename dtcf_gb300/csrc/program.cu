@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
+#include <set>
 
 #include "bodies.cuh"
 #include "launch.h"
@@ -586,12 +587,11 @@ int build_program(ProgRecorder& R, Program& P) {
 
 }  // namespace
 
-int prog_finish(ProgRecorder* r, ProgramPtr& out) {
-  std::unique_ptr<ProgRecorder> R(r);
+static int end_recording(ProgRecorder* r) {
   if (g_rec == r) g_rec = nullptr;
   cudaGraph_t g = nullptr;
-  cudaError_t e = cudaStreamEndCapture(R->cap, &g);
-  cudaStreamDestroy(R->cap);
+  cudaError_t e = cudaStreamEndCapture(r->cap, &g);
+  cudaStreamDestroy(r->cap);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture", __FILE__, __LINE__);
   size_t nodes = 0;
   if (g) {
@@ -599,9 +599,35 @@ int prog_finish(ProgRecorder* r, ProgramPtr& out) {
     cudaGraphDestroy(g);
   }
   if (nodes) return fail(GBX_EUNSUPPORTED, "program: %zu operations of the iteration were launched, not recorded", nodes);
+  return GBX_OK;
+}
+
+int prog_finish(ProgRecorder* r, ProgramPtr& out) {
+  std::unique_ptr<ProgRecorder> R(r);
+  GBX_TRY(end_recording(r));
   ProgramPtr P(new Program());
   GBX_TRY(build_program(*R, *P));
   out = std::move(P);
+  return GBX_OK;
+}
+
+int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps) {
+  std::unique_ptr<ProgRecorder> R(r);
+  GBX_TRY(end_recording(r));
+  std::vector<std::set<int>> all(nsteps), direct(nsteps);
+  for (const RecEntry& e : R->recs)
+    for (int d : e.deps) {
+      const int q = R->recs[d].step;
+      if (e.step < 0 || e.step >= nsteps || q > e.step) return fail(GBX_EINVAL, "program: record outside the steps");
+      if (q >= 0 && q != e.step) direct[e.step].insert(q);
+    }
+  deps.assign(nsteps, {});
+  for (int i = 0; i < nsteps; ++i) {
+    for (int d : direct[i]) all[i].insert(all[d].begin(), all[d].end());
+    for (int d : direct[i])
+      if (!all[i].count(d)) deps[i].push_back(d);
+    all[i].insert(direct[i].begin(), direct[i].end());
+  }
   return GBX_OK;
 }
 

@@ -209,6 +209,9 @@ cudaStream_t prog_stream(ProgRecorder* r);
 // Stops recording and builds the program (device tables uploaded); the
 // recorder is released in any case.
 int prog_finish(ProgRecorder* r, ProgramPtr& out);
+// Stops recording and gives, for each step, the earlier steps it has to wait
+// for (those that others of them already wait for left out); no program.
+int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps);
 // Enqueues one run of the program on st.
 int prog_run(const Program& p, cudaStream_t st);
 // Bound on every dependency wait of the program's memory launches (clock

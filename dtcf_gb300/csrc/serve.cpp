@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/gbx_serve.h"
+#include "cc.h"
 #include "common.h"
 
 namespace {
@@ -239,6 +240,15 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
   if (!s) return fail(GBX_EINVAL, "null server");
   if (s->ran) return fail(GBX_EINVAL, "the server has already run");
   s->ran = true;
+  // where the budget does not hold all jobs at once, memory comes first: one
+  // workspace region to a job, its steps in a chain
+  double all = 0.0;
+  for (const Job& j : s->jobs) all += j.footprint;
+  if (all > s->cfg.budget_bytes)
+    for (Job& j : s->jobs) {
+      j.cfg.use_graph = kGraphChain;
+      GBX_TRY(gbx_cc_footprint(&j.cfg, &j.footprint, nullptr, nullptr));
+    }
   GBX_CUDA(cudaGetDevice(&s->device));
   GBX_CUDA(cudaStreamCreateWithFlags(&s->mem_stream, cudaStreamNonBlocking));
   // a job's requests run in arrival order
