@@ -132,7 +132,6 @@ struct gbx_cc_job {
   bool branched = false;  // use_graph 1: independent steps are branches of the graph
   int record_steps(ProgRecorder** rec);
   int record_program();
-  int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps);
 
   ~gbx_cc_job() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -877,55 +876,6 @@ int gbx_cc_job::record_program() {
   return GBX_OK;
 }
 
-// Captures the steps as branches: each on a stream that ends in a step it
-// waits for, or on one of its own, with events for its other dependencies.
-// The streams and events serve the capture alone.
-int gbx_cc_job::capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps) {
-  struct Streams {
-    std::vector<cudaStream_t> s;
-    std::vector<cudaEvent_t> e;
-    ~Streams() {
-      for (cudaEvent_t x : e) cudaEventDestroy(x);
-      for (size_t i = 1; i < s.size(); ++i) cudaStreamDestroy(s[i]);
-    }
-    int event(cudaEvent_t* out) {
-      GBX_CUDA(cudaEventCreateWithFlags(out, cudaEventDisableTiming));
-      e.push_back(*out);
-      return GBX_OK;
-    }
-  } use;
-  use.s.push_back(cap);
-  cudaEvent_t begin;
-  GBX_TRY(use.event(&begin));
-  GBX_CUDA(cudaEventRecord(begin, cap));
-  const int n = (int)steps.size();
-  std::vector<int> last(1, -1), at(n, 0);  // a stream's last step; a step's stream
-  std::vector<cudaEvent_t> done(n);
-  for (int i = 0; i < n; ++i) {
-    int q = -1;
-    for (int d : deps[i])
-      if (last[at[d]] == d) q = at[d];  // the latest of them
-    if (q < 0 && i == 0) q = 0;
-    if (q < 0) {
-      cudaStream_t st;
-      GBX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-      q = (int)use.s.size();
-      use.s.push_back(st);
-      last.push_back(-1);
-      if (deps[i].empty()) GBX_CUDA(cudaStreamWaitEvent(st, begin, 0));
-    }
-    for (int d : deps[i])
-      if (last[q] != d) GBX_CUDA(cudaStreamWaitEvent(use.s[q], done[d], 0));
-    GBX_TRY(steps[i](use.s[q]));
-    GBX_TRY(use.event(&done[i]));
-    GBX_CUDA(cudaEventRecord(done[i], use.s[q]));
-    last[q] = i;
-    at[i] = q;
-  }
-  for (size_t q = 1; q < use.s.size(); ++q) GBX_CUDA(cudaStreamWaitEvent(cap, done[last[q]], 0));
-  return GBX_OK;
-}
-
 int gbx_cc_capture(gbx_cc_job* job) {
   if (!job) return fail(GBX_EINVAL, "null job");
   if (!job->cfg.use_graph || job->exec) return GBX_OK;
@@ -945,7 +895,7 @@ int gbx_cc_capture(gbx_cc_job* job) {
   if (job->prog) {
     rc = prog_run(*job->prog, cap);
   } else if (job->branched) {
-    rc = job->capture_branches(cap, deps);
+    rc = capture_branches(cap, deps, [&](int i, cudaStream_t st) { return job->steps[i](st); });
   } else {
     for (auto& s : job->steps) {
       rc = s(cap);

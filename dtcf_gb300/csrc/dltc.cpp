@@ -23,6 +23,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <set>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -30,6 +31,7 @@
 #include "../../include/gbx_dltc.h"
 #include "common.h"
 #include "plan.h"
+#include "program.h"
 #include "split.h"
 
 namespace gbx {
@@ -289,22 +291,28 @@ int run_moves_once(const std::vector<MoveDesc>& v, const double* src, double* ds
 // ws_a + ws_b + ws_c elements); g or sp: the product planned by the caller
 // (neither: a one-shot FP64 product).
 GemmProblem gemm_problem(const Op& op, const double* A, const double* B, double* C, double* ws);
+// stages: 1 what does not touch C (the packs, and the product where it goes
+// to the workspace), 2 the rest, 3 both.
 int run_mul_op(const Op& op, const double* A, const double* B, double* C, double* ws, const MoveSet* ma,
-               const MoveSet* mb, const MoveSet* mc, F64Gemm* g, SplitPlan* sp, cudaStream_t st) {
+               const MoveSet* mb, const MoveSet* mc, F64Gemm* g, SplitPlan* sp, cudaStream_t st, int stages = 3) {
   if (op.M == 0 || op.N == 0) return GBX_OK;
   double* wa = ws;
   double* wb = ws + op.ws_a;
   double* wc = ws + op.ws_a + op.ws_b;
-  if (op.pack_a && op.pack_b && ma && mb) {
-    GBX_TRY(run_moves_two(*ma, A, wa, *mb, B, wb, st));
-  } else {
-    if (op.pack_a) GBX_TRY(ma ? run_moves(*ma, A, wa, st) : run_moves_once(op.mv_a, A, wa, st));
-    if (op.pack_b) GBX_TRY(mb ? run_moves(*mb, B, wb, st) : run_moves_once(op.mv_b, B, wb, st));
+  if (stages & 1) {
+    if (op.pack_a && op.pack_b && ma && mb) {
+      GBX_TRY(run_moves_two(*ma, A, wa, *mb, B, wb, st));
+    } else {
+      if (op.pack_a) GBX_TRY(ma ? run_moves(*ma, A, wa, st) : run_moves_once(op.mv_a, A, wa, st));
+      if (op.pack_b) GBX_TRY(mb ? run_moves(*mb, B, wb, st) : run_moves_once(op.mv_b, B, wb, st));
+    }
   }
-  if (sp) GBX_TRY(run_split_plan(sp, true, true, st));
-  else if (g) GBX_TRY(g->run(st));
-  else GBX_TRY(run_f64_one(gemm_problem(op, A, B, C, ws), st));
-  if (op.unpack_c) GBX_TRY(mc ? run_moves(*mc, wc, C, st) : run_moves_once(op.mv_c, wc, C, st));
+  if (stages & (op.unpack_c ? 1 : 2)) {
+    if (sp) GBX_TRY(run_split_plan(sp, true, true, st));
+    else if (g) GBX_TRY(g->run(st));
+    else GBX_TRY(run_f64_one(gemm_problem(op, A, B, C, ws), st));
+  }
+  if ((stages & 2) && op.unpack_c) GBX_TRY(mc ? run_moves(*mc, wc, C, st) : run_moves_once(op.mv_c, wc, C, st));
   return GBX_OK;
 }
 
@@ -703,8 +711,22 @@ struct gbx_dltc_program {
   std::vector<std::unique_ptr<F64Gemm>> gemm;
   std::vector<SplitPlan*> split;
   double* ws = nullptr;
+  std::vector<int64_t> ws_at;  // an expression's workspace (all 0: one for all)
+  // the whole table as a graph, expressions that do not depend on one
+  // another as branches (where they have workspaces of their own)
+  cudaGraphExec_t exec = nullptr;
   double flops = 0.0;
+
+  int run_op(int i, cudaStream_t st, int stages = 3) {
+    const Op& op = ops[i];
+    if (op.kind == GBX_DLTC_SUM) return stages & 2 ? run_moves(*msum[i], data[op.a], data[op.c], st) : GBX_OK;
+    return run_mul_op(op, data[op.a], data[op.b], data[op.c], ws + ws_at[i], ma[i].get(), mb[i].get(), mc[i].get(),
+                      gemm[i].get(), split[i], st, stages);
+  }
+  int capture();
+
   ~gbx_dltc_program() {
+    if (exec) cudaGraphExecDestroy(exec);
     for (SplitPlan* p : split) destroy_split_plan(p);
     gemm.clear();
     dev_free(ws);
@@ -719,6 +741,65 @@ int upload_moves(const std::vector<MoveDesc>& v, std::unique_ptr<MoveSet>& out) 
   return out->upload();
 }
 }  // namespace
+
+// Workspace elements up to which expressions keep workspaces of their own (2
+// GB: under 1% of the GPU's memory) and the table runs as a graph of branches
+// instead of kernel after kernel through one workspace (per run of the CCD
+// table: O = 4, V = 6, FP64 70 / 37 us; O = 9, V = 15, split 218 / 68; O = 12,
+// V = 35, split 340 / 130; O = 12, V = 36, FP64 1060 / 954).
+constexpr int64_t kBranchElems = 250000000;
+
+// An expression is one step, or two: what does not touch its C, and the rest.
+// A C that several expressions add to is written in their order.
+int gbx_dltc_program::capture() {
+  struct Step {
+    int op, stages;
+  };
+  std::vector<Step> steps;
+  std::vector<std::set<int>> direct;
+  std::vector<int> writer(data.size(), -1);
+  std::vector<std::vector<int>> readers(data.size());
+  const auto add = [&](int op, int stages) {
+    steps.push_back({op, stages});
+    direct.emplace_back();
+    return (int)steps.size() - 1;
+  };
+  for (int i = 0; i < (int)ops.size(); ++i) {
+    const Op& op = ops[i];
+    const bool two = op.kind == GBX_DLTC_MUL && op.M && op.N && (op.pack_a || op.pack_b || op.unpack_c);
+    const int first = add(i, two ? 1 : 3), rest = two ? add(i, 2) : first;
+    if (two) direct[rest].insert(first);
+    const auto reads = [&](int t, bool packed) {
+      if (t < 0) return;
+      if (writer[t] >= 0) direct[first].insert(writer[t]);
+      readers[t].push_back(packed || op.unpack_c ? first : rest);
+    };
+    reads(op.a, op.pack_a);
+    reads(op.b, op.pack_b);
+    if (writer[op.c] >= 0) direct[rest].insert(writer[op.c]);
+    for (int r : readers[op.c])
+      if (r != rest && r != first) direct[rest].insert(r);
+    writer[op.c] = rest;
+    readers[op.c].clear();
+  }
+  std::vector<std::vector<int>> deps;
+  reduce_deps(direct, deps);
+  cudaStream_t cap;
+  GBX_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+  cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeRelaxed);
+  int rc = e == cudaSuccess ? GBX_OK : cuda_fail(e, "cudaStreamBeginCapture", __FILE__, __LINE__);
+  if (rc == GBX_OK) {
+    rc = capture_branches(cap, deps, [&](int k, cudaStream_t st) { return run_op(steps[k].op, st, steps[k].stages); });
+    cudaGraph_t g = nullptr;
+    e = cudaStreamEndCapture(cap, &g);
+    if (rc == GBX_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaStreamEndCapture", __FILE__, __LINE__);
+    if (rc == GBX_OK && (e = cudaGraphInstantiate(&exec, g, 0)) != cudaSuccess)
+      rc = cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__);
+    if (g) cudaGraphDestroy(g);
+  }
+  cudaStreamDestroy(cap);
+  return rc;
+}
 
 extern "C" {
 
@@ -793,7 +874,7 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
   }
   Ranges R;
   GBX_TRY(make_ranges(D, nullptr, nullptr, R));
-  int64_t ws = 0;
+  int64_t ws = 0, all = 0;
   for (const TableExpr& x : p->table.exprs) {
     // index names must fit the tensors' index types
     auto fits = [&](int t, const std::vector<int>& ids) {
@@ -813,12 +894,19 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
     op.c = x.c;
     op.a = x.a;
     op.b = x.b;
-    ws = std::max(ws, op.ws_a + op.ws_b + op.ws_c);
+    const int64_t need = (op.ws_a + op.ws_b + op.ws_c + 31) / 32 * 32;
+    p->ws_at.push_back(all);
+    all += need;
+    ws = std::max(ws, need);
     p->flops += op.flops;
     p->ops.push_back(op);
   }
+  const bool branched = all <= kBranchElems;
+  if (branched) ws = all;
+  else p->ws_at.assign(p->ops.size(), 0);
   GBX_TRY(dev_alloc((void**)&p->ws, sizeof(double) * std::max<int64_t>(ws, 1)));
-  for (Op& op : p->ops) {
+  for (size_t i = 0; i < p->ops.size(); ++i) {
+    const Op& op = p->ops[i];
     p->ma.emplace_back();
     p->mb.emplace_back();
     p->mc.emplace_back();
@@ -833,7 +921,7 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
     if (op.pack_a) GBX_TRY(upload_moves(op.mv_a, p->ma.back()));
     if (op.pack_b) GBX_TRY(upload_moves(op.mv_b, p->mb.back()));
     if (op.unpack_c) GBX_TRY(upload_moves(op.mv_c, p->mc.back()));
-    GemmProblem g = gemm_problem(op, p->data[op.a], p->data[op.b], p->data[op.c], p->ws);
+    GemmProblem g = gemm_problem(op, p->data[op.a], p->data[op.b], p->data[op.c], p->ws + p->ws_at[i]);
     if (mode == GBX_MODE_SPLIT) {
       GBX_TRY(make_split(op, g, &p->split.back()));
     } else {
@@ -841,6 +929,7 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
       GBX_TRY(p->gemm.back()->build({g}));
     }
   }
+  if (branched) GBX_TRY(p->capture());
   *out = p.release();
   return GBX_OK;
 }
@@ -859,15 +948,17 @@ int gbx_dltc_program_run(gbx_dltc_program* p, int first, int count, void* stream
   if (first < 0 || first + count > n) return fail(GBX_EINVAL, "expressions [%d, %d) outside [0, %d)", first,
                                                   first + count, n);
   cudaStream_t st = (cudaStream_t)stream;
-  for (int i = first; i < first + count; ++i) {
-    const Op& op = p->ops[i];
-    if (op.kind == GBX_DLTC_SUM) {
-      GBX_TRY(run_moves(*p->msum[i], p->data[op.a], p->data[op.c], st));
-      continue;
+  if (p->exec && first == 0 && count == n) {
+    // a caller's own capture takes the kernels themselves
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &c);
+    if (e == cudaSuccess && c == cudaStreamCaptureStatusNone) {
+      GBX_CUDA(cudaGraphLaunch(p->exec, st));
+      return GBX_OK;
     }
-    GBX_TRY(run_mul_op(op, p->data[op.a], p->data[op.b], p->data[op.c], p->ws, p->ma[i].get(), p->mb[i].get(),
-                       p->mc[i].get(), p->gemm[i].get(), p->split[i], st));
+    if (e != cudaSuccess) cudaGetLastError();
   }
+  for (int i = first; i < first + count; ++i) GBX_TRY(p->run_op(i, st));
   return GBX_OK;
 }
 

@@ -67,8 +67,11 @@ __device__ __forceinline__ bool wait_deps(const ProgLaunch& L, int r, uint32_t* 
           atomicCAS(L.err, 0, kProgErrWait);
           return false;
         }
+        // short sleeps: records of a small job take a few microseconds (CCSD
+        // at o = 12, v = 36: 330 us per iteration with sleeps of up to 1024
+        // ns, 318 so; at o = 48, v = 240 no difference)
         __nanosleep(ns);
-        if (ns < 1024) ns *= 2;
+        if (ns < 64) ns *= 2;
       }
     }
     if (cacheable) seen[d >> 5] |= 1u << (d & 31);
@@ -614,20 +617,73 @@ int prog_finish(ProgRecorder* r, ProgramPtr& out) {
 int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps) {
   std::unique_ptr<ProgRecorder> R(r);
   GBX_TRY(end_recording(r));
-  std::vector<std::set<int>> all(nsteps), direct(nsteps);
+  std::vector<std::set<int>> direct(nsteps);
   for (const RecEntry& e : R->recs)
     for (int d : e.deps) {
       const int q = R->recs[d].step;
       if (e.step < 0 || e.step >= nsteps || q > e.step) return fail(GBX_EINVAL, "program: record outside the steps");
       if (q >= 0 && q != e.step) direct[e.step].insert(q);
     }
-  deps.assign(nsteps, {});
-  for (int i = 0; i < nsteps; ++i) {
+  reduce_deps(direct, deps);
+  return GBX_OK;
+}
+
+void reduce_deps(const std::vector<std::set<int>>& direct, std::vector<std::vector<int>>& deps) {
+  const int n = (int)direct.size();
+  std::vector<std::set<int>> all(n);
+  deps.assign(n, {});
+  for (int i = 0; i < n; ++i) {
     for (int d : direct[i]) all[i].insert(all[d].begin(), all[d].end());
     for (int d : direct[i])
       if (!all[i].count(d)) deps[i].push_back(d);
     all[i].insert(direct[i].begin(), direct[i].end());
   }
+}
+
+int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps,
+                     const std::function<int(int, cudaStream_t)>& step) {
+  struct Streams {
+    std::vector<cudaStream_t> s;
+    std::vector<cudaEvent_t> e;
+    ~Streams() {
+      for (cudaEvent_t x : e) cudaEventDestroy(x);
+      for (size_t i = 1; i < s.size(); ++i) cudaStreamDestroy(s[i]);
+    }
+    int event(cudaEvent_t* out) {
+      GBX_CUDA(cudaEventCreateWithFlags(out, cudaEventDisableTiming));
+      e.push_back(*out);
+      return GBX_OK;
+    }
+  } use;
+  use.s.push_back(cap);
+  cudaEvent_t begin;
+  GBX_TRY(use.event(&begin));
+  GBX_CUDA(cudaEventRecord(begin, cap));
+  const int n = (int)deps.size();
+  std::vector<int> last(1, -1), at(n, 0);  // a stream's last step; a step's stream
+  std::vector<cudaEvent_t> done(n);
+  for (int i = 0; i < n; ++i) {
+    int q = -1;
+    for (int d : deps[i])
+      if (last[at[d]] == d) q = at[d];  // the latest of them
+    if (q < 0 && i == 0) q = 0;
+    if (q < 0) {
+      cudaStream_t st;
+      GBX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+      q = (int)use.s.size();
+      use.s.push_back(st);
+      last.push_back(-1);
+      if (deps[i].empty()) GBX_CUDA(cudaStreamWaitEvent(st, begin, 0));
+    }
+    for (int d : deps[i])
+      if (last[q] != d) GBX_CUDA(cudaStreamWaitEvent(use.s[q], done[d], 0));
+    GBX_TRY(step(i, use.s[q]));
+    GBX_TRY(use.event(&done[i]));
+    GBX_CUDA(cudaEventRecord(done[i], use.s[q]));
+    last[q] = i;
+    at[i] = q;
+  }
+  for (size_t q = 1; q < use.s.size(); ++q) GBX_CUDA(cudaStreamWaitEvent(cap, done[last[q]], 0));
   return GBX_OK;
 }
 

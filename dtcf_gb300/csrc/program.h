@@ -38,6 +38,7 @@
 #include <cstdint>
 #include <functional>
 #include <memory>
+#include <set>
 #include <vector>
 
 #include "cc.h"
@@ -212,6 +213,13 @@ int prog_finish(ProgRecorder* r, ProgramPtr& out);
 // Stops recording and gives, for each step, the earlier steps it has to wait
 // for (those that others of them already wait for left out); no program.
 int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps);
+// Dependencies on earlier steps without those that others imply.
+void reduce_deps(const std::vector<std::set<int>>& direct, std::vector<std::vector<int>>& deps);
+// Captures steps as branches of the graph that cap captures: each on a stream
+// that ends in a step it waits for, or on one of its own, with events for its
+// other dependencies.  The streams and events serve the capture alone.
+int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps,
+                     const std::function<int(int, cudaStream_t)>& step);
 // Enqueues one run of the program on st.
 int prog_run(const Program& p, cudaStream_t st);
 // Bound on every dependency wait of the program's memory launches (clock

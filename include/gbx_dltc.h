@@ -88,7 +88,8 @@ typedef struct gbx_dltc_program gbx_dltc_program;
 
 /* A table bound to device tensors of the given dims, zeroed (as GA_Zero
  * leaves them), with every expression prepared once: transposes, GEMM (mode
- * GBX_MODE_FP64 or GBX_MODE_SPLIT) and one shared workspace.
+ * GBX_MODE_FP64 or GBX_MODE_SPLIT) and its workspace (up to 2 GB together;
+ * beyond, one shared by all).
  * Replaces the setup half of ccd_t2 / ccsd_t1 / ccsd_t2 (Tensor2/Tensor4 +
  * allocGA + the Multiplication / Summation constructors). */
 GBX_API int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_dltc_program** out);
@@ -96,7 +97,9 @@ GBX_API int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mo
 GBX_API int gbx_dltc_program_tensor(gbx_dltc_program* p, int tensor, double** d_data, int64_t* elems);
 /* Enqueue expressions [first, first + count) of the execution order
  * (count < 0: to the end) on stream.  All of them = the layers of the
- * table one after the other (the Barriers become stream order).
+ * table one after the other (the Barriers become dependencies: expressions
+ * with workspaces of their own run as one graph, those that do not depend on
+ * one another side by side; in a stream that is being captured, one by one).
  * Replaces the exec / gtc_process half of ccd_t2 / ccsd_t1 / ccsd_t2. */
 GBX_API int gbx_dltc_program_run(gbx_dltc_program* p, int first, int count, void* stream);
 /* GBX_ETIMEOUT if a bounded device wait of the split engine ran out (syncs). */
