@@ -399,6 +399,7 @@ struct Program {
     int grid = 0;
   };
   std::vector<Op> ops;
+  std::vector<std::vector<int>> op_deps;  // the launches each one waits for
   std::vector<MemLaunch> mem;
   std::vector<SplitMerged*> merged;
   std::vector<std::function<int(cudaStream_t)>> ext;
@@ -475,6 +476,7 @@ int build_program(ProgRecorder& R, Program& P) {
   GBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, prog_mem_kernel, kProgThreads, 0));
   if (occ < 1) return fail(GBX_ECUDA, "program: memory kernel does not fit an SM");
   std::vector<int> local(n, -1);
+  std::vector<int> op_of(n, -1);  // the launch an entry is part of
   size_t words = 0;
   std::vector<size_t> ticket_off(nlev), done_off(nlev);
   int records = 0;
@@ -548,6 +550,7 @@ int build_program(ProgRecorder& R, Program& P) {
         GBX_TRY(dev_alloc((void**)&ml.d_deps, sizeof(uint32_t) * hd.size()));
         GBX_CUDA(cudaMemcpy(ml.d_deps, hd.data(), sizeof(uint32_t) * hd.size(), cudaMemcpyHostToDevice));
       }
+      for (int i : ids) op_of[i] = (int)P.ops.size();
       P.ops.push_back({0, (int)P.mem.size()});
       P.mem.push_back(ml);
       records += m;
@@ -562,7 +565,10 @@ int build_program(ProgRecorder& R, Program& P) {
     for (int c : classes) {
       std::vector<std::pair<SplitPlan*, int>> parts;
       for (int i = 0; i < n; ++i)
-        if (E[i].level == lv && E[i].cls == 1 && E[i].split_cls == c) parts.push_back({E[i].sp, E[i].launch});
+        if (E[i].level == lv && E[i].cls == 1 && E[i].split_cls == c) {
+          parts.push_back({E[i].sp, E[i].launch});
+          op_of[i] = (int)P.ops.size();
+        }
       SplitMerged* sm = nullptr;
       GBX_TRY(split_merge(parts, P.d_err, &sm));
       P.ops.push_back({1, (int)P.merged.size()});
@@ -571,11 +577,19 @@ int build_program(ProgRecorder& R, Program& P) {
     }
     for (int i = 0; i < n; ++i)
       if (E[i].level == lv && E[i].cls == 2) {
+        op_of[i] = (int)P.ops.size();
         P.ops.push_back({2, (int)P.ext.size()});
         P.ext.push_back(E[i].ext);
         ++records;
       }
   }
+  std::vector<std::set<int>> direct(P.ops.size());
+  for (int i = 0; i < n; ++i)
+    for (int d : E[i].deps) {
+      if (op_of[d] > op_of[i]) return fail(GBX_EINVAL, "program: a launch before one that it waits for");
+      if (op_of[d] != op_of[i]) direct[op_of[i]].insert(op_of[d]);
+    }
+  reduce_deps(direct, P.op_deps);
   P.counter_words = std::max<size_t>(words, 32);
   GBX_TRY(dev_alloc((void**)&P.d_counters, sizeof(uint32_t) * P.counter_words));
   GBX_CUDA(cudaMemset(P.d_counters, 0, sizeof(uint32_t) * P.counter_words));
@@ -687,28 +701,29 @@ int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps
   return GBX_OK;
 }
 
+// Launches that do not depend on one another -- the GEMM kernels of a level,
+// and the next level's records beside a GEMM that only later ones wait for --
+// are branches of the graph that st captures (one after another / so, per
+// iteration: CCSD at o = 12, v = 40, FP64 565 / 507 us; o = 12, v = 36 at 5
+// slices 318 / 287; o = 32, v = 160 1539 / 1479; o = 48, v = 240 5849 / 5739).
 int prog_run(const Program& P, cudaStream_t st) {
   GBX_CUDA(cudaMemsetAsync(P.d_counters, 0, sizeof(uint32_t) * P.counter_words, st));
-  for (const Program::Op& op : P.ops) {
-    if (op.type == 0) {
-      const Program::MemLaunch& m = P.mem[op.idx];
-      ProgLaunch L;
-      L.recs = m.d_recs;
-      L.deps = m.d_deps;
-      L.ticket = P.d_counters + m.ticket_off;
-      L.done = P.d_counters + m.done_off;
-      L.err = P.d_err;
-      L.limit = P.limit;
-      L.nrec = m.nrec;
-      L.total = m.total;
-      GBX_TRY(launch(prog_mem_kernel, (unsigned)m.grid, kProgThreads, st, L));
-    } else if (op.type == 1) {
-      GBX_TRY(split_merged_run(P.merged[op.idx], st));
-    } else {
-      GBX_TRY(P.ext[op.idx](st));
-    }
-  }
-  return GBX_OK;
+  return capture_branches(st, P.op_deps, [&](int i, cudaStream_t q) {
+    const Program::Op& op = P.ops[i];
+    if (op.type == 1) return split_merged_run(P.merged[op.idx], q);
+    if (op.type == 2) return P.ext[op.idx](q);
+    const Program::MemLaunch& m = P.mem[op.idx];
+    ProgLaunch L;
+    L.recs = m.d_recs;
+    L.deps = m.d_deps;
+    L.ticket = P.d_counters + m.ticket_off;
+    L.done = P.d_counters + m.done_off;
+    L.err = P.d_err;
+    L.limit = P.limit;
+    L.nrec = m.nrec;
+    L.total = m.total;
+    return launch(prog_mem_kernel, (unsigned)m.grid, kProgThreads, q, L);
+  });
 }
 
 void prog_set_wait_limit(Program& p, long long cycles) { p.limit = cycles > 0 ? cycles : kProgWaitCycles; }

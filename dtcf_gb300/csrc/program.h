@@ -19,7 +19,9 @@
 //     k-stationary launch, one per thin-K block width, ...) over all the
 //     problems of every contraction at that level;
 //   * anything else (the FP64 tensor-pipe GEMM kernels) is launched as it
-//     would be, in record order.
+//     would be.
+// The launches are captured as branches: each waits for those that hold
+// records its own depend on.
 //
 // A record depends on the record before it in the same step (the steps of
 // one contraction stay in order) and on every earlier record that touches a
