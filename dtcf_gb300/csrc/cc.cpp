@@ -883,10 +883,12 @@ int gbx_cc_capture(gbx_cc_job* job) {
   std::vector<std::vector<int>> deps;
   if (job->branched) {
     ProgRecorder* rec = nullptr;
-    const int rrc = job->record_steps(&rec);
-    const int frc = rec ? prog_finish_steps(rec, (int)job->steps.size(), deps) : GBX_OK;
-    GBX_TRY(rrc);
-    GBX_TRY(frc);
+    int rrc = job->record_steps(&rec);
+    if (rec) {
+      const int frc = prog_finish_steps(rec, (int)job->steps.size(), deps);
+      if (rrc == GBX_OK) rrc = frc;
+    }
+    job->branched = rrc == GBX_OK;  // else the chain, which needs no record
   }
   cudaStream_t cap;
   GBX_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));

@@ -929,7 +929,7 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
       GBX_TRY(p->gemm.back()->build({g}));
     }
   }
-  if (branched) GBX_TRY(p->capture());
+  if (branched && p->capture() != GBX_OK) cudaGetLastError();  // the table then runs kernel by kernel
   *out = p.release();
   return GBX_OK;
 }

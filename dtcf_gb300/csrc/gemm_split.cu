@@ -817,13 +817,13 @@ __global__ void __launch_bounds__(kThinThreads, 1) split_thin_kernel(const GemmP
 //
 // What bounds it is shared memory: at S = 4 a K step of 16 reads 16 KB of A
 // and 20 KB of B and TMA writes 24 KB, 60 KB at 128 bytes a clock against 320
-// clocks of MMAs.  9216 x 768 x 4096 runs at 1305 TFLOP/s of slice products
-// at S = 4 (58% of the tensor pipe; the bound above is 68%), 1250 at 5, 1240
-// at 6 and 1180 at 7, where the pair-by-pair kernel reaches 940.
+// clocks of MMAs.  9216 x 768 x 4096 runs at 1483 TFLOP/s of slice products
+// at S = 4 (66% of the tensor pipe; the bound above is 68%), 1366 at 5, 1332
+// at 6 and 1190 at 7, where the pair-by-pair kernel reaches 940.
 //
 // A k-block is 64 elements up to four slices (two stages or more); beyond
-// only one such stage would fit, so 32 (S = 4 takes 453 us with 32, 441 with
-// 64).
+// only one such stage would fit, so 32 (at S = 4 that took 453 us, and 64 took
+// 441).
 //
 // TMEM holds eight such accumulators.  Level l sums l + 1 products of at
 // most 2^14 per element, so 1024 / (l + 1) elements fit below 2^24 and are
