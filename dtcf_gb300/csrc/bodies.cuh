@@ -465,6 +465,16 @@ __device__ __forceinline__ void direct_elements(const DirSmem& sm, uint32_t e0, 
       }
     }
   }
+  if (kStore && fabs(alpha) == 1.0) {
+    // a store of +-1 times the sum: its sign bit, not another FP64 instruction
+    const long long flip = __double_as_longlong(alpha) & (long long)0x8000000000000000ull;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t e = e0 + (uint32_t)(k * kThr);
+      if (e < it.n) C[it.coff + e] = __longlong_as_double(__double_as_longlong(acc[k]) ^ flip);
+    }
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const uint32_t e = e0 + (uint32_t)(k * kThr);
@@ -1051,6 +1061,16 @@ __device__ __forceinline__ void splitk_reduce_body(const GemmProblem* __restrict
 constexpr int kCcThreads = 256;
 constexpr int kCcChunk = 2048;
 
+// 0 + x / 2 (-0 turned into +0) on the bits; zeros and values whose half is
+// not normal take the FP64 instruction, warp by warp.
+__device__ __forceinline__ double half_of(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), e = (hi >> 20) & 0x7FFu;
+  const bool zero = ((hi << 1) | (uint32_t)__double2loint(x)) == 0;
+  double h = zero ? 0.0 : __hiloint2double((int)(hi - (1u << 20)), __double2loint(x));
+  if (__any_sync(__activemask(), !zero && (e < 2 || e == 0x7FF))) h = __fma_rn(0.5, x, 0.0);
+  return h;
+}
+
 // tau, taut and Q from t2 and t1 (see CCAmpTile in cc.h).
 template <bool kCoh>
 __device__ __forceinline__ void cc_amp_body(const CCAmpTile* __restrict__ tiles, const CCAmpItem* __restrict__ items,
@@ -1064,6 +1084,28 @@ __device__ __forceinline__ void cc_amp_body(const CCAmpTile* __restrict__ tiles,
     const uint32_t ej = tl.fj.d, ea = tl.fa.d, eb = tl.fb.d;
     const int64_t o_ia = tl.t1[0], o_jb = tl.t1[1], o_ib = tl.t1[2], o_ja = tl.t1[3];
     const bool h1 = o_ia >= 0 && o_jb >= 0, h2 = o_ib >= 0 && o_ja >= 0;
+    // tiles no t1 block reaches (all but one in eight with eight irreps): a
+    // branch of its own, because the compiler evaluates both sides of `hd ? ..`
+    // and with that five FP64 instructions to every element (133 MB of t2 in
+    // 8 irreps: 165 us, 98 so)
+    if (!h1 && !h2) {
+      double x[kPer];
+#pragma unroll
+      for (int k = 0; k < kPer; ++k)
+        x[k] = ldin<kCoh>(t2 + tl.off + it.f0 + min((uint32_t)(threadIdx.x + k * kCcThreads), it.n - 1));
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t e = threadIdx.x + k * kCcThreads;
+        if (e >= it.n) continue;
+        const int64_t at = tl.off + it.f0 + e;
+        const unsigned long long xb = (unsigned long long)__double_as_longlong(x[k]);
+        const double x0 = __longlong_as_double((long long)(xb == 0x8000000000000000ull ? 0ull : xb));
+        tau[at] = x0;
+        taut[at] = x0;
+        Q[at] = half_of(x[k]);
+      }
+      continue;
+    }
     double x[kPer], p1[kPer], d[kPer];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
