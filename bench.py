@@ -46,7 +46,7 @@ def parse():
                         "iterations of the default workload, inside the 1e-10 Eh bound; 6: ~1e-16)")
     p.add_argument("--autotune", type=int, default=1,
                    help="1: the split job times each contraction's output tile widths when it is built")
-    p.add_argument("--graph", type=int, default=2, choices=[1, 2],
+    p.add_argument("--graph", type=int, default=1, choices=[1, 2],
                    help="iteration of the headline number -- 1: one CUDA graph of the iteration's kernels; "
                         "2: the persistent program (a few persistent launches off a device-side work queue, "
                         "captured as the graph); the other mode is timed beside it")

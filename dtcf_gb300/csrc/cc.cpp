@@ -96,6 +96,9 @@ struct gbx_cc_job {
   std::vector<CCAmpItem> amp_items;
   CCAmpSet amp;
   std::vector<std::function<int(cudaStream_t)>> steps;       // one iteration
+  // contractions that run in two stages: the product into the plan's
+  // workspace, and from there into the output
+  std::map<int, std::function<int(cudaStream_t, int)>> staged;
   std::vector<std::function<int(cudaStream_t)>> init_steps;  // once, after the MP2 guess
   std::set<std::string> dynamic_use;  // tensors read or written outside constant plan operands
   std::vector<std::pair<CCTensor*, CCTensor*>> plan_operands;  // A, B of each contraction plan
@@ -130,7 +133,8 @@ struct gbx_cc_job {
 
   bool persistent() const { return cfg.use_graph == 2; }
   bool branched = false;  // use_graph 1: independent steps are branches of the graph
-  int record_steps(ProgRecorder** rec);
+  using Steps = std::vector<std::function<int(cudaStream_t)>>;
+  int record_steps(const Steps& todo, ProgRecorder** rec);
   int record_program();
 
   ~gbx_cc_job() {
@@ -229,7 +233,9 @@ struct gbx_cc_job {
     flops += p->flops;
     gemm_flops += p->gemm_flops;
     ContractionPlan* pp = p.get();
-    steps.push_back([=](cudaStream_t st) { return pp->execute(A->d, B->d, C->d, alpha, st); });
+    const auto run = [=](cudaStream_t st, int stages) { return pp->execute(A->d, B->d, C->d, alpha, st, stages); };
+    if (!pp->direct) staged[(int)steps.size()] = run;
+    steps.push_back([=](cudaStream_t st) { return run(st, 3); });
     info.push_back({std::string(c) + "[" + lc + "]" + (stores ? "=" : "+=") + a + "[" + la + "]*" + b + "[" + lb + "]", 0,
                     pp->flops, 8.0 * (double)(A->L.nelem + B->L.nelem + (stores ? 1 : 2) * C->L.nelem),
                     (int)cplans.size()});
@@ -615,15 +621,14 @@ double up256d(double x) { return std::ceil(x / 256.0) * 256.0; }
 
 // Whether contractions may run side by side, each in its own region of the
 // arena (`regions` bytes together): always in a persistent program, in a
-// graph up to 2 GB of regions (under 1% of the GPU's memory).  Larger jobs
-// share one region and run in a chain: their kernels fill the GPU one after
-// another and their memory counts.  Per iteration, chain / branches: CCSD at
-// o = 8, v = 24, FP64 300 / 179 us (12 / 15 MB resident); o = 16, v = 64 in 8
-// irreps at 6 slices 486 / 277 (54 / 63 MB); o = 16, v = 64 at 5 slices 1219 /
-// 843 (457 / 721 MB); o = 32, v = 160 in 8 irreps at 4 slices 1691 / 1325 (1.4 /
-// 1.9 GB); o = 48, v = 240 in 8 irreps 5945 / 5722 (6.6 / 8.6 GB, beyond the
-// line).
-constexpr double kBranchBytes = 2e9;
+// graph up to 4 GB of regions (1.4% of the GPU's memory).  Larger jobs share
+// one region and run in a chain: their memory counts.  Per iteration, chain /
+// branches: CCSD at o = 8, v = 24, FP64 300 / 160 us (12 / 15 MB resident); o =
+// 16, v = 64 in 8 irreps at 6 slices 486 / 259 (54 / 63 MB); o = 16, v = 64 at
+// 5 slices 1219 / 787 (457 / 721 MB); o = 32, v = 160 in 8 irreps at 4 slices
+// 1691 / 1178 (1.4 / 1.9 GB); o = 48, v = 240 in 8 irreps 5880 / 5344 (6.6 /
+// 8.6 GB).
+constexpr double kBranchBytes = 4e9;
 bool side_by_side(int use_graph, double regions) {
   return use_graph == 2 || (use_graph == 1 && regions <= kBranchBytes);
 }
@@ -848,25 +853,25 @@ int gbx_cc_create(const gbx_cc_config* cfg, void* stream, gbx_cc_job** out) {
   return GBX_OK;
 }
 
-// Records the iteration's steps: the job's tensors are the buffers whose
-// conflicts order the records of different steps (every other buffer a step
-// touches belongs to that step's plan).
-int gbx_cc_job::record_steps(ProgRecorder** rec) {
+// Records steps: the job's tensors are the buffers whose conflicts order the
+// records of different steps (every other buffer a step touches belongs to
+// that step's plan).
+int gbx_cc_job::record_steps(const Steps& todo, ProgRecorder** rec) {
   std::vector<ProgBuffer> bufs;
   for (auto& kv : T)
     if (kv.second->d) bufs.push_back({kv.second->d, sizeof(double) * (size_t)std::max<int64_t>(1, kv.second->L.nelem)});
   GBX_TRY(prog_begin(bufs, rec));
   int rc = GBX_OK;
-  for (size_t i = 0; i < steps.size() && rc == GBX_OK; ++i) {
+  for (size_t i = 0; i < todo.size() && rc == GBX_OK; ++i) {
     prog_step(*rec, (int)i);
-    rc = steps[i](prog_stream(*rec));
+    rc = todo[i](prog_stream(*rec));
   }
   return rc;
 }
 
 int gbx_cc_job::record_program() {
   ProgRecorder* rec = nullptr;
-  const int rc = record_steps(&rec);
+  const int rc = record_steps(steps, &rec);
   if (!rec) return rc;
   ProgramPtr p;
   const int frc = prog_finish(rec, p);
@@ -880,12 +885,31 @@ int gbx_cc_capture(gbx_cc_job* job) {
   if (!job) return fail(GBX_EINVAL, "null job");
   if (!job->cfg.use_graph || job->exec) return GBX_OK;
   if (job->persistent() && !job->prog) GBX_TRY(job->record_program());
+  // branches: a contraction's product waits for its operands alone, and only
+  // what adds it to the output for what the output holds before (CCSD at o =
+  // 8, v = 24, FP64: 182 us per iteration with whole contractions, 161 so; o =
+  // 12, v = 36 at 5 slices 195 / 160; o = 32, v = 160 1303 / 1178)
+  gbx_cc_job::Steps parts;
   std::vector<std::vector<int>> deps;
   if (job->branched) {
+    std::vector<int> prev;
+    for (size_t i = 0; i < job->steps.size(); ++i) {
+      const auto two = job->staged.find((int)i);
+      if (two == job->staged.end()) {
+        parts.push_back(job->steps[i]);
+        prev.push_back(-1);
+        continue;
+      }
+      const auto run = two->second;
+      parts.push_back([run](cudaStream_t st) { return run(st, 1); });
+      prev.push_back(-1);
+      parts.push_back([run](cudaStream_t st) { return run(st, 2); });
+      prev.push_back((int)parts.size() - 2);
+    }
     ProgRecorder* rec = nullptr;
-    int rrc = job->record_steps(&rec);
+    int rrc = job->record_steps(parts, &rec);
     if (rec) {
-      const int frc = prog_finish_steps(rec, (int)job->steps.size(), deps);
+      const int frc = prog_finish_steps(rec, prev, deps);
       if (rrc == GBX_OK) rrc = frc;
     }
     job->branched = rrc == GBX_OK;  // else the chain, which needs no record
@@ -897,7 +921,7 @@ int gbx_cc_capture(gbx_cc_job* job) {
   if (job->prog) {
     rc = prog_run(*job->prog, cap);
   } else if (job->branched) {
-    rc = capture_branches(cap, deps, [&](int i, cudaStream_t st) { return job->steps[i](st); });
+    rc = capture_branches(cap, deps, [&](int i, cudaStream_t st) { return parts[i](st); });
   } else {
     for (auto& s : job->steps) {
       rc = s(cap);

@@ -940,7 +940,8 @@ int ContractionPlan::stage(const double* dA, const double* dB, cudaStream_t st) 
   return GBX_OK;
 }
 
-int ContractionPlan::execute(const double* dA, const double* dB, double* dC, double alpha, cudaStream_t st) {
+int ContractionPlan::execute(const double* dA, const double* dB, double* dC, double alpha, cudaStream_t st,
+                             int stages) {
   if (direct) {
     if (!dA || !dB || !dC) return fail(GBX_EINVAL, "contraction operand without device memory");
     return run_direct(d_dir_items, (int)dir_items.size(), d_dir_pairs, dA, dB, dC, alpha, dir_overwrite, st);
@@ -948,9 +949,12 @@ int ContractionPlan::execute(const double* dA, const double* dB, double* dC, dou
   if (f64.nprob == 0 && !split) return GBX_OK;
   const bool skipA = a_static && static_ready, skipB = b_static && static_ready;
   if ((!skipA && !dA) || (!skipB && !dB)) return fail(GBX_EINVAL, "contraction operand without device memory");
-  GBX_TRY(pack(!skipA, !skipB, dA, dB, st));
-  GBX_TRY(f64.run(st));
-  if (split) GBX_TRY(run_split_plan(split, !skipA, !skipB, st));
+  if (stages & 1) {
+    GBX_TRY(pack(!skipA, !skipB, dA, dB, st));
+    GBX_TRY(f64.run(st));
+    if (split) GBX_TRY(run_split_plan(split, !skipA, !skipB, st));
+  }
+  if (!(stages & 2)) return GBX_OK;
   return run_moves_scaled(unpackC, d_Cbig, dC, alpha * alpha_factor, st);
 }
 

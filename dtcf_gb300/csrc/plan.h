@@ -183,8 +183,9 @@ struct ContractionPlan {
   // Packs and splits the changing operands without running the GEMM (so a
   // GEMM can be timed alone on current data).
   int stage(const double* dA, const double* dB, cudaStream_t st);
-  // C += alpha * A * B.
-  int execute(const double* dA, const double* dB, double* dC, double alpha, cudaStream_t st);
+  // C += alpha * A * B.  stages: 1 the product into the workspace (packed
+  // engines), 2 from there into C, 3 both; direct plans know 3 only.
+  int execute(const double* dA, const double* dB, double* dC, double alpha, cudaStream_t st, int stages = 3);
   // Autotuner: times the split GEMMs (with their per-run splits) at output
   // tile widths 64, 128 and 256 against the current choice and keeps the
   // fastest.  Call right after prepare_static, while the static scratch

@@ -628,10 +628,13 @@ int prog_finish(ProgRecorder* r, ProgramPtr& out) {
   return GBX_OK;
 }
 
-int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps) {
+int prog_finish_steps(ProgRecorder* r, const std::vector<int>& prev, std::vector<std::vector<int>>& deps) {
   std::unique_ptr<ProgRecorder> R(r);
   GBX_TRY(end_recording(r));
+  const int nsteps = (int)prev.size();
   std::vector<std::set<int>> direct(nsteps);
+  for (int i = 0; i < nsteps; ++i)
+    if (prev[i] >= 0) direct[i].insert(prev[i]);
   for (const RecEntry& e : R->recs)
     for (int d : e.deps) {
       const int q = R->recs[d].step;

@@ -214,7 +214,8 @@ cudaStream_t prog_stream(ProgRecorder* r);
 int prog_finish(ProgRecorder* r, ProgramPtr& out);
 // Stops recording and gives, for each step, the earlier steps it has to wait
 // for (those that others of them already wait for left out); no program.
-int prog_finish_steps(ProgRecorder* r, int nsteps, std::vector<std::vector<int>>& deps);
+// prev: per step, one that it follows whatever they touch (-1: none).
+int prog_finish_steps(ProgRecorder* r, const std::vector<int>& prev, std::vector<std::vector<int>>& deps);
 // Dependencies on earlier steps without those that others imply.
 void reduce_deps(const std::vector<std::set<int>>& direct, std::vector<std::vector<int>>& deps);
 // Captures steps as branches of the graph that cap captures: each on a stream
