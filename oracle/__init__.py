@@ -27,8 +27,8 @@ _p = ctypes.c_void_p
 
 
 def build(ref=True):
-    """Compile liboracle.so, and oracle/_ref/libref.so when the reference tree
-    exists.  The tree's location is the Makefile's REF (DTCF_REFERENCE, when
+    """Compile liboracle.so, and oracle/_ref/libref.so when the reference tree's
+    sources exist.  The tree's location is the Makefile's REF (DTCF_REFERENCE, when
     set, overrides it); `make ref` reports a missing tree and builds nothing."""
     subprocess.run(["make", "-s", "-C", HERE, "liboracle.so"], check=True)
     if ref:
