@@ -28,7 +28,8 @@ def _sources():
 
 def _compile(src, verbose):
     obj = os.path.join(OBJ, os.path.basename(src) + ".o")
-    deps = [src] + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(os.path.dirname(HERE), "include", "*.h"))
+    deps = [src] + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "*.cuh"))
+    deps += glob.glob(os.path.join(os.path.dirname(HERE), "include", "*.h"))
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(d) for d in deps):
         return obj, ""
     cmd = [NVCC] + ARCH + FLAGS + ["-c", src, "-o", obj]
