@@ -256,12 +256,9 @@ int run_f64_one(const GemmProblem& p, cudaStream_t st, double* scratch = nullptr
 // Split-K partial-sum elements F64Gemm::build allocates for these problems
 // (model kernels).
 int64_t f64_partial_elems(const std::vector<GemmProblem>& probs);
-// Kernel choice shared by the host planner: 0 the tile kernel, 4 / 5 one
-// thread per row / column, 6 K <= 8.
+// Kernel of a product: 0 the tile kernel, 4 / 5 one thread per row / column,
+// 6 K <= 8, 7 at most 16 x 16 outputs with long K, 8 matrix-vector.
 int f64_variant(int m, int n, int k);
-// As f64_variant, plus variants 7 (at most 16 x 16 outputs, long K) and 8
-// (matrix-vector) for planned launches.
-int f64_variant_planned(int m, int n, int k);
 
 // Device scratch allocation helpers (the library's own allocations go
 // through these so that OOM surfaces as GBX_ENOMEM).

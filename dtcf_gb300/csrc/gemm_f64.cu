@@ -49,8 +49,14 @@ int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // the tile kernel reaches on such shapes).  Measured, tile / thin kernel:
 // 5000 x 6 x 30 12 / 23 us, 100000 x 6 x 30 78 / 54, 40000 x 24 x 64 143 /
 // 207, 100000 x 24 x 64 306 / 320, 300000 x 24 x 64 883 / 825.
+// Before either, variant 7: outputs of at most 16 x 16 with long K, one CTA
+// per K chunk holding the whole output (reduced in a fixed order), and 8:
+// matrix-vector shapes (one side <= 2, K > 64), one warp per output of the
+// wide side, the wide operand's rows read once and coalesced.
 int f64_variant(int m, int n, int k) {
   if (k <= kSmallK) return 6;
+  if (m <= kSmallOutDim && n <= kSmallOutDim && k >= kSmallOutMinK) return 7;
+  if (k > kGemvMinK && ((m <= kGemvDim && n > kSmallOutDim) || (n <= kGemvDim && m > kSmallOutDim))) return 8;
   const bool rows = n <= kThinN && m >= 4 * n, cols = m <= kThinN && n >= 4 * m;
   if (rows || cols) {
     const int wide = rows ? m : n, thin = rows ? n : m;
@@ -60,15 +66,6 @@ int f64_variant(int m, int n, int k) {
     if (filled > 0.9 * real) return rows ? 4 : 5;
   }
   return 0;
-}
-// Planned launches also use variant 7: outputs of at most 16 x 16 with long
-// K, one CTA per K chunk holding the whole output (reduced in a fixed order).
-int f64_variant_planned(int m, int n, int k) {
-  if (m <= kSmallOutDim && n <= kSmallOutDim && k >= kSmallOutMinK) return 7;
-  // matrix-vector shapes (one side <= 2, K > 64): one warp per output of the
-  // wide side, the wide operand's rows read once and coalesced
-  if (k > kGemvMinK && ((m <= kGemvDim && n > kSmallOutDim) || (n <= kGemvDim && m > kSmallOutDim))) return 8;
-  return f64_variant(m, n, k);
 }
 
 // One thread per row (variant 4) or per column (variant 5) of C; the thin
@@ -386,6 +383,15 @@ __global__ void __launch_bounds__(256) small_k_one_f64_kernel(const __grid_const
   begin_dependent();
   dev::small_k_body<false>(&a.p, 1, &a.zero, total, blockIdx.x, gridDim.x);
 }
+__global__ void __launch_bounds__(256) gemv_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  begin_dependent();
+  dev::gemv_body<false>(&a.p, 1, &a.zero, total, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(256) small_out_one_f64_kernel(const __grid_constant__ OneProblem a, int total) {
+  begin_dependent();
+  __shared__ dev::SmallOutSmem sm;
+  dev::small_out_body<false>(&a.p, 1, &a.zero, total, blockIdx.x, gridDim.x, sm);
+}
 __global__ void __launch_bounds__(kRedThreads) splitk_reduce_one_kernel(const __grid_constant__ OneProblem a,
                                                                         uint32_t nchunks) {
   begin_dependent();
@@ -468,6 +474,21 @@ void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
 
 int64_t dmma_count(const GemmProblem& q) { return tile_count(q, 8) * ceil_div(q.k, 4); }
 
+// Small outputs: K chunks that give every SM four of all problems' `total_k`,
+// of at least 64.
+int small_out_chunk(int64_t total_k) { return (int)std::max<int64_t>(64, total_k / (4 * kSms) / 64 * 64); }
+
+// Matrix-vector problems: K ranges when the outputs are few.
+void gemv_ksplit(GemmProblem& q) {
+  const int64_t wide = q.m <= kGemvDim && q.m <= q.n ? q.n : q.m;
+  const int64_t groups = (wide + 7) / 8;
+  int ks = 1;
+  if (groups < kGemvItems && q.k > 2 * kGemvMinChunk)
+    ks = (int)std::min<int64_t>((kGemvItems + groups - 1) / groups, ceil_div(q.k, kGemvMinChunk));
+  q.kchunk = ceil_div(ceil_div(q.k, ks), 32) * 32;
+  q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
+}
+
 constexpr int kPlannedLeast = 96;   // about 25 us of one quarter: two reduction launches
 constexpr int kOneShotLeast = 512;  // a one-shot call also allocates the partial sums
 
@@ -478,7 +499,7 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
   int64_t dmmas = 0, small_k = 0;
   for (size_t i = 0; i < probs.size(); ++i) {
     GemmProblem& q = probs[i];
-    q.pad_ = want[i] >= 0 ? want[i] : f64_variant_planned(q.m, q.n, q.k);
+    q.pad_ = want[i] >= 0 ? want[i] : f64_variant(q.m, q.n, q.k);
     if (q.pad_ == 0) {
       tiles.push_back(&q);
       dmmas += dmma_count(q);
@@ -488,7 +509,7 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
   tp = tile_plan(tiles);
   // small outputs: chunks of up to 2048, shorter where all problems together
   // would leave CTAs without one
-  const int chunk7 = (int)std::max<int64_t>(64, std::min<int64_t>(kSmallOutChunk, small_k / (4 * kSms) / 64 * 64));
+  const int chunk7 = std::min(kSmallOutChunk, small_out_chunk(small_k));
   int64_t part = 0;
   for (GemmProblem& q : probs) {
     q.ksplit = 1;
@@ -497,14 +518,8 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
     if (q.pad_ == 7) {
       q.ksplit = std::max(1, ceil_div(q.k, chunk7));
       q.kchunk = chunk7;
-    } else if (q.pad_ == 8) {  // matrix-vector: K ranges when the outputs are few
-      const int64_t wide = q.m <= kGemvDim && q.m <= q.n ? q.n : q.m;
-      const int64_t groups = (wide + 7) / 8;
-      int ks = 1;
-      if (groups < kGemvItems && q.k > 2 * kGemvMinChunk)
-        ks = (int)std::min<int64_t>((kGemvItems + groups - 1) / groups, ceil_div(q.k, kGemvMinChunk));
-      q.kchunk = ceil_div(ceil_div(q.k, ks), 32) * 32;
-      q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
+    } else if (q.pad_ == 8) {
+      gemv_ksplit(q);
     } else if (q.pad_ == 0) {
       tile_ksplit(q, tp, dmmas, kPlannedLeast);
     }
@@ -721,6 +736,26 @@ int F64Gemm::run_each(cudaStream_t st) const {
   return GBX_OK;
 }
 
+// Kernel of a one-call product: a planned one's, but for the shapes whose few
+// outputs and short K the tile kernel's clusters finish first (the kernels for
+// long K add their K ranges' partial sums in a launch of their own, and
+// matrix-vector warps walk short K one after another).  Tile kernel /
+// matrix-vector or small-output kernel, one call of many: 2000 x 1 x 2000 73 /
+// 22 us, 5000 x 2 x 5000 447 / 113 (149 with the wide operand stored down its
+// columns), 700 x 1 x 300 9.1 / 4.9, 20 x 1 x 200000 156 / 31, 1 x 1 x 10^6
+// 159 / 41, 12 x 9 x 10^5 122 / 39; the other way round 20 x 1 x 2000 8.4 /
+// 16, 300 x 2 x 1200 12.5 / 15, 2000 x 2 x 70 4.7 / 6.6, 1 x 1 x 4096 12.9 /
+// 16.6.
+int one_call_variant(int m, int n, int k) {
+  const int v = f64_variant(m, n, k);
+  if (v == 7 && m == 1 && n == 1 && k < 6144) return 0;
+  if (v == 8 && k < 4608) {
+    const int wide = std::max(m, n);
+    if (wide < 400 || (int64_t)ceil_div(wide, 8) * ceil_div(k, 4) < 5000) return 0;
+  }
+  return v;
+}
+
 // One problem, one call: the descriptor travels in the kernel's arguments.
 // The partial sums of long K with few outputs come from `scratch` (at most
 // scratch_elems) when given, else from a stream-ordered temporary.
@@ -730,7 +765,7 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
   GemmProblem& q = a.p;
   q = in;
   if (q.m <= 0 || q.n <= 0) return GBX_OK;
-  q.pad_ = f64_variant(q.m, q.n, q.k);
+  q.pad_ = one_call_variant(q.m, q.n, q.k);
   q.ksplit = 1;
   q.kchunk = std::max(q.k, 4);
   q.partial = nullptr;
@@ -738,15 +773,20 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
   double* own = nullptr;
   if (q.pad_ == 0) {
     tile_ksplit(q, tp, dmma_count(q), kOneShotLeast);
-    if (scratch && (int64_t)q.ksplit * q.m * q.n > scratch_elems) {
-      const int64_t ks = std::max<int64_t>(1, scratch_elems / ((int64_t)q.m * q.n));
-      q.kchunk = 4 * ceil_div(ceil_div(q.k, 4), ks);
-      q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
-    }
-    if (q.ksplit > 1) {
-      if (!scratch) GBX_CUDA(cudaMallocAsync((void**)&own, sizeof(double) * q.ksplit * q.m * q.n, st));
-      q.partial = scratch ? scratch : own;
-    }
+  } else if (q.pad_ == 7) {
+    q.kchunk = small_out_chunk(q.k);
+    q.ksplit = ceil_div(q.k, q.kchunk);
+  } else if (q.pad_ == 8) {
+    gemv_ksplit(q);
+  }
+  if (scratch && (int64_t)q.ksplit * q.m * q.n > scratch_elems) {
+    const int64_t ks = std::max<int64_t>(1, scratch_elems / ((int64_t)q.m * q.n));
+    q.kchunk = 4 * ceil_div(ceil_div(q.k, 4), ks);
+    q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
+  }
+  if (q.ksplit > 1) {
+    if (!scratch) GBX_CUDA(cudaMallocAsync((void**)&own, sizeof(double) * q.ksplit * q.m * q.n, st));
+    q.partial = scratch ? scratch : own;
   }
   const int64_t items = f64_items(q, tp.ts);
   if (items >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "FP64 GEMM has too many work items");
@@ -759,6 +799,8 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
       break;
     case 4: rc = launch(thin_one_f64_kernel<true>, (unsigned)grid, 256, st, a, (int)items); break;
     case 6: rc = launch(small_k_one_f64_kernel, (unsigned)grid, 256, st, a, (int)items); break;
+    case 7: rc = launch(small_out_one_f64_kernel, (unsigned)grid, 256, st, a, (int)items); break;
+    case 8: rc = launch(gemv_one_f64_kernel, (unsigned)grid, 256, st, a, (int)items); break;
     default: rc = launch(thin_one_f64_kernel<false>, (unsigned)grid, 256, st, a, (int)items); break;
   }
   if (rc == GBX_OK && q.ksplit > 1) {
