@@ -124,9 +124,9 @@ int run_moves_two(const MoveSet& ma, const double* srcA, double* dstA, const Mov
 // One move; an accumulating one uses scale * alpha.
 int run_move_one(const MoveDesc& md, const double* src, double* dst, double alpha, cudaStream_t st);
 // nblocks blocks of block_elems elements, block b moved by moves[which[b]]
-// (at most 16 moves, offsets relative to the block; which unused for one).
-int run_block_moves(const std::vector<MoveDesc>& moves, const uint8_t* which, int64_t nblocks, int64_t block_elems,
-                    const double* src, double* dst, cudaStream_t st);
+// (offsets relative to the block).
+int run_block_moves(const std::vector<MoveDesc>& moves, const std::vector<int>& which, int64_t nblocks,
+                    int64_t block_elems, const double* src, double* dst, cudaStream_t st);
 // Tiles of rows x cols elements into (or out of) one row-major matrix of
 // nrows x ncols tiles; position i of the grid holds tile slots[i].
 int run_pack(int64_t rows, int64_t cols, int64_t nrows, int64_t ncols, const std::vector<int>& slots, bool to_big,

@@ -298,10 +298,17 @@ int gbx_transpose_blocks(const double* d_in, double* d_out, int num_blocks, cons
   int64_t bs = 1;
   for (int i = 0; i < dims; ++i) bs *= widths[i];
   // every permutation as one word (three bits a dimension), checked when it
-  // first occurs
-  std::vector<uint32_t> key(num_blocks);
+  // first occurs; which: the blocks' numbers among them, found through a hash
+  // table that is kept at most half full
+  std::vector<int> which(num_blocks);
   std::vector<uint32_t> known;
-  uint32_t prev = ~0u;
+  std::vector<int> table(64, -1);
+  std::vector<MoveDesc> mv;
+  const auto place = [&](uint32_t k) {
+    size_t at = (k * 0x9E3779B1u >> 7) & (table.size() - 1);
+    while (table[at] >= 0 && known[table[at]] != k) at = (at + 1) & (table.size() - 1);
+    return at;
+  };
   for (int b = 0; b < num_blocks; ++b) {
     const int* p = perms + (int64_t)b * dims;
     if (b == 0) GBX_TRY(check_perm(dims, p));  // dims too
@@ -312,36 +319,21 @@ int gbx_transpose_blocks(const double* d_in, double* d_out, int num_blocks, cons
       stray |= p[d] & ~7;
     }
     if (stray) return check_perm(dims, p);
-    if (k != prev && std::find(known.begin(), known.end(), k) == known.end()) {
-      GBX_TRY(check_perm(dims, p));
-      known.push_back(k);
+    const size_t at = place(k);
+    if (table[at] >= 0) {
+      which[b] = table[at];
+      continue;
     }
-    key[b] = prev = k;
+    GBX_TRY(check_perm(dims, p));
+    which[b] = table[at] = (int)known.size();
+    known.push_back(k);
+    mv.push_back(permute_move(dims, p, widths, 0, 0));
+    if (2 * known.size() > table.size()) {
+      table.assign(2 * table.size(), -1);
+      for (size_t i = 0; i < known.size(); ++i) table[place(known[i])] = (int)i;
+    }
   }
-  // the blocks' numbers among the permutations of a launch; more than 16 go
-  // out in several launches of consecutive blocks
-  std::vector<MoveDesc> mv;
-  std::vector<uint32_t> seen;
-  std::vector<uint8_t> which(num_blocks);
-  cudaStream_t st = (cudaStream_t)stream;
-  int b0 = 0;
-  for (int b = 0; b < num_blocks; ++b) {
-    size_t i = 0;
-    while (i < seen.size() && seen[i] != key[b]) ++i;
-    if (i == 16) {
-      GBX_TRY(run_block_moves(mv, which.data() + b0, b - b0, bs, d_in + b0 * bs, d_out + b0 * bs, st));
-      mv.clear();
-      seen.clear();
-      b0 = b;
-      i = 0;
-    }
-    if (i == seen.size()) {
-      seen.push_back(key[b]);
-      mv.push_back(permute_move(dims, perms + (int64_t)b * dims, widths, 0, 0));
-    }
-    which[b] = (uint8_t)i;
-  }
-  return run_block_moves(mv, which.data() + b0, num_blocks - b0, bs, d_in + b0 * bs, d_out + b0 * bs, st);
+  return run_block_moves(mv, which, num_blocks, bs, d_in, d_out, (cudaStream_t)stream);
 }
 
 int gbx_dltc_transpose(const double* d_x, const int* ids_x, double* d_y, const int* ids_y, int dim,
