@@ -48,7 +48,10 @@ int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // its waves of 152 CTAs are fuller than the blocks are real (times 0.9, what
 // the tile kernel reaches on such shapes).  Measured, tile / thin kernel:
 // 5000 x 6 x 30 12 / 23 us, 100000 x 6 x 30 78 / 54, 40000 x 24 x 64 143 /
-// 207, 100000 x 24 x 64 306 / 320, 300000 x 24 x 64 883 / 825.
+// 207, 100000 x 24 x 64 306 / 320, 300000 x 24 x 64 883 / 825.  K beyond one
+// stage only where the rows are very many: a thread walks K alone, and few
+// CTAs have too few loads in flight for that (13000 x 3 x 75 23 / 39 us, 16000
+// x 3 x 100 31 / 44, 14000 x 3 x 2000 431 / 1033).
 // Before either, variant 7: outputs of at most 16 x 16 with long K, one CTA
 // per K chunk holding the whole output (reduced in a fixed order), and 8:
 // matrix-vector shapes (one side <= 2, K > 64), one warp per output of the
@@ -63,7 +66,7 @@ int f64_variant(int m, int n, int k) {
     const int ctas = ceil_div(wide, 256);
     const double filled = (double)ctas / ((double)kSms * ceil_div(ctas, kSms));
     const double real = (double)thin / (8.0 * ceil_div(thin, 8)) * (double)k / (4.0 * ceil_div(k, 4));
-    if (filled > 0.9 * real) return rows ? 4 : 5;
+    if ((k <= kThinK || wide >= kThinMinWide) && filled > 0.9 * real) return rows ? 4 : 5;
   }
   return 0;
 }
