@@ -443,7 +443,7 @@ struct TilePlan {
 
 int64_t tile_count(const GemmProblem& q, int ts) { return (int64_t)ceil_div(q.m, ts) * ceil_div(q.n, ts); }
 
-TilePlan tile_plan(const std::vector<const GemmProblem*>& probs) {
+TilePlan tile_plan(const std::vector<const GemmProblem*>& probs, bool warp_tiles = true) {
   TilePlan t;
   int64_t n16 = 0, n8 = 0;
   int kmax = 0;
@@ -453,7 +453,8 @@ TilePlan tile_plan(const std::vector<const GemmProblem*>& probs) {
     kmax = std::max(kmax, q->k);
   }
   const int64_t waves = (n16 + kQuarters - 1) / kQuarters;
-  if (waves >= 16 || (waves >= 4 && n16 >= 0.92 * (double)(waves * kQuarters))) t.ts = 0;
+  if (!warp_tiles) t.ts = 16;
+  else if (waves >= 16 || (waves >= 4 && n16 >= 0.92 * (double)(waves * kQuarters))) t.ts = 0;
   if (t.ts == 0 || n16 >= 12 * kSms) return t;
   t.ts = 8;
   while (t.cluster < 8 && n8 * t.cluster <= kSms && ceil_div(kmax, 4) >= 48 * t.cluster) t.cluster *= 2;
@@ -477,6 +478,16 @@ void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
 
 int64_t dmma_count(const GemmProblem& q) { return tile_count(q, 8) * ceil_div(q.k, 4); }
 
+// A tile that one warp would walk long after the others of its launch are
+// done: more than twice their average DMMAs, and more than a quarter of an
+// even share of the launch.  Such problems get a launch of their own, with
+// their K shared (10000 products of 32 x 32 x 32 and one of 32 x 32 x 10^6:
+// 317 ms before, 5.1 so, 73 with 16 x 16 tiles from a work queue; with one of 32 x 32 x 10^5 32 ms, 1.1 and 8.1).
+bool outlasts(const GemmProblem& q, int64_t dmmas, int64_t tiles) {
+  const int64_t item = std::min(2, ceil_div(q.m, 8)) * std::min(2, ceil_div(q.n, 8)) * ceil_div(q.k, 4);
+  return item > 2 * dmmas / tiles && item > dmmas / kQuarters / 4;
+}
+
 // Small outputs: K chunks that give every SM four of all problems' `total_k`,
 // of at least 64.
 int small_out_chunk(int64_t total_k) { return (int)std::max<int64_t>(64, total_k / (4 * kSms) / 64 * 64); }
@@ -495,11 +506,14 @@ void gemv_ksplit(GemmProblem& q) {
 constexpr int kPlannedLeast = 96;   // about 25 us of one quarter: two reduction launches
 constexpr int kOneShotLeast = 512;  // a one-shot call also allocates the partial sums
 
-// Variant, K ranges and tile schedule of every problem; partial sums are
-// numbered from 0 in q.partial (offset + 1, 0 = none).  Returns their count.
-int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& want, TilePlan& tp) {
-  std::vector<const GemmProblem*> tiles;
-  int64_t dmmas = 0, small_k = 0;
+constexpr int kLongTiles = 1;  // variant number of tile-kernel problems with a launch of their own
+
+// Variant, K ranges and tile schedule of every problem (tp[1]: of those with
+// kLongTiles); partial sums are numbered from 0 in q.partial (offset + 1, 0 =
+// none).  Returns their count.
+int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& want, TilePlan (&tp)[2]) {
+  std::vector<const GemmProblem*> tiles, long_tiles;
+  int64_t dmmas = 0, long_dmmas = 0, small_k = 0;
   for (size_t i = 0; i < probs.size(); ++i) {
     GemmProblem& q = probs[i];
     q.pad_ = want[i] >= 0 ? want[i] : f64_variant(q.m, q.n, q.k);
@@ -509,7 +523,18 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
     }
     if (q.pad_ == 7) small_k += q.k;
   }
-  tp = tile_plan(tiles);
+  tp[0] = tile_plan(tiles);
+  if (tp[0].ts == 0) {
+    int64_t n16 = 0;
+    for (const GemmProblem* q : tiles) n16 += tile_count(*q, 16);
+    for (GemmProblem& q : probs)
+      if (q.pad_ == 0 && outlasts(q, dmmas, n16)) {
+        q.pad_ = kLongTiles;
+        long_tiles.push_back(&q);
+        long_dmmas += dmma_count(q);
+      }
+    tp[1] = tile_plan(long_tiles, false);
+  }
   // small outputs: chunks of up to 2048, shorter where all problems together
   // would leave CTAs without one
   const int chunk7 = std::min(kSmallOutChunk, small_out_chunk(small_k));
@@ -524,7 +549,9 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
     } else if (q.pad_ == 8) {
       gemv_ksplit(q);
     } else if (q.pad_ == 0) {
-      tile_ksplit(q, tp, dmmas, kPlannedLeast);
+      tile_ksplit(q, tp[0], dmmas, kPlannedLeast);
+    } else if (q.pad_ == kLongTiles) {
+      tile_ksplit(q, tp[1], long_dmmas, kPlannedLeast);
     }
     if (q.ksplit > 1) {
       q.partial = (double*)(intptr_t)(part + 1);
@@ -564,7 +591,7 @@ int64_t f64_partial_elems(const std::vector<GemmProblem>& in) {
   std::vector<GemmProblem> probs;
   for (auto& q : in)
     if (q.m > 0 && q.n > 0) probs.push_back(q);
-  TilePlan tp;
+  TilePlan tp[2];
   return f64_schedule(probs, std::vector<int>(probs.size(), -1), tp);
 }
 
@@ -588,7 +615,7 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
   }
   nprob = (int)probs.size();
   if (nprob == 0) return GBX_OK;
-  TilePlan tp;
+  TilePlan tp[2];
   const int64_t part_elems = f64_schedule(probs, want, tp);
   std::vector<int> red;
   std::vector<uint32_t> red_first;
@@ -623,7 +650,8 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
   for (auto& q : probs)
     if (q.partial) q.partial = d_partial + ((intptr_t)q.partial - 1);
   // one launch per kernel
-  for (int v : {0, 4, 5, 6, 7, 8}) {
+  for (int v : {0, kLongTiles, 4, 5, 6, 7, 8}) {
+    const TilePlan& t = tp[v == kLongTiles ? 1 : 0];
     std::vector<GemmProblem> vp;
     std::vector<int> first;
     int64_t tiles = 0;
@@ -631,7 +659,7 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
       if (q.pad_ != v) continue;
       vp.push_back(q);
       first.push_back((int)tiles);
-      tiles += f64_items(q, tp.ts);
+      tiles += f64_items(q, t.ts);
       if (tiles >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "grouped GEMM has too many work items");
     }
     if (vp.empty()) continue;
@@ -639,8 +667,8 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
     sb.variant = v;
     sb.nprob = (int)vp.size();
     sb.total_tiles = (int)tiles;
-    sb.ts = tp.ts;
-    sb.cluster = tp.cluster;
+    sb.ts = t.ts;
+    sb.cluster = t.cluster;
     GBX_TRY(alloc((void**)&sb.d_probs, sizeof(GemmProblem) * vp.size()));
     GBX_TRY(alloc((void**)&sb.d_first, sizeof(int) * vp.size()));
     GBX_TRY(copy(sb.d_probs, vp.data(), sizeof(GemmProblem) * vp.size()));
@@ -700,6 +728,7 @@ int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first,
   const int grid = std::min(tiles, kSms * 8);
   switch (v) {
     case 0:
+    case kLongTiles:
       return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8> : tp.ts ? tile_gemm_f64_kernel<16> : tile_gemm_f64_kernel<0>,
                           tp, tiles, st, probs, nprob, first);
     case 4: return launch(thin_gemm_f64_kernel<true>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
