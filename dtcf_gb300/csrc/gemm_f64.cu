@@ -435,6 +435,8 @@ namespace {
 // 16 x 16).  While those leave fewer than two CTAs per SM, clusters share a
 // tile's K steps, at least six for every warp (64 x 64 x 432: 10.3 us without,
 // 8.3 with four; 192 x 192 x 192, 576 tiles: 17.2 without, 18.7 with two).
+// Work that fills every quarter for longer than K ranges cost takes those
+// alone: single CTAs spread evenly, clusters of eight do not (below).
 // 64 x 48 x 96 takes 3.9 us on the GPU so (one 64 x 64 tile: 125), 1021 x 765
 // x 1531 2.29 ms, 1.045 TFLOP/s (64 x 64 tiles: 2.36 ms).
 struct TilePlan {
@@ -443,46 +445,71 @@ struct TilePlan {
 
 int64_t tile_count(const GemmProblem& q, int ts) { return (int64_t)ceil_div(q.m, ts) * ceil_div(q.n, ts); }
 
-TilePlan tile_plan(const std::vector<const GemmProblem*>& probs, bool warp_tiles = true) {
+int64_t dmma_count(const GemmProblem& q) { return tile_count(q, 8) * ceil_div(q.k, 4); }
+
+// least: DMMAs of a warp that K ranges have to be worth (tile_ksplit).
+TilePlan tile_plan(const std::vector<const GemmProblem*>& probs, int least, bool warp_tiles = true) {
   TilePlan t;
-  int64_t n16 = 0, n8 = 0;
+  int64_t n16 = 0, n8 = 0, dmmas = 0;
   int kmax = 0;
   for (const GemmProblem* q : probs) {
     n16 += tile_count(*q, 16);
     n8 += tile_count(*q, 8);
     kmax = std::max(kmax, q->k);
+    dmmas += dmma_count(*q);
   }
   const int64_t waves = (n16 + kQuarters - 1) / kQuarters;
   if (!warp_tiles) t.ts = 16;
   else if (waves >= 16 || (waves >= 4 && n16 >= 0.92 * (double)(waves * kQuarters))) t.ts = 0;
   if (t.ts == 0 || n16 >= 12 * kSms) return t;
   t.ts = 8;
+  if (dmmas / kQuarters >= 2 * least) return t;
   while (t.cluster < 8 && n8 * t.cluster <= kSms && ceil_div(kmax, 4) >= 48 * t.cluster) t.cluster *= 2;
   return t;
 }
 
+// Clusters that get SMs of their own side by side: sixteen of eight CTAs did
+// not (32 x 32 x 20000: 94 us, fifteen tiles of 17 x 40 half as long per
+// product).
+int clusters_apart(int cluster) { return cluster == 8 ? 15 : cluster == 4 ? 36 : kSms / cluster; }
+
 // K ranges of one problem: cut where one CTA's share of a tile would outlast
 // an even share of the whole launch (of `dmmas` DMMAs) and `least` DMMAs per
 // warp, the cost that the partial sums and their reduction have to be worth.
+// A problem that is most of its launch also counts how often its clusters
+// come round to an SM, and is cut to even that out (planned, tiles cut by
+// their share alone / so: 32 x 32 x 10^6 4422 / 1872 us, 100 x 100 x 50000 1774 /
+// 1041, 110 x 110 x 2000 74 / 53).
 void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
   const int steps = ceil_div(q.k, 4), workers = 4 * t.cluster;
   if (t.ts == 0) return;
   const int64_t blocks = t.ts == 16 ? std::min(2, ceil_div(q.m, 8)) * std::min(2, ceil_div(q.n, 8)) : 1;
   const int64_t item = blocks * ceil_div(steps, workers);
   const int64_t share = std::max<int64_t>(dmmas / kQuarters, least);
-  int64_t ks = std::max<int64_t>(1, std::min<int64_t>((item + share / 2) / share, steps / (8 * workers)));
+  const int64_t most = std::max(1, steps / (8 * workers));
+  int64_t ks = std::max<int64_t>(1, std::min<int64_t>((item + share / 2) / share, most));
+  if (2 * dmma_count(q) >= dmmas) {
+    // the DMMAs of the SM quarter with the most
+    const auto load = [&](int64_t k) {
+      return ceil_div(tile_count(q, t.ts) * k, clusters_apart(t.cluster)) * blocks * ceil_div(ceil_div(steps, k), workers);
+    };
+    if (2 * load(1) >= 3 * share) {
+      const int64_t to = std::min(most, 8 * std::max<int64_t>(ks, 2));
+      int64_t best = load(ks);
+      for (int64_t k = ks; k <= to; ++k) best = std::min(best, load(k));
+      while (ks < to && 20 * load(ks) > 21 * best) ++ks;
+    }
+  }
   const int chunk = 4 * ceil_div(steps, ks);
   q.ksplit = std::max(1, ceil_div(q.k, std::max(chunk, 4)));
   q.kchunk = std::max(chunk, 4);
 }
 
-int64_t dmma_count(const GemmProblem& q) { return tile_count(q, 8) * ceil_div(q.k, 4); }
-
 // A tile that one warp would walk long after the others of its launch are
 // done: more than twice their average DMMAs, and more than a quarter of an
 // even share of the launch.  Such problems get a launch of their own, with
 // their K shared (10000 products of 32 x 32 x 32 and one of 32 x 32 x 10^6:
-// 317 ms before, 5.1 so, 73 with 16 x 16 tiles from a work queue; with one of 32 x 32 x 10^5 32 ms, 1.1 and 8.1).
+// 317 ms in one launch, 2.5 so; with one of 32 x 32 x 10^5 32 and 0.85).
 bool outlasts(const GemmProblem& q, int64_t dmmas, int64_t tiles) {
   const int64_t item = std::min(2, ceil_div(q.m, 8)) * std::min(2, ceil_div(q.n, 8)) * ceil_div(q.k, 4);
   return item > 2 * dmmas / tiles && item > dmmas / kQuarters / 4;
@@ -523,7 +550,7 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
     }
     if (q.pad_ == 7) small_k += q.k;
   }
-  tp[0] = tile_plan(tiles);
+  tp[0] = tile_plan(tiles, kPlannedLeast);
   if (tp[0].ts == 0) {
     int64_t n16 = 0;
     for (const GemmProblem* q : tiles) n16 += tile_count(*q, 16);
@@ -533,7 +560,7 @@ int64_t f64_schedule(std::vector<GemmProblem>& probs, const std::vector<int>& wa
         long_tiles.push_back(&q);
         long_dmmas += dmma_count(q);
       }
-    tp[1] = tile_plan(long_tiles, false);
+    tp[1] = tile_plan(long_tiles, kPlannedLeast, false);
   }
   // small outputs: chunks of up to 2048, shorter where all problems together
   // would leave CTAs without one
@@ -801,7 +828,7 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
   q.ksplit = 1;
   q.kchunk = std::max(q.k, 4);
   q.partial = nullptr;
-  const TilePlan tp = tile_plan({&q});
+  const TilePlan tp = tile_plan({&q}, kOneShotLeast);
   double* own = nullptr;
   if (q.pad_ == 0) {
     tile_ksplit(q, tp, dmma_count(q), kOneShotLeast);
