@@ -493,8 +493,11 @@ __device__ __forceinline__ void direct_elements(const DirSmem& sm, uint32_t e0, 
 // other one is (mostly) a broadcast.  Items of at most kThr elements (the
 // planner cuts small outputs so, see direct_step) take one element per
 // thread, warps beyond the end none, and several contracted indices at once.
-// Every output element is the same sequence of fused multiply-adds either
-// way.
+// A warp whose kDirPer elements do not all lie inside a larger item takes
+// those that do one after another in the same way: lanes beyond the end would
+// issue their multiply-adds all the same (outputs of 16 x 16 x 48 x 48 in
+// items of 896: 46 us with all kDirPer, 24 so).  Every output element is the
+// same sequence of fused multiply-adds either way.
 // kStore: C = alpha * sum (the items cover every element of C, which holds
 // no earlier value), else C += alpha * sum -- a template parameter, so that
 // the accumulating kernel's C loads are scheduled as without the choice.
@@ -518,8 +521,16 @@ __device__ __forceinline__ void direct_body(const DirItem* __restrict__ items, i
       continue;
     }
 #pragma unroll 1
-    for (int pass = 0; pass < kPasses; ++pass)
-      direct_elements<kThr, kDirPer, 1, kCoh, kStore>(sm, (uint32_t)(pass * kThr * kDirPer) + threadIdx.x, A, B, C, alpha);
+    for (int pass = 0; pass < kPasses; ++pass) {
+      const uint32_t e0 = (uint32_t)(pass * kThr * kDirPer) + threadIdx.x, w0 = e0 & ~31u;
+      if (w0 + (kDirPer - 1) * kThr < it.n) {
+        direct_elements<kThr, kDirPer, 1, kCoh, kStore>(sm, e0, A, B, C, alpha);
+        continue;
+      }
+#pragma unroll 1
+      for (uint32_t k = 0; k < kDirPer * kThr && w0 + k < it.n; k += kThr)
+        direct_elements<kThr, 1, 8, kCoh, kStore>(sm, e0 + k, A, B, C, alpha);
+    }
   }
 }
 

@@ -297,10 +297,13 @@ ContractionPlan::~ContractionPlan() {
 
 // Output elements of a direct work item: enough items for four to an SM, at
 // least a warp for each of an SM's quarters (27648 outputs of 64 products:
-// 33 us in 14 items of 2048, 10 in 216 of 128).
+// 33 us in 14 items of 2048, 10 in 216 of 128).  Between an element to each
+// of a CTA's threads and the largest item there is nothing to gain: outputs of
+// 16 x 16 x 48 x 48, 16 contracted, in items of 896 / 512 24.0 / 21.0 us.
 static int64_t direct_step(int64_t outputs) {
   const int64_t even = outputs / (4 * 152) / 128 * 128;
-  return std::max<int64_t>(128, std::min<int64_t>(kDirItemElems, even));
+  if (even > kDirItemElems / 2) return kDirItemElems;
+  return std::max<int64_t>(128, std::min<int64_t>(kDirItemElems / 4, even));
 }
 
 bool find_contraction_pair(const TensorLayout& A, const TensorLayout& B, const std::vector<std::string>& la,
