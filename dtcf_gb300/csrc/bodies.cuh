@@ -254,13 +254,129 @@ struct FsSmem {
   FsTerm terms[kFsMaxTerms];
 };
 
-// One CTA per work item (grid-stride over items).  Threads hold kFsPer
-// destination elements each, in destination order, and add the terms one
-// after the other: rows of slabs that are contiguous in the source's own
-// order are read directly (coalesced); slabs stored transposed are first
-// copied into shared memory in source order and read back transposed, so
-// both sides stay coalesced; anything else is gathered.  Stores are
-// coalesced along the destination.
+// One work item.  Threads hold kPer destination elements each, in destination
+// order, and add the terms one after the other: rows of slabs that are
+// contiguous in the source's own order are read directly (coalesced); slabs
+// stored transposed are first copied into shared memory in source order and
+// read back transposed, so both sides stay coalesced; anything else is
+// gathered.  Stores are coalesced along the destination.  kPer is what the
+// item needs: a slot past its end loads and adds like the others (the
+// residual's sum at o = 10, v = 40 with kFsPer slots to every item: 26.6 us
+// in items of 2048, 32.8 of 512, 16.2 so of 1024; o = 8, v = 32: 24.6 / 20.5 /
+// 12.3).
+template <bool kCoh, int kPer>
+__device__ __forceinline__ void fused_item(const double* __restrict__ scale, double* __restrict__ out, FsSmem& sm) {
+  const FsItem& it = sm.item;
+  const uint32_t E = it.fE.d, ea = it.fea.d, eb = it.feb.d, O1 = it.fo1.d;
+  double acc[kPer];
+  // element k of this thread: e = tid + k * threads (lanes past the end
+  // repeat the last element: valid addresses, no store); the outer indices
+  // of its slab, packed as o0 << 16 | o1, and its index q within the slab
+  uint32_t oo[kPer], qk[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    acc[k] = 0.0;
+    const uint32_t f = it.f0 + min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
+    const uint32_t sg = it.fE.div(f);
+    const uint32_t o0 = it.fo1.div(sg);
+    qk[k] = f - sg * E;
+    oo[k] = (o0 << 16) | (sg - o0 * O1);
+  }
+#define FS_ELEM(k, o0, o1, q)      \
+  const uint32_t o0 = oo[k] >> 16;  \
+  const uint32_t o1 = oo[k] & 0xFFFFu; \
+  const uint32_t q = qk[k]
+  // offsets inside a source tile are 32-bit (a tile holds fewer than 2^31
+  // elements): one multiply-add each instead of 64-bit products
+  auto gather = [&](const FsTerm& tm, double* x) {
+    const double* __restrict__ p = sm.base[tm.slot] + tm.off;
+    const uint32_t so0 = (uint32_t)tm.so0, so1 = (uint32_t)tm.so1;
+    if (tm.mode == 1 && it.whole) {
+      const uint32_t pa = ea | 1u, sp = eb * pa;
+      const uint32_t s_first = it.fE.div(it.f0);
+      __syncthreads();  // earlier reads of stage are done
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t e = min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
+        const uint32_t sl = it.fE.div(e);
+        const uint32_t sg = s_first + sl, o0 = it.fo1.div(sg), o1 = sg - o0 * O1;
+        x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + (e - sl * E)));
+      }
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t e = threadIdx.x + k * kFsThreads;
+        if (e < it.n) {
+          const uint32_t sl = it.fE.div(e);
+          const uint32_t qq = e - sl * E;  // source order within the slab: b * ea + a
+          const uint32_t b = it.fea.div(qq);
+          sm.stage[sl * sp + b * pa + (qq - b * ea)] = x[k];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t e = min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
+        const uint32_t sl = it.fE.div(e), q = qk[k];
+        const uint32_t a = it.feb.div(q);
+        x[k] = sm.stage[sl * sp + (q - a * eb) * pa + a];
+      }
+    } else if (tm.mode == 0) {
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        FS_ELEM(k, o0, o1, q);
+        x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + q));
+      }
+    } else {
+      const uint32_t sa = (uint32_t)tm.sa, sb = (uint32_t)tm.sb;
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        FS_ELEM(k, o0, o1, q);
+        const uint32_t a = it.feb.div(q);
+        x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + a * sa + (q - a * eb) * sb));
+      }
+    }
+  };
+  // FP64 instructions are the scarce resource here (the FP64 pipe issues
+  // about 1.6 per clock per SM, fewer than the elements HBM delivers): the
+  // first term of a +-1 coefficient is a sign flip on the bits (0 + c x
+  // with -0 turned into +0), every other term one fused multiply-add --
+  // the separately rounded product and sum whenever c x is exact, as it is
+  // for c = +-2^k
+  uint32_t t0 = 0;
+  if (it.nterm > 0) {
+    const unsigned long long cbits = (unsigned long long)__double_as_longlong(sm.terms[0].coef);
+    if ((cbits & 0x7FFFFFFFFFFFFFFFull) == 0x3FF0000000000000ull) {
+      double x[kPer];
+      gather(sm.terms[0], x);
+      const unsigned long long sign = cbits & 0x8000000000000000ull;
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(x[k]) ^ sign;
+        acc[k] = __longlong_as_double((long long)(b == 0x8000000000000000ull ? 0ull : b));
+      }
+      t0 = 1;
+    }
+  }
+  for (uint32_t t = t0; t < it.nterm; ++t) {
+    double x[kPer];
+    gather(sm.terms[t], x);
+    const double c = sm.terms[t].coef;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) acc[k] = __fma_rn(c, x[k], acc[k]);
+  }
+#undef FS_ELEM
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const uint32_t e = threadIdx.x + k * kFsThreads;
+    if (e < it.n) {
+      double v = acc[k];
+      if (scale) v = __dmul_rn(v, ldin<kCoh>(scale + it.dst + e));
+      out[it.dst + e] = v;
+    }
+  }
+}
+
+// One CTA per work item (grid-stride over items).
 template <bool kCoh>
 __device__ __forceinline__ void fused_sum_body(const FsItem* __restrict__ items, int nitems,
                                                const FsTerm* __restrict__ terms, const FsSrc& src,
@@ -274,116 +390,13 @@ __device__ __forceinline__ void fused_sum_body(const FsItem* __restrict__ items,
     __syncthreads();  // the previous item is finished with the item, its terms and stage
     if (threadIdx.x == 0) sm.item = items[i];
     __syncthreads();
-    const FsItem& it = sm.item;
-    if (threadIdx.x < it.nterm) sm.terms[threadIdx.x] = terms[it.term0 + threadIdx.x];
+    if (threadIdx.x < sm.item.nterm) sm.terms[threadIdx.x] = terms[sm.item.term0 + threadIdx.x];
     __syncthreads();
-    const uint32_t E = it.fE.d, ea = it.fea.d, eb = it.feb.d, O1 = it.fo1.d;
-    double acc[kFsPer];
-    // element k of this thread: e = tid + k * threads (lanes past the end
-    // repeat the last element: valid addresses, no store); the outer indices
-    // of its slab, packed as o0 << 16 | o1, and its index q within the slab
-    uint32_t oo[kFsPer], qk[kFsPer];
-#pragma unroll
-    for (int k = 0; k < kFsPer; ++k) {
-      acc[k] = 0.0;
-      const uint32_t f = it.f0 + min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
-      const uint32_t sg = it.fE.div(f);
-      const uint32_t o0 = it.fo1.div(sg);
-      qk[k] = f - sg * E;
-      oo[k] = (o0 << 16) | (sg - o0 * O1);
-    }
-#define FS_ELEM(k, o0, o1, q)      \
-  const uint32_t o0 = oo[k] >> 16;  \
-  const uint32_t o1 = oo[k] & 0xFFFFu; \
-  const uint32_t q = qk[k]
-    // offsets inside a source tile are 32-bit (a tile holds fewer than 2^31
-    // elements): one multiply-add each instead of 64-bit products
-    auto gather = [&](const FsTerm& tm, double* x) {
-      const double* __restrict__ p = sm.base[tm.slot] + tm.off;
-      const uint32_t so0 = (uint32_t)tm.so0, so1 = (uint32_t)tm.so1;
-      if (tm.mode == 1 && it.whole) {
-        const uint32_t pa = ea | 1u, sp = eb * pa;
-        const uint32_t s_first = it.fE.div(it.f0);
-        __syncthreads();  // earlier reads of stage are done
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          const uint32_t e = min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
-          const uint32_t sl = it.fE.div(e);
-          const uint32_t sg = s_first + sl, o0 = it.fo1.div(sg), o1 = sg - o0 * O1;
-          x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + (e - sl * E)));
-        }
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          const uint32_t e = threadIdx.x + k * kFsThreads;
-          if (e < it.n) {
-            const uint32_t sl = it.fE.div(e);
-            const uint32_t qq = e - sl * E;  // source order within the slab: b * ea + a
-            const uint32_t b = it.fea.div(qq);
-            sm.stage[sl * sp + b * pa + (qq - b * ea)] = x[k];
-          }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          const uint32_t e = min((uint32_t)(threadIdx.x + k * kFsThreads), it.n - 1);
-          const uint32_t sl = it.fE.div(e), q = qk[k];
-          const uint32_t a = it.feb.div(q);
-          x[k] = sm.stage[sl * sp + (q - a * eb) * pa + a];
-        }
-      } else if (tm.mode == 0) {
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          FS_ELEM(k, o0, o1, q);
-          x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + q));
-        }
-      } else {
-        const uint32_t sa = (uint32_t)tm.sa, sb = (uint32_t)tm.sb;
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          FS_ELEM(k, o0, o1, q);
-          const uint32_t a = it.feb.div(q);
-          x[k] = ldin<kCoh>(p + (o0 * so0 + o1 * so1 + a * sa + (q - a * eb) * sb));
-        }
-      }
-    };
-    // FP64 instructions are the scarce resource here (the FP64 pipe issues
-    // about 1.6 per clock per SM, fewer than the elements HBM delivers): the
-    // first term of a +-1 coefficient is a sign flip on the bits (0 + c x
-    // with -0 turned into +0), every other term one fused multiply-add --
-    // the separately rounded product and sum whenever c x is exact, as it is
-    // for c = +-2^k
-    uint32_t t0 = 0;
-    if (it.nterm > 0) {
-      const unsigned long long cbits = (unsigned long long)__double_as_longlong(sm.terms[0].coef);
-      if ((cbits & 0x7FFFFFFFFFFFFFFFull) == 0x3FF0000000000000ull) {
-        double x[kFsPer];
-        gather(sm.terms[0], x);
-        const unsigned long long sign = cbits & 0x8000000000000000ull;
-#pragma unroll
-        for (int k = 0; k < kFsPer; ++k) {
-          const unsigned long long b = (unsigned long long)__double_as_longlong(x[k]) ^ sign;
-          acc[k] = __longlong_as_double((long long)(b == 0x8000000000000000ull ? 0ull : b));
-        }
-        t0 = 1;
-      }
-    }
-    for (uint32_t t = t0; t < it.nterm; ++t) {
-      double x[kFsPer];
-      gather(sm.terms[t], x);
-      const double c = sm.terms[t].coef;
-#pragma unroll
-      for (int k = 0; k < kFsPer; ++k) acc[k] = __fma_rn(c, x[k], acc[k]);
-    }
-#undef FS_ELEM
-#pragma unroll
-    for (int k = 0; k < kFsPer; ++k) {
-      const uint32_t e = threadIdx.x + k * kFsThreads;
-      if (e < it.n) {
-        double v = acc[k];
-        if (scale) v = __dmul_rn(v, ldin<kCoh>(scale + it.dst + e));
-        out[it.dst + e] = v;
-      }
-    }
+    const uint32_t n = sm.item.n;
+    if (n > 4 * kFsThreads) fused_item<kCoh, kFsPer>(scale, out, sm);
+    else if (n > 2 * kFsThreads) fused_item<kCoh, 4>(scale, out, sm);
+    else if (n > kFsThreads) fused_item<kCoh, 2>(scale, out, sm);
+    else fused_item<kCoh, 1>(scale, out, sm);
   }
 }
 

@@ -1087,10 +1087,12 @@ int plan_fused_sum(const TensorLayout& C, const std::vector<std::string>& lc, co
   auto p = std::make_unique<FusedSumPlan>();
   p->C = C;
   p->nslots = nslots;
-  // elements of an item: smaller ones where the largest would leave SMs idle
+  // elements of an item: half, a quarter or an eighth of the largest (what a
+  // CTA's threads hold evenly) where larger ones were fewer than the SMs
   int64_t outputs = 0;
   for (const Coords& c : C.tiles) outputs += C.tile_size(c.data());
-  const int64_t most = std::max<int64_t>(256, std::min<int64_t>(kFsItemElems, outputs / (2 * 152) / 256 * 256));
+  int64_t most = 256;
+  while (most < kFsItemElems && outputs >= 2 * 152 * most) most *= 2;
   std::vector<int> order(C.tiles.size());
   for (size_t t = 0; t < order.size(); ++t) order[t] = (int)t;
   if (r == 4) {
