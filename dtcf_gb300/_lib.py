@@ -68,6 +68,7 @@ SIGNATURES = {
     "gbx_cc_time_gemm": (_i, [_p, _i, _i, _p, _p, _p, _p, _p]),
     "gbx_cc_contraction_error": (_i, [_p, _i, _p, _p, _p]),
     "gbx_cc_program_info": (_i, [_p, ctypes.POINTER(_i), ctypes.POINTER(_i), ctypes.POINTER(_i)]),
+    "gbx_cc_branches": (_i, [_p, _ip]),
     "gbx_cc_program_selftest": (_i, [ctypes.c_longlong, _p]),
     "gbx_dltc_mul_orders": (_i, [_i, _p, _i, _p, _p, _p, _p, _p, _p, _p]),
     "gbx_dltc_task_mul": (_i, [_d, _i, _p, _p, _i, _p, _p, _i, _p, _p, _p, _p, _p, _i, _p]),
@@ -77,6 +78,7 @@ SIGNATURES = {
     "gbx_dltc_program_tensor": (_i, [_p, _i, _p, _p]),
     "gbx_dltc_program_run": (_i, [_p, _i, _i, _p]),
     "gbx_dltc_program_check": (_i, [_p]),
+    "gbx_dltc_program_branches": (_i, [_p, _ip]),
     "gbx_dltc_program_flops": (_d, [_p]),
     "gbx_dltc_program_destroy": (_i, [_p]),
 }

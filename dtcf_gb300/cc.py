@@ -155,6 +155,12 @@ class Job:
         check(lib().gbx_cc_program_info(self.handle, *[ctypes.byref(x) for x in v]))
         return dict(zip(("records", "levels", "launches"), (x.value for x in v)))
 
+    def branches(self):
+        """Branches of the iteration's graph: 1 for a chain, 0 without a graph."""
+        n = ctypes.c_int()
+        check(lib().gbx_cc_branches(self.handle, ctypes.byref(n)))
+        return n.value
+
     def close(self):
         if getattr(self, "handle", None) and self.handle.value:
             lib().gbx_cc_destroy(self.handle)

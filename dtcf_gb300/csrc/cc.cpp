@@ -133,6 +133,8 @@ struct gbx_cc_job {
 
   bool persistent() const { return cfg.use_graph == 2; }
   bool branched = false;  // use_graph 1: independent steps are branches of the graph
+  int branches = 0;       // of the captured graph (1: a chain)
+  std::string chain_why;  // the failure that made a chain of branches
   using Steps = std::vector<std::function<int(cudaStream_t)>>;
   int record_steps(const Steps& todo, ProgRecorder** rec);
   int record_program();
@@ -913,16 +915,18 @@ int gbx_cc_capture(gbx_cc_job* job) {
       if (rrc == GBX_OK) rrc = frc;
     }
     job->branched = rrc == GBX_OK;  // else the chain, which needs no record
+    if (rrc != GBX_OK) job->chain_why = gbx_last_error();
   }
   cudaStream_t cap;
   GBX_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   GBX_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
   int rc = GBX_OK;
   if (job->prog) {
-    rc = prog_run(*job->prog, cap);
+    rc = prog_run(*job->prog, cap, &job->branches);
   } else if (job->branched) {
-    rc = capture_branches(cap, deps, [&](int i, cudaStream_t st) { return parts[i](st); });
+    rc = capture_branches(cap, deps, [&](int i, cudaStream_t st) { return parts[i](st); }, &job->branches);
   } else {
+    job->branches = 1;
     for (auto& s : job->steps) {
       rc = s(cap);
       if (rc != GBX_OK) break;
@@ -977,6 +981,14 @@ int gbx_cc_program_info(gbx_cc_job* job, int* records, int* levels, int* launche
   if (records) *records = s.records;
   if (levels) *levels = s.levels;
   if (launches) *launches = s.launches;
+  return GBX_OK;
+}
+
+int gbx_cc_branches(gbx_cc_job* job, int* branches) {
+  if (!job || !branches) return fail(GBX_EINVAL, "null argument");
+  GBX_TRY(gbx_cc_capture(job));
+  *branches = job->branches;
+  if (!job->chain_why.empty()) set_error("%s", job->chain_why.c_str());
   return GBX_OK;
 }
 

@@ -715,6 +715,8 @@ struct gbx_dltc_program {
   // the whole table as a graph, expressions that do not depend on one
   // another as branches (where they have workspaces of their own)
   cudaGraphExec_t exec = nullptr;
+  int branches = 0;       // of the graph (0: none)
+  std::string chain_why;  // the failure that left the table without one
   double flops = 0.0;
 
   int run_op(int i, cudaStream_t st, int stages = 3) {
@@ -789,7 +791,8 @@ int gbx_dltc_program::capture() {
   cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeRelaxed);
   int rc = e == cudaSuccess ? GBX_OK : cuda_fail(e, "cudaStreamBeginCapture", __FILE__, __LINE__);
   if (rc == GBX_OK) {
-    rc = capture_branches(cap, deps, [&](int k, cudaStream_t st) { return run_op(steps[k].op, st, steps[k].stages); });
+    rc = capture_branches(cap, deps, [&](int k, cudaStream_t st) { return run_op(steps[k].op, st, steps[k].stages); },
+                          &branches);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(cap, &g);
     if (rc == GBX_OK && e != cudaSuccess) rc = cuda_fail(e, "cudaStreamEndCapture", __FILE__, __LINE__);
@@ -929,7 +932,11 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
       GBX_TRY(p->gemm.back()->build({g}));
     }
   }
-  if (branched && p->capture() != GBX_OK) cudaGetLastError();  // the table then runs kernel by kernel
+  if (branched && p->capture() != GBX_OK) {  // the table then runs kernel by kernel
+    cudaGetLastError();
+    p->branches = 0;
+    p->chain_why = gbx_last_error();
+  }
   *out = p.release();
   return GBX_OK;
 }
@@ -968,6 +975,13 @@ int gbx_dltc_program_check(gbx_dltc_program* p) {
     const int err = split_plan_error(sp);
     if (err != 0) return fail(GBX_ETIMEOUT, "split GEMM: a bounded device wait ran out (stage %d)", err);
   }
+  return GBX_OK;
+}
+
+int gbx_dltc_program_branches(const gbx_dltc_program* p, int* branches) {
+  if (!p || !branches) return fail(GBX_EINVAL, "null argument");
+  *branches = p->branches;
+  if (!p->chain_why.empty()) set_error("%s", p->chain_why.c_str());
   return GBX_OK;
 }
 

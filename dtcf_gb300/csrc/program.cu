@@ -658,7 +658,7 @@ void reduce_deps(const std::vector<std::set<int>>& direct, std::vector<std::vect
 }
 
 int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps,
-                     const std::function<int(int, cudaStream_t)>& step) {
+                     const std::function<int(int, cudaStream_t)>& step, int* branches) {
   struct Streams {
     std::vector<cudaStream_t> s;
     std::vector<cudaEvent_t> e;
@@ -701,6 +701,7 @@ int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps
     at[i] = q;
   }
   for (size_t q = 1; q < use.s.size(); ++q) GBX_CUDA(cudaStreamWaitEvent(cap, done[last[q]], 0));
+  if (branches) *branches = (int)use.s.size();
   return GBX_OK;
 }
 
@@ -709,7 +710,7 @@ int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps
 // are branches of the graph that st captures (one after another / so, per
 // iteration: CCSD at o = 12, v = 40, FP64 565 / 507 us; o = 12, v = 36 at 5
 // slices 318 / 287; o = 32, v = 160 1539 / 1479; o = 48, v = 240 5849 / 5739).
-int prog_run(const Program& P, cudaStream_t st) {
+int prog_run(const Program& P, cudaStream_t st, int* branches) {
   GBX_CUDA(cudaMemsetAsync(P.d_counters, 0, sizeof(uint32_t) * P.counter_words, st));
   return capture_branches(st, P.op_deps, [&](int i, cudaStream_t q) {
     const Program::Op& op = P.ops[i];
@@ -726,7 +727,7 @@ int prog_run(const Program& P, cudaStream_t st) {
     L.nrec = m.nrec;
     L.total = m.total;
     return launch(prog_mem_kernel, (unsigned)m.grid, kProgThreads, q, L);
-  });
+  }, branches);
 }
 
 void prog_set_wait_limit(Program& p, long long cycles) { p.limit = cycles > 0 ? cycles : kProgWaitCycles; }

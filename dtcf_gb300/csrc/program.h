@@ -221,10 +221,11 @@ void reduce_deps(const std::vector<std::set<int>>& direct, std::vector<std::vect
 // Captures steps as branches of the graph that cap captures: each on a stream
 // that ends in a step it waits for, or on one of its own, with events for its
 // other dependencies.  The streams and events serve the capture alone.
+// branches (optional): the streams it took.
 int capture_branches(cudaStream_t cap, const std::vector<std::vector<int>>& deps,
-                     const std::function<int(int, cudaStream_t)>& step);
+                     const std::function<int(int, cudaStream_t)>& step, int* branches = nullptr);
 // Enqueues one run of the program on st.
-int prog_run(const Program& p, cudaStream_t st);
+int prog_run(const Program& p, cudaStream_t st, int* branches = nullptr);
 // Bound on every dependency wait of the program's memory launches (clock
 // cycles; default about one second).
 void prog_set_wait_limit(Program& p, long long cycles);

@@ -135,6 +135,12 @@ class Program:
     def check(self):
         check(lib().gbx_dltc_program_check(self.handle))
 
+    def branches(self):
+        """Branches of the whole table's graph, 0 where it runs kernel by kernel."""
+        n = ctypes.c_int()
+        check(lib().gbx_dltc_program_branches(self.handle, ctypes.byref(n)))
+        return n.value
+
     @property
     def flops(self):
         return lib().gbx_dltc_program_flops(self.handle)

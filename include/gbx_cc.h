@@ -140,6 +140,10 @@ GBX_API int gbx_cc_contraction_error(gbx_cc_job* job, int contraction, double* r
  * (DLTC/ccd-t2.cc:97-134) -- a task pool per dependency layer, barriers
  * between layers -- with a device-side work queue. */
 GBX_API int gbx_cc_program_info(gbx_cc_job* job, int* records, int* levels, int* launches);
+/* Branches of the iteration's graph (captured on first use): the streams its
+ * capture took, 1 for a chain, 0 without a graph.  Where a failure made a
+ * chain of it, gbx_last_error() then tells which. */
+GBX_API int gbx_cc_branches(gbx_cc_job* job, int* branches);
 /* Self-test of the persistent program's bounded dependency wait: runs a
  * two-record launch whose one wait can never be met, bounded by
  * limit_cycles; returns GBX_ETIMEOUT when the wait ran out as it must (the

@@ -104,6 +104,10 @@ GBX_API int gbx_dltc_program_tensor(gbx_dltc_program* p, int tensor, double** d_
 GBX_API int gbx_dltc_program_run(gbx_dltc_program* p, int first, int count, void* stream);
 /* GBX_ETIMEOUT if a bounded device wait of the split engine ran out (syncs). */
 GBX_API int gbx_dltc_program_check(gbx_dltc_program* p);
+/* Branches of the whole table's graph (the streams its capture took), 0 where
+ * it runs kernel by kernel; where a failure is the reason, gbx_last_error()
+ * then tells which. */
+GBX_API int gbx_dltc_program_branches(const gbx_dltc_program* p, int* branches);
 /* 2 * M * N * K summed over the Multiplications. */
 GBX_API double gbx_dltc_program_flops(const gbx_dltc_program* p);
 GBX_API int gbx_dltc_program_destroy(gbx_dltc_program* p);
