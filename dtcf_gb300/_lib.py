@@ -14,6 +14,7 @@ _ip = ctypes.POINTER(ctypes.c_int)
 SIGNATURES = {
     "gbx_last_error": (ctypes.c_char_p, []),
     "gbx_version": (ctypes.c_char_p, []),
+    "gbx_alloc_budget": (_i, [ctypes.c_int64]),
     "gbx_transpose": (_i, [_p, _p, _p, _i, _p, _p]),
     "gbx_transpose_blocks": (_i, [_p, _p, _i, _p, _i, _p, _p]),
     "gbx_dltc_transpose": (_i, [_p, _p, _p, _p, _i, _p, _p]),

@@ -132,6 +132,7 @@ struct gbx_cc_job {
   ProgramPtr prog;
 
   bool persistent() const { return cfg.use_graph == 2; }
+  bool chain = false;     // one region for all contractions, whatever use_graph says
   bool branched = false;  // use_graph 1: independent steps are branches of the graph
   int branches = 0;       // of the captured graph (1: a chain)
   std::string chain_why;  // the failure that made a chain of branches
@@ -734,8 +735,8 @@ int gbx_cc_job::materialize(cudaStream_t st) {
     widest = std::max(widest, w);
     scratch_bytes = std::max(scratch_bytes, sc);
   }
-  branched = cfg.use_graph == 1 && side_by_side(1, (double)arena_bytes);
-  if (!side_by_side(cfg.use_graph, (double)arena_bytes)) {
+  branched = cfg.use_graph == 1 && !chain && side_by_side(1, (double)arena_bytes);
+  if (chain || !side_by_side(cfg.use_graph, (double)arena_bytes)) {
     arena_bytes = widest;
     arena_off.assign(cplans.size(), 0);
   }
@@ -844,11 +845,21 @@ int gbx_cc_create(const gbx_cc_config* cfg, void* stream, gbx_cc_job** out) {
   if (!out) return fail(GBX_EINVAL, "null argument");
   *out = nullptr;
   std::unique_ptr<gbx_cc_job> job;
-  GBX_TRY(cc_setup(cfg, job));
-  {
+  const auto build = [&] {
     AllocAccount acct(&job->account);
-    GBX_TRY(job->materialize(0));
+    return job->materialize(0);
+  };
+  GBX_TRY(cc_setup(cfg, job));
+  int rc = build();
+  if (rc == GBX_ENOMEM && job->branched) {
+    // regions of their own did not fit: one for all contractions, in a chain
+    const std::string why = gbx_last_error();
+    GBX_TRY(cc_setup(cfg, job));
+    job->chain = true;
+    job->chain_why = why;
+    rc = build();
   }
+  GBX_TRY(rc);
   job->nenergies = 1;
   (void)stream;
   *out = job.release();

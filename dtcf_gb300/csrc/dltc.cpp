@@ -855,12 +855,11 @@ int gbx_dltc_table(int which, gbx_dltc_expr* exprs, int* nexpr, int* types, int*
   return GBX_OK;
 }
 
-int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_dltc_program** out) {
-  if (!out) return fail(GBX_EINVAL, "out is NULL");
-  *out = nullptr;
-  GBX_TRY(check_dims(dims));
-  if (mode != GBX_MODE_FP64 && mode != GBX_MODE_SPLIT) return fail(GBX_EINVAL, "mode must be FP64 or SPLIT");
-  std::unique_ptr<gbx_dltc_program> p(new gbx_dltc_program());
+// branched: workspaces of their own wanted (up to kBranchElems together) /
+// had.
+static int build_program(int which, const gbx_dltc_dims* dims, int mode, bool& branched,
+                         std::unique_ptr<gbx_dltc_program>& p) {
+  p.reset(new gbx_dltc_program());
   GBX_TRY(get_table(which, p->table));
   p->D = Dims{dims->O, dims->V, dims->wbO, dims->wbV, dims->nocc_names};
   p->mode = mode;
@@ -904,7 +903,7 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
     p->flops += op.flops;
     p->ops.push_back(op);
   }
-  const bool branched = all <= kBranchElems;
+  branched = branched && all <= kBranchElems;
   if (branched) ws = all;
   else p->ws_at.assign(p->ops.size(), 0);
   GBX_TRY(dev_alloc((void**)&p->ws, sizeof(double) * std::max<int64_t>(ws, 1)));
@@ -937,6 +936,25 @@ int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_
     p->branches = 0;
     p->chain_why = gbx_last_error();
   }
+  return GBX_OK;
+}
+
+int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_dltc_program** out) {
+  if (!out) return fail(GBX_EINVAL, "out is NULL");
+  *out = nullptr;
+  GBX_TRY(check_dims(dims));
+  if (mode != GBX_MODE_FP64 && mode != GBX_MODE_SPLIT) return fail(GBX_EINVAL, "mode must be FP64 or SPLIT");
+  std::unique_ptr<gbx_dltc_program> p;
+  bool branched = true;
+  int rc = build_program(which, dims, mode, branched, p);
+  if (rc == GBX_ENOMEM && branched) {
+    // workspaces of their own did not fit: one for all expressions
+    const std::string why = gbx_last_error();
+    branched = false;
+    rc = build_program(which, dims, mode, branched, p);
+    p->chain_why = why;
+  }
+  GBX_TRY(rc);
   *out = p.release();
   return GBX_OK;
 }

@@ -64,6 +64,7 @@ std::unordered_map<void*, AllocRec> g_allocs;
 thread_local std::atomic<int64_t>* g_account = nullptr;
 thread_local bool g_ordered = false;
 thread_local cudaStream_t g_order_stream = nullptr;
+thread_local int64_t g_budget = -1;  // bytes this thread's calls may still allocate (gbx_alloc_budget)
 }  // namespace
 
 AllocAccount::AllocAccount(std::atomic<int64_t>* acc) : prev(g_account) { g_account = acc; }
@@ -81,6 +82,8 @@ StreamOrderedAlloc::~StreamOrderedAlloc() {
 int dev_alloc(void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return GBX_OK;
+  if (g_budget >= 0 && (int64_t)bytes > g_budget)
+    return fail(GBX_ENOMEM, "device allocation of %zu bytes: %lld left of the thread's budget", bytes, (long long)g_budget);
   cudaError_t e;
   if (g_ordered) {
     // the allocation completes before the memory is handed out, so any
@@ -99,6 +102,7 @@ int dev_alloc(void** p, size_t bytes) {
   std::lock_guard<std::mutex> lk(g_alloc_mu);
   g_allocs[*p] = AllocRec{bytes, g_account, g_order_stream, g_ordered};
   if (g_account) g_account->fetch_add((int64_t)bytes);
+  if (g_budget >= 0) g_budget -= (int64_t)bytes;
   return GBX_OK;
 }
 
@@ -111,6 +115,7 @@ void dev_free(void* p) {
     auto it = g_allocs.find(p);
     if (it != g_allocs.end()) {
       if (it->second.account) it->second.account->fetch_sub((int64_t)it->second.bytes);
+      if (g_budget >= 0) g_budget += (int64_t)it->second.bytes;
       ordered = it->second.ordered;
       st = it->second.stream;
       g_allocs.erase(it);
@@ -282,6 +287,11 @@ using namespace gbx;
 extern "C" {
 
 const char* gbx_last_error(void) { return t_err.c_str(); }
+
+int gbx_alloc_budget(int64_t bytes) {
+  g_budget = std::max<int64_t>(bytes, -1);
+  return GBX_OK;
+}
 
 const char* gbx_version(void) { return "dtcf_gb300 0.1 (sm_103a)"; }
 

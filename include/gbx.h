@@ -36,6 +36,11 @@ extern "C" {
 GBX_API const char* gbx_last_error(void);
 /* Library version string. */
 GBX_API const char* gbx_version(void);
+/* Bytes that the calling thread's calls may from now on allocate beyond what
+ * they free, as on a GPU with that much free memory (negative: no limit, the
+ * default): a larger request fails with GBX_ENOMEM.  For what jobs, plans and
+ * programs keep; stream-ordered temporaries of one call do not count. */
+GBX_API int gbx_alloc_budget(int64_t bytes);
 
 /* ---- leaf entry points ------------------------------------------------- */
 

@@ -32,7 +32,8 @@ typedef struct {
     int slices;          /* split engine: bf16 slices per operand (0 = default) */
     int use_graph;       /* 0: launch kernel by kernel; 1: capture one iteration as a CUDA graph of its
                             kernels, steps that do not depend on one another as branches where the
-                            contractions' own workspaces for that stay below 4 GB; 2: run the iteration as a persistent program -- a few persistent
+                            contractions' own workspaces for that stay below 4 GB and can be had
+                            (else one workspace and a chain); 2: run the iteration as a persistent program -- a few persistent
                             launches driven by a device-side work queue (one per dependency level of
                             the memory-bound work, one per GEMM kernel and level) -- captured as the
                             graph; each contraction then keeps its own workspace */

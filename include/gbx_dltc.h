@@ -89,7 +89,7 @@ typedef struct gbx_dltc_program gbx_dltc_program;
 /* A table bound to device tensors of the given dims, zeroed (as GA_Zero
  * leaves them), with every expression prepared once: transposes, GEMM (mode
  * GBX_MODE_FP64 or GBX_MODE_SPLIT) and its workspace (up to 2 GB together;
- * beyond, one shared by all).
+ * beyond, or where memory is short, one shared by all).
  * Replaces the setup half of ccd_t2 / ccsd_t1 / ccsd_t2 (Tensor2/Tensor4 +
  * allocGA + the Multiplication / Summation constructors). */
 GBX_API int gbx_dltc_program_create(int which, const gbx_dltc_dims* dims, int mode, gbx_dltc_program** out);
