@@ -841,6 +841,18 @@ int gbx_cc_footprint(const gbx_cc_config* cfg, double* resident_bytes, double* p
   return job->footprint(resident_bytes, peak_bytes);
 }
 
+}  // extern "C"
+
+int gbx::cc_footprints(const gbx_cc_config& cfg, double* branches, double* chain) {
+  std::unique_ptr<gbx_cc_job> job;
+  GBX_TRY(cc_setup(&cfg, job));
+  GBX_TRY(job->footprint(branches, nullptr));
+  job->cfg.use_graph = kGraphChain;
+  return job->footprint(chain, nullptr);
+}
+
+extern "C" {
+
 int gbx_cc_create(const gbx_cc_config* cfg, void* stream, gbx_cc_job** out) {
   if (!out) return fail(GBX_EINVAL, "null argument");
   *out = nullptr;

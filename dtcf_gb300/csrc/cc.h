@@ -42,6 +42,8 @@ namespace gbx {
 // use_graph of a server's jobs: the kernel graph with its steps in one chain
 // (every value but 0, 1 and 2 means so).
 constexpr int kGraphChain = 3;
+// Planned resident bytes of a use_graph 1 job, as configured and as a chain.
+int cc_footprints(const gbx_cc_config& cfg, double* branches, double* chain);
 
 struct CCTile {
   int64_t off;

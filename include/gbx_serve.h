@@ -61,8 +61,8 @@ typedef struct gbx_server gbx_server;
 GBX_API int gbx_server_create(const gbx_serve_config* cfg, gbx_server** out);
 /* Registers a job (host planning only; nothing is allocated yet);
  * footprint_bytes receives its planned resident bytes (where the budget does
- * not hold all jobs of a run at once, they take one workspace region each and
- * less memory than that). */
+ * not hold all jobs of a run at once, those with the larger workspaces take one
+ * region each and less memory than that). */
 GBX_API int gbx_server_add_job(gbx_server* s, const gbx_cc_config* cfg, int* job_id, double* footprint_bytes);
 /* One iteration request of job_id arriving arrival_s seconds after
  * gbx_server_run starts.  Submit every request before running. */
