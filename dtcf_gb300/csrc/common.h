@@ -211,6 +211,7 @@ struct GemmProblem {
   int m, n, k;
   double alpha;
   int accumulate;
+  int twice;  // products of the first `twice` of the k columns count twice (variant 0 only)
   // split-K and kernel (filled by F64Gemm::build)
   int ksplit, kchunk, pad_;
   double* partial;
@@ -224,6 +225,7 @@ struct F64Gemm {
     int* d_first = nullptr;
     int nprob = 0, total_tiles = 0, variant = 0;
     int ts = 16, cluster = 1;  // tile kernel: tile edge, CTAs per tile
+    bool twice = false;        // some problem has columns that count twice
     std::vector<int> first;  // host copy of d_first (per-problem launches)
   };
   std::vector<Sub> subs;

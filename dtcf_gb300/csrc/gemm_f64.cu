@@ -168,11 +168,10 @@ struct TileSmem {
   double sum[256];
 };
 
-// MB x NB blocks of 8 x 8 over K steps [s0, s1) of the range [kbeg, kend);
-// out(row, col, two sums) takes the results, rows and columns within the tile.
-template <int MB, int NB, class Out>
-__device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, int kbeg, int kend, int s0, int s1,
-                                          Out&& out) {
+// Adds K steps [s0, s1) of the range [kbeg, kend) to MB x NB blocks of 8 x 8.
+template <int MB, int NB>
+__device__ __forceinline__ void tile_steps(const GemmProblem& p, int m0, int n0, int kbeg, int kend, int s0, int s1,
+                                           double (&acc)[MB][NB][2]) {
   const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
   const int64_t acs = p.a_cs, bcs = p.b_cs;
   const double* pa[MB];
@@ -183,11 +182,6 @@ __device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, 
   for (int i = 0; i < MB; ++i) pa[i] = p.A + (int64_t)min(m0 + 8 * i + r, p.m - 1) * p.a_rs + k0 * acs;
 #pragma unroll
   for (int j = 0; j < NB; ++j) pb[j] = p.B + (int64_t)min(n0 + 8 * j + r, p.n - 1) * p.b_rs + k0 * bcs;
-  double acc[MB][NB][2];
-#pragma unroll
-  for (int i = 0; i < MB; ++i)
-#pragma unroll
-    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   double a[2][kTileUnroll][MB], b[2][kTileUnroll][NB];
   auto load = [&](int buf, int s) {
 #pragma unroll
@@ -217,6 +211,49 @@ __device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, 
     if (s + 2 * kTileUnroll < s1) load(0, s + 2 * kTileUnroll);
     if (s + kTileUnroll < s1) mma(1, s + kTileUnroll);
   }
+}
+
+// K steps of the range [kbeg, kend): with kTwice those of its columns that
+// count twice, then the others (no step holds both).
+__device__ __forceinline__ int steps_twice(const GemmProblem& p, int kbeg, int kend) {
+  return (max(min(kend, p.twice) - kbeg, 0) + 3) / 4;
+}
+template <bool kTwice>
+__device__ __forceinline__ int k_steps(const GemmProblem& p, int kbeg, int kend) {
+  if (!kTwice) return (max(kend - kbeg, 0) + 3) / 4;
+  return steps_twice(p, kbeg, kend) + (max(kend - max(kbeg, p.twice), 0) + 3) / 4;
+}
+
+// MB x NB blocks of 8 x 8 over K steps [s0, s1) of the range [kbeg, kend);
+// out(row, col, two sums) takes the results, rows and columns within the tile.
+template <int MB, int NB, bool kTwice, class Out>
+__device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, int kbeg, int kend, int s0, int s1,
+                                          Out&& out) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  double acc[MB][NB][2];
+#pragma unroll
+  for (int i = 0; i < MB; ++i)
+#pragma unroll
+    for (int j = 0; j < NB; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  if constexpr (!kTwice) {
+    tile_steps<MB, NB>(p, m0, n0, kbeg, kend, s0, s1, acc);
+  } else {
+    const int n2 = steps_twice(p, kbeg, kend);
+#pragma unroll 1
+    for (bool dbl = s0 < n2;; dbl = false) {
+      tile_steps<MB, NB>(p, m0, n0, dbl ? kbeg : max(kbeg, p.twice), dbl ? min(kend, p.twice) : kend,
+                         dbl ? s0 : max(s0 - n2, 0), dbl ? min(s1, n2) : max(s1 - n2, 0), acc);
+      if (!dbl) break;
+      // what counts twice: the sums so far, doubled exactly
+#pragma unroll
+      for (int i = 0; i < MB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j) {
+          acc[i][j][0] = __dadd_rn(acc[i][j][0], acc[i][j][0]);
+          acc[i][j][1] = __dadd_rn(acc[i][j][1], acc[i][j][1]);
+        }
+    }
+  }
 #pragma unroll
   for (int i = 0; i < MB; ++i)
 #pragma unroll
@@ -224,22 +261,23 @@ __device__ __forceinline__ void tile_loop(const GemmProblem& p, int m0, int n0, 
 }
 
 // The 8 x 8 blocks of a 16 x 16 tile that hold real outputs.
-template <class Out>
+template <bool kTwice, class Out>
 __device__ __forceinline__ void tile_blocks(const GemmProblem& p, bool m2, bool n2, int m0, int n0, int kbeg, int kend,
                                             int s0, int s1, Out&& out) {
-  if (m2 && n2) tile_loop<2, 2>(p, m0, n0, kbeg, kend, s0, s1, out);
-  else if (m2) tile_loop<2, 1>(p, m0, n0, kbeg, kend, s0, s1, out);
-  else if (n2) tile_loop<1, 2>(p, m0, n0, kbeg, kend, s0, s1, out);
-  else tile_loop<1, 1>(p, m0, n0, kbeg, kend, s0, s1, out);
+  if (m2 && n2) tile_loop<2, 2, kTwice>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else if (m2) tile_loop<2, 1, kTwice>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else if (n2) tile_loop<1, 2, kTwice>(p, m0, n0, kbeg, kend, s0, s1, out);
+  else tile_loop<1, 1, kTwice>(p, m0, n0, kbeg, kend, s0, s1, out);
 }
 
 // Work item `local` of problem p when every warp has a 16 x 16 tile of its own.
+template <bool kTwice>
 __device__ __forceinline__ void warp_tile_item(const GemmProblem& p, int64_t local) {
   const int ntn = (p.n + 15) / 16, ntm = (p.m + 15) / 16;
   const int64_t t = local * kTileWarps + (threadIdx.x >> 5);
   if (t >= (int64_t)ntm * ntn) return;
   const int m0 = (int)(t / ntn) * 16, n0 = (int)(t % ntn) * 16;
-  tile_blocks(p, p.m - m0 > 8, p.n - n0 > 8, m0, n0, 0, p.k, 0, (p.k + 3) / 4, [&](int i, int j, double x, double y) {
+  tile_blocks<kTwice>(p, p.m - m0 > 8, p.n - n0 > 8, m0, n0, 0, p.k, 0, k_steps<kTwice>(p, 0, p.k), [&](int i, int j, double x, double y) {
     const int64_t gm = m0 + i, gn = n0 + j;
     if (gm >= p.m) return;
     double* c = p.C + gm * p.c_rs + gn;
@@ -250,10 +288,10 @@ __device__ __forceinline__ void warp_tile_item(const GemmProblem& p, int64_t loc
 
 // One work item of problem p: output tile and K range `local`.  TS: tile
 // edge, 16 or 8; 0: a tile per warp.
-template <int TS>
+template <int TS, bool kTwice>
 __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, TileSmem& sm) {
   if constexpr (TS == 0) {
-    warp_tile_item(p, local);
+    warp_tile_item<kTwice>(p, local);
     return;
   }
   constexpr int ts = TS;
@@ -266,7 +304,7 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, T
   const int t = (int)(local - kc * per_k);
   const int m0 = t / ntn * ts, n0 = (t % ntn) * ts;
   const int kbeg = kc * p.kchunk, kend = min(p.k, kbeg + p.kchunk);
-  const int steps = (max(kend - kbeg, 0) + 3) / 4;
+  const int steps = k_steps<kTwice>(p, kbeg, kend);
   const int per = (steps + csize * kTileWarps - 1) / (csize * kTileWarps);
   const int s0 = min(steps, (crank * kTileWarps + warp) * per), s1 = min(steps, s0 + per);
   const bool m2 = ts == 16 && p.m - m0 > 8, n2 = ts == 16 && p.n - n0 > 8;
@@ -274,8 +312,8 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, T
   const auto keep = [&](int i, int j, double x, double y) {
     *reinterpret_cast<double2*>(part + i * 16 + j) = make_double2(x, y);
   };
-  if constexpr (TS == 8) tile_loop<1, 1>(p, m0, n0, kbeg, kend, s0, s1, keep);
-  else tile_blocks(p, m2, n2, m0, n0, kbeg, kend, s0, s1, keep);
+  if constexpr (TS == 8) tile_loop<1, 1, kTwice>(p, m0, n0, kbeg, kend, s0, s1, keep);
+  else tile_blocks<kTwice>(p, m2, n2, m0, n0, kbeg, kend, s0, s1, keep);
   __syncthreads();
   const int rows = min(ts, p.m - m0), cols = min(ts, p.n - n0);
   const auto add = [&](int e) {
@@ -316,7 +354,7 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, T
 
 // All problems of a launch, one work item per cluster: the item's problem is
 // found by a 32-way search of the first-item table.
-template <int TS>
+template <int TS, bool kTwice>
 __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
     tile_gemm_f64_kernel(const GemmProblem* __restrict__ probs, int nprob, const int* __restrict__ first) {
   begin_dependent();
@@ -331,7 +369,7 @@ __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
     n = min(step, lo + n - nlo);
     lo = nlo;
   }
-  tile_item<TS>(probs[lo], item - first[lo], sm);
+  tile_item<TS, kTwice>(probs[lo], item - first[lo], sm);
 }
 
 // A one-problem launch with its descriptor in the kernel's arguments: nothing to upload, no search.
@@ -347,7 +385,7 @@ __global__ void __launch_bounds__(kTileThreads, TS == 8 ? 8 : 4)
     tile_one_f64_kernel(const __grid_constant__ OneProblem a) {
   begin_dependent();
   __shared__ TileSmem sm;
-  tile_item<TS>(a.p, blockIdx.x / cg::this_cluster().num_blocks(), sm);
+  tile_item<TS, false>(a.p, blockIdx.x / cg::this_cluster().num_blocks(), sm);
 }
 
 // K <= 8 (dev::small_k_body).
@@ -680,11 +718,13 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
   for (int v : {0, kLongTiles, 4, 5, 6, 7, 8}) {
     const TilePlan& t = tp[v == kLongTiles ? 1 : 0];
     std::vector<GemmProblem> vp;
+    bool twice = false;
     std::vector<int> first;
     int64_t tiles = 0;
     for (auto& q : probs) {
       if (q.pad_ != v) continue;
       vp.push_back(q);
+      twice = twice || q.twice > 0;
       first.push_back((int)tiles);
       tiles += f64_items(q, t.ts);
       if (tiles >= (1ll << 31)) return fail(GBX_EUNSUPPORTED, "grouped GEMM has too many work items");
@@ -696,6 +736,7 @@ int F64Gemm::build(const std::vector<GemmProblem>& in, bool async, cudaStream_t 
     sb.total_tiles = (int)tiles;
     sb.ts = t.ts;
     sb.cluster = t.cluster;
+    sb.twice = twice;
     GBX_TRY(alloc((void**)&sb.d_probs, sizeof(GemmProblem) * vp.size()));
     GBX_TRY(alloc((void**)&sb.d_first, sizeof(int) * vp.size()));
     GBX_TRY(copy(sb.d_probs, vp.data(), sizeof(GemmProblem) * vp.size()));
@@ -751,12 +792,17 @@ int F64Gemm::run(cudaStream_t st) const {
 namespace {
 // The kernel of variant v over problems [probs, probs + nprob) and their `tiles` work items.
 int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first, int tiles, const TilePlan& tp,
-                   cudaStream_t st) {
+                   bool twice, cudaStream_t st) {
   const int grid = std::min(tiles, kSms * 8);
   switch (v) {
     case 0:
     case kLongTiles:
-      return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8> : tp.ts ? tile_gemm_f64_kernel<16> : tile_gemm_f64_kernel<0>,
+      if (twice)
+        return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8, true> : tp.ts ? tile_gemm_f64_kernel<16, true>
+                                                                              : tile_gemm_f64_kernel<0, true>,
+                            tp, tiles, st, probs, nprob, first);
+      return launch_tiles(tp.ts == 8 ? tile_gemm_f64_kernel<8, false> : tp.ts ? tile_gemm_f64_kernel<16, false>
+                                                                             : tile_gemm_f64_kernel<0, false>,
                           tp, tiles, st, probs, nprob, first);
     case 4: return launch(thin_gemm_f64_kernel<true>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
     case 6: return launch(small_k_gemm_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
@@ -771,7 +817,7 @@ int F64Gemm::run_sub(const Sub& sb, cudaStream_t st) {
   TilePlan tp;
   tp.ts = sb.ts;
   tp.cluster = sb.cluster;
-  return launch_variant(sb.variant, sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles, tp, st);
+  return launch_variant(sb.variant, sb.d_probs, sb.nprob, sb.d_first, sb.total_tiles, tp, sb.twice, st);
 }
 
 int F64Gemm::run_each(cudaStream_t st) const {
@@ -784,7 +830,7 @@ int F64Gemm::run_each(cudaStream_t st) const {
       TilePlan tp;
       tp.ts = sb.ts;
       tp.cluster = sb.cluster;
-      GBX_TRY(launch_variant(sb.variant, sb.d_probs + i, 1, sb.d_first, sb.first[i + 1] - sb.first[i], tp, st));
+      GBX_TRY(launch_variant(sb.variant, sb.d_probs + i, 1, sb.d_first, sb.first[i + 1] - sb.first[i], tp, sb.twice, st));
     }
   }
   if (nred) {

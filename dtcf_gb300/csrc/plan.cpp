@@ -406,22 +406,8 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
   for (auto& kv : rows) assign(kv.second, dA);
   for (auto& kv : cols) assign(kv.second, dB);
   for (auto& kv : ks) assign(kv.second, dK);
-  // the diagonal block pairs' columns first
-  int64_t k_diag = 0;
-  if (pair && pair->exact) {
-    if (rows.size() > 1 || ks.size() > 1) return fail(GBX_EINVAL, "symmetric pair over several irreps");
-    for (auto& kv : ks) {
-      int64_t off = 0;
-      for (bool diag : {true, false}) {
-        for (auto& t : kv.second.off)
-          if ((t.first[px] == t.first[py]) == diag) {
-            t.second = off;
-            off += tuple_size(dK, t.first);
-          }
-        if (diag) k_diag = off;
-      }
-    }
-  }
+  if (pair && pair->exact && (rows.size() > 1 || ks.size() > 1))
+    return fail(GBX_EINVAL, "symmetric pair over several irreps");
   for (auto& kv : ks_full) assign(kv.second, dK);
   // irrep groups present in rows, cols and K
   int64_t ao = 0, bo = 0, co = 0;
@@ -453,15 +439,25 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
     g.engine = whole.engine;
     g.swap = whole.swap;
   }
-  bool halve = false;  // the diagonal pairs in one operand's pack
   if (pair && pair->exact && !p->groups.empty()) {
-    if (p->groups[0].engine == 1) {
-      p->dbl_from = k_diag;
-      p->dbl_plan_b = pair->scale_b;
-    } else {
-      halve = true;
-      p->alpha_factor = 2.0;
+    GroupBlock& g = p->groups[0];
+    // only the FP64 tile kernel counts columns twice
+    if (g.engine == 0 && f64_variant((int)g.M, (int)g.N, (int)g.K) != 0)
+      return plan_contraction(A, B, C, la, lb, lc, e, nslices, out, split_all, defer, nullptr);
+    // the diagonal block pairs' columns first for the split engine, last for
+    // the tile kernel
+    TupleIndex& kt = ks[g.h];
+    int64_t off = 0;
+    for (const bool diag : {g.engine == 1, g.engine != 1}) {
+      for (auto& t : kt.off)
+        if ((t.first[px] == t.first[py]) == diag) {
+          t.second = off;
+          off += tuple_size(dK, t.first);
+        }
+      if (diag && g.engine == 1) p->dbl_from = off;
+      if (!diag && g.engine == 0) p->twice = off;
     }
+    p->dbl_plan_b = pair->scale_b;
   }
 
   // pack moves: A (rows = extA tuples of irrep h, cols = K tuples of irrep h)
@@ -509,11 +505,7 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
           for (size_t i = 0; i < contr_dims.size(); ++i) dstr[contr_dims[i]] = sK[i];
           int64_t dst = (isA ? g.a_off : g.b_off) + rv.second * g.K + kvv.second;
           // off-diagonal block pairs of a symmetric contracted pair count twice
-          // (or the diagonal ones half)
-          if (pair_scaled && px >= 0) {
-            if (pair->exact) factor *= halve && kvv.first[px] == kvv.first[py] ? 0.5 : 1.0;
-            else if (kvv.first[px] > kvv.first[py]) factor *= 2.0;
-          }
+          if (pair_scaled && px >= 0 && !pair->exact && kvv.first[px] > kvv.first[py]) factor *= 2.0;
           ms.host.push_back(make_move(T.rank, ext, sstr, dstr, T.off[id], dst, 0, factor));
         }
       }
@@ -838,6 +830,7 @@ int ContractionPlan::build(unsigned char* arena, unsigned char* static_scratch) 
     q.k = (int)g.K;
     q.alpha = 1.0;
     q.accumulate = 0;
+    q.twice = (int)twice;
     probs.push_back(q);
   }
   GBX_TRY(f64.build(probs));
@@ -958,7 +951,7 @@ int ContractionPlan::execute(const double* dA, const double* dB, double* dC, dou
     if (split) GBX_TRY(run_split_plan(split, !skipA, !skipB, st));
   }
   if (!(stages & 2)) return GBX_OK;
-  return run_moves_scaled(unpackC, d_Cbig, dC, alpha * alpha_factor, st);
+  return run_moves_scaled(unpackC, d_Cbig, dC, alpha, st);
 }
 
 bool ContractionPlan::set_overwrite(double alpha, int64_t c_elems) {
@@ -978,7 +971,7 @@ bool ContractionPlan::set_overwrite(double alpha, int64_t c_elems) {
     // stores of alpha * the product (a store move ignores the run-time factor)
     for (MoveDesc& m : unpackC.host) {
       m.op = 0;
-      m.scale = alpha * alpha_factor;
+      m.scale = alpha;
     }
     store_scale = alpha;
   }

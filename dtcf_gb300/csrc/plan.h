@@ -156,9 +156,9 @@ struct ContractionPlan {
   // Nonzero: the unpack stores store_scale * A B into C, whatever factor
   // execute is given (set_overwrite on a packed plan).
   double store_scale = 0.0;
-  // exact pairs: the unpack's factor (FP64 groups), the columns whose
-  // products count twice (split groups; -1: none)
-  double alpha_factor = 1.0;
+  // exact pairs: the columns whose products count twice, the first `twice` of
+  // an FP64 group or those from dbl_from on of a split one (-1: none)
+  int64_t twice = 0;
   int64_t dbl_from = -1;
   bool dbl_plan_b = true;
   // Makes the plan write C = alpha A B instead of accumulating, when it writes
@@ -210,10 +210,10 @@ constexpr double kDirectMaxK = 16.0;
 // so the packed GEMMs run over block pairs X >= Y only, the off-diagonal ones
 // weighted 2 in one operand's pack (scale_b: B's, else A's) -- close to half
 // the contracted extent.  Both indices must have the same blocking.
-// exact: no value is scaled up for it.  The FP64 engine computes 2 (sum_{X>Y}
-// + 1/2 sum_{X=Y}), the diagonal pairs weighted 1/2 in the pack and the
-// unpack's factor doubled (the FP64 ladder at o = 16, v = 48 in blocks of 8:
-// 1193 -> 710 us); the split engine doubles the off-diagonal columns' digits
+// exact: no operand or factor is scaled for it, so values at the ends of the
+// FP64 range stay as they are.  The FP64 tile kernel doubles its sums between
+// the off-diagonal columns and the diagonal ones (the ladder at o = 16, v = 48
+// in blocks of 8: 1193 -> 665 us); the split engine doubles the off-diagonal columns' digits
 // (SplitProblem::dbl_from; o = 32, v = 128, blocks of 16: 5033 -> 3132 us).
 // Needs operands of one irrep; the engine is chosen as for the whole sum.
 struct ContractionPair {
