@@ -277,23 +277,20 @@ __device__ __forceinline__ void warp_tile_item(const GemmProblem& p, int64_t loc
   const int64_t t = local * kTileWarps + (threadIdx.x >> 5);
   if (t >= (int64_t)ntm * ntn) return;
   const int m0 = (int)(t / ntn) * 16, n0 = (int)(t % ntn) * 16;
-  tile_blocks<kTwice>(p, p.m - m0 > 8, p.n - n0 > 8, m0, n0, 0, p.k, 0, k_steps<kTwice>(p, 0, p.k), [&](int i, int j, double x, double y) {
+  const auto store = [&](int i, int j, double x, double y) {
     const int64_t gm = m0 + i, gn = n0 + j;
     if (gm >= p.m) return;
     double* c = p.C + gm * p.c_rs + gn;
     if (gn < p.n) c[0] = p.accumulate ? __dadd_rn(c[0], __dmul_rn(p.alpha, x)) : __dmul_rn(p.alpha, x);
     if (gn + 1 < p.n) c[1] = p.accumulate ? __dadd_rn(c[1], __dmul_rn(p.alpha, y)) : __dmul_rn(p.alpha, y);
-  });
+  };
+  tile_blocks<kTwice>(p, p.m - m0 > 8, p.n - n0 > 8, m0, n0, 0, p.k, 0, k_steps<kTwice>(p, 0, p.k), store);
 }
 
-// One work item of problem p: output tile and K range `local`.  TS: tile
-// edge, 16 or 8; 0: a tile per warp.
+// One work item of problem p: output tile of edge TS (16 or 8) and K range
+// `local`.
 template <int TS, bool kTwice>
-__device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, TileSmem& sm) {
-  if constexpr (TS == 0) {
-    warp_tile_item<kTwice>(p, local);
-    return;
-  }
+__device__ __forceinline__ void cluster_tile_item(const GemmProblem& p, int64_t local, TileSmem& sm) {
   constexpr int ts = TS;
   const cg::cluster_group cl = cg::this_cluster();
   const int csize = (int)cl.num_blocks(), crank = (int)cl.block_rank();
@@ -350,6 +347,13 @@ __device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, T
       store(e, v);
     }
   cl.sync();  // no CTA leaves while another reads its sums
+}
+
+// Work item `local` of problem p; TS 0: a tile per warp.
+template <int TS, bool kTwice>
+__device__ __forceinline__ void tile_item(const GemmProblem& p, int64_t local, TileSmem& sm) {
+  if constexpr (TS == 0) warp_tile_item<kTwice>(p, local);
+  else cluster_tile_item<TS, kTwice>(p, local, sm);
 }
 
 // All problems of a launch, one work item per cluster: the item's problem is

@@ -863,7 +863,8 @@ struct KsCfg {
   static constexpr int kStages = (220 * 1024 / kStageBytes) < 8 ? 220 * 1024 / kStageBytes : 8;
   static constexpr int kCut = S <= 5 ? 0 : S - 4;  // levels below this go to the upper sum
   // the drains' level loops: unrolled, their TMEM reads overlap the sums
-  // before (S = 6: 978 instead of 1019 us); at S = 4 that spills
+  // before (S = 6: 978 instead of 1019 us, although at 168 registers it spills
+  // 224 bytes and S = 7 60); at S = 4, faster without, it would spill too
   static constexpr int kUnroll = S <= 4 ? 1 : S;
 };
 

@@ -67,9 +67,6 @@ __global__ void __launch_bounds__(256) apply_kernel(const ApplyDesc* __restrict_
 struct Choice {
   int engine = 0, variant = -1, width = 0;
   bool swap = false;
-  bool operator<(const Choice& o) const {
-    return std::tie(engine, variant, width, swap) < std::tie(o.engine, o.variant, o.width, o.swap);
-  }
 };
 
 bool split_capable(const gbx_triple& t) { return t.a_cs == 1 && t.b_cs == 1; }

@@ -36,9 +36,14 @@ constexpr int kBoxSmem = 5120;    // with its pitches made odd
 constexpr int kBoxDims = 6;       // dimensions a box may extend in
 constexpr int kBoxPer = 8;        // elements in flight per thread
 constexpr int kSetDescs = 16;     // permutations of one launch
-constexpr int kSetBlocks = 16384; // blocks of one launch
-constexpr int kListBlocks = 4096; // with the blocks' numbers beside their permutations
-constexpr int kPackTiles = 14336; // tiles of one pack launch (slots below 65536; half as many beyond)
+// Entries of a launch's tables: about what fits into 32 KB of kernel arguments
+// beside the descriptors, and for calls of fewer blocks or tiles (kSmallSet,
+// kSmallPack) a few KB, since the host fills all of the arguments it launches
+// with (2000 4^4 blocks 14.3 us, 16.0 with the large table; 81 packed tiles
+// 9.1 and 9.6).
+constexpr int kSetBlocks = 16384, kSmallSet = 2048;
+constexpr int kListBlocks = 4096;  // with the blocks' numbers beside their permutations
+constexpr int kPackTiles = 14336, kSmallPack = 1536;  // (slots below 65536; kPackTiles / 2 beyond)
 
 // One dimension of a walk over a box: extent, ceil(2^32 / extent) for the
 // division (exact: index x extent < 2^32), the tensor stride and the
@@ -560,9 +565,9 @@ int run_block_moves(const std::vector<MoveDesc>& moves, const std::vector<int>& 
         std::copy(which.begin() + b0, which.begin() + b0 + nb, a.which);
         return launch(kernel, grid, kBoxThreads, st, a, s, d);
       };
-      if (nb <= 2048) {
-        MoveTable<2048> a;
-        GBX_TRY(run(a, box_set_kernel<2048>));
+      if (nb <= kSmallSet) {
+        MoveTable<kSmallSet> a;
+        GBX_TRY(run(a, box_set_kernel<kSmallSet>));
       } else {
         MoveTable<kSetBlocks> a;
         GBX_TRY(run(a, box_set_kernel<kSetBlocks>));
@@ -657,8 +662,8 @@ int run_pack(int64_t rows, int64_t cols, int64_t nrows, int64_t ncols, const std
     if (wide) {
       PackTable<uint32_t, kPackTiles / 2> a;
       GBX_TRY(go(a, t0, nt));
-    } else if (nt <= 1536) {
-      PackTable<uint16_t, 1536> a;
+    } else if (nt <= kSmallPack) {
+      PackTable<uint16_t, kSmallPack> a;
       GBX_TRY(go(a, t0, nt));
     } else {
       PackTable<uint16_t, kPackTiles> a;

@@ -242,11 +242,8 @@ void sub_strides(const std::vector<int64_t>& ext, int64_t base, std::vector<int6
 }  // namespace
 
 namespace {
-// FP64 seconds of an m x n x k product for the engine choice, as an FP64
-// engine of 64- and 16-wide output tiles would take them.  The FP64 kernels
-// have since become faster than this on small and ragged shapes, but the
-// line between the engines stays: a group that moved from slices to FP64 or
-// back would change a job's results by the slices' error, not by rounding.
+// FP64 seconds of an m x n x k product for the engine choice (choose_engine),
+// as an FP64 engine of 64- and 16-wide output tiles would take them.
 double f64_model_seconds(int64_t M, int64_t N, int64_t K) {
   auto up = [](int64_t x, int64_t m) { return (double)((x + m - 1) / m * m); };
   const double flops = 2.0 * (double)M * (double)N * (double)K, wide = (double)std::max(M, N) * (double)K * 8.0;

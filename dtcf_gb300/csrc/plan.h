@@ -103,9 +103,12 @@ struct GroupBlock {   // one irrep block of the packed operands
   bool swap = false;            // split engine computes C^T = B A^T (C block stored N x M)
 };
 
-// Engine and orientation of one packed GEMM from a throughput model of this
-// GPU: FP64 DMMA near 0.95 TFLOP/s on 64x64 tiles, the split engine near
-// 1 PFLOP/s of bf16 slice products on 128x64 tiles (S(S+1)/2 products).
+// Engine and orientation of one packed GEMM.  The line between the engines is
+// a fixed one, not a model of the present kernels: FP64 at 0.95 TFLOP/s on
+// 64x64 tiles, the split engine at 1 PFLOP/s of bf16 slice products on 128x64
+// tiles (S(S+1)/2 products) with its slices streamed once for each.  Both
+// engines have since become faster, but a group that changed sides would
+// change a job's results by the slices' error.
 void choose_engine(GroupBlock& g, bool split_engine, bool split_all, int slices);
 
 enum class Engine { F64 = 0, Split = 1 };
