@@ -521,7 +521,7 @@ int clusters_apart(int cluster) { return cluster == 8 ? 15 : cluster == 4 ? 36 :
 // A problem that is most of its launch also counts how often its clusters
 // come round to an SM, and is cut to even that out (planned, tiles cut by
 // their share alone / so: 32 x 32 x 10^6 4422 / 1872 us, 100 x 100 x 50000 1774 /
-// 1041, 110 x 110 x 2000 74 / 53).
+// 1041, 110 x 110 x 2000 74 / 53, 28 x 3 x 17508 43 / 18).
 void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
   const int steps = ceil_div(q.k, 4), workers = 4 * t.cluster;
   if (t.ts == 0) return;
@@ -531,11 +531,14 @@ void tile_ksplit(GemmProblem& q, const TilePlan& t, int64_t dmmas, int least) {
   const int64_t most = std::max(1, steps / (8 * workers));
   int64_t ks = std::max<int64_t>(1, std::min<int64_t>((item + share / 2) / share, most));
   if (2 * dmma_count(q) >= dmmas) {
-    // the DMMAs of the SM quarter with the most
+    // the DMMAs of the SM quarter with the most (clusters beyond two rounds
+    // share the SMs about evenly)
     const auto load = [&](int64_t k) {
-      return ceil_div(tile_count(q, t.ts) * k, clusters_apart(t.cluster)) * blocks * ceil_div(ceil_div(steps, k), workers);
+      const int64_t n = tile_count(q, t.ts) * k, apart = clusters_apart(t.cluster);
+      const int64_t each = blocks * ceil_div(ceil_div(steps, k), workers);
+      return t.cluster > 1 && n > 2 * apart ? n * each / apart : ceil_div(n, apart) * each;
     };
-    if (2 * load(1) >= 3 * share) {
+    if (2 * load(1) >= 3 * (dmmas / kQuarters) && load(1) >= least) {
       const int64_t to = std::min(most, 8 * std::max<int64_t>(ks, 2));
       int64_t best = load(ks);
       for (int64_t k = ks; k <= to; ++k) best = std::min(best, load(k));

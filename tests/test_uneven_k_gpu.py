@@ -43,6 +43,7 @@ def test_launches_and_results(long_shapes, launched):
 @pytest.mark.parametrize("m,n,k,ctas,reduced", [
     (32, 32, 100000, 304, True),   # K ranges without clusters: two CTAs to every SM
     (100, 100, 50000, 608, True),  # 169 tiles, a few more than SMs
+    (28, 3, 17508, 96, True),      # four tiles
     (17, 40, 30001, 120, False), (24, 24, 3456, 72, False), (48, 48, 1500, 288, False),  # clusters, K whole
 ])
 def test_one_long_product(m, n, k, ctas, reduced):
