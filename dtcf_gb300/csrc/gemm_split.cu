@@ -1440,10 +1440,13 @@ int split_layout(const std::vector<SplitProblem>& probs, int S, bool static_a, b
     // whole exact-accumulation chunks: 16 k-blocks for the pair-by-pair
     // kernel, 256 elements for the k-stationary one (so few-tile problems --
     // matrix-vector shapes, small outputs with long K -- spread over many more
-    // CTAs instead of walking K serially)
+    // CTAs instead of walking K serially).  Only K that fills the accumulators
+    // more than twice is worth the partial sums (two slices: 1024 elements; 3052
+    // x 718 x 518 at 2 and 3 slices 53 and 60 us in ranges, 28 and 33 whole)
     const int chunk = o.ks_kernel ? 256 / o.kb : kChunkKb;
+    const int least = o.ks_kernel ? std::max(chunk, 16 / S * BK / o.kb) : chunk;
     int ks = 1;
-    if (!o.thin && out_tiles < kSplitFill && nkb > 2 * chunk) {
+    if (!o.thin && out_tiles < kSplitFill && nkb > 2 * least) {
       int want = (int)((kSplitFill + out_tiles - 1) / out_tiles);
       ks = std::max(1, std::min(want, nkb / chunk));
     }
