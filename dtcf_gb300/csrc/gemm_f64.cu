@@ -868,6 +868,39 @@ int one_call_variant(int m, int n, int k) {
   return v;
 }
 
+namespace {
+// Stream-ordered temporaries of one-call products, from a pool of their own
+// that keeps up to kTempKeep bytes of a device between calls: the default pool
+// gives its memory back at every synchronisation, and a call after one then
+// waits 150 us for the driver (16 x 16 x 5000 alone: 181 us, 24 so).  The
+// pool is the CUDA runtime's, safe with any number of threads and streams.
+constexpr uint64_t kTempKeep = 32ull << 20;
+
+int temp_alloc(double** p, size_t bytes, cudaStream_t st) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[256] = {nullptr};
+  int dev = 0;
+  GBX_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 256) return fail(GBX_EUNSUPPORTED, "device ordinal %d out of range", dev);
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!pools[dev]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      GBX_CUDA(cudaMemPoolCreate(&pools[dev], &props));
+      uint64_t keep = kTempKeep;
+      GBX_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    pool = pools[dev];
+  }
+  GBX_CUDA(cudaMallocFromPoolAsync((void**)p, bytes, pool, st));
+  return GBX_OK;
+}
+}  // namespace
+
 // One problem, one call: the descriptor travels in the kernel's arguments.
 // The partial sums of long K with few outputs come from `scratch` (at most
 // scratch_elems) when given, else from a stream-ordered temporary.
@@ -897,7 +930,7 @@ int run_f64_one(const GemmProblem& in, cudaStream_t st, double* scratch, int64_t
     q.ksplit = std::max(1, ceil_div(q.k, q.kchunk));
   }
   if (q.ksplit > 1) {
-    if (!scratch) GBX_CUDA(cudaMallocAsync((void**)&own, sizeof(double) * q.ksplit * q.m * q.n, st));
+    if (!scratch) GBX_TRY(temp_alloc(&own, sizeof(double) * q.ksplit * q.m * q.n, st));
     q.partial = scratch ? scratch : own;
   }
   const int64_t items = f64_items(q, tp.ts);

@@ -73,7 +73,9 @@ GBX_API int gbx_dltc_transpose(const double* d_x, const int* ids_x, double* d_y,
  * Replaces: void local_contraction(int,int,int,double*,double*,double*,int,int,double)
  *           localcontract.h:13 (localcontract.cc:3-20), with the leading
  *           dimension of a transposed operand corrected (the reference passes
- *           n_b, right only when n_b == n_k). */
+ *           n_b, right only when n_b == n_k).
+ * Few outputs with long K take a stream-ordered temporary, from a pool of
+ * which the library keeps up to 32 MB of a device between calls. */
 GBX_API int gbx_local_contraction(int n_a, int n_b, int n_k, const double* d_A, const double* d_B, double* d_C,
                           int at, int bt, double alpha, void* stream);
 
