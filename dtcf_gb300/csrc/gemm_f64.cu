@@ -56,10 +56,10 @@ int ceil_div(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 // per K chunk holding the whole output (reduced in a fixed order), and 8:
 // matrix-vector shapes (one side <= 2, K > 64), one warp per output of the
 // wide side, the wide operand's rows read once and coalesced.
-int f64_variant(int m, int n, int k) {
+static int variant_of(int m, int n, int k, int gemv_min_k) {
   if (k <= kSmallK) return 6;
   if (m <= kSmallOutDim && n <= kSmallOutDim && k >= kSmallOutMinK) return 7;
-  if (k > kGemvMinK && ((m <= kGemvDim && n > kSmallOutDim) || (n <= kGemvDim && m > kSmallOutDim))) return 8;
+  if (k > gemv_min_k && ((m <= kGemvDim && n > kSmallOutDim) || (n <= kGemvDim && m > kSmallOutDim))) return 8;
   const bool rows = n <= kThinN && m >= 4 * n, cols = m <= kThinN && n >= 4 * m;
   if (rows || cols) {
     const int wide = rows ? m : n, thin = rows ? n : m;
@@ -70,6 +70,7 @@ int f64_variant(int m, int n, int k) {
   }
   return 0;
 }
+int f64_variant(int m, int n, int k) { return variant_of(m, n, k, kGemvMinK); }
 
 // One thread per row (variant 4) or per column (variant 5) of C; the thin
 // operand (at most kThinN rows) is staged through shared memory kThinK
@@ -851,15 +852,16 @@ int F64Gemm::run_each(cudaStream_t st) const {
 // Kernel of a one-call product: a planned one's, but for the shapes whose few
 // outputs and short K the tile kernel's clusters finish first (the kernels for
 // long K add their K ranges' partial sums in a launch of their own, and
-// matrix-vector warps walk short K one after another).  Tile kernel /
+// matrix-vector warps walk short K one after another), and for the K up to 128
+// that leave a matrix-vector warp little but its reduction.  Tile kernel /
 // matrix-vector or small-output kernel, one call of many: 2000 x 1 x 2000 73 /
-// 22 us, 5000 x 2 x 5000 447 / 113 (149 with the wide operand stored down its
+// 22 us, 5000 x 2 x 5000 447 / 113 (150 with the wide operand stored down its
 // columns), 700 x 1 x 300 9.1 / 4.9, 20 x 1 x 200000 156 / 31, 1 x 1 x 10^6
-// 159 / 41, 12 x 9 x 10^5 122 / 39; the other way round 20 x 1 x 2000 8.4 /
-// 16, 300 x 2 x 1200 12.5 / 15, 2000 x 2 x 70 4.7 / 6.6, 1 x 1 x 4096 12.9 /
-// 16.6.
+// 159 / 45, 12 x 9 x 10^5 122 / 36; the other way round 20 x 1 x 2000 8.4 /
+// 16, 300 x 2 x 1200 12.5 / 15, 1 x 1 x 4096 12.9 / 16.6, and against the thin
+// kernel 100000 x 2 x 100 99 / 169, 50000 x 1 x 70 30 / 43.
 int one_call_variant(int m, int n, int k) {
-  const int v = f64_variant(m, n, k);
+  const int v = variant_of(m, n, k, 2 * kGemvMinK);
   if (v == 7 && m == 1 && n == 1 && k < 6144) return 0;
   if (v == 8 && k < 4608) {
     const int wide = std::max(m, n);

@@ -33,6 +33,7 @@ def call(noalloc, m, n, k, dA, dB, dC, at, bt, alpha, stream):
     (400, 1, 400, "gemv"), (399, 1, 400, "tile"), (400, 2, 399, "gemv"), (400, 2, 396, "tile"), (2000, 1, 2000, "gemv"),
     (1, 2000, 2049, "gemv"), (2, 1999, 2500, "gemv"), (5000, 2, 600, "gemv"), (17, 1, 4608, "gemv"), (2, 17, 4607, "tile"),
     (1, 1, 6144, "small_out"), (1, 1, 6143, "tile"), (1, 2, 4096, "small_out"), (16, 16, 4097, "small_out"),
+    (20000, 1, 129, "gemv"), (20000, 1, 128, "thin"), (2, 20000, 128, "thin"), (2, 20000, 129, "gemv"),
     (5, 3, 100001, "small_out"), (16, 16, 4095, "tile"), (17, 3, 65, "tile"),
 ])
 def test_kernel_and_result(m, n, k, kernel, at, bt, noalloc):
