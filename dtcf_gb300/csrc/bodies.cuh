@@ -900,7 +900,9 @@ __device__ __forceinline__ int find_problem(const int* __restrict__ first, int n
 // Eight warps per CTA: a work item is eight consecutive wide-side outputs
 // over one K range; with several ranges (few outputs, long K) each writes
 // its raw sums to a partial slab that the split-K reduction adds in order.
-template <bool kCoh>
+// kTwice: some columns count twice (code of its own: with the second loop the
+// other products were 15% slower).
+template <bool kCoh, bool kTwice = false>
 __device__ __forceinline__ void gemv_body(const GemmProblem* __restrict__ probs, int nprob,
                                           const int* __restrict__ block_first, int total_blocks, uint32_t bid,
                                           uint32_t nblk) {
@@ -924,7 +926,20 @@ __device__ __forceinline__ void gemv_body(const GemmProblem* __restrict__ probs,
     double acc[kGemvDim];
 #pragma unroll
     for (int j = 0; j < kGemvDim; ++j) acc[j] = 0.0;
-    for (int64_t k = k0 + lane; k < k1; k += 32) {
+    int64_t k = k0 + lane;
+    if constexpr (kTwice) {  // the columns that count twice first, their sums doubled
+      const int64_t end = min(k1, (int64_t)p.twice);
+      for (; k < end; k += 32) {
+        const double x = ldin<kCoh>(W + k * wcs);
+#pragma unroll
+        for (int j = 0; j < kGemvDim; ++j)
+          if (j < tn) acc[j] = fma(x, ldin<kCoh>(T + j * trs + k * tcs), acc[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < kGemvDim; ++j) acc[j] = __dadd_rn(acc[j], acc[j]);
+      // (k itself is the lane's next column)
+    }
+    for (; k < k1; k += 32) {
       const double x = ldin<kCoh>(W + k * wcs);
 #pragma unroll
       for (int j = 0; j < kGemvDim; ++j)
@@ -1026,8 +1041,10 @@ __device__ __forceinline__ void small_out_body(const GemmProblem* __restrict__ p
     const int i = out / p.n, j = out - i * p.n;
     const int k0 = c * p.kchunk, k1 = min(p.k, k0 + p.kchunk);
     double acc = 0.0;
-    for (int kk = k0; kk < k1; kk += 64) {
-      const int kc = min(64, k1 - kk);
+    // slices end with the columns that count twice
+    const int twice = min(k1, p.twice);
+    for (int kk = k0, kc; kk < k1; kk += kc) {
+      kc = min(64, (kk < twice ? twice : k1) - kk);
       __syncthreads();
       for (int e = tid; e < p.m * 64; e += 256) {
         const int r = e >> 6, q = e & 63;
@@ -1040,6 +1057,7 @@ __device__ __forceinline__ void small_out_body(const GemmProblem* __restrict__ p
       __syncthreads();
       if (active)
         for (int q = lane; q < kc; q += lanes) acc = fma(sm.As[i][q], sm.Bs[j][q], acc);
+      if (kk + kc == twice) acc = __dadd_rn(acc, acc);
     }
     __syncthreads();
     sm.red[tid] = active ? acc : 0.0;

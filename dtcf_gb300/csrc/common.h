@@ -211,7 +211,7 @@ struct GemmProblem {
   int m, n, k;
   double alpha;
   int accumulate;
-  int twice;  // products of the first `twice` of the k columns count twice (variant 0 only)
+  int twice;  // products of the first `twice` of the k columns count twice (not for K <= 8)
   // split-K and kernel (filled by F64Gemm::build)
   int ksplit, kchunk, pad_;
   double* partial;

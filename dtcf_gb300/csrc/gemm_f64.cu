@@ -98,8 +98,8 @@ __device__ __forceinline__ void thin_body(const GemmProblem* __restrict__ probs,
     double acc[kThinN];
 #pragma unroll
     for (int j = 0; j < kThinN; ++j) acc[j] = 0.0;
-    for (int k0 = 0; k0 < p.k; k0 += kThinK) {
-      const int kc = min(kThinK, p.k - k0);
+    for (int k0 = 0, kc; k0 < p.k; k0 += kc) {
+      kc = min(kThinK, (k0 < p.twice ? p.twice : p.k) - k0);  // a stage ends with the columns that count twice
       __syncthreads();
       for (int e = threadIdx.x; e < tn * kc; e += 256)
         Ts[e] = __ldg(T + (int64_t)(e / kc) * trs + (int64_t)(k0 + e % kc) * tcs);
@@ -111,6 +111,11 @@ __device__ __forceinline__ void thin_body(const GemmProblem* __restrict__ probs,
           for (int j = 0; j < kThinN; ++j)
             if (j < tn) acc[j] = fma(w, Ts[j * kc + k], acc[j]);
         }
+      }
+      if (k0 + kc == p.twice) {
+#pragma unroll
+        for (int j = 0; j < kThinN; ++j)
+          if (j < tn) acc[j] = __dadd_rn(acc[j], acc[j]);
       }
     }
     if (i < wide) {
@@ -134,10 +139,11 @@ __global__ void __launch_bounds__(256) thin_gemm_f64_kernel(const GemmProblem* _
 }
 
 // Matrix-vector shapes (variant 8): dev::gemv_body.
+template <bool kTwice>
 __global__ void __launch_bounds__(256) gemv_f64_kernel(const GemmProblem* __restrict__ probs, int nprob,
                                                        const int* __restrict__ block_first, int total_blocks) {
   begin_dependent();
-  dev::gemv_body<false>(probs, nprob, block_first, total_blocks, blockIdx.x, gridDim.x);
+  dev::gemv_body<false, kTwice>(probs, nprob, block_first, total_blocks, blockIdx.x, gridDim.x);
 }
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
@@ -771,6 +777,7 @@ int F64Gemm::run(cudaStream_t st) const {
     // the CUDA-core shapes become records of the persistent program (static
     // schedule over their work items); the tile and thin kernels keep their own launches
     for (const Sub& sb : subs) {
+      if (sb.twice) return fail(GBX_EUNSUPPORTED, "columns that count twice in a program");
       const int kind = sb.variant == 6 ? PK_SMALLK : sb.variant == 7 ? PK_SMALLOUT : sb.variant == 8 ? PK_GEMV : -1;
       if (kind >= 0) {
         ProgArgs a;
@@ -815,7 +822,8 @@ int launch_variant(int v, const GemmProblem* probs, int nprob, const int* first,
     case 4: return launch(thin_gemm_f64_kernel<true>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
     case 6: return launch(small_k_gemm_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
     case 7: return launch(small_out_gemm_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
-    case 8: return launch(gemv_f64_kernel, (unsigned)grid, 256, st, probs, nprob, first, tiles);
+    case 8:
+      return launch(twice ? gemv_f64_kernel<true> : gemv_f64_kernel<false>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
     default: return launch(thin_gemm_f64_kernel<false>, (unsigned)grid, 256, st, probs, nprob, first, tiles);
   }
 }

@@ -438,11 +438,11 @@ int plan_contraction(const TensorLayout& A, const TensorLayout& B, const TensorL
   }
   if (pair && pair->exact && !p->groups.empty()) {
     GroupBlock& g = p->groups[0];
-    // only the FP64 tile kernel counts columns twice
-    if (g.engine == 0 && f64_variant((int)g.M, (int)g.N, (int)g.K) != 0)
+    // every FP64 kernel but the one for K <= 8 counts columns twice
+    if (g.engine == 0 && f64_variant((int)g.M, (int)g.N, (int)g.K) == 6)
       return plan_contraction(A, B, C, la, lb, lc, e, nslices, out, split_all, defer, nullptr);
     // the diagonal block pairs' columns first for the split engine, last for
-    // the tile kernel
+    // the FP64 kernels
     TupleIndex& kt = ks[g.h];
     int64_t off = 0;
     for (const bool diag : {g.engine == 1, g.engine != 1}) {

@@ -214,7 +214,7 @@ constexpr double kDirectMaxK = 16.0;
 // weighted 2 in one operand's pack (scale_b: B's, else A's) -- close to half
 // the contracted extent.  Both indices must have the same blocking.
 // exact: no operand or factor is scaled for it, so values at the ends of the
-// FP64 range stay as they are.  The FP64 tile kernel doubles its sums between
+// FP64 range stay as they are.  The FP64 kernels double their sums between
 // the off-diagonal columns and the diagonal ones (the ladder at o = 16, v = 48
 // in blocks of 8: 1193 -> 665 us); the split engine doubles the off-diagonal columns' digits
 // (SplitProblem::dbl_from; o = 32, v = 128, blocks of 16: 5033 -> 3132 us).

@@ -68,3 +68,37 @@ def test_exact_integers(v, vb, o, ob):
     C = make("aabb", (v, v, o, o), (v // vb, v // vb, o // ob, o // ob), ints)
     got, want = result(A, B, C, 2.0, -1)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("kernel,ta,tb,tc", [
+    # (symmetry, extents, block extents, indices) of A, B and C
+    ("gemv", ("aabb", (45,) * 4, (9,) * 4, "a,b,e,f"), ("aacc", (45, 45, 1, 1), (9, 9, 1, 1), "e,f,i,j"),
+     ("aacc", (45, 45, 1, 1), (9, 9, 1, 1), "a,b,i,j")),
+    ("gemv", ("aac", (33, 33, 2), (11, 11, 2), "e,f,i"), ("aacc", (33, 33, 10, 20), (11, 11, 10, 20), "e,f,j,k"),
+     ("ccc", (2, 10, 20), (2, 10, 20), "i,j,k")),
+    ("small_out", ("aacc", (28, 28, 22, 9), (7, 7, 11, 9), "e,f,g,i"), ("aacc", (28, 28, 22, 13), (7, 7, 11, 13), "e,f,g,j"),
+     ("cc", (9, 13), (9, 13), "i,j")),
+    ("thin", ("ccaa", (150, 150, 10, 10), (50, 50, 5, 5), "a,b,e,f"), ("aac", (10, 10, 5), (5, 5, 5), "e,f,i"),
+     ("ccc", (150, 150, 5), (50, 50, 5), "a,b,i")),
+    ("thin", ("aac", (10, 10, 5), (5, 5, 5), "e,f,i"), ("aacc", (10, 10, 150, 150), (5, 5, 50, 50), "e,f,a,b"),
+     ("ccc", (5, 150, 150), (5, 50, 50), "i,a,b")),
+])
+def test_every_kernel_counts_twice(kernel, ta, tb, tc):
+    """The thin kernels too run over block pairs x >= y, at half the products, with exact sums."""
+    from dtcf_gb300.rrr import Plan
+    from launches import launches
+    rng = np.random.default_rng(len(kernel))
+    A, B, C = (make(s, size, tuple(n // b for n, b in zip(size, blk)), lambda k: rng.integers(-9, 10, k).astype(np.float64))
+               for s, size, blk, _ in (ta, tb, tc))
+    names = [t[3] for t in (ta, tb, tc)]
+    want = oracle.rrr.contract(as_oracle(A), as_oracle(B), as_oracle(C), *names, 2.0, -1)
+    start = C.tiles.clone()
+    plan = Plan(A, B, C, *names, mode="fp64", sign=-1)
+    made = launches(lambda st: plan.execute(A, B, C, 2.0, stream=st))
+    assert any(kernel in name for name, _ in made), made
+    torch.cuda.synchronize()
+    C.tiles.copy_(start)
+    plan.execute(A, B, C, 2.0)
+    torch.cuda.synchronize()
+    assert np.array_equal(C.tiles.cpu().numpy().reshape(want.shape), want)
+    assert np.abs(want - start.cpu().numpy().reshape(want.shape)).max() > 0
