@@ -57,7 +57,7 @@ def test_exact_at_the_ends(ea, eb, alpha):
 @pytest.mark.parametrize("v,vb,o,ob", [(6, 3, 6, 3), (10, 5, 10, 5), (21, 7, 7, 7), (33, 11, 11, 11), (65, 13, 5, 5),
                                        (48, 8, 16, 8), (90, 10, 10, 10), (45, 9, 1, 1), (8, 1, 9, 1)])
 def test_exact_integers(v, vb, o, ob):
-    """Block pairs of every remainder by four, from one tile to several to an SM, and outputs too thin to be paired."""
+    """Block pairs of every remainder by four, from one tile to several to an SM, and thin outputs."""
     rng = np.random.default_rng(v)
 
     def ints(k):
