@@ -900,9 +900,15 @@ int temp_alloc(double** p, size_t bytes, cudaStream_t st) {
       props.allocType = cudaMemAllocationTypePinned;
       props.location.type = cudaMemLocationTypeDevice;
       props.location.id = dev;
-      GBX_CUDA(cudaMemPoolCreate(&pools[dev], &props));
+      // (also in the first call of a capture, this thread's or another's)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      GBX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      cudaError_t e = cudaMemPoolCreate(&pool, &props);
       uint64_t keep = kTempKeep;
-      GBX_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) return cuda_fail(e, "pool of one-call temporaries", __FILE__, __LINE__);
+      pools[dev] = pool;
     }
     pool = pools[dev];
   }

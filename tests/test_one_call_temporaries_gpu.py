@@ -1,7 +1,10 @@
 """The partial sums of one-call products: no wait for the driver in a call
 after a synchronisation, captured and replayed, and from several threads and
 streams at once."""
+import os
 import statistics
+import subprocess
+import sys
 import threading
 import time
 
@@ -60,6 +63,28 @@ def test_captured_and_replayed(m, n, k):
         graph.replay()
     torch.cuda.synchronize()
     check(c, A, B, 4)
+
+
+FIRST = """
+import numpy as np, torch
+import dtcf_gb300 as gbx
+rng = np.random.default_rng(1)
+A, B = rng.integers(-9, 10, (16, 5000)).astype(float), rng.integers(-9, 10, (16, 5000)).astype(float)
+a, b = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+c = torch.zeros(16, 16, dtype=torch.float64, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, capture_error_mode="global"):
+    gbx.local_contraction(16, 16, 5000, a, b, c, 0, 1, 1.0, stream=torch.cuda.current_stream())
+graph.replay()
+torch.cuda.synchronize()
+assert np.array_equal(c.cpu().numpy(), A @ B.T)
+"""
+
+
+def test_the_first_call_of_a_process_may_be_captured():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", FIRST], check=True, timeout=300, cwd=root)
 
 
 def test_threads_and_streams():
