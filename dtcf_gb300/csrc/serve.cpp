@@ -4,7 +4,9 @@
 // completion events, admits waiting jobs by planned footprint against the
 // byte budget, and puts the earliest runnable request on every free stream
 // slot: one graph launch of the job's iteration, an asynchronous read of its
-// energy into pinned memory, then an event.  Three builder threads create
+// energy into pinned memory, then an event.  While a slot stays free, a running
+// job's next request goes behind it on the same stream, so that the GPU goes
+// from one iteration to the next without this thread between them.  Three builder threads create
 // admitted jobs (host planning, integrals, constant operands, graph capture;
 // up to three at once, so one large job does not hold up the others), evict
 // idle jobs and check and destroy finished ones, so that none of this stalls
@@ -42,6 +44,7 @@ using Clock = std::chrono::steady_clock;
 
 constexpr int kPending = 1;  // request status while it has not finished
 constexpr int kBuilders = 3;  // builder threads: job builds in flight at once
+constexpr int kDepth = 2;     // requests of one job on a slot's stream
 
 struct Req {
   int job = 0, iter = 0;
@@ -294,16 +297,22 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
 
   const int nslot = s->cfg.slots;
   std::vector<cudaStream_t> streams(nslot, nullptr);
-  std::vector<cudaEvent_t> events(nslot, nullptr);
-  std::vector<int> slot_req(nslot, -1);
+  // a slot's requests, all of one job: the running one and one behind it
+  struct Slot {
+    int req[kDepth];
+    int head = 0, n = 0;
+    int at(int k) const { return (head + k) % kDepth; }
+  };
+  std::vector<Slot> slots(nslot);
+  std::vector<cudaEvent_t> events(nslot * kDepth, nullptr);  // and pinned: of a slot's places
   double* pinned = nullptr;
   int rc = GBX_OK;
-  for (int i = 0; i < nslot && rc == GBX_OK; ++i) {
-    if (cudaStreamCreateWithFlags(&streams[i], cudaStreamNonBlocking) != cudaSuccess ||
+  for (int i = 0; i < nslot * kDepth && rc == GBX_OK; ++i) {
+    if ((i < nslot && cudaStreamCreateWithFlags(&streams[i], cudaStreamNonBlocking) != cudaSuccess) ||
         cudaEventCreateWithFlags(&events[i], cudaEventDisableTiming) != cudaSuccess)
       rc = fail(GBX_ECUDA, "stream or event creation failed");
   }
-  if (rc == GBX_OK && cudaMallocHost((void**)&pinned, sizeof(double) * nslot) != cudaSuccess)
+  if (rc == GBX_OK && cudaMallocHost((void**)&pinned, sizeof(double) * nslot * kDepth) != cudaSuccess)
     rc = fail(GBX_ECUDA, "pinned buffer allocation failed");
   std::vector<std::thread> workers;
   if (rc == GBX_OK)
@@ -379,17 +388,20 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
     bool progress = false;
     // completions
     for (int i = 0; i < nslot; ++i) {
-      if (slot_req[i] < 0) continue;
-      const cudaError_t q = cudaEventQuery(events[i]);
+      Slot& sl = slots[i];
+      if (sl.n == 0) continue;
+      const int place = i * kDepth + sl.head;
+      const cudaError_t q = cudaEventQuery(events[place]);
       if (q == cudaErrorNotReady) continue;
-      Req& r = s->reqs[slot_req[i]];
+      Req& r = s->reqs[sl.req[sl.head]];
       Job& j = s->jobs[r.job];
       r.end = t;
-      r.energy = pinned[i];
+      r.energy = pinned[place];
       r.status = q == cudaSuccess ? GBX_OK : GBX_ECUDA;
       ++finished_reqs;
       ++j.done;
-      slot_req[i] = -1;
+      sl.head = sl.at(1);
+      --sl.n;
       progress = true;
       if (q != cudaSuccess) {
         rc = cuda_fail(q, "iteration request", __FILE__, __LINE__);
@@ -401,7 +413,7 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
         std::lock_guard<std::mutex> lk(s->mu);
         s->to_destroy.push_back(r.job);
         s->cv.notify_one();
-      } else {
+      } else if (sl.n == 0) {
         j.state = JobState::Ready;
       }
     }
@@ -467,9 +479,26 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
         break;
       }
     }
-    // dispatch: the earliest arrived runnable request on every free slot
+    const auto dispatch = [&](int i, int pick) {
+      Slot& sl = slots[i];
+      const int k = sl.at(sl.n), place = i * kDepth + k;
+      Req& q = s->reqs[pick];
+      Job& j = s->jobs[q.job];
+      GBX_TRY(gbx_cc_enqueue(j.h, 1, streams[i]));
+      GBX_TRY(gbx_cc_read_energy(j.h, pinned + place, streams[i]));
+      if (cudaEventRecord(events[place], streams[i]) != cudaSuccess) return fail(GBX_ECUDA, "event record failed");
+      q.start = now();
+      q.slot = i;
+      ++j.next;
+      j.state = JobState::Busy;
+      sl.req[k] = pick;
+      ++sl.n;
+      progress = true;
+      return (int)GBX_OK;
+    };
+    // the earliest arrived runnable request on every free slot
     for (int i = 0; i < nslot && rc == GBX_OK; ++i) {
-      if (slot_req[i] >= 0) continue;
+      if (slots[i].n > 0) continue;
       int pick = -1;
       for (int r : order) {
         const Req& q = s->reqs[r];
@@ -481,19 +510,16 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
         break;
       }
       if (pick < 0) break;
-      Req& q = s->reqs[pick];
-      Job& j = s->jobs[q.job];
-      rc = gbx_cc_enqueue(j.h, 1, streams[i]);
-      if (rc == GBX_OK) rc = gbx_cc_read_energy(j.h, pinned + i, streams[i]);
-      if (rc == GBX_OK && cudaEventRecord(events[i], streams[i]) != cudaSuccess)
-        rc = fail(GBX_ECUDA, "event record failed");
-      if (rc != GBX_OK) break;
-      q.start = now();
-      q.slot = i;
-      ++j.next;
-      j.state = JobState::Busy;
-      slot_req[i] = pick;
-      progress = true;
+      rc = dispatch(i, pick);
+    }
+    // nothing else waits for the slots that are left: the running jobs' next
+    // requests (a slot stays free, so no later arrival waits for them)
+    const bool spare = std::any_of(slots.begin(), slots.end(), [](const Slot& x) { return x.n == 0; });
+    for (int i = 0; i < nslot && spare && rc == GBX_OK; ++i) {
+      const Slot& sl = slots[i];
+      if (sl.n == 0 || sl.n == kDepth) continue;
+      const Job& j = s->jobs[s->reqs[sl.req[sl.head]].job];
+      if (j.next < (int)j.reqs.size() && s->reqs[j.reqs[j.next]].arrival <= t) rc = dispatch(i, j.reqs[j.next]);
     }
     if (time_limit_s > 0 && now() > time_limit_s) {
       timed_out = true;
@@ -505,14 +531,13 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
   for (int i = 0; i < nslot; ++i)
     if (streams[i]) cudaStreamSynchronize(streams[i]);
   const double tend = now();
-  for (int i = 0; i < nslot; ++i) {
-    if (slot_req[i] < 0) continue;
-    Req& r = s->reqs[slot_req[i]];
-    r.end = tend;
-    r.energy = pinned[i];
-    r.status = GBX_OK;
-    slot_req[i] = -1;
-  }
+  for (int i = 0; i < nslot; ++i)
+    for (; slots[i].n > 0; slots[i].head = slots[i].at(1), --slots[i].n) {
+      Req& r = s->reqs[slots[i].req[slots[i].head]];
+      r.end = tend;
+      r.energy = pinned[i * kDepth + slots[i].head];
+      r.status = GBX_OK;
+    }
   for (auto& r : s->reqs)
     if (r.status == kPending) r.status = timed_out ? GBX_ETIMEOUT : GBX_EINVAL;
   if (!workers.empty()) {
@@ -533,10 +558,10 @@ int gbx_server_run(gbx_server* s, double time_limit_s) {
     for (auto& w : workers) w.join();
     collect();
   }
-  for (int i = 0; i < nslot; ++i) {
-    if (events[i]) cudaEventDestroy(events[i]);
-    if (streams[i]) cudaStreamDestroy(streams[i]);
-  }
+  for (cudaEvent_t e : events)
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t st : streams)
+    if (st) cudaStreamDestroy(st);
   if (pinned) cudaFreeHost(pinned);
   cudaStreamSynchronize(s->mem_stream);
   // statistics

@@ -7,8 +7,9 @@
  * (gbx_cc_footprint) against a byte budget, and batches continuously: a
  * request starts as soon as a stream slot is free and its job is resident
  * and idle, so requests that arrive while others run overlap with them on the
- * device.  A job's iterations run in order; its state is released after its
- * last request.  Every request's latency is recorded.
+ * device (while a slot is free, a job's next request is put behind its running
+ * one).  A job's iterations run in order; its state is released after its last
+ * request.  Every request's latency is recorded.
  *
  * The reference has no serving layer (its jobs are single MPI runs); this is
  * the request loop around the node-local contraction path.  A resident job
@@ -26,7 +27,7 @@ extern "C" {
 
 typedef struct {
     double budget_bytes; /* device bytes the resident job states may take together */
-    int slots;           /* requests in flight on the GPU at once (one CUDA stream each) */
+    int slots;           /* jobs with an iteration in flight at once (one CUDA stream each) */
     int reserved;
 } gbx_serve_config;
 
